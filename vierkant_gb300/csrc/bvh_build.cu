@@ -10,7 +10,8 @@
 //   k_radix_*      stable LSD radix sort of (code, triangle id), 8 bits per pass
 //   k_karras       Karras 2012 radix tree (equal codes split by index)
 //   k_refit        bottom-up boxes, second arriving child finishes the parent
-//   k_collapse     breadth-first collapse to 8-wide nodes + 8-bit box quantisation (one CTA)
+//   k_topology     breadth-first collapse to 8-wide nodes: which BVH2 nodes become children, numbering
+//   k_quantise     the nodes' boxes (8 bits a side) and child words, eight lanes per node
 //   k_tri_records  48-byte triangle records (v0, e1, e2, id) in sorted order
 // Data layout in HBM: nodes (96 B each) and triangle records (48 B each) are contiguous arrays read
 // with 16-byte vector loads by the traversal kernels.
@@ -47,6 +48,15 @@ enum : uint32_t
     BUILD_ERR_INDEX = 1u,    // an index >= num_vertices (triangles) / a BLAS index >= num_blas (instances)
     BUILD_ERR_CAPACITY = 2u, // node capacity exceeded
     BUILD_ERR_SINGULAR = 4u, // an instance transform that cannot be inverted
+    BUILD_ERR_WAIT = 8u,     // a grid barrier of k_topology was not reached in time
+};
+
+// an internal node of the binary radix tree: what the collapse reads of it, in one 16-byte load
+struct alignas(16) bvh2_node
+{
+    uint32_t left, right; // LEAF_BIT | sorted position, or internal node
+    float area;           // half the surface area of its box (written by k_refit)
+    uint32_t count;       // primitives below it
 };
 
 __global__ void k_tri_boxes(const float *__restrict__ xyz, uint32_t nv, const uint32_t *__restrict__ idx, uint32_t n,
@@ -131,9 +141,8 @@ __global__ void k_morton(const box6 *__restrict__ tbox, uint32_t n, const uint32
     morton_out[i] = code;
 }
 
-__global__ void k_karras(const uint32_t *__restrict__ codes, uint32_t n, uint32_t *__restrict__ left,
-                         uint32_t *__restrict__ right, uint32_t *__restrict__ first, uint32_t *__restrict__ last,
-                         uint32_t *__restrict__ iparent, uint32_t *__restrict__ lparent)
+__global__ void k_karras(const uint32_t *__restrict__ codes, uint32_t n, bvh2_node *__restrict__ tree,
+                         uint32_t *__restrict__ first, uint32_t *__restrict__ iparent, uint32_t *__restrict__ lparent)
 {
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if(i >= (int64_t)n - 1) return;
@@ -157,10 +166,8 @@ __global__ void k_karras(const uint32_t *__restrict__ codes, uint32_t n, uint32_
     int64_t lo = i < j ? i : j, hi = i < j ? j : i;
     uint32_t lc = (lo == gamma) ? (LEAF_BIT | (uint32_t)gamma) : (uint32_t)gamma;
     uint32_t rc = (hi == gamma + 1) ? (LEAF_BIT | (uint32_t)(gamma + 1)) : (uint32_t)(gamma + 1);
-    left[i] = lc;
-    right[i] = rc;
+    *reinterpret_cast<uint4 *>(&tree[i]) = make_uint4(lc, rc, 0u, (uint32_t)(hi - lo) + 1u);
     first[i] = (uint32_t)lo;
-    last[i] = (uint32_t)hi;
     if(lc & LEAF_BIT) lparent[lc & ~LEAF_BIT] = (uint32_t)i;
     else iparent[lc] = (uint32_t)i;
     if(rc & LEAF_BIT) lparent[rc & ~LEAF_BIT] = (uint32_t)i;
@@ -186,9 +193,14 @@ __device__ __forceinline__ box6 load_box_cg(const box6 *p)
     return b;
 }
 
-__global__ void k_refit(const uint32_t *__restrict__ lparent, const uint32_t *__restrict__ iparent,
-                        const uint32_t *__restrict__ left, const uint32_t *__restrict__ right, const box6 *lbox,
-                        box6 *ibox, uint32_t *visits, uint32_t n)
+__device__ __forceinline__ float box_area(const box6 &b)
+{
+    float dx = fsub(b.hi[0], b.lo[0]), dy = fsub(b.hi[1], b.lo[1]), dz = fsub(b.hi[2], b.lo[2]);
+    return fadd(fadd(fmul(dx, dy), fmul(dy, dz)), fmul(dz, dx));
+}
+
+__global__ void k_refit(const uint32_t *__restrict__ lparent, const uint32_t *__restrict__ iparent, bvh2_node *tree,
+                        const box6 *lbox, box6 *ibox, uint32_t *visits, uint32_t n)
 {
     uint32_t leaf = blockIdx.x * blockDim.x + threadIdx.x;
     if(leaf >= n || n < 2) return;
@@ -199,7 +211,8 @@ __global__ void k_refit(const uint32_t *__restrict__ lparent, const uint32_t *__
         __threadfence();
         if(atomicAdd(&visits[p], 1u) == 0u) return; // first arrival: the sibling finishes p
         __threadfence();                            // acquire: the sibling's box is visible now
-        uint32_t l = left[p], r = right[p];
+        const uint2 lr = *reinterpret_cast<const uint2 *>(&tree[p]);
+        const uint32_t l = lr.x, r = lr.y;
         box6 a = (l & LEAF_BIT) ? load_box_cg(&lbox[l & ~LEAF_BIT]) : load_box_cg(&ibox[l]);
         box6 b = (r & LEAF_BIT) ? load_box_cg(&lbox[r & ~LEAF_BIT]) : load_box_cg(&ibox[r]);
         box6 u;
@@ -214,51 +227,97 @@ __global__ void k_refit(const uint32_t *__restrict__ lparent, const uint32_t *__
             __stcg(dst + k, u.lo[k]);
             __stcg(dst + 3 + k, u.hi[k]);
         }
+        tree[p].area = box_area(u);
         if(p == 0) return;
         p = iparent[p];
     }
 }
 
-// ---- breadth-first collapse to 8-wide nodes (one CTA, deterministic numbering) ----------------
+// ---- breadth-first collapse to 8-wide nodes (deterministic numbering) -----------------------------
 struct collapse_args
 {
-    const uint32_t *left, *right, *first, *last;
+    const bvh2_node *tree;
+    const uint32_t *first;
     const box6 *ibox, *lbox;
     uint32_t n, leaf_max, capacity;
     const uint32_t *scene_enc;
-    uint32_t *node_ref; // [capacity] BVH2 reference of each 8-wide node
-    node8 *nodes;       // [capacity]
-    uint32_t *out_info; // [0] num_nodes, [1] depth, [2] error flags
+    uint32_t *node_ref;  // [capacity] BVH2 reference of each 8-wide node
+    node8 *nodes;        // [capacity]
+    uint32_t *out_info;  // [0] num_nodes, [1] depth, [2] error flags, [3] grid barrier (zero at launch)
+    uint32_t *block_sum; // [grid] children of a block's nodes in the current level
     float *out_margin;
 };
 
 __device__ __forceinline__ uint32_t ref_count(const collapse_args &A, uint32_t r)
 {
-    return (r & LEAF_BIT) ? 1u : (A.last[r] - A.first[r] + 1u);
-}
-__device__ __forceinline__ uint32_t ref_first(const collapse_args &A, uint32_t r)
-{
-    return (r & LEAF_BIT) ? (r & ~LEAF_BIT) : A.first[r];
-}
-__device__ __forceinline__ box6 ref_box(const collapse_args &A, uint32_t r)
-{
-    return (r & LEAF_BIT) ? A.lbox[r & ~LEAF_BIT] : A.ibox[r];
-}
-__device__ __forceinline__ float box_area(const box6 &b)
-{
-    float dx = fsub(b.hi[0], b.lo[0]), dy = fsub(b.hi[1], b.lo[1]), dz = fsub(b.hi[2], b.lo[2]);
-    return fadd(fadd(fmul(dx, dy), fmul(dy, dz)), fmul(dz, dx));
+    return (r & LEAF_BIT) ? 1u : A.tree[r].count;
 }
 
-constexpr int COLLAPSE_THREADS = 1024;
-
-__global__ void __launch_bounds__(COLLAPSE_THREADS) k_collapse(collapse_args A)
+// Grid barrier of a cooperative launch: arrival `target` = grid size x barriers so far. false when
+// the others did not arrive within the try limit (a few seconds), which it reports to them.
+__device__ bool grid_barrier(uint32_t *arrived, uint32_t target, uint32_t *err)
 {
-    __shared__ uint32_t s_warp[32];
-    __shared__ uint32_t s_level_end, s_next, s_err;
-    __shared__ float s_margin;
-    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
-    if(tid == 0)
+    __shared__ uint32_t s_ok;
+    __syncthreads();
+    if(threadIdx.x == 0)
+    {
+        s_ok = 1u;
+        __threadfence();
+        atomicAdd(arrived, 1u);
+        uint32_t tries = 0;
+        while(*reinterpret_cast<volatile uint32_t *>(arrived) < target)
+            if(++tries > (1u << 23) || (*reinterpret_cast<volatile uint32_t *>(err) & BUILD_ERR_WAIT))
+            {
+                atomicOr(err, BUILD_ERR_WAIT);
+                s_ok = 0u;
+                break;
+            }
+        __threadfence();
+    }
+    __syncthreads();
+    return s_ok != 0u;
+}
+
+constexpr int COLLAPSE_THREADS = 512;
+// nodes per block below which further blocks would only add to the barriers
+constexpr uint32_t COLLAPSE_PRIMS_PER_BLOCK = 2048;
+
+// inclusive scan of x over the block; `total` receives the block's sum
+__device__ __forceinline__ uint32_t block_scan(uint32_t x, uint32_t *s_warp, uint32_t &total)
+{
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    for(int o = 1; o < 32; o <<= 1)
+    {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+        if(lane >= (uint32_t)o) x += y;
+    }
+    __syncthreads(); // s_warp may still be read for the call before
+    if(lane == 31) s_warp[warp] = x;
+    __syncthreads();
+    uint32_t before = 0;
+    total = 0;
+    for(uint32_t w = 0; w < COLLAPSE_THREADS / 32; ++w)
+    {
+        const uint32_t v = s_warp[w];
+        before += w < warp ? v : 0u;
+        total += v;
+    }
+    return before + x;
+}
+
+// Level by level, every 8-wide node of the level opens its BVH2 node until eight children are found or
+// only leaves are left (the largest box first); the internal children of a level, in node and slot
+// order, are the next level's nodes. A level's nodes are split over the blocks in contiguous runs;
+// one scan over the blocks' child counts numbers the next level exactly as one block would.
+// Between this kernel and k_quantise a node holds: child[] = its BVH2 references, origin[0] = index
+// of its first internal child, origin[1] = bit mask of the internal children, nchild.
+// Bound by the latency of the dependent loads of a node's opening (7 steps) and of two grid barriers
+// a level. One block did all of this and the quantisation before, 4.76 ms for 522,242 triangles.
+__global__ void __launch_bounds__(COLLAPSE_THREADS) k_topology(collapse_args A)
+{
+    __shared__ uint32_t s_warp[COLLAPSE_THREADS / 32];
+    const uint32_t tid = threadIdx.x;
+    if(blockIdx.x == 0 && tid == 0)
     {
         float lo[3], hi[3];
         scene_box(A.scene_enc, lo, hi);
@@ -268,162 +327,219 @@ __global__ void __launch_bounds__(COLLAPSE_THREADS) k_collapse(collapse_args A)
             ext = fmaxf(ext, fsub(hi[a], lo[a]));
             amax = fmaxf(amax, fmaxf(fabsf(lo[a]), fabsf(hi[a])));
         }
-        s_margin = fmul(fmaxf(ext, amax), 3.0517578125e-05f); // 2^-15
-        *A.out_margin = s_margin;
-        A.node_ref[0] = (A.n == 1) ? (LEAF_BIT | 0u) : 0u;
-        s_next = 1;
-        s_err = 0;
+        *A.out_margin = fmul(fmaxf(ext, amax), 3.0517578125e-05f); // 2^-15
+        __stcg(&A.node_ref[0], (A.n == 1) ? (LEAF_BIT | 0u) : 0u);
     }
     __syncthreads();
-    const float m = s_margin;
-    uint32_t begin = 0, end = 1, depth = 0;
+    uint32_t begin = 0, end = 1, depth = 0, barriers = 0, err = 0;
     while(begin < end)
     {
         ++depth;
-        if(tid == 0) s_level_end = end;
-        __syncthreads();
-        for(uint32_t cbase = begin; cbase < end; cbase += COLLAPSE_THREADS)
+        // whole rounds of the block per block: a level of few nodes stays with few blocks
+        const uint32_t rounds = (end - begin + COLLAPSE_THREADS - 1) / COLLAPSE_THREADS;
+        const uint32_t per = (rounds + gridDim.x - 1) / gridDim.x * COLLAPSE_THREADS;
+        const uint32_t lo = min(begin + blockIdx.x * per, end), hi = min(lo + per, end);
+        uint32_t carry = 0;
+        for(uint32_t base = lo; base < hi; base += COLLAPSE_THREADS)
         {
-            uint32_t ni = cbase + tid;
-            bool active = ni < end;
-            uint32_t slots[8];
-            uint32_t ns = 0, nint = 0;
+            const uint32_t ni = base + tid;
+            const bool active = ni < hi;
+            uint32_t slot[8], ns = 0, inner = 0;
             if(active)
             {
-                uint32_t r = A.node_ref[ni];
-                if((r & LEAF_BIT) || ref_count(A, r) <= 1u) { slots[ns++] = r; }
+                // per slot: its reference, the box area (-1: not to be opened) and its children
+                float area[8];
+                uint32_t left[8], right[8];
+                const uint32_t r = __ldcg(&A.node_ref[ni]);
+#pragma unroll
+                for(int k = 0; k < 8; ++k)
+                {
+                    slot[k] = left[k] = right[k] = 0u;
+                    area[k] = -1.f;
+                }
+                auto put = [&](int at, uint32_t ref) {
+                    uint4 v = make_uint4(0u, 0u, __float_as_uint(-1.f), 1u);
+                    if(!(ref & LEAF_BIT)) v = *reinterpret_cast<const uint4 *>(&A.tree[ref]);
+                    const bool open = v.w > A.leaf_max;
+#pragma unroll
+                    for(int k = 0; k < 8; ++k)
+                        if(k == at)
+                        {
+                            slot[k] = ref;
+                            left[k] = v.x;
+                            right[k] = v.y;
+                            area[k] = open ? __uint_as_float(v.z) : -1.f;
+                        }
+                    inner = (inner & ~(1u << at)) | (open ? 1u << at : 0u);
+                };
+                // (only the root of a single primitive is a leaf)
+                if(r & LEAF_BIT) put((int)ns++, r);
                 else
                 {
-                    slots[ns++] = A.left[r];
-                    slots[ns++] = A.right[r];
-                    while(ns < 8)
+                    const uint2 lr = *reinterpret_cast<const uint2 *>(&A.tree[r]);
+                    put(0, lr.x);
+                    put(1, lr.y);
+                    for(ns = 2; ns < 8; ++ns)
                     {
                         int best = -1;
                         float best_area = -1.f;
-                        for(uint32_t k = 0; k < ns; ++k)
-                        {
-                            uint32_t s = slots[k];
-                            if((s & LEAF_BIT) || ref_count(A, s) <= A.leaf_max) continue;
-                            float a = box_area(A.ibox[s]);
-                            if(a > best_area)
+                        uint32_t bl = 0, br = 0;
+#pragma unroll
+                        for(int k = 0; k < 8; ++k)
+                            if(area[k] > best_area)
                             {
-                                best_area = a;
-                                best = (int)k;
+                                best_area = area[k];
+                                best = k;
+                                bl = left[k];
+                                br = right[k];
                             }
-                        }
                         if(best < 0) break;
-                        uint32_t s = slots[best];
-                        slots[best] = A.left[s];
-                        slots[ns++] = A.right[s];
+                        put(best, bl);
+                        put((int)ns, br);
                     }
                 }
-                for(uint32_t k = 0; k < ns; ++k) nint += ref_count(A, slots[k]) > A.leaf_max ? 1u : 0u;
             }
-            // block exclusive scan of nint
-            uint32_t x = nint;
-            for(int o = 1; o < 32; o <<= 1)
-            {
-                uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-                if(lane >= (uint32_t)o) x += y;
-            }
-            if(lane == 31) s_warp[warp] = x;
-            __syncthreads();
-            if(warp == 0)
-            {
-                uint32_t w = s_warp[lane];
-                for(int o = 1; o < 32; o <<= 1)
-                {
-                    uint32_t y = __shfl_up_sync(0xffffffffu, w, o);
-                    if(lane >= (uint32_t)o) w += y;
-                }
-                s_warp[lane] = w;
-            }
-            __syncthreads();
-            uint32_t prefix = (warp ? s_warp[warp - 1] : 0u) + x - nint;
-            uint32_t chunk_total = s_warp[31];
-            uint32_t child_base = s_next + prefix;
+            uint32_t total;
+            const uint32_t nint = __popc(inner), incl = block_scan(nint, s_warp, total);
             if(active)
             {
-                node8 nd;
-                nd.nchild = (uint8_t)ns;
-                box6 gb[8];
-                box6 nb;
-                for(int a = 0; a < 3; ++a)
-                {
-                    nb.lo[a] = __int_as_float(0x7f800000);
-                    nb.hi[a] = __int_as_float(0xff800000);
-                }
-                for(uint32_t k = 0; k < 8; ++k)
-                {
-                    if(k >= ns) break;
-                    box6 b = ref_box(A, slots[k]);
-                    for(int a = 0; a < 3; ++a)
-                    {
-                        gb[k].lo[a] = fsub(b.lo[a], m);
-                        gb[k].hi[a] = fadd(b.hi[a], m);
-                        nb.lo[a] = fminf(nb.lo[a], gb[k].lo[a]);
-                        nb.hi[a] = fmaxf(nb.hi[a], gb[k].hi[a]);
-                    }
-                }
-                for(int a = 0; a < 3; ++a)
-                {
-                    float range = fsub(nb.hi[a], nb.lo[a]);
-                    float xq = fdiv(range, 255.0f);
-                    uint32_t e = ((__float_as_uint(xq) >> 23) & 0xFFu) + 1u;
-                    if(e > 254u) e = 254u;
-                    nd.origin[a] = nb.lo[a];
-                    nd.exps[a] = (uint8_t)e;
-                    float inv_s = exp_scale(254u - e);
-                    for(uint32_t k = 0; k < 8; ++k)
-                    {
-                        uint8_t ql = 0, qh = 0;
-                        if(k < ns)
-                        {
-                            float fl = floorf(fmul(fsub(gb[k].lo[a], nb.lo[a]), inv_s));
-                            float fh = ceilf(fmul(fsub(gb[k].hi[a], nb.lo[a]), inv_s));
-                            ql = (uint8_t)(fl < 0.f ? 0.f : (fl > 255.f ? 255.f : fl));
-                            qh = (uint8_t)(fh < 0.f ? 0.f : (fh > 255.f ? 255.f : fh));
-                        }
-                        nd.qlo[a][k] = ql;
-                        nd.qhi[a][k] = qh;
-                    }
-                }
-                uint32_t c = child_base;
-                for(uint32_t k = 0; k < 8; ++k)
-                {
-                    uint32_t word = 0u;
-                    if(k < ns)
-                    {
-                        uint32_t s = slots[k];
-                        uint32_t cnt = ref_count(A, s);
-                        if(cnt <= A.leaf_max) { word = LEAF_BIT | ((cnt - 1u) << 27) | ref_first(A, s); }
-                        else
-                        {
-                            if(c < A.capacity) A.node_ref[c] = s;
-                            else atomicOr(&s_err, BUILD_ERR_CAPACITY);
-                            word = c++;
-                        }
-                    }
-                    nd.child[k] = word;
-                }
-                A.nodes[ni] = nd;
+                node8 *nd = A.nodes + ni;
+                uint4 *w = reinterpret_cast<uint4 *>(nd);
+                w[0] = make_uint4(carry + incl - nint, inner, 0u, ns << 24);
+                w[4] = make_uint4(slot[0], slot[1], slot[2], slot[3]);
+                w[5] = make_uint4(slot[4], slot[5], slot[6], slot[7]);
             }
-            __syncthreads();
-            if(tid == 0) s_next += chunk_total;
+            carry += total;
+        }
+        uint32_t before = 0, next = 0; // children of the blocks before this one / of all
+        if(gridDim.x > 1)
+        {
+            if(tid == 0) __stcg(&A.block_sum[blockIdx.x], carry);
+            if(!grid_barrier(&A.out_info[3], gridDim.x * ++barriers, &A.out_info[2])) return;
+            uint32_t b = 0, t = 0;
+            for(uint32_t k = tid; k < gridDim.x; k += COLLAPSE_THREADS)
+            {
+                const uint32_t v = __ldcg(&A.block_sum[k]);
+                b += k < blockIdx.x ? v : 0u;
+                t += v;
+            }
+            block_scan(b, s_warp, before);
+            block_scan(t, s_warp, next);
+        }
+        else
+        {
+            next = carry;
             __syncthreads();
         }
-        __threadfence_block();
-        __syncthreads();
+        const uint32_t room = A.capacity - min(end, A.capacity);
+        if(next > room)
+        {
+            err = BUILD_ERR_CAPACITY;
+            end += next;
+            break;
+        }
+        for(uint32_t ni = lo + tid; ni < hi; ni += COLLAPSE_THREADS)
+        {
+            uint32_t *w = reinterpret_cast<uint32_t *>(A.nodes + ni);
+            const uint32_t c0 = end + before + w[0];
+            uint32_t c = c0;
+            for(uint32_t m = w[1]; m; m &= m - 1u) __stcg(&A.node_ref[c++], w[16 + __ffs(m) - 1]);
+            w[0] = c0;
+        }
         begin = end;
-        end = s_next;
-        if(s_err) break;
-        __syncthreads();
+        end += next;
+        if(gridDim.x > 1 && begin < end)
+        {
+            if(!grid_barrier(&A.out_info[3], gridDim.x * ++barriers, &A.out_info[2])) return;
+        }
+        else
+            __syncthreads();
     }
-    if(tid == 0)
+    if(blockIdx.x == 0 && tid == 0)
     {
-        A.out_info[0] = s_next;
+        A.out_info[0] = end;
         A.out_info[1] = depth;
-        A.out_info[2] = s_err;
+        if(err) atomicOr(&A.out_info[2], err);
+    }
+}
+
+// The nodes' quantised boxes and child words. Eight lanes per node, one child each: the child boxes are
+// read side by side, the node's box is a three-step shuffle reduction, and every field of the node is
+// written by neighbouring lanes.
+__global__ void __launch_bounds__(256) k_quantise(collapse_args A)
+{
+    if(A.out_info[2]) return;
+    const uint32_t num = A.out_info[0], lane = threadIdx.x & 31u, k = lane & 7u;
+    const float m = *A.out_margin;
+    const uint32_t warps = gridDim.x * (blockDim.x / 32u);
+    for(uint32_t n0 = 4u * (blockIdx.x * (blockDim.x / 32u) + (threadIdx.x >> 5)); n0 < num; n0 += 4u * warps)
+    {
+        const uint32_t ni = n0 + (lane >> 3);
+        const bool active = ni < num;
+        uint32_t ref = 0, ns = 0, inner = 0, c0 = 0;
+        if(active)
+        {
+            const uint32_t *w = reinterpret_cast<const uint32_t *>(A.nodes + ni);
+            c0 = w[0];
+            inner = w[1];
+            ns = w[3] >> 24;
+            ref = w[16 + k];
+        }
+        const bool valid = k < ns;
+        float lo[3], hi[3], nlo[3], nhi[3];
+        box6 b;
+        if(valid) b = (ref & LEAF_BIT) ? A.lbox[ref & ~LEAF_BIT] : A.ibox[ref];
+#pragma unroll
+        for(int a = 0; a < 3; ++a)
+        {
+            lo[a] = valid ? fsub(b.lo[a], m) : __int_as_float(0x7f800000);
+            hi[a] = valid ? fadd(b.hi[a], m) : __int_as_float(0xff800000);
+            nlo[a] = lo[a];
+            nhi[a] = hi[a];
+#pragma unroll
+            for(int o = 1; o < 8; o <<= 1)
+            {
+                nlo[a] = fminf(nlo[a], __shfl_xor_sync(0xffffffffu, nlo[a], o));
+                nhi[a] = fmaxf(nhi[a], __shfl_xor_sync(0xffffffffu, nhi[a], o));
+            }
+        }
+        __syncwarp(); // every lane has read the node's words
+        if(!active) continue;
+        uint8_t *out = reinterpret_cast<uint8_t *>(A.nodes + ni);
+        uint32_t exps = 0;
+#pragma unroll
+        for(int a = 0; a < 3; ++a)
+        {
+            const float xq = fdiv(fsub(nhi[a], nlo[a]), 255.0f);
+            uint32_t e = ((__float_as_uint(xq) >> 23) & 0xFFu) + 1u;
+            if(e > 254u) e = 254u;
+            exps |= e << (8 * a);
+            const float inv_s = exp_scale(254u - e);
+            uint8_t ql = 0, qh = 0;
+            if(valid)
+            {
+                const float fl = floorf(fmul(fsub(lo[a], nlo[a]), inv_s));
+                const float fh = ceilf(fmul(fsub(hi[a], nlo[a]), inv_s));
+                ql = (uint8_t)(fl < 0.f ? 0.f : (fl > 255.f ? 255.f : fl));
+                qh = (uint8_t)(fh < 0.f ? 0.f : (fh > 255.f ? 255.f : fh));
+            }
+            out[16 + 8 * a + k] = ql;
+            out[40 + 8 * a + k] = qh;
+        }
+        uint32_t word = 0u;
+        if(valid)
+        {
+            if((inner >> k) & 1u) word = c0 + __popc(inner & ((1u << k) - 1u));
+            else
+            {
+                const uint32_t cnt = ref_count(A, ref), at = (ref & LEAF_BIT) ? (ref & ~LEAF_BIT) : A.first[ref];
+                word = LEAF_BIT | ((cnt - 1u) << 27) | at;
+            }
+        }
+        reinterpret_cast<uint32_t *>(out)[16 + k] = word;
+        if(k == 0)
+            *reinterpret_cast<uint4 *>(out) = make_uint4(__float_as_uint(nlo[0]), __float_as_uint(nlo[1]),
+                                                         __float_as_uint(nlo[2]), exps | (ns << 24));
     }
 }
 
@@ -625,6 +741,24 @@ __global__ void k_instance_records(const vkg_instance *__restrict__ inst, const 
     by_id[id] = r;
 }
 
+// both kernels of the collapse. max_blocks 1 keeps to plain launches; more blocks need a cooperative
+// one, as they wait for each other (all of them fit on the device at once: one per SM)
+cudaError_t launch_collapse(const collapse_args &A, uint32_t max_blocks, cudaStream_t st)
+{
+    uint32_t grid = std::min(max_blocks, (A.n + COLLAPSE_PRIMS_PER_BLOCK - 1) / COLLAPSE_PRIMS_PER_BLOCK);
+    if(grid > 1)
+    {
+        void *args[] = {const_cast<collapse_args *>(&A)};
+        const cudaError_t e = cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(k_topology), dim3(grid),
+                                                          dim3(COLLAPSE_THREADS), args, 0, st);
+        if(e != cudaSuccess) return e;
+    }
+    else
+        k_topology<<<1, COLLAPSE_THREADS, 0, st>>>(A);
+    k_quantise<<<std::min((A.n + 31u) / 32u, 1216u), 256, 0, st>>>(A);
+    return cudaGetLastError();
+}
+
 // The primitive-independent part of a build: make_boxes(tbox, scene_enc, err) fills the n primitive
 // boxes, the scene box (ordered uints) and error bits; Morton codes, the radix sort, the Karras tree,
 // the refit and the 8-wide collapse follow; make_records(sorted) writes the leaf records in sorted
@@ -642,8 +776,9 @@ vkg_status build_core(vkg_ctx *ctx, vkg_bvh *bvh, uint32_t n, uint32_t leaf_max,
     // scratch
     box6 *tbox = nullptr, *lbox = nullptr, *ibox = nullptr;
     uint32_t *keys0 = nullptr, *keys1 = nullptr, *vals0 = nullptr, *vals1 = nullptr, *counts = nullptr;
-    uint32_t *left = nullptr, *right = nullptr, *first = nullptr, *last = nullptr, *iparent = nullptr,
-             *lparent = nullptr, *visits = nullptr, *node_ref = nullptr, *small = nullptr;
+    uint32_t *first = nullptr, *iparent = nullptr, *lparent = nullptr, *visits = nullptr, *node_ref = nullptr,
+             *block_sum = nullptr, *small = nullptr;
+    bvh2_node *tree = nullptr;
     node8 *nodes_tmp = nullptr;
     float *d_margin = nullptr;
     const uint32_t nblocks = (n + SORT_TILE - 1) / SORT_TILE;
@@ -661,10 +796,9 @@ vkg_status build_core(vkg_ctx *ctx, vkg_bvh *bvh, uint32_t n, uint32_t leaf_max,
     chk(dalloc(&vals0, n, st));
     chk(dalloc(&vals1, n, st));
     chk(dalloc(&counts, (size_t)256 * nblocks, st));
-    chk(dalloc(&left, ni, st));
-    chk(dalloc(&right, ni, st));
+    chk(dalloc(&tree, ni, st));
     chk(dalloc(&first, ni, st));
-    chk(dalloc(&last, ni, st));
+    chk(dalloc(&block_sum, (size_t)ctx->num_sms, st));
     chk(dalloc(&iparent, ni, st));
     chk(dalloc(&lparent, n, st));
     chk(dalloc(&visits, ni, st));
@@ -700,12 +834,12 @@ vkg_status build_core(vkg_ctx *ctx, vkg_bvh *bvh, uint32_t n, uint32_t leaf_max,
     k_gather_leaf_boxes<<<g, T, 0, st>>>(tbox, vin, n, lbox);
     if(n > 1)
     {
-        k_karras<<<(ni + T - 1) / T, T, 0, st>>>(kin, n, left, right, first, last, iparent, lparent);
-        k_refit<<<g, T, 0, st>>>(lparent, iparent, left, right, lbox, ibox, visits, n);
+        k_karras<<<(ni + T - 1) / T, T, 0, st>>>(kin, n, tree, first, iparent, lparent);
+        k_refit<<<g, T, 0, st>>>(lparent, iparent, tree, lbox, ibox, visits, n);
     }
-    collapse_args A{left, right, first, last, ibox, lbox, n, leaf_max, capacity, small, node_ref, nodes_tmp,
-                    small + 8, d_margin};
-    k_collapse<<<1, COLLAPSE_THREADS, 0, st>>>(A);
+    collapse_args A{tree,     first,     ibox,      lbox,      n,        leaf_max, capacity, small,
+                    node_ref, nodes_tmp, small + 8, block_sum, d_margin};
+    chk(launch_collapse(A, (uint32_t)ctx->num_sms, st));
     make_records(static_cast<const uint32_t *>(vin));
     chk(cudaGetLastError());
 
@@ -733,7 +867,7 @@ vkg_status build_core(vkg_ctx *ctx, vkg_bvh *bvh, uint32_t n, uint32_t leaf_max,
                                 st));
     }
     for(void *p: {(void *)tbox, (void *)lbox, (void *)ibox, (void *)keys0, (void *)keys1, (void *)vals0,
-                  (void *)vals1, (void *)counts, (void *)left, (void *)right, (void *)first, (void *)last,
+                  (void *)vals1, (void *)counts, (void *)tree, (void *)first, (void *)block_sum,
                   (void *)iparent, (void *)lparent, (void *)visits, (void *)node_ref, (void *)nodes_tmp,
                   (void *)small, (void *)d_margin})
         cudaFreeAsync(p, st);
@@ -744,6 +878,7 @@ vkg_status build_core(vkg_ctx *ctx, vkg_bvh *bvh, uint32_t n, uint32_t leaf_max,
     cudaEventDestroy(ev1);
     if(e != cudaSuccess) return cuda_check(ctx, e, "BVH build");
     err_bits = info[6];
+    if(info[10] & BUILD_ERR_WAIT) return set_error(ctx, VKG_ERR_TIMEOUT, "BVH build: a grid barrier ran out");
     if(info[10] & BUILD_ERR_CAPACITY) return set_error(ctx, VKG_ERR_CAPACITY, "BVH build: node capacity exceeded");
     const uint32_t max_depth = (TRAVERSAL_STACK - 1) / 7 + 1;
     if(bvh->depth > max_depth)
@@ -1001,7 +1136,8 @@ struct noalloc_scratch
     box6 tbox[NOALLOC_MAX_TRIS], lbox[NOALLOC_MAX_TRIS], ibox[NOALLOC_MAX_TRIS];
     uint32_t keys0[NOALLOC_MAX_TRIS], keys1[NOALLOC_MAX_TRIS], vals0[NOALLOC_MAX_TRIS], vals1[NOALLOC_MAX_TRIS];
     uint32_t counts[256 * NOALLOC_SORT_BLOCKS];
-    uint32_t left[NOALLOC_MAX_TRIS], right[NOALLOC_MAX_TRIS], first[NOALLOC_MAX_TRIS], last[NOALLOC_MAX_TRIS];
+    bvh2_node tree[NOALLOC_MAX_TRIS];
+    uint32_t first[NOALLOC_MAX_TRIS];
     uint32_t iparent[NOALLOC_MAX_TRIS], lparent[NOALLOC_MAX_TRIS], visits[NOALLOC_MAX_TRIS];
     uint32_t node_ref[NOALLOC_MAX_TRIS + 8];
     uint32_t morton[NOALLOC_MAX_TRIS];
@@ -1111,14 +1247,13 @@ extern "C" vkg_status vkg_bvh_build_noalloc(const float *d_xyz, uint32_t num_ver
     k_gather_leaf_boxes<<<g, T, 0, st>>>(s->tbox, vin, n, s->lbox);
     if(n > 1)
     {
-        k_karras<<<(n - 1 + T - 1) / T, T, 0, st>>>(kin, n, s->left, s->right, s->first, s->last, s->iparent,
-                                                      s->lparent);
-        k_refit<<<g, T, 0, st>>>(s->lparent, s->iparent, s->left, s->right, s->lbox, s->ibox, s->visits, n);
+        k_karras<<<(n - 1 + T - 1) / T, T, 0, st>>>(kin, n, s->tree, s->first, s->iparent, s->lparent);
+        k_refit<<<g, T, 0, st>>>(s->lparent, s->iparent, s->tree, s->lbox, s->ibox, s->visits, n);
     }
     const uint32_t capacity = std::min<uint32_t>(node_capacity, NOALLOC_MAX_TRIS + 8);
-    collapse_args A{s->left, s->right, s->first, s->last, s->ibox, s->lbox, n, leaf_max, capacity, s->small,
-                    s->node_ref, static_cast<node8 *>(d_nodes), s->small + 8, s->margin};
-    k_collapse<<<1, COLLAPSE_THREADS, 0, st>>>(A);
+    collapse_args A{s->tree, s->first, s->ibox, s->lbox, n, leaf_max, capacity, s->small, s->node_ref,
+                    static_cast<node8 *>(d_nodes), s->small + 8, nullptr, s->margin};
+    if(launch_collapse(A, 1, st) != cudaSuccess) return VKG_ERR_CUDA;
     k_tri_records<<<g, T, 0, st>>>(d_xyz, num_vertices, d_indices, vin, n, static_cast<tri_rec *>(d_tris));
     k_noalloc_info<<<1, 1, 0, st>>>(s, n, d_info);
     return cudaGetLastError() == cudaSuccess ? VKG_OK : VKG_ERR_CUDA;
