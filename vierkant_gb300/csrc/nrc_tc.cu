@@ -590,27 +590,34 @@ __global__ void __launch_bounds__(TC_THREADS)
 // ---- weight gradients on tcgen05 --------------------------------------------------------------
 // dW_l[k][o] = sum over records s of H_l[s][k] * G_l[s][o] (H_0 = the encoded inputs X, G_l the
 // gradient of layer l's pre-activation, both BF16 as the backward stored them). As one UMMA chain per
-// layer and chunk of 128 records: D (128 x N_l, FP32 in TMEM) += A (128 x 128) * B (N_l x 128)^T with
-// A = H_l^T zero-padded to 128 rows and B = G_l^T, both K-major over the records. The six
-// accumulators (336 TMEM columns) stay resident while the CTA walks its chunks; two shared-memory
-// buffer pairs let the staging of one layer overlap the MMAs of the previous one.
-constexpr uint32_t WG_TC_THREADS = 256, WG_TC_CHUNK = 128, WG_TC_TMEM = 512;
-constexpr uint32_t WG_A_BYTES = 128 * WG_TC_CHUNK * 2, WG_B_BYTES = 64 * WG_TC_CHUNK * 2;
-// two buffer pairs (96 KB) padded so that a single CTA fits per SM (its TMEM allocation takes all 512
-// columns)
-constexpr uint32_t WG_TC_SMEM = 120u * 1024u;
+// layer and chunk of 64 records: D (128 x N_l, FP32 in TMEM) += A (128 x 64) * B (N_l x 64)^T with
+// A = H_l^T and B = G_l^T. A record's features are contiguous, so both operands are MN-major: a core
+// matrix is 8 records x 8 features (16 bytes a record), and the rows of X, H and G go to shared memory
+// as they are, 16 bytes at a time by cp.async. One stage holds a chunk's X, H1..H5, G0..G4, G5 (92
+// feature groups, 94 KB); the next chunk's loads run during this chunk's MMAs. A layer with 64 inputs
+// still reads 128 rows: rows past its inputs are the following groups' data, and the accumulator
+// lanes that they give are never read. The six accumulators (336 TMEM columns) stay resident while
+// the CTA walks its chunks.
+// Bound by the loads (1.47 KB a record from L2). 65,536 records took 121 us when each record's features
+// were scattered into K-major operands with 2-byte shared-memory stores.
+constexpr uint32_t WG_TC_THREADS = 256, WG_TC_CHUNK = 64, WG_TC_TMEM = 512;
+constexpr uint32_t WG_X = IN / 8, WG_H = ACT / 8, WG_G = GRAD / 8; // 16-byte groups of a record: 10, 40, 42
+// a group's records, and 16 bytes that spread the groups of a record over the banks
+constexpr uint32_t WG_GROUP = WG_TC_CHUNK * 16 + 16;
+constexpr uint32_t WG_STAGE = (WG_X + WG_H + WG_G) * WG_GROUP, WG_TC_SMEM = 2 * WG_STAGE;
+static_assert(WG_X + 8 * 4 + 16 <= WG_X + WG_H + WG_G, "the last layer's 128 operand rows stay in the stage");
 
 __device__ __forceinline__ uint32_t tmem_col(int l) { return l < NLAYER - 1 ? 64u * (uint32_t)l : 320u; }
 
-// 16 BF16 values (8 u32) of record s into rows [r0, r0 + 16) of a K-major operand (K = 128 records)
-__device__ __forceinline__ void scatter16(uint8_t *buf, uint32_t r0, uint32_t s, const uint4 (&v)[2])
+// groups [g0, g0 + GROUPS) of a stage: rows [r0, r0 + 64) of src (GROUPS x 16 bytes each), zeros past n
+template<uint32_t GROUPS>
+__device__ __forceinline__ void wg_load(const uint32_t *__restrict__ src, uint32_t r0, uint32_t n, uint32_t dst)
 {
-    const uint32_t w[8] = {v[0].x, v[0].y, v[0].z, v[0].w, v[1].x, v[1].y, v[1].z, v[1].w};
-#pragma unroll
-    for(int j = 0; j < 8; ++j)
+    for(uint32_t i = threadIdx.x; i < GROUPS * WG_TC_CHUNK; i += WG_TC_THREADS)
     {
-        *reinterpret_cast<uint16_t *>(buf + tc::canon_offset(r0 + 2 * j, s, WG_TC_CHUNK)) = (uint16_t)(w[j] & 0xFFFFu);
-        *reinterpret_cast<uint16_t *>(buf + tc::canon_offset(r0 + 2 * j + 1, s, WG_TC_CHUNK)) = (uint16_t)(w[j] >> 16);
+        const uint32_t s = i / GROUPS, p = i - s * GROUPS;
+        const bool valid = r0 + s < n;
+        tc::cp_async16(dst + p * WG_GROUP + s * 16u, src + (valid ? ((size_t)(r0 + s) * GROUPS + p) * 4u : 0u), valid);
     }
 }
 
@@ -621,114 +628,82 @@ __global__ void __launch_bounds__(WG_TC_THREADS)
     extern __shared__ __align__(1024) uint8_t smem[];
     __shared__ uint64_t mbar[2];
     __shared__ uint32_t tslot;
-    uint8_t *sA[2] = {smem, smem + WG_A_BYTES}, *sB[2] = {smem + 2 * WG_A_BYTES, smem + 2 * WG_A_BYTES + WG_B_BYTES};
-    const uint32_t tid = threadIdx.x, warp = tid >> 5, s = tid & (WG_TC_CHUNK - 1), h = tid >> 7;
-    // A rows past a layer's inputs stay zero: clear both A buffers once
-    for(uint32_t i = tid; i < 2 * WG_A_BYTES / 16; i += WG_TC_THREADS)
-        reinterpret_cast<uint4 *>(smem)[i] = make_uint4(0u, 0u, 0u, 0u);
+    const uint32_t tid = threadIdx.x, warp = tid >> 5, h = tid >> 7;
+    const uint32_t n = d_n ? min(*d_n, n_cap) : n_cap;
+    const uint32_t chunks = (n + WG_TC_CHUNK - 1) / WG_TC_CHUNK;
+    const uint32_t base = tc::smem_addr(smem);
+    auto load = [&](uint32_t c, uint32_t b) {
+        const uint32_t r0 = c * WG_TC_CHUNK, st = base + b * WG_STAGE;
+        wg_load<WG_X>(X, r0, n, st);
+        wg_load<WG_H>(H, r0, n, st + WG_X * WG_GROUP);
+        wg_load<WG_G>(G, r0, n, st + (WG_X + WG_H) * WG_GROUP);
+    };
+    if(blockIdx.x < chunks) load(blockIdx.x, 0);
+    tc::cp_async_commit();
     if(warp == 0) tc::tmem_alloc(&tslot, WG_TC_TMEM);
     if(tid == 0)
     {
         tc::mbar_init(&mbar[0], 1);
         tc::mbar_init(&mbar[1], 1);
     }
-    tc::fence_async_smem();
     tc::fence_before_sync();
     __syncthreads();
     tc::fence_after_sync();
     const uint32_t tmem = tslot;
-    const uint32_t n = d_n ? min(*d_n, n_cap) : n_cap;
-    const uint32_t chunks = (n + WG_TC_CHUNK - 1) / WG_TC_CHUNK;
-    uint32_t phase[2] = {0u, 0u};
-    bool used[2] = {false, false}, failed = false, any = false;
-    for(uint32_t c = blockIdx.x; c < chunks && !failed; c += gridDim.x)
+    uint32_t phase[2] = {0u, 0u}, k = 0;
+    bool failed = false;
+    for(uint32_t c = blockIdx.x; c < chunks; c += gridDim.x, ++k)
     {
-        const uint32_t r = c * WG_TC_CHUNK + s;
-        const bool valid = r < n;
-#pragma unroll 1
-        for(int l = 0; l < NLAYER; ++l)
+        const uint32_t b = k & 1u, o = b ^ 1u;
+        if(k > 0)
         {
-            const uint32_t b = (uint32_t)l & 1u, K = layer_in(l), N = layer_out(l);
-            if(used[b])
+            // the chunk before read the other stage: its MMAs must be done before that is refilled
+            const bool ok = tc::mbar_wait(&mbar[o], phase[o]);
+            if(__syncthreads_or(!ok))
             {
-                // the MMAs that read this buffer pair last must be done before it is overwritten
-                const bool ok = tc::mbar_wait(&mbar[b], phase[b]);
-                if(__syncthreads_or(!ok))
-                {
-                    failed = true;
-                    break;
-                }
-                phase[b] ^= 1u;
-                used[b] = false;
+                failed = true;
+                break;
             }
-            // A: this record's layer inputs in blocks of 16 rows, the two halves of the CTA alternating
-            const uint32_t *arow = l == 0 ? X + (size_t)r * 40 : H + (size_t)r * 160 + 32 * (l - 1);
-            for(uint32_t k0 = 16 * h; k0 < K; k0 += 32)
-            {
-                uint4 v[2] = {make_uint4(0u, 0u, 0u, 0u), make_uint4(0u, 0u, 0u, 0u)};
-                if(valid)
-                {
-                    v[0] = *reinterpret_cast<const uint4 *>(arow + k0 / 2);
-                    v[1] = *reinterpret_cast<const uint4 *>(arow + k0 / 2 + 4);
-                }
-                scatter16(sA[b], k0, s, v);
-            }
-            if(b == 0 && l > 0 && h == 1)
-                // rows 64..79 of buffer 0 still hold layer 0's last inputs
-                for(uint32_t k = 64; k < 80; ++k)
-                    *reinterpret_cast<uint16_t *>(sA[b] + tc::canon_offset(k, s, WG_TC_CHUNK)) = 0;
-            // B: this record's output gradients in blocks of 16 rows
-            const uint32_t *grow = G + (size_t)r * 168 + (l == NLAYER - 1 ? 160 : 32 * l);
-            for(uint32_t o0 = 16 * h; o0 < N; o0 += 32)
-            {
-                uint4 v[2] = {make_uint4(0u, 0u, 0u, 0u), make_uint4(0u, 0u, 0u, 0u)};
-                if(valid)
-                {
-                    v[0] = *reinterpret_cast<const uint4 *>(grow + o0 / 2);
-                    v[1] = *reinterpret_cast<const uint4 *>(grow + o0 / 2 + 4);
-                }
-                scatter16(sB[b], o0, s, v);
-            }
-            tc::fence_async_smem();
-            tc::fence_before_sync();
-            __syncthreads();
-            if(tid == 0)
-            {
-                tc::fence_after_sync();
-                const uint32_t idesc = tc::idesc_bf16(128, N);
-                const uint32_t a0 = tc::smem_addr(sA[b]), b0 = tc::smem_addr(sB[b]);
-                for(uint32_t k = 0; k < WG_TC_CHUNK / 16; ++k)
-                    tc::mma_bf16(tmem + tmem_col(l), tc::smem_desc(a0 + 256u * k, 128u, WG_TC_CHUNK * 16u),
-                                 tc::smem_desc(b0 + 256u * k, 128u, WG_TC_CHUNK * 16u), idesc, any || k > 0);
-                tc::mma_commit(&mbar[b]);
-            }
-            used[b] = true;
+            phase[o] ^= 1u;
         }
-        any = true;
+        if(c + gridDim.x < chunks) load(c + gridDim.x, o);
+        tc::cp_async_commit();
+        tc::cp_async_wait<1>(); // this chunk's own groups have landed
+        tc::fence_async_smem();
+        tc::fence_before_sync();
+        __syncthreads();
+        if(tid == 0)
+        {
+            tc::fence_after_sync();
+            const uint32_t st = base + b * WG_STAGE, gr = st + (WG_X + WG_H) * WG_GROUP;
+            for(int l = 0; l < NLAYER; ++l)
+            {
+                const uint32_t idesc = tc::idesc_bf16(128, layer_out(l)) | tc::IDESC_A_MN | tc::IDESC_B_MN;
+                const uint32_t a0 = l == 0 ? st : st + (WG_X + 8u * (l - 1)) * WG_GROUP, b0 = gr + 8u * l * WG_GROUP;
+                for(uint32_t q = 0; q < WG_TC_CHUNK / 16; ++q)
+                    tc::mma_bf16(tmem + tmem_col(l), tc::smem_desc(a0 + 256u * q, 128u, WG_GROUP),
+                                 tc::smem_desc(b0 + 256u * q, 128u, WG_GROUP), idesc, k > 0 || q > 0);
+            }
+            tc::mma_commit(&mbar[b]);
+        }
     }
-    // the last MMAs of both buffers
-    for(int b = 0; b < 2 && !failed; ++b)
-        if(used[b])
-        {
-            const bool ok = tc::mbar_wait(&mbar[b], phase[b]);
-            if(__syncthreads_or(!ok)) failed = true;
-            else
-            {
-                phase[b] ^= 1u;
-                used[b] = false;
-            }
-        }
+    tc::cp_async_wait<0>();
+    // the last chunk's MMAs (after a wait that ran out: the chunk's before it, once more)
+    if(k > 0)
+    {
+        const uint32_t b = (k - 1u) & 1u;
+        const bool ok = tc::mbar_wait(&mbar[b], phase[b]);
+        if(__syncthreads_or(!ok)) failed = true;
+    }
     if(failed)
     {
         if(tid == 0) atomicOr(err, TC_TIMEOUT);
-        for(int b = 0; b < 2; ++b)
-            if(used[b]) tc::mbar_wait(&mbar[b], phase[b]);
     }
-    else if(any)
+    else if(k > 0)
     {
         tc::fence_after_sync();
-        // lane k = 32 (warp mod 4) + lane of TMEM holds row k of every layer's accumulator
-        const uint32_t k = 32u * (warp & 3u) + (tid & 31u), lane_base = (32u * (warp & 3u)) << 16;
+        // lane r = 32 (warp mod 4) + lane of TMEM holds row r of every layer's accumulator
+        const uint32_t r = 32u * (warp & 3u) + (tid & 31u), lane_base = (32u * (warp & 3u)) << 16;
 #pragma unroll 1
         for(int l = 0; l < NLAYER; ++l)
         {
@@ -738,9 +713,11 @@ __global__ void __launch_bounds__(WG_TC_THREADS)
                 float v[16];
                 tc::tmem_ld16(tmem + lane_base + tmem_col(l) + c0, v);
                 tc::tmem_ld_wait();
-                if(k < K)
-                    for(int j = 0; j < 16; ++j)
-                        if(c0 + j < N) atomicAdd(&dW[layer_off(l) + k * N + c0 + j], v[j]);
+                float4 *out = reinterpret_cast<float4 *>(dW + layer_off(l) + r * N + c0);
+                if(r < K)
+#pragma unroll
+                    for(int j = 0; j < 4; ++j)
+                        atomicAdd(out + j, make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]));
             }
         }
     }
