@@ -99,12 +99,53 @@ __device__ __forceinline__ void layer(const uint32_t (&a)[KT][4], const uint2 *_
 
 __device__ __forceinline__ uint32_t eff_count(uint32_t n, const uint32_t *d_n) { return d_n ? min(*d_n, n) : n; }
 
-__global__ void k_encode(const float *__restrict__ feats, uint32_t n, const uint32_t *__restrict__ d_n, grid_config gc,
-                         const __half2 *__restrict__ grid, uint32_t *__restrict__ X)
+// The 80 BF16 inputs of a record as 40 u32 (BF16 pairs): 16 levels x 2 hash-grid features, 16 SH
+// coefficients of the direction, 16 of the normal, roughness, albedo, zero padding. A CTA encodes 64
+// records; four warp pairs take four levels each, and one of the other parts. Records come in and
+// encoded rows go out through shared memory, so that both streams are coalesced (row by row, a warp's
+// 40 stores and 13 loads touched 32 lines each). Rows of 44 words keep the 16-byte stores free of
+// bank conflicts.
+constexpr int ENC_ROWS = 64, ENC_THREADS = 4 * ENC_ROWS, ENC_STRIDE = 44;
+__global__ void __launch_bounds__(ENC_THREADS)
+        k_encode(const float *__restrict__ feats, uint32_t n_cap, const uint32_t *__restrict__ d_n, grid_config gc,
+                 const __half2 *__restrict__ grid, uint32_t *__restrict__ X)
 {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if(i >= eff_count(n, d_n)) return;
-    encode_record(gc, grid, feats + (size_t)FEAT * i, X + (size_t)(IN / 2) * i);
+    __shared__ float sf[ENC_ROWS * FEAT];
+    __shared__ __align__(16) uint32_t sx[ENC_ROWS * ENC_STRIDE];
+    const uint32_t n = eff_count(n_cap, d_n), row0 = blockIdx.x * ENC_ROWS;
+    if(row0 >= n) return;
+    const uint32_t rows = min((uint32_t)ENC_ROWS, n - row0), tid = threadIdx.x;
+    for(uint32_t i = tid; i < rows * FEAT; i += ENC_THREADS) sf[i] = __ldg(feats + (size_t)row0 * FEAT + i);
+    __syncthreads();
+    const uint32_t r = tid & (ENC_ROWS - 1), part = tid / ENC_ROWS;
+    if(r < rows)
+    {
+        const float *f = sf + FEAT * r;
+        uint4 *out = reinterpret_cast<uint4 *>(sx + ENC_STRIDE * r);
+        float px, py, pz;
+        normalised_pos(gc, f, px, py, pz);
+        uint32_t v[4];
+#pragma unroll
+        for(uint32_t j = 0; j < 4; ++j)
+            v[j] = 4 * part + j < gc.levels ? encode_level(gc, grid, 4 * part + j, px, py, pz) : 0u;
+        out[part] = make_uint4(v[0], v[1], v[2], v[3]);
+        if(part < 2)
+        {
+            uint32_t s[8];
+            encode_sh(f + 3 + 3 * part, s);
+            out[4 + 2 * part] = make_uint4(s[0], s[1], s[2], s[3]);
+            out[5 + 2 * part] = make_uint4(s[4], s[5], s[6], s[7]);
+        }
+        else if(part == 2)
+            out[8] = make_uint4(pack_bf16(f[9], f[10]), pack_bf16(f[11], f[12]), 0u, 0u);
+        else
+            out[9] = make_uint4(0u, 0u, 0u, 0u);
+    }
+    __syncthreads();
+    uint4 *dst = reinterpret_cast<uint4 *>(X + (size_t)(IN / 2) * row0);
+    const uint4 *src = reinterpret_cast<const uint4 *>(sx);
+    for(uint32_t i = tid; i < rows * (IN / 8); i += ENC_THREADS)
+        dst[i] = src[(i / (IN / 8)) * (ENC_STRIDE / 4) + i % (IN / 8)];
 }
 
 // ---- fused forward -------------------------------------------------------------------------------
@@ -542,7 +583,7 @@ vkg_status nrc_ensure(vkg_nrc *c, uint32_t n)
 vkg_status nrc_encode(vkg_nrc *c, const float *feats, uint32_t n, const uint32_t *d_n, uint32_t *X, cudaStream_t st)
 {
     if(n == 0) return VKG_OK;
-    k_encode<<<(n + 127) / 128, 128, 0, st>>>(feats, n, d_n, c->gc, c->grid_h, X);
+    k_encode<<<(n + ENC_ROWS - 1) / ENC_ROWS, ENC_THREADS, 0, st>>>(feats, n, d_n, c->gc, c->grid_h, X);
     return cuda_check(c->ctx, cudaGetLastError(), "k_encode");
 }
 
@@ -689,6 +730,7 @@ vkg_status vkg_nrc_create(vkg_ctx *ctx, const vkg_nrc_config *cfg, vkg_nrc **out
     c->gc.growth = cfg->levels > 1 ? expf((logf((float)cfg->max_resolution) - logf((float)cfg->base_resolution)) /
                                           (float)(cfg->levels - 1))
                                    : 1.f;
+    for(uint32_t l = 0; l < 16; ++l) c->gc.res[l] = l < cfg->levels ? level_res(c->gc, l) : 1u;
     for(int a = 0; a < 3; ++a)
     {
         c->gc.smin[a] = cfg->scene_min[a];

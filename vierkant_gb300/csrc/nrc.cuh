@@ -64,6 +64,7 @@ struct grid_config
     uint32_t levels, log2_t, base_res;
     float growth;
     float smin[3], sinv[3]; // position normalisation: p = (x - smin) * sinv
+    uint32_t res[16];       // level_res() of every level
 };
 
 __host__ __device__ inline uint32_t level_res(const grid_config &g, uint32_t l)

@@ -48,7 +48,7 @@ struct corner_iter
 __device__ __forceinline__ corner_iter level_setup(const grid_config &gc, uint32_t l, float px, float py, float pz)
 {
     corner_iter c;
-    c.res = level_res(gc, l);
+    c.res = gc.res[l];
     c.table = 1u << gc.log2_t;
     const uint64_t r1 = (uint64_t)c.res + 1;
     c.dense = r1 * r1 * r1 <= (uint64_t)c.table;
@@ -74,6 +74,46 @@ __device__ __forceinline__ uint32_t corner_index(const corner_iter &c, int k, fl
     return (x * 1u ^ y * 2654435761u ^ z * 805459861u) & (c.table - 1u);
 }
 
+__device__ __forceinline__ uint32_t quad_word(const uint4 &q, uint32_t i)
+{
+    const uint32_t a = (i & 1u) ? q.y : q.x, b = (i & 1u) ? q.w : q.z;
+    return (i & 2u) ? b : a;
+}
+
+// BF16 feature pair of one level: the eight corners' entries interpolated. The gathers are bound by
+// L1 lookups (one line a cycle and SM: 128 entries a record took 916 us for 2,073,600 records), so an
+// entry is read with the aligned four that hold it: corners k and k + 1 of an x pair differ in the low
+// bits of their index only (dense levels: by one), and lie in one four in three cases of four.
+__device__ __forceinline__ uint32_t encode_level(const grid_config &gc, const __half2 *__restrict__ grid, uint32_t l,
+                                                 float px, float py, float pz)
+{
+    const corner_iter c = level_setup(gc, l, px, py, pz);
+    const uint32_t *tab = reinterpret_cast<const uint32_t *>(grid) + ((size_t)l << gc.log2_t);
+    float w[8];
+    uint32_t idx[8], e[8];
+    uint4 q[4];
+#pragma unroll
+    for(int k = 0; k < 8; ++k) idx[k] = corner_index(c, k, w[k]);
+#pragma unroll
+    for(int p = 0; p < 4; ++p) q[p] = __ldg(reinterpret_cast<const uint4 *>(tab) + (idx[2 * p] >> 2));
+#pragma unroll
+    for(int p = 0; p < 4; ++p)
+    {
+        e[2 * p] = quad_word(q[p], idx[2 * p]);
+        e[2 * p + 1] = quad_word(q[p], idx[2 * p + 1]);
+        if((idx[2 * p] ^ idx[2 * p + 1]) >> 2) e[2 * p + 1] = __ldg(tab + idx[2 * p + 1]);
+    }
+    float f0 = 0.f, f1 = 0.f;
+#pragma unroll
+    for(int k = 0; k < 8; ++k)
+    {
+        const float2 v = __half22float2(*reinterpret_cast<const __half2 *>(&e[k]));
+        f0 += w[k] * v.x;
+        f1 += w[k] * v.y;
+    }
+    return pack_bf16(f0, f1);
+}
+
 __device__ __forceinline__ void normalised_pos(const grid_config &gc, const float *f, float &px, float &py, float &pz)
 {
     px = fminf(fmaxf((f[0] - gc.smin[0]) * gc.sinv[0], 0.f), 1.f);
@@ -87,55 +127,28 @@ template<int L0, int L1>
 __device__ __forceinline__ void encode_levels(const grid_config &gc, const __half2 *__restrict__ grid, float px,
                                               float py, float pz, uint32_t *out)
 {
-    const uint32_t T = 1u << gc.log2_t;
 #pragma unroll
-    for(int l = L0; l < L1; ++l)
-    {
-        uint32_t word = 0u;
-        if((uint32_t)l < gc.levels)
-        {
-            corner_iter c = level_setup(gc, l, px, py, pz);
-            float f0 = 0.f, f1 = 0.f;
+    for(int l = L0; l < L1; ++l) out[l - L0] = (uint32_t)l < gc.levels ? encode_level(gc, grid, l, px, py, pz) : 0u;
+}
+
+// the 16 SH coefficients of a direction as BF16 pairs
+__device__ __forceinline__ void encode_sh(const float *d, uint32_t *out)
+{
+    float s[16];
+    sh4(d[0], d[1], d[2], s);
 #pragma unroll
-            for(int k = 0; k < 8; ++k)
-            {
-                float w;
-                const uint32_t idx = corner_index(c, k, w);
-                const float2 v = __half22float2(grid[(size_t)l * T + idx]);
-                f0 += w * v.x;
-                f1 += w * v.y;
-            }
-            word = pack_bf16(f0, f1);
-        }
-        out[l - L0] = word;
-    }
+    for(int k = 0; k < 8; ++k) out[k] = pack_bf16(s[2 * k], s[2 * k + 1]);
 }
 
 // the non-grid inputs (words 16..39): SH of the direction and of the normal, roughness, albedo, padding
 __device__ __forceinline__ void encode_rest(const float *f, uint32_t *out)
 {
-    float s[16];
-    sh4(f[3], f[4], f[5], s);
-#pragma unroll
-    for(int k = 0; k < 8; ++k) out[k] = pack_bf16(s[2 * k], s[2 * k + 1]);
-    sh4(f[6], f[7], f[8], s);
-#pragma unroll
-    for(int k = 0; k < 8; ++k) out[8 + k] = pack_bf16(s[2 * k], s[2 * k + 1]);
+    encode_sh(f + 3, out);
+    encode_sh(f + 6, out + 8);
     out[16] = pack_bf16(f[9], f[10]);
     out[17] = pack_bf16(f[11], f[12]);
 #pragma unroll
     for(int k = 18; k < 24; ++k) out[k] = 0u;
-}
-
-// the 80 BF16 inputs of one feature record as 40 u32 (BF16 pairs): 16 levels x 2 hash-grid features,
-// 16 SH coefficients of the direction, 16 of the normal, roughness, albedo, zero padding
-__device__ __forceinline__ void encode_record(const grid_config &gc, const __half2 *__restrict__ grid, const float *f,
-                                              uint32_t *out)
-{
-    float px, py, pz;
-    normalised_pos(gc, f, px, py, pz);
-    encode_levels<0, 16>(gc, grid, px, py, pz, out);
-    encode_rest(f, out + 16);
 }
 
 }// namespace nrc
