@@ -1,0 +1,77 @@
+"""The radiance cache's encoding, hash-grid gradients and weight gradients at ragged record counts (one
+record, around the 64-record CTA and chunk, several chunks per CTA) and level counts."""
+import ctypes as C
+
+import numpy as np
+import pytest
+import torch
+
+from nrc_reference import encode, forward, level_resolutions, random_features, relative_l2, split_weights
+from vierkant_gb300.nrc import NeuralRadianceCache
+from vierkant_gb300.raytracing import _cudart
+
+pytestmark = pytest.mark.gpu
+
+COUNTS = [1, 63, 64, 65, 129, 64 * 152 + 1, 64 * 152 * 2 + 77]
+
+
+def _read(address, count):
+    out = torch.empty(count, dtype=torch.float32, device="cuda")
+    torch.cuda.synchronize()
+    assert _cudart().cudaMemcpy(C.c_void_p(out.data_ptr()), C.c_void_p(address), C.c_size_t(4 * count), 3) == 0
+    return out
+
+
+def _cache(ctx, levels):
+    cfg = NeuralRadianceCache.default_config()
+    cfg.levels, cfg.log2_table_size = levels, 12
+    cache = NeuralRadianceCache(ctx, cfg)
+    i = cache.info()
+    g = torch.Generator(device="cuda").manual_seed(levels)
+    grid = torch.rand(i.num_grid_params, generator=g, device="cuda") * 2 - 1
+    cache.load_params(None, grid)
+    torch.cuda.synchronize()
+    return cache, _read(i.d_mlp_params, i.num_mlp_params), grid
+
+
+def _reference_inputs(cfg, feats, grid, levels):
+    """the 80 inputs; the columns of levels past the cache's count are zero"""
+    res = level_resolutions(levels) if levels > 1 else [16]
+    x = encode(feats, grid, res, 1 << cfg.log2_table_size, list(cfg.scene_min), list(cfg.scene_max), half_grid=False)
+    pad = torch.zeros((x.shape[0], 32 - 2 * levels), dtype=x.dtype, device=x.device)
+    return torch.cat([x[:, :2 * levels], pad, x[:, 2 * levels:]], dim=1)[:, :80]
+
+
+@pytest.mark.parametrize("n", COUNTS)
+@pytest.mark.parametrize("levels", [16, 5])
+def test_gradients(ctx, n, levels):
+    """against FP64 autograd of the same network: BF16 activations (8 bits) through six layers give
+    gradients of the right direction; the cosine bound is the one of the full-size gradient tests"""
+    cache, mlp, grid = _cache(ctx, levels)
+    feats = random_features(n, n)
+    targets = torch.rand((n, 3), generator=torch.Generator(device="cuda").manual_seed(n), device="cuda")
+    cache.backward(feats, targets)
+    i = cache.info()
+    assert i.kernel_error == 0
+    w, gr = mlp.double().requires_grad_(True), grid.double().requires_grad_(True)
+    y = forward(_reference_inputs(cache.config, feats, gr, levels), split_weights(w), emulate_bf16=False)
+    gw, gg = torch.autograd.grad(relative_l2(y, targets.double()), (w, gr))
+    for got, want in ((_read(i.d_mlp_grads, i.num_mlp_params), gw), (_read(i.d_grid_grads, i.num_grid_params), gg)):
+        got = got.double()
+        assert torch.isfinite(got).all()
+        cos = float((got * want).sum() / (got.norm() * want.norm()))
+        assert cos > 0.99
+        assert abs(float(got.norm() / want.norm()) - 1) < 0.05
+    cache.close()
+
+
+@pytest.mark.parametrize("n", COUNTS)
+def test_inference(ctx, n):
+    cache, mlp, grid = _cache(ctx, 16)
+    feats = random_features(n, n + 1)
+    got = cache.infer(feats).double().cpu().numpy()
+    x = _reference_inputs(cache.config, feats, grid.to(torch.float16).double(), 16)
+    want = forward(x, split_weights(mlp.double())).cpu().numpy()
+    # the emulated BF16 network: only FP32 sums and a rounding flip of a BF16 activation (2^-8 of it) differ
+    assert np.abs(got - want).max() <= 0.05 * max(1.0, np.abs(want).max())
+    cache.close()

@@ -429,27 +429,36 @@ __global__ void __launch_bounds__(WG_THREADS)
     }
 }
 
-__global__ void k_grid_backward(const float *__restrict__ feats, uint32_t n, const uint32_t *__restrict__ d_n,
-                                grid_config gc, const float *__restrict__ dXg, float *__restrict__ grid_g)
+// Hash-grid gradients: one thread per (record, level), 16 neighbouring lanes per record, so that the
+// incoming gradients are read by line. Bound by the atomics (16 per level as scalars): a feature pair is
+// one two-wide atomic, and an x pair of corners whose entries form an aligned pair (every other cell)
+// one four-wide atomic, 6 per level on average.
+__global__ void __launch_bounds__(256)
+        k_grid_backward(const float *__restrict__ feats, uint32_t n, const uint32_t *__restrict__ d_n, grid_config gc,
+                        const float *__restrict__ dXg, float *__restrict__ grid_g)
 {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if(i >= eff_count(n, d_n)) return;
+    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x, i = t >> 4, l = t & 15u;
+    if(i >= eff_count(n, d_n) || l >= gc.levels) return;
+    const float2 g = *reinterpret_cast<const float2 *>(dXg + (size_t)i * 32 + 2 * l);
+    if(g.x == 0.f && g.y == 0.f) return;
     float px, py, pz;
     normalised_pos(gc, feats + (size_t)FEAT * i, px, py, pz);
-    const uint32_t T = 1u << gc.log2_t;
-    for(uint32_t l = 0; l < gc.levels; ++l)
-    {
-        const float g0 = dXg[(size_t)i * 32 + 2 * l], g1 = dXg[(size_t)i * 32 + 2 * l + 1];
-        if(g0 == 0.f && g1 == 0.f) continue;
-        corner_iter c = level_setup(gc, l, px, py, pz);
+    const corner_iter c = level_setup(gc, l, px, py, pz);
+    float2 *tab = reinterpret_cast<float2 *>(grid_g) + ((size_t)l << gc.log2_t);
 #pragma unroll
-        for(int k = 0; k < 8; ++k)
+    for(int k = 0; k < 8; k += 2)
+    {
+        float w0, w1;
+        const uint32_t i0 = corner_index(c, k, w0), i1 = corner_index(c, k + 1, w1);
+        if((i0 ^ i1) == 1u)
         {
-            float w;
-            const uint32_t idx = corner_index(c, k, w);
-            float *p = grid_g + 2 * ((size_t)l * T + idx);
-            atomicAdd(p, w * g0);
-            atomicAdd(p + 1, w * g1);
+            const float wa = i0 & 1u ? w1 : w0, wb = i0 & 1u ? w0 : w1;
+            atomicAdd(reinterpret_cast<float4 *>(tab + (i0 & ~1u)), make_float4(wa * g.x, wa * g.y, wb * g.x, wb * g.y));
+        }
+        else
+        {
+            atomicAdd(tab + i0, make_float2(w0 * g.x, w0 * g.y));
+            atomicAdd(tab + i1, make_float2(w1 * g.x, w1 * g.y));
         }
     }
 }
@@ -629,7 +638,7 @@ vkg_status nrc_backward(vkg_nrc *c, const float *feats, const float *targets, ui
         const uint32_t wg = std::min<uint32_t>((n + WG_CHUNK - 1) / WG_CHUNK, (uint32_t)c->ctx->num_sms * 2);
         k_wgrad<<<wg, WG_THREADS, 0, st>>>(c->X, c->H, c->G, n, d_n, c->w_g);
     }
-    k_grid_backward<<<(n + 127) / 128, 128, 0, st>>>(feats, n, d_n, c->gc, c->dXg, c->grid_g);
+    k_grid_backward<<<(n + 15) / 16, 256, 0, st>>>(feats, n, d_n, c->gc, c->dXg, c->grid_g);
     return cuda_check(c->ctx, cudaGetLastError(), "nrc backward");
 }
 
