@@ -9,6 +9,7 @@
 // Work per ray (the roofline's algorithmic unit): 32 B ray in + 16 B hit out from HBM, plus
 // 96 B per node visit and 48 B per triangle test from L2/L1.
 #include "traverse.cuh"
+#include "traverse_group.cuh"
 
 #include <algorithm>
 #include <cstdlib>
@@ -60,6 +61,27 @@ __global__ void __launch_bounds__(TRACE_THREADS)
             atomicAdd(&counters[1], tests);
         }
     }
+}
+
+// eight lanes per ray (traverse_group.cuh): batches of at most GROUP_MAX_RAYS
+template<bool ANY, int STACK>
+__global__ void __launch_bounds__(TRACE_THREADS)
+        k_trace_group(const node8 *__restrict__ nodes, const tri_rec *__restrict__ tris,
+                      const vkg_ray *__restrict__ rays, uint32_t n, vkg_hit *__restrict__ hits,
+                      uint32_t *__restrict__ occluded, int cull, unsigned long long *__restrict__ counters)
+{
+    __shared__ uint2 stack[TRACE_THREADS / GROUP_LANES][group_stack_entries<STACK>];
+    const uint32_t group = threadIdx.x / GROUP_LANES, i = blockIdx.x * (TRACE_THREADS / GROUP_LANES) + group;
+    const bool active = i < n;
+    const float4 *rp = reinterpret_cast<const float4 *>(rays + (active ? i : 0u));
+    const float4 r0 = __ldg(rp), r1 = __ldg(rp + 1);
+    const trace_result r = trace_group<ANY, STACK>(active, nodes, tris, r0.x, r0.y, r0.z, r0.w, r1.x, r1.y, r1.z, r1.w,
+                                                   cull, stack[group], counters);
+    if(!active || (threadIdx.x & (GROUP_LANES - 1))) return;
+    if(ANY) occluded[i] = r.occluded ? 1u : 0u;
+    else
+        reinterpret_cast<uint4 *>(hits)[i] =
+                make_uint4(r.prim, __float_as_uint(r.t), __float_as_uint(r.u), __float_as_uint(r.v));
 }
 
 // Persistent variant: a fixed grid of warps; every lane whose ray has finished takes the next ray
@@ -485,6 +507,17 @@ vkg_status launch_trace(vkg_ctx *ctx, const vkg_bvh *bvh, const vkg_ray *d_rays,
     }
     const int cull = (flags & VKG_RAY_CULL_BACK_FACES) ? 1 : 0;
     const bool stats = (flags & VKG_RAY_COUNT_STATS) != 0;
+    const bool small = bvh->depth <= 10;
+    if(!stats && !use_persistent() && n <= GROUP_MAX_RAYS)
+    {
+        auto go = [&](auto kern) {
+            kern<<<(n * GROUP_LANES + TRACE_THREADS - 1) / TRACE_THREADS, TRACE_THREADS, 0, st>>>(
+                    bvh->d_nodes, bvh->d_tris, d_rays, n, d_hits, d_occ, cull, ctx->d_counters);
+        };
+        if(d_occ) small ? go(k_trace_group<true, 64>) : go(k_trace_group<true, (int)TRAVERSAL_STACK>);
+        else small ? go(k_trace_group<false, 64>) : go(k_trace_group<false, (int)TRAVERSAL_STACK>);
+        return cuda_check(ctx, cudaGetLastError(), "k_trace_group");
+    }
     // reordered: device word, the number of tiles the binning reordered (0: trace in the given order)
     const uint32_t *reordered = nullptr;
     const uint32_t *perm = bin_rays(ctx, bvh, d_rays, n, nullptr, flags, st, &reordered);
@@ -503,7 +536,6 @@ vkg_status launch_trace(vkg_ctx *ctx, const vkg_bvh *bvh, const vkg_ray *d_rays,
         if(perm) bin_rays_done(ctx, st);
         return cuda_check(ctx, cudaGetLastError(), "k_trace_persistent");
     }
-    const bool small = bvh->depth <= 10;
     if(d_occ)
     {
         if(stats) launch_simple<true, true>(small, grid, st, bvh, d_rays, n, nullptr, d_occ, cull, ctx->d_counters, perm, reordered);
