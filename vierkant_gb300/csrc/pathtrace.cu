@@ -1239,6 +1239,14 @@ vkg_status vkg_tracer_render(vkg_tracer *t, const vkg_scene *sc, const vkg_camer
         P.train_base = last && train_paths ? n_render : 0xFFFFFFFFu;
         const uint32_t grid = (uint32_t)std::min<size_t>((n + PT_THREADS - 1) / PT_THREADS, (size_t)ctx->num_sms * 16);
         const single_scene SS{P};
+        // Short queues of single-level scenes without alpha-tested materials are traced by groups of eight
+        // lanes (k_pt_extend_group). A wave of at most PT_GROUP_MAX_WAVE paths is always; a larger wave's
+        // later queues may be short, which only the device knows: both kernels are launched from the
+        // first bounce on (a binned queue is long), and the queue's count picks the one that runs.
+        const bool can_group = sc->bvh && !alpha;
+        const bool groups = can_group && n <= PT_GROUP_MAX_WAVE;
+        const uint32_t group_grid = (uint32_t)std::min<size_t>(((size_t)n * GROUP_LANES + PT_THREADS - 1) / PT_THREADS,
+                                                               (size_t)ctx->num_sms * 64);
         if(cache_render) VKG_TRY_CUDA(ctx, cudaMemsetAsync(cnt_q, 0, sizeof(uint32_t), st));
         k_pt_generate<<<grid, PT_THREADS, 0, st>>>(P, n, t->q_ray[0], t->q_pid[0], t->rng, t->beta_pdf, t->radiance,
                                                    t->counters, t->vcount);
@@ -1268,18 +1276,27 @@ vkg_status vkg_tracer_render(vkg_tracer *t, const vkg_scene *sc, const vkg_camer
                 const bool bin_queue = depth == 1 || (sc->tlas && depth == 2);
                 const uint32_t *perm =
                         bin_queue ? bin_rays(ctx, bounds, t->q_ray[a], n, cnt_in, 0u, st, &reordered) : nullptr;
-                if(alpha && small_stack)
-                    k_pt_extend<single_scene, 64, true><<<grid, PT_THREADS, 0, st>>>(
-                            SS, t->q_ray[a], t->q_pid[a], cnt_in, t->hits, t->hit_inst, perm, reordered, t->rng, depth);
+                const bool by_count = can_group && !groups && depth > 0 && !perm;
+                auto extend = [&](auto kern) {
+                    kern<<<grid, PT_THREADS, 0, st>>>(SS, t->q_ray[a], t->q_pid[a], cnt_in, t->hits, t->hit_inst, perm,
+                                                      reordered, t->rng, depth, by_count ? PT_GROUP_MAX_QUEUE : 0u);
+                };
+                auto extend_group = [&](auto kern) {
+                    kern<<<group_grid, PT_THREADS, 0, st>>>(SS, t->q_ray[a], cnt_in, t->hits,
+                                                            by_count ? PT_GROUP_MAX_QUEUE : 0xFFFFFFFFu);
+                };
+                constexpr int BIG = (int)TRAVERSAL_STACK;
+                using T1 = single_scene;
+                if(sc->tlas)
+                    alpha ? extend(k_pt_extend<T1, BIG, true, LEVELS_TWO>) : extend(k_pt_extend<T1, BIG, false, LEVELS_TWO>);
                 else if(alpha)
-                    k_pt_extend<single_scene, (int)TRAVERSAL_STACK, true><<<grid, PT_THREADS, 0, st>>>(
-                            SS, t->q_ray[a], t->q_pid[a], cnt_in, t->hits, t->hit_inst, perm, reordered, t->rng, depth);
-                else if(small_stack)
-                    k_pt_extend<single_scene, 64><<<grid, PT_THREADS, 0, st>>>(SS, t->q_ray[a], t->q_pid[a], cnt_in,
-                                                                                t->hits, t->hit_inst, perm, reordered);
-                else
-                    k_pt_extend<<<grid, PT_THREADS, 0, st>>>(SS, t->q_ray[a], t->q_pid[a], cnt_in, t->hits, t->hit_inst,
-                                                             perm, reordered);
+                    small_stack ? extend(k_pt_extend<T1, 64, true, LEVELS_ONE>)
+                                : extend(k_pt_extend<T1, BIG, true, LEVELS_ONE>);
+                else if(!groups)
+                    small_stack ? extend(k_pt_extend<T1, 64, false, LEVELS_ONE>)
+                                : extend(k_pt_extend<T1, BIG, false, LEVELS_ONE>);
+                if(groups || by_count)
+                    small_stack ? extend_group(k_pt_extend_group<64>) : extend_group(k_pt_extend_group<BIG>);
                 if(perm) bin_rays_done(ctx, st);
             }
             VKG_TRY_CUDA(ctx, cudaMemsetAsync(cnt_out, 0, sizeof(uint32_t), st));
@@ -1329,31 +1346,43 @@ vkg_status vkg_tracer_render(vkg_tracer *t, const vkg_scene *sc, const vkg_camer
                 const uint32_t *s_perm = (mode == MODE_PLAIN && depth <= 1)
                                                  ? bin_rays(ctx, s_bounds, t->s_ray, n, cnt_s, 0u, st, &s_reordered)
                                                  : nullptr;
-                if(alpha && small_stack)
-                    k_pt_shadow<single_scene, 64, true><<<grid, PT_THREADS, 0, st>>>(
-                            SS, t->s_ray, t->s_pid, t->s_contrib, cnt_s, t->radiance, s_perm, s_reordered, t->rng);
+                const bool by_count = can_group && !groups && depth > 0 && !s_perm;
+                auto shadow = [&](auto kern) {
+                    kern<<<grid, PT_THREADS, 0, st>>>(SS, t->s_ray, t->s_pid, t->s_contrib, cnt_s, t->radiance, s_perm,
+                                                      s_reordered, t->rng, by_count ? PT_GROUP_MAX_QUEUE : 0u);
+                };
+                auto shadow_group = [&](auto kern) {
+                    kern<<<group_grid, PT_THREADS, 0, st>>>(SS, t->s_ray, t->s_pid, t->s_contrib, cnt_s, t->radiance,
+                                                            by_count ? PT_GROUP_MAX_QUEUE : 0xFFFFFFFFu);
+                };
+                constexpr int BIG = (int)TRAVERSAL_STACK;
+                using T1 = single_scene;
+                if(sc->tlas)
+                    alpha ? shadow(k_pt_shadow<T1, BIG, true, LEVELS_TWO>) : shadow(k_pt_shadow<T1, BIG, false, LEVELS_TWO>);
                 else if(alpha)
-                    k_pt_shadow<single_scene, (int)TRAVERSAL_STACK, true><<<grid, PT_THREADS, 0, st>>>(
-                            SS, t->s_ray, t->s_pid, t->s_contrib, cnt_s, t->radiance, s_perm, s_reordered, t->rng);
-                else if(small_stack)
-                    k_pt_shadow<single_scene, 64><<<grid, PT_THREADS, 0, st>>>(SS, t->s_ray, t->s_pid, t->s_contrib,
-                                                                                cnt_s, t->radiance, s_perm, s_reordered);
-                else
-                    k_pt_shadow<<<grid, PT_THREADS, 0, st>>>(SS, t->s_ray, t->s_pid, t->s_contrib, cnt_s, t->radiance,
-                                                             s_perm, s_reordered);
+                    small_stack ? shadow(k_pt_shadow<T1, 64, true, LEVELS_ONE>)
+                                : shadow(k_pt_shadow<T1, BIG, true, LEVELS_ONE>);
+                else if(!groups)
+                    small_stack ? shadow(k_pt_shadow<T1, 64, false, LEVELS_ONE>)
+                                : shadow(k_pt_shadow<T1, BIG, false, LEVELS_ONE>);
+                if(groups || by_count)
+                    small_stack ? shadow_group(k_pt_shadow_group<64>) : shadow_group(k_pt_shadow_group<BIG>);
                 if(s_perm) bin_rays_done(ctx, st);
             }
             if(cnt_l && !empty)
             {
-                if(alpha && small_stack)
-                    k_pt_light_shadow<single_scene, 64, true><<<grid, PT_THREADS, 0, st>>>(SS, lq, t->radiance, t->rng);
+                auto light = [&](auto kern) { kern<<<grid, PT_THREADS, 0, st>>>(SS, lq, t->radiance, t->rng); };
+                constexpr int BIG = (int)TRAVERSAL_STACK;
+                using T1 = single_scene;
+                if(sc->tlas)
+                    alpha ? light(k_pt_light_shadow<T1, BIG, true, LEVELS_TWO>)
+                          : light(k_pt_light_shadow<T1, BIG, false, LEVELS_TWO>);
                 else if(alpha)
-                    k_pt_light_shadow<single_scene, (int)TRAVERSAL_STACK, true>
-                            <<<grid, PT_THREADS, 0, st>>>(SS, lq, t->radiance, t->rng);
-                else if(small_stack)
-                    k_pt_light_shadow<single_scene, 64><<<grid, PT_THREADS, 0, st>>>(SS, lq, t->radiance);
+                    small_stack ? light(k_pt_light_shadow<T1, 64, true, LEVELS_ONE>)
+                                : light(k_pt_light_shadow<T1, BIG, true, LEVELS_ONE>);
                 else
-                    k_pt_light_shadow<<<grid, PT_THREADS, 0, st>>>(SS, lq, t->radiance);
+                    small_stack ? light(k_pt_light_shadow<T1, 64, false, LEVELS_ONE>)
+                                : light(k_pt_light_shadow<T1, BIG, false, LEVELS_ONE>);
             }
             k_pt_tally<<<1, 1, 0, st>>>(cnt_in, cnt_s, cnt_l, t->totals);
             a = 1 - a;

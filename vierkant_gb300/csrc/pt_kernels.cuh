@@ -13,6 +13,7 @@
 #include "texture.cuh"
 #include "tlas.cuh"
 #include "traverse.cuh"
+#include "traverse_group.cuh"
 
 #include <cmath>
 #include <limits>
@@ -378,16 +379,32 @@ __global__ void __launch_bounds__(PT_THREADS)
     if(blockIdx.x == 0 && threadIdx.x == 0) counters[0] = n;
 }
 
+// The levels of a scene's BVH that a tracer is compiled for: one that holds both traversals spills in
+// the shorter (96 bytes a thread in the 64-entry k_pt_extend), so only job tables, whose jobs
+// may be of either kind, choose per path.
+enum scene_levels : int
+{
+    LEVELS_ANY = 0,
+    LEVELS_ONE = 1,
+    LEVELS_TWO = 2
+};
+template<int LEVELS>
+__device__ __forceinline__ bool two_level(const pt_params &P)
+{
+    return LEVELS == LEVELS_ANY ? P.two_level != 0u : LEVELS == LEVELS_TWO;
+}
+
 // ALPHA: the scene has alpha-tested materials (alpha_filter); rng and depth then give each ray its
 // segment's first uniform
-template<class J, int STACK = (int)TRAVERSAL_STACK, bool ALPHA = false>
+template<class J, int STACK = (int)TRAVERSAL_STACK, bool ALPHA = false, int LEVELS = LEVELS_ANY>
 __global__ void __launch_bounds__(PT_THREADS, STACK <= 64 ? 8 : 6) // 64 / 85 registers
         k_pt_extend(J S, const vkg_ray *__restrict__ q_ray, const uint32_t *__restrict__ q_pid,
                     const uint32_t *__restrict__ count, vkg_hit *__restrict__ hits, uint32_t *__restrict__ hit_inst,
                     const uint32_t *__restrict__ perm = nullptr, const uint32_t *__restrict__ reordered = nullptr,
-                    const uint64_t *__restrict__ rng = nullptr, uint32_t depth = 0)
+                    const uint64_t *__restrict__ rng = nullptr, uint32_t depth = 0, uint32_t groups_up_to = 0)
 {
     const uint32_t n = *count;
+    if(n <= groups_up_to) return; // k_pt_extend_group traces it
     const uint32_t stride = gridDim.x * blockDim.x;
     // a binned queue (bin_rays): position j traces entry perm[j]; results stay in the entry's slot
     if(perm && *reordered == 0u) perm = nullptr;
@@ -401,7 +418,7 @@ __global__ void __launch_bounds__(PT_THREADS, STACK <= 64 ? 8 : 6) // 64 / 85 re
         using F = std::conditional_t<ALPHA, alpha_filter, no_filter>;
         F f{};
         if constexpr(ALPHA) f = alpha_filter{&P, 0ull, peek_uniform(P, rng[pid], S.inc(pid), depth), 0u, false};
-        if(P.two_level)
+        if(two_level<LEVELS>(P))
         {
             const tlas_result r = trace_tlas<false, F>(P.tl_nodes, P.tl_inst, P.tl_blas, r0.x, r0.y, r0.z, r0.w, r1.x,
                                                        r1.y, r1.z, r1.w, CULL_BACK_UNLESS_TWOSIDED, f);
@@ -415,6 +432,37 @@ __global__ void __launch_bounds__(PT_THREADS, STACK <= 64 ? 8 : 6) // 64 / 85 re
                                                            r1.w, CULL_BACK_UNLESS_TWOSIDED, v, t, nullptr, f);
         reinterpret_cast<uint4 *>(hits)[i] =
                 make_uint4(r.prim, __float_as_uint(r.t), __float_as_uint(r.u), __float_as_uint(r.v));
+    }
+}
+
+// The same for short queues, eight lanes per ray (traverse_group.cuh); single-level scenes without
+// alpha-tested materials, queues of at most `up_to` rays (k_pt_extend traces longer ones).
+// The bounds: a 720p-like Cornell frame of one sample and six segments takes 542 against 1,065 us at 58,101
+// paths, 921 against 1,283 us at 256,000 with every queue traced by groups; at 516,000 the first two
+// queues are faster with a thread per ray and the later ones by groups (1,478 us; none 1,654, all 1,517).
+// Incoherent queues break even at 64,000 to 190,000 rays.
+constexpr uint32_t PT_GROUP_MAX_WAVE = 1u << 18, PT_GROUP_MAX_QUEUE = 1u << 17;
+template<int STACK>
+__global__ void __launch_bounds__(PT_THREADS)
+        k_pt_extend_group(single_scene S, const vkg_ray *__restrict__ q_ray, const uint32_t *__restrict__ count,
+                          vkg_hit *__restrict__ hits, uint32_t up_to)
+{
+    __shared__ uint2 stack[PT_THREADS / GROUP_LANES][group_stack_entries<STACK>];
+    constexpr uint32_t PER = PT_THREADS / GROUP_LANES;
+    const pt_params &P = S.params(0u);
+    const uint32_t n = *count, group = threadIdx.x / GROUP_LANES;
+    if(n > up_to) return;
+    for(uint32_t base = blockIdx.x * PER; base < n; base += gridDim.x * PER)
+    {
+        const uint32_t i = base + group;
+        const bool active = i < n;
+        const float4 *rp = reinterpret_cast<const float4 *>(q_ray + (active ? i : base));
+        const float4 r0 = __ldg(rp), r1 = __ldg(rp + 1);
+        const trace_result r = trace_group<false, STACK>(active, P.nodes, P.tris, r0.x, r0.y, r0.z, r0.w, r1.x, r1.y,
+                                                         r1.z, r1.w, CULL_BACK_UNLESS_TWOSIDED, stack[group], nullptr);
+        if(active && !(threadIdx.x & (GROUP_LANES - 1)))
+            reinterpret_cast<uint4 *>(hits)[i] =
+                    make_uint4(r.prim, __float_as_uint(r.t), __float_as_uint(r.u), __float_as_uint(r.v));
     }
 }
 
@@ -1206,14 +1254,16 @@ __global__ void __launch_bounds__(PT_THREADS)
 }
 
 // ALPHA: alpha-tested materials (alpha_filter), each candidate's uniform hashed from rng[path]
-template<class J, int STACK = (int)TRAVERSAL_STACK, bool ALPHA = false>
+template<class J, int STACK = (int)TRAVERSAL_STACK, bool ALPHA = false, int LEVELS = LEVELS_ANY>
 __global__ void __launch_bounds__(PT_THREADS, STACK <= 64 ? 8 : 6) // 64 / 85 registers
         k_pt_shadow(J S, const vkg_ray *__restrict__ s_ray, const uint32_t *__restrict__ s_pid,
                     const float4 *__restrict__ s_contrib, const uint32_t *__restrict__ count,
                     float4 *__restrict__ radiance, const uint32_t *__restrict__ perm = nullptr,
-                    const uint32_t *__restrict__ reordered = nullptr, const uint64_t *__restrict__ rng = nullptr)
+                    const uint32_t *__restrict__ reordered = nullptr, const uint64_t *__restrict__ rng = nullptr,
+                    uint32_t groups_up_to = 0)
 {
     const uint32_t n = *count;
+    if(n <= groups_up_to) return; // k_pt_shadow_group traces it
     const uint32_t stride = gridDim.x * blockDim.x;
     // a binned queue (bin_rays): position j tests entry perm[j] (each path has one entry per launch)
     if(perm && *reordered == 0u) perm = nullptr;
@@ -1229,7 +1279,7 @@ __global__ void __launch_bounds__(PT_THREADS, STACK <= 64 ? 8 : 6) // 64 / 85 re
         F f{};
         if constexpr(ALPHA) f = alpha_filter{&P, rng[s_pid[i]], 0.f, ALPHA_SALT_SHADOW, false};
         bool occluded;
-        if(P.two_level)
+        if(two_level<LEVELS>(P))
             occluded = trace_tlas<true, F>(P.tl_nodes, P.tl_inst, P.tl_blas, r0.x, r0.y, r0.z, r0.w, r1.x, r1.y, r1.z,
                                            r1.w, cull, f)
                                .occluded;
@@ -1252,6 +1302,41 @@ __global__ void __launch_bounds__(PT_THREADS, STACK <= 64 ? 8 : 6) // 64 / 85 re
     }
 }
 
+// the same for short queues, eight lanes per ray (k_pt_extend_group)
+template<int STACK>
+__global__ void __launch_bounds__(PT_THREADS)
+        k_pt_shadow_group(single_scene S, const vkg_ray *__restrict__ s_ray, const uint32_t *__restrict__ s_pid,
+                          const float4 *__restrict__ s_contrib, const uint32_t *__restrict__ count,
+                          float4 *__restrict__ radiance, uint32_t up_to)
+{
+    __shared__ uint2 stack[PT_THREADS / GROUP_LANES][group_stack_entries<STACK>];
+    constexpr uint32_t PER = PT_THREADS / GROUP_LANES;
+    const pt_params &P = S.params(0u);
+    const uint32_t n = *count, group = threadIdx.x / GROUP_LANES;
+    if(n > up_to) return;
+    for(uint32_t base = blockIdx.x * PER; base < n; base += gridDim.x * PER)
+    {
+        const bool active = base + group < n;
+        const uint32_t i = active ? base + group : base;
+        const float4 *rp = reinterpret_cast<const float4 *>(s_ray + i);
+        const float4 r0 = __ldg(rp), r1 = __ldg(rp + 1);
+        const float4 c = s_contrib[i];
+        const bool occluded = trace_group<true, STACK>(active, P.nodes, P.tris, r0.x, r0.y, r0.z, r0.w, r1.x, r1.y,
+                                                       r1.z, r1.w, c.w != 0.f ? CULL_BACK : CULL_NONE, stack[group],
+                                                       nullptr)
+                                      .occluded;
+        if(active && !occluded && !(threadIdx.x & (GROUP_LANES - 1)))
+        {
+            const uint32_t pid = s_pid[i];
+            float4 L = radiance[pid];
+            L.x += c.x;
+            L.y += c.y;
+            L.z += c.z;
+            radiance[pid] = L;
+        }
+    }
+}
+
 // light-NEE visibility (transmittance_test, visibility_test.slang:94-131): 0 at the first opaque
 // surface on the segment, else the product of transmission x base colour over the transmissive
 // surfaces it crosses; null surfaces pass unattenuated. Scenes without transmissive materials take one any-hit query; single-level
@@ -1260,7 +1345,7 @@ __global__ void __launch_bounds__(PT_THREADS, STACK <= 64 ? 8 : 6) // 64 / 85 re
 // environment shadow kernel, so each path's radiance has one writer at a time.
 constexpr int PT_MAX_CROSSINGS = 32;
 
-template<class J, int STACK = (int)TRAVERSAL_STACK, bool ALPHA = false>
+template<class J, int STACK = (int)TRAVERSAL_STACK, bool ALPHA = false, int LEVELS = LEVELS_ANY>
 __global__ void __launch_bounds__(PT_THREADS, STACK <= 64 ? 8 : 6) // 64 / 85 registers
         k_pt_light_shadow(J S, light_queue lq, float4 *__restrict__ radiance, const uint64_t *__restrict__ rng = nullptr)
 {
@@ -1282,7 +1367,7 @@ __global__ void __launch_bounds__(PT_THREADS, STACK <= 64 ? 8 : 6) // 64 / 85 re
         if constexpr(ALPHA) f = alpha_filter{&P, rng[pid], 0.f, ALPHA_SALT_LIGHT_SHADOW, true};
         if(!P.transmissive)
         {
-            const bool occ = P.two_level ? trace_tlas<true, F>(P.tl_nodes, P.tl_inst, P.tl_blas, r0.x, r0.y, r0.z, r0.w,
+            const bool occ = two_level<LEVELS>(P) ? trace_tlas<true, F>(P.tl_nodes, P.tl_inst, P.tl_blas, r0.x, r0.y, r0.z, r0.w,
                                                                r1.x, r1.y, r1.z, r1.w, cull, f)
                                                    .occluded
                                          : trace_ray<true, false, STACK, F>(P.nodes, P.tris, r0.x, r0.y, r0.z, r0.w,
@@ -1291,7 +1376,7 @@ __global__ void __launch_bounds__(PT_THREADS, STACK <= 64 ? 8 : 6) // 64 / 85 re
                                                    .occluded;
             if(occ) T = f3(0.f, 0.f, 0.f);
         }
-        else if(!P.two_level)
+        else if(!two_level<LEVELS>(P))
         {
             // Beer-Lambert through transmissive volumes: optical depth -sigma_t t at an entry (front
             // face), +sigma_t t at an exit, clamped at 0 (visibility_test.slang:123-129, :161-162)
@@ -1327,7 +1412,7 @@ __global__ void __launch_bounds__(PT_THREADS, STACK <= 64 ? 8 : 6) // 64 / 85 re
             {
                 uint32_t prim, mat, inst = 0;
                 float t, hu = 0.f, hv = 0.f;
-                if(P.two_level)
+                if(two_level<LEVELS>(P))
                 {
                     const tlas_result r = trace_tlas<false, F>(P.tl_nodes, P.tl_inst, P.tl_blas, r0.x, r0.y, r0.z,
                                                                tmin, r1.x, r1.y, r1.z, r1.w, cull, f);
