@@ -41,3 +41,21 @@ def test_build_equals_the_cpu_statement(ctx, n, kind, leaf_max):
     assert _device_bytes(inf.d_nodes, 96 * inf.num_nodes) == cb.node_bytes()
     assert _device_bytes(inf.d_tris, 48 * n) == cb.tri_bytes()
     b.close()
+
+
+def test_destroying_a_bvh_waits_for_its_queries(ctx):
+    """a BVH destroyed right after a query was queued on it: the query still reads the tree (a destroy
+    that did not wait handed the memory back under it)"""
+    xyz, idx = _mesh(60000, "spread")
+    x, i = torch.from_numpy(xyz).cuda(), torch.from_numpy(idx.astype(np.int32)).cuda()
+    g = torch.Generator(device="cuda").manual_seed(1)
+    rays = torch.randn((1_000_000, 8), generator=g, device="cuda")
+    rays[:, 3], rays[:, 7] = 0.0, 1e30
+    keep = BVH(ctx, x, i)
+    want = keep.closest_hit(rays)
+    for _ in range(3):
+        b = BVH(ctx, x, i)
+        got = b.closest_hit(rays)
+        b.close()
+        assert torch.equal(got, want)
+    keep.close()

@@ -569,9 +569,31 @@ __global__ void k_tri_records(const float *__restrict__ xyz, uint32_t nv, const 
 }
 
 template<typename T>
-cudaError_t dalloc(T **p, size_t count, cudaStream_t s)
+cudaError_t dalloc(vkg_ctx *ctx, T **p, size_t count, cudaStream_t s)
 {
-    return cudaMallocAsync(reinterpret_cast<void **>(p), count * sizeof(T) + 16, s);
+    return ctx_alloc(ctx, reinterpret_cast<void **>(p), count * sizeof(T) + 16, s);
+}
+
+// hands out 256-byte aligned pieces of one allocation (of no allocation yet: only adds up their sizes)
+struct arena
+{
+    uintptr_t base = 0;
+    size_t used = 0;
+    template<typename T>
+    void take(T *&p, size_t count)
+    {
+        p = reinterpret_cast<T *>(base + used);
+        used += (count * sizeof(T) + 255) & ~size_t(255);
+    }
+};
+
+// what a build starts from: [0..5] the empty scene box (ordered uints: +inf, -inf), [6] error bits of the
+// primitives, [8..10] the collapse's info, [11] its grid barrier, [12] the margin
+__global__ void k_build_init(uint32_t *__restrict__ visits, uint32_t n, uint32_t *__restrict__ small)
+{
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if(i < n) visits[i] = 0u;
+    if(i < 16) small[i] = i < 3 ? 0xFF800000u : (i < 6 ? 0x007FFFFFu : 0u);
 }
 
 // ---- instances (two-level BVH) -------------------------------------------------------------------
@@ -773,49 +795,55 @@ vkg_status build_core(vkg_ctx *ctx, vkg_bvh *bvh, uint32_t n, uint32_t leaf_max,
     cudaEventCreate(&ev1);
     cudaEventRecord(ev0, st);
 
-    // scratch
-    box6 *tbox = nullptr, *lbox = nullptr, *ibox = nullptr;
-    uint32_t *keys0 = nullptr, *keys1 = nullptr, *vals0 = nullptr, *vals1 = nullptr, *counts = nullptr;
-    uint32_t *first = nullptr, *iparent = nullptr, *lparent = nullptr, *visits = nullptr, *node_ref = nullptr,
-             *block_sum = nullptr, *small = nullptr;
-    bvh2_node *tree = nullptr;
-    node8 *nodes_tmp = nullptr;
-    float *d_margin = nullptr;
+    // scratch, one allocation
+    box6 *tbox, *lbox, *ibox;
+    uint32_t *keys0, *keys1, *vals0, *vals1, *counts, *first, *iparent, *lparent, *visits, *node_ref, *block_sum, *small;
+    bvh2_node *tree;
+    node8 *nodes_tmp;
     const uint32_t nblocks = (n + SORT_TILE - 1) / SORT_TILE;
     const uint32_t ni = n > 1 ? n - 1 : 1;
     const uint32_t capacity = n + 8;
+    arena mem;
+    auto lay_out = [&]() {
+        mem.used = 0;
+        mem.take(tbox, n);
+        mem.take(lbox, n);
+        mem.take(ibox, ni);
+        mem.take(keys0, n);
+        mem.take(keys1, n);
+        mem.take(vals0, n);
+        mem.take(vals1, n);
+        mem.take(counts, (size_t)256 * nblocks);
+        mem.take(tree, ni);
+        mem.take(first, ni);
+        mem.take(iparent, ni);
+        mem.take(lparent, n);
+        mem.take(visits, ni);
+        mem.take(node_ref, capacity);
+        mem.take(nodes_tmp, capacity);
+        mem.take(block_sum, (size_t)ctx->num_sms);
+        mem.take(small, 16);
+    };
+    lay_out();
+    void *scratch = nullptr;
     cudaError_t e = cudaSuccess;
     auto chk = [&](cudaError_t x) {
         if(e == cudaSuccess) e = x;
     };
-    chk(dalloc(&tbox, n, st));
-    chk(dalloc(&lbox, n, st));
-    chk(dalloc(&ibox, ni, st));
-    chk(dalloc(&keys0, n, st));
-    chk(dalloc(&keys1, n, st));
-    chk(dalloc(&vals0, n, st));
-    chk(dalloc(&vals1, n, st));
-    chk(dalloc(&counts, (size_t)256 * nblocks, st));
-    chk(dalloc(&tree, ni, st));
-    chk(dalloc(&first, ni, st));
-    chk(dalloc(&block_sum, (size_t)ctx->num_sms, st));
-    chk(dalloc(&iparent, ni, st));
-    chk(dalloc(&lparent, n, st));
-    chk(dalloc(&visits, ni, st));
-    chk(dalloc(&node_ref, capacity, st));
-    chk(dalloc(&nodes_tmp, capacity, st));
-    chk(dalloc(&small, 16, st));
-    chk(dalloc(&d_margin, 1, st));
-    chk(dalloc(&bvh->d_morton, n, st));
-    chk(dalloc(&bvh->d_sorted, n, st));
+    chk(ctx_alloc(ctx, &scratch, mem.used, st));
+    if(e == cudaSuccess) chk(dalloc(ctx, &bvh->d_morton, n, st));
+    if(e == cudaSuccess) chk(dalloc(ctx, &bvh->d_sorted, n, st));
     if(e != cudaSuccess)
+    {
+        if(scratch) cudaFreeAsync(scratch, st);
+        cudaEventDestroy(ev0);
+        cudaEventDestroy(ev1);
+        cudaGetLastError();
         return set_error(ctx, VKG_ERR_OUT_OF_MEMORY, "BVH build: device allocation failed (%s)", cudaGetErrorString(e));
-    // small[0..5] scene box (ordered uints), [6] error flags, [8..10] collapse info
-    uint32_t init[16] = {0xFF800000u, 0xFF800000u, 0xFF800000u, 0x007FFFFFu, 0x007FFFFFu, 0x007FFFFFu, 0, 0,
-                         0,           0,           0,           0,           0,           0,           0, 0};
-    // +inf encodes as 0xFF800000, -inf as 0x007FFFFF
-    chk(cudaMemcpyAsync(small, init, sizeof(init), cudaMemcpyHostToDevice, st));
-    chk(cudaMemsetAsync(visits, 0, sizeof(uint32_t) * ni, st));
+    }
+    mem.base = reinterpret_cast<uintptr_t>(scratch);
+    lay_out();
+    k_build_init<<<(std::max(ni, 16u) + 255) / 256, 256, 0, st>>>(visits, ni, small);
 
     const int T = 256;
     const uint32_t g = (n + T - 1) / T;
@@ -838,21 +866,19 @@ vkg_status build_core(vkg_ctx *ctx, vkg_bvh *bvh, uint32_t n, uint32_t leaf_max,
         k_refit<<<g, T, 0, st>>>(lparent, iparent, tree, lbox, ibox, visits, n);
     }
     collapse_args A{tree,     first,     ibox,      lbox,      n,        leaf_max, capacity, small,
-                    node_ref, nodes_tmp, small + 8, block_sum, d_margin};
+                    node_ref, nodes_tmp, small + 8, block_sum, reinterpret_cast<float *>(small + 12)};
     chk(launch_collapse(A, (uint32_t)ctx->num_sms, st));
     make_records(static_cast<const uint32_t *>(vin));
     chk(cudaGetLastError());
 
     uint32_t info[16];
-    float margin = 0.f;
     chk(cudaMemcpyAsync(info, small, sizeof(info), cudaMemcpyDeviceToHost, st));
-    chk(cudaMemcpyAsync(&margin, d_margin, sizeof(float), cudaMemcpyDeviceToHost, st));
     chk(cudaStreamSynchronize(st));
     if(e == cudaSuccess)
     {
         bvh->num_nodes = info[8];
         bvh->depth = info[9];
-        bvh->margin = margin;
+        std::memcpy(&bvh->margin, &info[12], 4);
         for(int a = 0; a < 3; ++a)
         {
             uint32_t lo = info[a], hi = info[3 + a];
@@ -861,16 +887,12 @@ vkg_status build_core(vkg_ctx *ctx, vkg_bvh *bvh, uint32_t n, uint32_t leaf_max,
             std::memcpy(&bvh->scene_min[a], &lb, 4);
             std::memcpy(&bvh->scene_max[a], &hb, 4);
         }
-        chk(dalloc(&bvh->d_nodes, bvh->num_nodes, st));
+        chk(dalloc(ctx, &bvh->d_nodes, bvh->num_nodes, st));
         if(e == cudaSuccess)
             chk(cudaMemcpyAsync(bvh->d_nodes, nodes_tmp, sizeof(node8) * bvh->num_nodes, cudaMemcpyDeviceToDevice,
                                 st));
     }
-    for(void *p: {(void *)tbox, (void *)lbox, (void *)ibox, (void *)keys0, (void *)keys1, (void *)vals0,
-                  (void *)vals1, (void *)counts, (void *)tree, (void *)first, (void *)block_sum,
-                  (void *)iparent, (void *)lparent, (void *)visits, (void *)node_ref, (void *)nodes_tmp,
-                  (void *)small, (void *)d_margin})
-        cudaFreeAsync(p, st);
+    cudaFreeAsync(scratch, st);
     cudaEventRecord(ev1, st);
     chk(cudaEventSynchronize(ev1));
     cudaEventElapsedTime(&bvh->build_ms, ev0, ev1);
@@ -919,7 +941,7 @@ extern "C" vkg_status vkg_bvh_build(vkg_ctx *ctx, const float *d_xyz, uint32_t n
         return VKG_OK;
     }
     const uint32_t n = num_tris;
-    if(cudaMallocAsync(reinterpret_cast<void **>(&bvh->d_tris), n * sizeof(tri_rec) + 16, st) != cudaSuccess)
+    if(dalloc(ctx, &bvh->d_tris, n, st) != cudaSuccess)
     {
         vkg_bvh_destroy(ctx, bvh);
         return set_error(ctx, VKG_ERR_OUT_OF_MEMORY, "vkg_bvh_build: device allocation failed");
@@ -975,6 +997,7 @@ extern "C" vkg_status vkg_bvh_destroy(vkg_ctx *ctx, vkg_bvh *bvh)
 {
     if(!bvh) return VKG_OK;
     if(ctx) bind_device(ctx);
+    cudaDeviceSynchronize(); // cudaFree does not wait for work that still reads stream-ordered memory
     cudaFree(bvh->d_nodes);
     cudaFree(bvh->d_tris);
     cudaFree(bvh->d_morton);
@@ -1028,27 +1051,27 @@ extern "C" vkg_status vkg_tlas_build(vkg_ctx *ctx, const vkg_bvh *const *blas, u
     cudaError_t e = cudaSuccess;
     if(num_blas)
     {
-        e = cudaMalloc(&t->d_blas, num_blas * sizeof(blas_ref));
-        if(e == cudaSuccess) e = cudaMalloc(&d_bb, num_blas * sizeof(blas_box));
+        e = dalloc(ctx, &t->d_blas, num_blas, st);
+        if(e == cudaSuccess) e = dalloc(ctx, &d_bb, num_blas, st);
         if(e == cudaSuccess)
             e = cudaMemcpyAsync(t->d_blas, refs.data(), num_blas * sizeof(blas_ref), cudaMemcpyHostToDevice, st);
         if(e == cudaSuccess) e = cudaMemcpyAsync(d_bb, boxes.data(), num_blas * sizeof(blas_box), cudaMemcpyHostToDevice, st);
     }
     if(e == cudaSuccess && num_instances)
     {
-        e = cudaMalloc(&t->d_inst, num_instances * sizeof(inst_rec));
-        if(e == cudaSuccess) e = cudaMalloc(&t->d_inst_by_id, num_instances * sizeof(inst_rec));
+        e = dalloc(ctx, &t->d_inst, num_instances, st);
+        if(e == cudaSuccess) e = dalloc(ctx, &t->d_inst_by_id, num_instances, st);
     }
     if(e != cudaSuccess)
     {
-        cudaFree(d_bb);
+        if(d_bb) cudaFreeAsync(d_bb, st);
         vkg_tlas_destroy(ctx, t);
         return cuda_check(ctx, e, "vkg_tlas_build");
     }
     if(num_instances == 0)
     {
         cudaStreamSynchronize(st);
-        cudaFree(d_bb);
+        if(d_bb) cudaFreeAsync(d_bb, st);
         *out = t;
         return VKG_OK;
     }
@@ -1065,7 +1088,7 @@ extern "C" vkg_status vkg_tlas_build(vkg_ctx *ctx, const vkg_bvh *const *blas, u
                 k_instance_records<<<g, T, 0, st>>>(d_instances, sorted, n, num_blas, t->d_inst, t->d_inst_by_id);
             },
             err_bits);
-    cudaFree(d_bb);
+    if(d_bb) cudaFreeAsync(d_bb, st);
     t->top.num_tris = n;
     if(s == VKG_OK && (err_bits & BUILD_ERR_INDEX))
         s = set_error(ctx, VKG_ERR_INVALID_ARGUMENT, "vkg_tlas_build: an instance's BLAS index >= %u", num_blas);
@@ -1107,6 +1130,7 @@ extern "C" vkg_status vkg_tlas_destroy(vkg_ctx *ctx, vkg_tlas *t)
 {
     if(!t) return VKG_OK;
     if(ctx) bind_device(ctx);
+    cudaDeviceSynchronize(); // as in vkg_bvh_destroy
     cudaFree(t->top.d_nodes);
     cudaFree(t->top.d_morton);
     cudaFree(t->top.d_sorted);
@@ -1142,7 +1166,6 @@ struct noalloc_scratch
     uint32_t node_ref[NOALLOC_MAX_TRIS + 8];
     uint32_t morton[NOALLOC_MAX_TRIS];
     uint32_t small[16];
-    float margin[4];
 };
 
 // ~2.2 MB, held by every GPU that loads libvkg until the process exits. Host code must not use the
@@ -1170,19 +1193,6 @@ vkg_status noalloc_scratch_for_current_device(noalloc_scratch **out)
     return VKG_OK;
 }
 
-// the scratch keeps the previous call's contents: reset what the build expects to start at zero
-__global__ void k_noalloc_reset(noalloc_scratch *s, uint32_t n)
-{
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if(i < n) s->visits[i] = 0u;
-    if(i < 16)
-    {
-        const uint32_t init = i < 3 ? 0xFF800000u : (i < 6 ? 0x007FFFFFu : 0u); // +inf / -inf encodings, flags
-        s->small[i] = init;
-    }
-    if(i == 0) s->margin[0] = 0.f;
-}
-
 // info words: [0] nodes, [1] depth, [2] error flags (1 = index >= num_vertices, 2 = node capacity),
 // [3] margin (float bits), [4..6] scene min, [7..9] scene max (float bits)
 constexpr uint32_t NOALLOC_FLAG_DEPTH = 4u;
@@ -1197,7 +1207,7 @@ __global__ void k_noalloc_info(const noalloc_scratch *s, uint32_t n, uint32_t *i
     info[2] = s->small[10] | s->small[6];
     // deeper than the traversal stack supports (the limit vkg_bvh_build enforces)
     if(s->small[9] > (TRAVERSAL_STACK - 1) / 7 + 1) info[2] |= NOALLOC_FLAG_DEPTH;
-    info[3] = __float_as_uint(s->margin[0]);
+    info[3] = s->small[12];
     for(int a = 0; a < 3; ++a)
     {
         info[4 + a] = __float_as_uint(fdec(s->small[a]));
@@ -1232,7 +1242,8 @@ extern "C" vkg_status vkg_bvh_build_noalloc(const float *d_xyz, uint32_t num_ver
     const int T = 256;
     const uint32_t g = (n + T - 1) / T;
     const uint32_t nblocks = (n + SORT_TILE - 1) / SORT_TILE;
-    k_noalloc_reset<<<(n + 15 + T - 1) / T, T, 0, st>>>(s, n);
+    // (the scratch keeps the previous call's contents)
+    k_build_init<<<(n + 15 + T - 1) / T, T, 0, st>>>(s->visits, n, s->small);
     k_tri_boxes<<<g, T, 0, st>>>(d_xyz, num_vertices, d_indices, n, s->tbox, s->small, s->small + 6);
     k_morton<<<g, T, 0, st>>>(s->tbox, n, s->small, s->keys0, s->vals0, s->morton);
     uint32_t *kin = s->keys0, *kout = s->keys1, *vin = s->vals0, *vout = s->vals1;
@@ -1252,7 +1263,7 @@ extern "C" vkg_status vkg_bvh_build_noalloc(const float *d_xyz, uint32_t num_ver
     }
     const uint32_t capacity = std::min<uint32_t>(node_capacity, NOALLOC_MAX_TRIS + 8);
     collapse_args A{s->tree, s->first, s->ibox, s->lbox, n, leaf_max, capacity, s->small, s->node_ref,
-                    static_cast<node8 *>(d_nodes), s->small + 8, nullptr, s->margin};
+                    static_cast<node8 *>(d_nodes), s->small + 8, nullptr, reinterpret_cast<float *>(s->small + 12)};
     if(launch_collapse(A, 1, st) != cudaSuccess) return VKG_ERR_CUDA;
     k_tri_records<<<g, T, 0, st>>>(d_xyz, num_vertices, d_indices, vin, n, static_cast<tri_rec *>(d_tris));
     k_noalloc_info<<<1, 1, 0, st>>>(s, n, d_info);

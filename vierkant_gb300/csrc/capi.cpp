@@ -69,6 +69,17 @@ vkg_status vkg_ctx_create(int device, vkg_ctx **out)
         delete ctx;
         return VKG_ERR_CUDA;
     }
+    cudaMemPoolProps props{};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = device;
+    uint64_t keep = vkg::POOL_KEEP;
+    if(cudaMemPoolCreate(&ctx->pool, &props) != cudaSuccess ||
+       cudaMemPoolSetAttribute(ctx->pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess)
+    {
+        vkg_ctx_destroy(ctx);
+        return VKG_ERR_CUDA;
+    }
     *out = ctx;
     return VKG_OK;
 }
@@ -90,6 +101,7 @@ vkg_status vkg_ctx_destroy(vkg_ctx *ctx)
     cudaFree(ctx->bins.tile_counts);
     cudaFree(ctx->bins.bin_totals);
     if(ctx->bins.done) cudaEventDestroy(ctx->bins.done);
+    if(ctx->pool) cudaMemPoolDestroy(ctx->pool); // (memory still allocated from it stays valid until freed)
     delete ctx;
     return VKG_OK;
 }
