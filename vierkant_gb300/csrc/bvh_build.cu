@@ -812,7 +812,6 @@ vkg_status build_core(vkg_ctx *ctx, vkg_bvh *bvh, uint32_t n, uint32_t leaf_max,
     uint32_t *keys0, *keys1, *vals0, *vals1, *counts, *first, *iparent, *lparent, *visits, *node_ref, *block_sum, *small;
     bvh2_node *tree;
     node8 *nodes_tmp;
-    const uint32_t nblocks = (n + SORT_TILE - 1) / SORT_TILE;
     const uint32_t ni = n > 1 ? n - 1 : 1;
     const uint32_t capacity = n + 8;
     arena mem;
@@ -825,7 +824,7 @@ vkg_status build_core(vkg_ctx *ctx, vkg_bvh *bvh, uint32_t n, uint32_t leaf_max,
         mem.take(keys1, n);
         mem.take(vals0, n);
         mem.take(vals1, n);
-        mem.take(counts, (size_t)256 * nblocks);
+        mem.take(counts, sort_count_words(n));
         mem.take(tree, ni);
         mem.take(first, ni);
         mem.take(iparent, ni);
@@ -862,14 +861,7 @@ vkg_status build_core(vkg_ctx *ctx, vkg_bvh *bvh, uint32_t n, uint32_t leaf_max,
     make_boxes(tbox, small, small + 6);
     k_morton<<<g, T, 0, st>>>(tbox, n, small, keys0, vals0, bvh->d_morton);
     uint32_t *kin = keys0, *kout = keys1, *vin = vals0, *vout = vals1;
-    for(int shift = 0; shift < 30; shift += 8)
-    {
-        k_radix_hist<<<nblocks, SORT_THREADS, 0, st>>>(kin, n, shift, counts, nblocks);
-        k_scan_exclusive<<<1, 1024, 0, st>>>(counts, 256u * nblocks, nullptr);
-        k_radix_scatter<<<nblocks, SORT_THREADS, 0, st>>>(kin, vin, n, shift, counts, nblocks, kout, vout);
-        std::swap(kin, kout);
-        std::swap(vin, vout);
-    }
+    radix_sort(kin, vin, kout, vout, n, 30, counts, st);
     chk(cudaMemcpyAsync(bvh->d_sorted, vin, sizeof(uint32_t) * n, cudaMemcpyDeviceToDevice, st));
     k_gather_leaf_boxes<<<g, T, 0, st>>>(tbox, vin, n, lbox);
     if(n > 1)
@@ -1165,13 +1157,12 @@ namespace
 {
 
 constexpr uint32_t NOALLOC_MAX_TRIS = 16384;
-constexpr uint32_t NOALLOC_SORT_BLOCKS = (NOALLOC_MAX_TRIS + SORT_TILE - 1) / SORT_TILE;
 
 struct noalloc_scratch
 {
     box6 tbox[NOALLOC_MAX_TRIS], lbox[NOALLOC_MAX_TRIS], ibox[NOALLOC_MAX_TRIS];
     uint32_t keys0[NOALLOC_MAX_TRIS], keys1[NOALLOC_MAX_TRIS], vals0[NOALLOC_MAX_TRIS], vals1[NOALLOC_MAX_TRIS];
-    uint32_t counts[256 * NOALLOC_SORT_BLOCKS];
+    uint32_t counts[sort_count_words(NOALLOC_MAX_TRIS)];
     bvh2_node tree[NOALLOC_MAX_TRIS];
     uint32_t first[NOALLOC_MAX_TRIS];
     uint32_t iparent[NOALLOC_MAX_TRIS], lparent[NOALLOC_MAX_TRIS], visits[NOALLOC_MAX_TRIS];
@@ -1253,20 +1244,12 @@ extern "C" vkg_status vkg_bvh_build_noalloc(const float *d_xyz, uint32_t num_ver
     }
     const int T = 256;
     const uint32_t g = (n + T - 1) / T;
-    const uint32_t nblocks = (n + SORT_TILE - 1) / SORT_TILE;
     // (the scratch keeps the previous call's contents)
     k_build_init<<<(n + 15 + T - 1) / T, T, 0, st>>>(s->visits, n, s->small);
     k_tri_boxes<<<g, T, 0, st>>>(d_xyz, num_vertices, d_indices, n, s->tbox, s->small, s->small + 6);
     k_morton<<<g, T, 0, st>>>(s->tbox, n, s->small, s->keys0, s->vals0, s->morton);
     uint32_t *kin = s->keys0, *kout = s->keys1, *vin = s->vals0, *vout = s->vals1;
-    for(int shift = 0; shift < 30; shift += 8)
-    {
-        k_radix_hist<<<nblocks, SORT_THREADS, 0, st>>>(kin, n, shift, s->counts, nblocks);
-        k_scan_exclusive<<<1, 1024, 0, st>>>(s->counts, 256u * nblocks, nullptr);
-        k_radix_scatter<<<nblocks, SORT_THREADS, 0, st>>>(kin, vin, n, shift, s->counts, nblocks, kout, vout);
-        std::swap(kin, kout);
-        std::swap(vin, vout);
-    }
+    radix_sort(kin, vin, kout, vout, n, 30, s->counts, st);
     k_gather_leaf_boxes<<<g, T, 0, st>>>(s->tbox, vin, n, s->lbox);
     if(n > 1)
     {
