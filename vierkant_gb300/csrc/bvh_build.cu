@@ -763,7 +763,9 @@ __global__ void __launch_bounds__(256)
 
 // instance records in leaf (sorted) order and in input order
 __global__ void k_instance_records(const vkg_instance *__restrict__ inst, const uint32_t *__restrict__ sorted,
-                                   uint32_t n, uint32_t nblas, inst_rec *__restrict__ out, inst_rec *__restrict__ by_id)
+                                   uint32_t n, uint32_t nblas, const box6 *__restrict__ lbox,
+                                   const float *__restrict__ margin, inst_rec *__restrict__ out,
+                                   inst_rec *__restrict__ by_id, float4 *__restrict__ box)
 {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if(i >= n) return;
@@ -778,6 +780,10 @@ __global__ void k_instance_records(const vkg_instance *__restrict__ inst, const 
     r.material = I.material;
     out[i] = r;
     by_id[id] = r;
+    const box6 b = lbox[i];
+    const float m = *margin;
+    box[2 * (size_t)i] = make_float4(fsub(b.lo[0], m), fsub(b.lo[1], m), fsub(b.lo[2], m), fadd(b.hi[0], m));
+    box[2 * (size_t)i + 1] = make_float4(fadd(b.hi[1], m), fadd(b.hi[2], m), 0.f, 0.f);
 }
 
 // both kernels of the collapse. max_blocks 1 keeps to plain launches; more blocks need a cooperative
@@ -800,8 +806,8 @@ cudaError_t launch_collapse(const collapse_args &A, uint32_t max_blocks, cudaStr
 
 // The primitive-independent part of a build: make_boxes(tbox, scene_enc, err) fills the n primitive
 // boxes, the scene box (ordered uints) and error bits; Morton codes, the radix sort, the Karras tree,
-// the refit and the 8-wide collapse follow; make_records(sorted) writes the leaf records in sorted
-// order. On success bvh holds the nodes, Morton codes, sorted order, scene box, margin and depth, and
+// the refit and the 8-wide collapse follow; make_records(sorted, lbox, margin) writes the leaf
+// records in sorted order (lbox: the boxes in that order). On success bvh holds the nodes, Morton codes, sorted order, scene box, margin and depth, and
 // err_bits the error bits that make_boxes raised. The caller frees bvh on failure.
 template<class MakeBoxes, class MakeRecords>
 vkg_status build_core(vkg_ctx *ctx, vkg_bvh *bvh, uint32_t n, uint32_t leaf_max, cudaStream_t st,
@@ -877,7 +883,7 @@ vkg_status build_core(vkg_ctx *ctx, vkg_bvh *bvh, uint32_t n, uint32_t leaf_max,
     collapse_args A{tree,     first,     ibox,      lbox,      n,        leaf_max, capacity, small,
                     node_ref, nodes_tmp, small + 8, block_sum, reinterpret_cast<float *>(small + 12)};
     chk(launch_collapse(A, (uint32_t)ctx->num_sms, st));
-    make_records(static_cast<const uint32_t *>(vin));
+    make_records(static_cast<const uint32_t *>(vin), lbox, reinterpret_cast<const float *>(small + 12));
     chk(cudaGetLastError());
 
     uint32_t info[16];
@@ -963,7 +969,7 @@ extern "C" vkg_status vkg_bvh_build(vkg_ctx *ctx, const float *d_xyz, uint32_t n
             [&](box6 *tbox, uint32_t *scene_enc, uint32_t *err) {
                 k_tri_boxes<<<g, T, 0, st>>>(d_xyz, num_vertices, d_indices, n, tbox, scene_enc, err);
             },
-            [&](const uint32_t *sorted) {
+            [&](const uint32_t *sorted, const box6 *, const float *) {
                 k_tri_records<<<g, T, 0, st>>>(d_xyz, num_vertices, d_indices, sorted, n, bvh->d_tris);
             },
             err_bits);
@@ -1054,6 +1060,7 @@ extern "C" vkg_status vkg_tlas_build(vkg_ctx *ctx, const vkg_bvh *const *blas, u
             boxes[b].hi[a] = blas[b]->scene_max[a];
         }
         boxes[b].num_tris = blas[b]->num_tris;
+        t->max_blas_depth = std::max(t->max_blas_depth, blas[b]->depth);
         boxes[b].nodes = blas[b]->d_nodes;
     }
     blas_box *d_bb = nullptr;
@@ -1070,6 +1077,7 @@ extern "C" vkg_status vkg_tlas_build(vkg_ctx *ctx, const vkg_bvh *const *blas, u
     {
         e = dalloc(ctx, &t->d_inst, num_instances, st);
         if(e == cudaSuccess) e = dalloc(ctx, &t->d_inst_by_id, num_instances, st);
+        if(e == cudaSuccess) e = dalloc(ctx, &t->d_inst_box, 2 * (size_t)num_instances, st);
     }
     if(e != cudaSuccess)
     {
@@ -1093,8 +1101,9 @@ extern "C" vkg_status vkg_tlas_build(vkg_ctx *ctx, const vkg_bvh *const *blas, u
             [&](box6 *tbox, uint32_t *scene_enc, uint32_t *err) {
                 k_instance_boxes<<<(n + 7) / 8, 256, 0, st>>>(d_instances, n, d_bb, num_blas, tbox, scene_enc, err);
             },
-            [&](const uint32_t *sorted) {
-                k_instance_records<<<g, T, 0, st>>>(d_instances, sorted, n, num_blas, t->d_inst, t->d_inst_by_id);
+            [&](const uint32_t *sorted, const box6 *lbox, const float *margin) {
+                k_instance_records<<<g, T, 0, st>>>(d_instances, sorted, n, num_blas, lbox, margin, t->d_inst,
+                                                    t->d_inst_by_id, t->d_inst_box);
             },
             err_bits);
     if(d_bb) cudaFreeAsync(d_bb, st);
@@ -1110,7 +1119,7 @@ extern "C" vkg_status vkg_tlas_build(vkg_ctx *ctx, const vkg_bvh *const *blas, u
         vkg_tlas_destroy(ctx, t);
         return s;
     }
-    t->top.bytes = sizeof(node8) * t->top.num_nodes + 2 * sizeof(inst_rec) * (size_t)n;
+    t->top.bytes = sizeof(node8) * t->top.num_nodes + (2 * sizeof(inst_rec) + 2 * sizeof(float4)) * (size_t)n;
     *out = t;
     return VKG_OK;
 }
@@ -1145,6 +1154,7 @@ extern "C" vkg_status vkg_tlas_destroy(vkg_ctx *ctx, vkg_tlas *t)
     cudaFree(t->top.d_sorted);
     cudaFree(t->d_inst);
     cudaFree(t->d_inst_by_id);
+    cudaFree(t->d_inst_box);
     cudaFree(t->d_blas);
     delete t;
     return VKG_OK;

@@ -93,8 +93,10 @@ struct vkg_tlas
     vkg_bvh top;                       // 8-wide BVH over the instances' world boxes (no triangle records)
     vkg::inst_rec *d_inst = nullptr;   // instance records in sorted (leaf) order
     vkg::inst_rec *d_inst_by_id = nullptr; // the same records in input order
+    float4 *d_inst_box = nullptr;      // world boxes in leaf order, grown by the margin: {lo xyz, hi x}, {hi yz, -, -}
     vkg::blas_ref *d_blas = nullptr;
     uint32_t num_instances = 0, num_blas = 0;
+    uint32_t max_blas_depth = 0; // depth of the deepest mesh BVH
 };
 
 namespace vkg

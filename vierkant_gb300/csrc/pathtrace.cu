@@ -1213,6 +1213,7 @@ vkg_status vkg_tracer_render(vkg_tracer *t, const vkg_scene *sc, const vkg_camer
     const bool bin_materials = pt_binning_selected();
     // a 64-entry traversal stack serves BVHs up to 10 levels deep (7 (depth - 1) + 1 entries)
     const bool small_stack = sc->bvh && sc->bvh->depth <= 10;
+    const bool tl_small_stack = sc->tlas && tl_group_small_stack(sc->tlas);
     uint32_t tl_grid = 0;
     if(tl_persistent)
     {
@@ -1239,11 +1240,11 @@ vkg_status vkg_tracer_render(vkg_tracer *t, const vkg_scene *sc, const vkg_camer
         P.train_base = last && train_paths ? n_render : 0xFFFFFFFFu;
         const uint32_t grid = (uint32_t)std::min<size_t>((n + PT_THREADS - 1) / PT_THREADS, (size_t)ctx->num_sms * 16);
         const single_scene SS{P};
-        // Short queues of single-level scenes without alpha-tested materials are traced by groups of eight
+        // Short queues of scenes without alpha-tested materials are traced by groups of eight
         // lanes (k_pt_extend_group). A wave of at most PT_GROUP_MAX_WAVE paths is always; a larger wave's
         // later queues may be short, which only the device knows: both kernels are launched from the
         // first bounce on (a binned queue is long), and the queue's count picks the one that runs.
-        const bool can_group = sc->bvh && !alpha;
+        const bool can_group = !alpha && !empty && !tl_persistent;
         const bool groups = can_group && n <= PT_GROUP_MAX_WAVE;
         const uint32_t group_grid = (uint32_t)std::min<size_t>(((size_t)n * GROUP_LANES + PT_THREADS - 1) / PT_THREADS,
                                                                (size_t)ctx->num_sms * 64);
@@ -1282,12 +1283,12 @@ vkg_status vkg_tracer_render(vkg_tracer *t, const vkg_scene *sc, const vkg_camer
                                                       reordered, t->rng, depth, by_count ? PT_GROUP_MAX_QUEUE : 0u);
                 };
                 auto extend_group = [&](auto kern) {
-                    kern<<<group_grid, PT_THREADS, 0, st>>>(SS, t->q_ray[a], cnt_in, t->hits,
+                    kern<<<group_grid, PT_THREADS, 0, st>>>(SS, t->q_ray[a], cnt_in, t->hits, t->hit_inst,
                                                             by_count ? PT_GROUP_MAX_QUEUE : 0xFFFFFFFFu);
                 };
                 constexpr int BIG = (int)TRAVERSAL_STACK;
                 using T1 = single_scene;
-                if(sc->tlas)
+                if(sc->tlas && !groups)
                     alpha ? extend(k_pt_extend<T1, BIG, true, LEVELS_TWO>) : extend(k_pt_extend<T1, BIG, false, LEVELS_TWO>);
                 else if(alpha)
                     small_stack ? extend(k_pt_extend<T1, 64, true, LEVELS_ONE>)
@@ -1295,8 +1296,12 @@ vkg_status vkg_tracer_render(vkg_tracer *t, const vkg_scene *sc, const vkg_camer
                 else if(!groups)
                     small_stack ? extend(k_pt_extend<T1, 64, false, LEVELS_ONE>)
                                 : extend(k_pt_extend<T1, BIG, false, LEVELS_ONE>);
-                if(groups || by_count)
-                    small_stack ? extend_group(k_pt_extend_group<64>) : extend_group(k_pt_extend_group<BIG>);
+                if((groups || by_count) && sc->tlas)
+                    tl_small_stack ? extend_group(k_pt_extend_group<TL_GROUP_SMALL_STACK, LEVELS_TWO>)
+                                   : extend_group(k_pt_extend_group<TL_GROUP_STACK, LEVELS_TWO>);
+                else if(groups || by_count)
+                    small_stack ? extend_group(k_pt_extend_group<64, LEVELS_ONE>)
+                                : extend_group(k_pt_extend_group<BIG, LEVELS_ONE>);
                 if(perm) bin_rays_done(ctx, st);
             }
             VKG_TRY_CUDA(ctx, cudaMemsetAsync(cnt_out, 0, sizeof(uint32_t), st));
@@ -1357,7 +1362,7 @@ vkg_status vkg_tracer_render(vkg_tracer *t, const vkg_scene *sc, const vkg_camer
                 };
                 constexpr int BIG = (int)TRAVERSAL_STACK;
                 using T1 = single_scene;
-                if(sc->tlas)
+                if(sc->tlas && !groups)
                     alpha ? shadow(k_pt_shadow<T1, BIG, true, LEVELS_TWO>) : shadow(k_pt_shadow<T1, BIG, false, LEVELS_TWO>);
                 else if(alpha)
                     small_stack ? shadow(k_pt_shadow<T1, 64, true, LEVELS_ONE>)
@@ -1365,8 +1370,12 @@ vkg_status vkg_tracer_render(vkg_tracer *t, const vkg_scene *sc, const vkg_camer
                 else if(!groups)
                     small_stack ? shadow(k_pt_shadow<T1, 64, false, LEVELS_ONE>)
                                 : shadow(k_pt_shadow<T1, BIG, false, LEVELS_ONE>);
-                if(groups || by_count)
-                    small_stack ? shadow_group(k_pt_shadow_group<64>) : shadow_group(k_pt_shadow_group<BIG>);
+                if((groups || by_count) && sc->tlas)
+                    tl_small_stack ? shadow_group(k_pt_shadow_group<TL_GROUP_SMALL_STACK, LEVELS_TWO>)
+                                   : shadow_group(k_pt_shadow_group<TL_GROUP_STACK, LEVELS_TWO>);
+                else if(groups || by_count)
+                    small_stack ? shadow_group(k_pt_shadow_group<64, LEVELS_ONE>)
+                                : shadow_group(k_pt_shadow_group<BIG, LEVELS_ONE>);
                 if(s_perm) bin_rays_done(ctx, st);
             }
             if(cnt_l && !empty)

@@ -12,6 +12,7 @@
 #include "pixel.cuh"
 #include "texture.cuh"
 #include "tlas.cuh"
+#include "tlas_group.cuh"
 #include "traverse.cuh"
 #include "traverse_group.cuh"
 
@@ -85,6 +86,7 @@ struct pt_params
     // and the meshes' vertex / index arrays; two_level selects them
     const node8 *tl_nodes;
     const inst_rec *tl_inst, *tl_by_id;
+    const float4 *tl_box; // the instances' world boxes, in leaf order
     const blas_ref *tl_blas;
     const mesh_ref *meshes;
     uint32_t two_level;
@@ -420,7 +422,7 @@ __global__ void __launch_bounds__(PT_THREADS, STACK <= 64 ? 8 : 6) // 64 / 85 re
         if constexpr(ALPHA) f = alpha_filter{&P, 0ull, peek_uniform(P, rng[pid], S.inc(pid), depth), 0u, false};
         if(two_level<LEVELS>(P))
         {
-            const tlas_result r = trace_tlas<false, F>(P.tl_nodes, P.tl_inst, P.tl_blas, r0.x, r0.y, r0.z, r0.w, r1.x,
+            const tlas_result r = trace_tlas<false, F>(P.tl_nodes, P.tl_inst, P.tl_box, P.tl_blas, r0.x, r0.y, r0.z, r0.w, r1.x,
                                                        r1.y, r1.z, r1.w, CULL_BACK_UNLESS_TWOSIDED, f);
             reinterpret_cast<uint4 *>(hits)[i] =
                     make_uint4(r.prim, __float_as_uint(r.t), __float_as_uint(r.u), __float_as_uint(r.v));
@@ -435,17 +437,17 @@ __global__ void __launch_bounds__(PT_THREADS, STACK <= 64 ? 8 : 6) // 64 / 85 re
     }
 }
 
-// The same for short queues, eight lanes per ray (traverse_group.cuh); single-level scenes without
+// The same for short queues, eight lanes per ray (traverse_group.cuh, tlas_group.cuh); scenes without
 // alpha-tested materials, queues of at most `up_to` rays (k_pt_extend traces longer ones).
 // The bounds: a 720p-like Cornell frame of one sample and six segments takes 542 against 1,065 us at 58,101
 // paths, 921 against 1,283 us at 256,000 with every queue traced by groups; at 516,000 the first two
 // queues are faster with a thread per ray and the later ones by groups (1,478 us; none 1,654, all 1,517).
 // Incoherent queues break even at 64,000 to 190,000 rays.
 constexpr uint32_t PT_GROUP_MAX_WAVE = 1u << 18, PT_GROUP_MAX_QUEUE = 1u << 17;
-template<int STACK>
+template<int STACK, int LEVELS>
 __global__ void __launch_bounds__(PT_THREADS)
         k_pt_extend_group(single_scene S, const vkg_ray *__restrict__ q_ray, const uint32_t *__restrict__ count,
-                          vkg_hit *__restrict__ hits, uint32_t up_to)
+                          vkg_hit *__restrict__ hits, uint32_t *__restrict__ hit_inst, uint32_t up_to)
 {
     __shared__ uint2 stack[PT_THREADS / GROUP_LANES][group_stack_entries<STACK>];
     constexpr uint32_t PER = PT_THREADS / GROUP_LANES;
@@ -458,11 +460,26 @@ __global__ void __launch_bounds__(PT_THREADS)
         const bool active = i < n;
         const float4 *rp = reinterpret_cast<const float4 *>(q_ray + (active ? i : base));
         const float4 r0 = __ldg(rp), r1 = __ldg(rp + 1);
-        const trace_result r = trace_group<false, STACK>(active, P.nodes, P.tris, r0.x, r0.y, r0.z, r0.w, r1.x, r1.y,
-                                                         r1.z, r1.w, CULL_BACK_UNLESS_TWOSIDED, stack[group], nullptr);
-        if(active && !(threadIdx.x & (GROUP_LANES - 1)))
-            reinterpret_cast<uint4 *>(hits)[i] =
-                    make_uint4(r.prim, __float_as_uint(r.t), __float_as_uint(r.u), __float_as_uint(r.v));
+        const bool writes = active && !(threadIdx.x & (GROUP_LANES - 1));
+        auto trace = [&]() {
+            if constexpr(LEVELS == LEVELS_TWO)
+            {
+                const tlas_result r = trace_tlas_group<false, STACK>(active, P.tl_nodes, P.tl_inst, P.tl_box, P.tl_blas,
+                                                                     r0.x, r0.y, r0.z, r0.w, r1.x, r1.y, r1.z, r1.w,
+                                                                     CULL_BACK_UNLESS_TWOSIDED, stack[group]);
+                if(writes) hit_inst[i] = r.inst;
+                return make_uint4(r.prim, __float_as_uint(r.t), __float_as_uint(r.u), __float_as_uint(r.v));
+            }
+            else
+            {
+                const trace_result r = trace_group<false, STACK>(active, P.nodes, P.tris, r0.x, r0.y, r0.z, r0.w, r1.x,
+                                                                 r1.y, r1.z, r1.w, CULL_BACK_UNLESS_TWOSIDED,
+                                                                 stack[group], nullptr);
+                return make_uint4(r.prim, __float_as_uint(r.t), __float_as_uint(r.u), __float_as_uint(r.v));
+            }
+        };
+        const uint4 h = trace();
+        if(writes) reinterpret_cast<uint4 *>(hits)[i] = h;
     }
 }
 
@@ -1280,7 +1297,7 @@ __global__ void __launch_bounds__(PT_THREADS, STACK <= 64 ? 8 : 6) // 64 / 85 re
         if constexpr(ALPHA) f = alpha_filter{&P, rng[s_pid[i]], 0.f, ALPHA_SALT_SHADOW, false};
         bool occluded;
         if(two_level<LEVELS>(P))
-            occluded = trace_tlas<true, F>(P.tl_nodes, P.tl_inst, P.tl_blas, r0.x, r0.y, r0.z, r0.w, r1.x, r1.y, r1.z,
+            occluded = trace_tlas<true, F>(P.tl_nodes, P.tl_inst, P.tl_box, P.tl_blas, r0.x, r0.y, r0.z, r0.w, r1.x, r1.y, r1.z,
                                            r1.w, cull, f)
                                .occluded;
         else
@@ -1303,7 +1320,7 @@ __global__ void __launch_bounds__(PT_THREADS, STACK <= 64 ? 8 : 6) // 64 / 85 re
 }
 
 // the same for short queues, eight lanes per ray (k_pt_extend_group)
-template<int STACK>
+template<int STACK, int LEVELS>
 __global__ void __launch_bounds__(PT_THREADS)
         k_pt_shadow_group(single_scene S, const vkg_ray *__restrict__ s_ray, const uint32_t *__restrict__ s_pid,
                           const float4 *__restrict__ s_contrib, const uint32_t *__restrict__ count,
@@ -1321,10 +1338,16 @@ __global__ void __launch_bounds__(PT_THREADS)
         const float4 *rp = reinterpret_cast<const float4 *>(s_ray + i);
         const float4 r0 = __ldg(rp), r1 = __ldg(rp + 1);
         const float4 c = s_contrib[i];
-        const bool occluded = trace_group<true, STACK>(active, P.nodes, P.tris, r0.x, r0.y, r0.z, r0.w, r1.x, r1.y,
-                                                       r1.z, r1.w, c.w != 0.f ? CULL_BACK : CULL_NONE, stack[group],
-                                                       nullptr)
-                                      .occluded;
+        const int cull = c.w != 0.f ? CULL_BACK : CULL_NONE;
+        bool occluded;
+        if constexpr(LEVELS == LEVELS_TWO)
+            occluded = trace_tlas_group<true, STACK>(active, P.tl_nodes, P.tl_inst, P.tl_box, P.tl_blas, r0.x, r0.y, r0.z,
+                                                     r0.w, r1.x, r1.y, r1.z, r1.w, cull, stack[group])
+                               .occluded;
+        else
+            occluded = trace_group<true, STACK>(active, P.nodes, P.tris, r0.x, r0.y, r0.z, r0.w, r1.x, r1.y, r1.z, r1.w,
+                                                cull, stack[group], nullptr)
+                               .occluded;
         if(active && !occluded && !(threadIdx.x & (GROUP_LANES - 1)))
         {
             const uint32_t pid = s_pid[i];
@@ -1367,7 +1390,7 @@ __global__ void __launch_bounds__(PT_THREADS, STACK <= 64 ? 8 : 6) // 64 / 85 re
         if constexpr(ALPHA) f = alpha_filter{&P, rng[pid], 0.f, ALPHA_SALT_LIGHT_SHADOW, true};
         if(!P.transmissive)
         {
-            const bool occ = two_level<LEVELS>(P) ? trace_tlas<true, F>(P.tl_nodes, P.tl_inst, P.tl_blas, r0.x, r0.y, r0.z, r0.w,
+            const bool occ = two_level<LEVELS>(P) ? trace_tlas<true, F>(P.tl_nodes, P.tl_inst, P.tl_box, P.tl_blas, r0.x, r0.y, r0.z, r0.w,
                                                                r1.x, r1.y, r1.z, r1.w, cull, f)
                                                    .occluded
                                          : trace_ray<true, false, STACK, F>(P.nodes, P.tris, r0.x, r0.y, r0.z, r0.w,
@@ -1414,7 +1437,7 @@ __global__ void __launch_bounds__(PT_THREADS, STACK <= 64 ? 8 : 6) // 64 / 85 re
                 float t, hu = 0.f, hv = 0.f;
                 if(two_level<LEVELS>(P))
                 {
-                    const tlas_result r = trace_tlas<false, F>(P.tl_nodes, P.tl_inst, P.tl_blas, r0.x, r0.y, r0.z,
+                    const tlas_result r = trace_tlas<false, F>(P.tl_nodes, P.tl_inst, P.tl_box, P.tl_blas, r0.x, r0.y, r0.z,
                                                                tmin, r1.x, r1.y, r1.z, r1.w, cull, f);
                     prim = r.prim;
                     t = r.t;
@@ -1594,7 +1617,7 @@ __global__ void __launch_bounds__(PT_THREADS)
         }
         const bool active = cur != 0xFFFFFFFFu;
         if(!__any_sync(0xffffffffu, active)) break;
-        if(active && !tl_step<SHADOW>(s, P.tl_nodes, P.tl_inst, P.tl_blas, cull))
+        if(active && !tl_step<SHADOW>(s, P.tl_nodes, P.tl_inst, P.tl_box, P.tl_blas, cull))
         {
             if constexpr(SHADOW)
             {
@@ -1786,6 +1809,7 @@ inline pt_params make_params(const vkg_scene *sc, const vkg_camera &cam, const v
         P.two_level = 1;
         P.tl_nodes = sc->tlas->top.d_nodes;
         P.tl_inst = sc->tlas->d_inst;
+        P.tl_box = sc->tlas->d_inst_box;
         P.tl_by_id = sc->tlas->d_inst_by_id;
         P.tl_blas = sc->tlas->d_blas;
         P.meshes = sc->d_meshes;

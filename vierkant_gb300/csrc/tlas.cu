@@ -1,6 +1,6 @@
 // Two-level ray queries (vkg_tlas_closest_hit / vkg_tlas_any_hit): one thread per ray through
-// trace_tlas (tlas.cuh). The top-level build lives with the other builds in bvh_build.cu.
-#include "tlas.cuh"
+// trace_tlas (tlas.cuh), or eight lanes per ray for small batches (tlas_group.cuh). The top-level build lives with the other builds in bvh_build.cu.
+#include "tlas_group.cuh"
 
 namespace vkg
 {
@@ -12,16 +12,40 @@ constexpr int TLAS_THREADS = 128;
 template<bool ANY>
 __global__ void __launch_bounds__(TLAS_THREADS)
         k_tlas_trace(const node8 *__restrict__ tnodes, const inst_rec *__restrict__ inst,
-                     const blas_ref *__restrict__ blas, const vkg_ray *__restrict__ rays, uint32_t n,
+                     const float4 *__restrict__ box, const blas_ref *__restrict__ blas, const vkg_ray *__restrict__ rays, uint32_t n,
                      vkg_inst_hit *__restrict__ hits, uint32_t *__restrict__ occluded, int cull)
 {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if(i >= n) return;
     const float4 *rp = reinterpret_cast<const float4 *>(rays + i);
     const float4 r0 = __ldg(rp), r1 = __ldg(rp + 1);
-    const tlas_result r = trace_tlas<ANY>(tnodes, inst, blas, r0.x, r0.y, r0.z, r0.w, r1.x, r1.y, r1.z, r1.w, cull);
+    const tlas_result r = trace_tlas<ANY>(tnodes, inst, box, blas, r0.x, r0.y, r0.z, r0.w, r1.x, r1.y, r1.z, r1.w, cull);
     if(ANY)
         occluded[i] = r.occluded ? 1u : 0u;
+    else
+    {
+        uint4 *o = reinterpret_cast<uint4 *>(hits + i);
+        o[0] = make_uint4(r.prim, r.inst, __float_as_uint(r.t), __float_as_uint(r.u));
+        o[1] = make_uint4(__float_as_uint(r.v), 0u, 0u, 0u);
+    }
+}
+
+template<bool ANY, int STACK>
+__global__ void __launch_bounds__(TLAS_THREADS)
+        k_tlas_trace_group(const node8 *__restrict__ tnodes, const inst_rec *__restrict__ inst,
+                           const float4 *__restrict__ box, const blas_ref *__restrict__ blas,
+                           const vkg_ray *__restrict__ rays, uint32_t n, vkg_inst_hit *__restrict__ hits,
+                           uint32_t *__restrict__ occluded, int cull)
+{
+    __shared__ uint2 stack[TLAS_THREADS / GROUP_LANES][group_stack_entries<STACK>];
+    const uint32_t group = threadIdx.x / GROUP_LANES, i = blockIdx.x * (TLAS_THREADS / GROUP_LANES) + group;
+    const bool active = i < n;
+    const float4 *rp = reinterpret_cast<const float4 *>(rays + (active ? i : 0u));
+    const float4 r0 = __ldg(rp), r1 = __ldg(rp + 1);
+    const tlas_result r = trace_tlas_group<ANY, STACK>(active, tnodes, inst, box, blas, r0.x, r0.y, r0.z, r0.w, r1.x,
+                                                       r1.y, r1.z, r1.w, cull, stack[group]);
+    if(!active || (threadIdx.x & (GROUP_LANES - 1))) return;
+    if(ANY) occluded[i] = r.occluded ? 1u : 0u;
     else
     {
         uint4 *o = reinterpret_cast<uint4 *>(hits + i);
@@ -50,12 +74,19 @@ vkg_status launch(vkg_ctx *ctx, const vkg_tlas *t, const vkg_ray *rays, uint32_t
         return set_error(ctx, VKG_ERR_INVALID_ARGUMENT, "two-level query: buffers must be 16-byte aligned");
     if(vkg_status s = bind_device(ctx); s != VKG_OK) return s;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    const uint32_t grid = (n + TLAS_THREADS - 1) / TLAS_THREADS;
     if(t->num_instances == 0)
-        k_tlas_miss<<<grid, TLAS_THREADS, 0, st>>>(n, ANY ? nullptr : hits, ANY ? occ : nullptr);
+        k_tlas_miss<<<(n + TLAS_THREADS - 1) / TLAS_THREADS, TLAS_THREADS, 0, st>>>(n, ANY ? nullptr : hits, ANY ? occ : nullptr);
     else
-        k_tlas_trace<ANY><<<grid, TLAS_THREADS, 0, st>>>(t->top.d_nodes, t->d_inst, t->d_blas, rays, n, hits, occ,
-                                                         (flags & VKG_RAY_CULL_BACK_FACES) ? CULL_BACK : CULL_NONE);
+    {
+        const int cull = (flags & VKG_RAY_CULL_BACK_FACES) ? CULL_BACK : CULL_NONE;
+        auto go = [&](auto kern, uint32_t lanes) {
+            kern<<<(n * lanes + TLAS_THREADS - 1) / TLAS_THREADS, TLAS_THREADS, 0, st>>>(
+                    t->top.d_nodes, t->d_inst, t->d_inst_box, t->d_blas, rays, n, hits, occ, cull);
+        };
+        if(n > TL_GROUP_MAX_RAYS) go(k_tlas_trace<ANY>, 1u);
+        else if(tl_group_small_stack(t)) go(k_tlas_trace_group<ANY, TL_GROUP_SMALL_STACK>, GROUP_LANES);
+        else go(k_tlas_trace_group<ANY, TL_GROUP_STACK>, GROUP_LANES);
+    }
     return cuda_check(ctx, cudaGetLastError(), "k_tlas_trace");
 }
 

@@ -85,7 +85,8 @@ __device__ __forceinline__ void tl_init(tl_state &s, const node8 *tnodes, float 
 // is >= +0 (key_pos): the child keys are the entry distances' float bits
 template<bool ANY, class F = no_filter, bool POS = false>
 __device__ __forceinline__ bool tl_step(tl_state &s, const node8 *__restrict__ tnodes, const inst_rec *__restrict__ inst,
-                                        const blas_ref *__restrict__ blas, int cull, const F &f = F())
+                                        const float4 *__restrict__ box, const blas_ref *__restrict__ blas, int cull,
+                                        const F &f = F())
 {
     while(s.sp > 0 && !s.done)
     {
@@ -107,6 +108,15 @@ __device__ __forceinline__ bool tl_step(tl_state &s, const node8 *__restrict__ t
         if(__uint_as_float(ent.y) > s.best_t) continue;
         if(!s.in_blas && (e & INST_BIT))
         {
+            // a leaf's instances were pushed for the box they share: each is entered only if the ray hits
+            // its own (20,000 spheres, 518,400 camera rays: 1,175 -> 1,095 us)
+            const float4 b0 = __ldg(box + 2 * (e & ~INST_BIT)), b1 = __ldg(box + 2 * (e & ~INST_BIT) + 1);
+            const float x0 = (b0.x - s.wo[0]) * s.wi[0], x1 = (b0.w - s.wo[0]) * s.wi[0];
+            const float y0 = (b0.y - s.wo[1]) * s.wi[1], y1 = (b1.x - s.wo[1]) * s.wi[1];
+            const float z0 = (b0.z - s.wo[2]) * s.wi[2], z1 = (b1.y - s.wo[2]) * s.wi[2];
+            const float tn = fmaxf(fmaxf(fminf(x0, x1), fminf(y0, y1)), fmaxf(fminf(z0, z1), s.tmin));
+            const float tf = fminf(fminf(fmaxf(x0, x1), fmaxf(y0, y1)), fminf(fmaxf(z0, z1), s.best_t));
+            if(!(tn <= tf)) continue;
             // enter an instance: object-space ray, RETURN marker, BLAS root
             const float4 *mp = reinterpret_cast<const float4 *>(inst + (e & ~INST_BIT));
             const uint4 meta = __ldg(reinterpret_cast<const uint4 *>(mp + 6));
@@ -208,7 +218,7 @@ __device__ __forceinline__ bool tl_step(tl_state &s, const node8 *__restrict__ t
 
 template<bool ANY, class F = no_filter>
 __device__ __forceinline__ tlas_result trace_tlas(const node8 *__restrict__ tnodes, const inst_rec *__restrict__ inst,
-                                                  const blas_ref *__restrict__ blas, float ox, float oy, float oz,
+                                                  const float4 *__restrict__ box, const blas_ref *__restrict__ blas, float ox, float oy, float oz,
                                                   float tmin, float dx, float dy, float dz, float tmax, int cull,
                                                   const F &f = F())
 {
@@ -217,9 +227,9 @@ __device__ __forceinline__ tlas_result trace_tlas(const node8 *__restrict__ tnod
     s.st = stack;
     tl_init(s, tnodes, ox, oy, oz, tmin, dx, dy, dz, tmax);
     if(key_pos(tmin))
-        while(tl_step<ANY, F, true>(s, tnodes, inst, blas, cull, f)) {}
+        while(tl_step<ANY, F, true>(s, tnodes, inst, box, blas, cull, f)) {}
     else
-        while(tl_step<ANY, F, false>(s, tnodes, inst, blas, cull, f)) {}
+        while(tl_step<ANY, F, false>(s, tnodes, inst, box, blas, cull, f)) {}
     tlas_result R;
     R.occluded = s.done;
     R.prim = s.best_prim;
