@@ -123,10 +123,15 @@ constexpr uint32_t TRAVERSAL_STACK = 128;
 // d_n is a device-side count <= n -- so that neighbouring threads follow similar paths through bvh:
 // perm[position] = ray, valid when *reordered_out (a device word) is non-zero; otherwise the rays
 // are to be traced as given. Returns nullptr (trace as given) for VKG_RAY_KEEP_ORDER, batches below
-// 2^19 rays, a stream being captured, or scratch that cannot be allocated. The scratch is the
+// min_rays, a stream being captured, or scratch that cannot be allocated. The scratch is the
 // context's; calls on different streams are ordered by an event recorded by bin_rays_done().
 const uint32_t *bin_rays(vkg_ctx *ctx, const vkg_bvh *bvh, const vkg_ray *d_rays, uint32_t n, const uint32_t *d_n,
-                         uint32_t flags, cudaStream_t st, const uint32_t **reordered_out);
+                         uint32_t flags, uint32_t min_rays, cudaStream_t st, const uint32_t **reordered_out);
+// Batches from which binning pays. The binning itself takes 40-90 us; a closest-hit traversal of incoherent
+// rays gains more than that from 2^19 rays on (600,000: 441 -> 414 us, 784,000: 531 -> 494 us), an any-hit
+// traversal, which ends at the first hit, from about 1.5 million (600,000: 164 -> 184 us, 784,000: 209 ->
+// 218 us, 1,200,000: 351 either way, 1,800,000: 551 -> 534 us).
+constexpr uint32_t BIN_MIN_CLOSEST = 1u << 19, BIN_MIN_ANY = 3u << 19;
 // after the launch that reads the order: the scratch may be reused once the stream reaches here
 inline void bin_rays_done(vkg_ctx *ctx, cudaStream_t st) { cudaEventRecord(ctx->bins.done, st); }
 }// namespace vkg

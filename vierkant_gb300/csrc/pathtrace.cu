@@ -1276,7 +1276,7 @@ vkg_status vkg_tracer_render(vkg_tracer *t, const vkg_scene *sc, const vkg_camer
                 const vkg_bvh *bounds = sc->bvh ? sc->bvh : (sc->tlas ? &sc->tlas->top : nullptr);
                 const bool bin_queue = depth == 1 || (sc->tlas && depth == 2);
                 const uint32_t *perm =
-                        bin_queue ? bin_rays(ctx, bounds, t->q_ray[a], n, cnt_in, 0u, st, &reordered) : nullptr;
+                        bin_queue ? bin_rays(ctx, bounds, t->q_ray[a], n, cnt_in, 0u, BIN_MIN_CLOSEST, st, &reordered) : nullptr;
                 const bool by_count = can_group && !groups && depth > 0 && !perm;
                 auto extend = [&](auto kern) {
                     kern<<<grid, PT_THREADS, 0, st>>>(SS, t->q_ray[a], t->q_pid[a], cnt_in, t->hits, t->hit_inst, perm,
@@ -1349,7 +1349,7 @@ vkg_status vkg_tracer_render(vkg_tracer *t, const vkg_scene *sc, const vkg_camer
                 const uint32_t *s_reordered = nullptr;
                 const vkg_bvh *s_bounds = sc->bvh ? sc->bvh : (sc->tlas ? &sc->tlas->top : nullptr);
                 const uint32_t *s_perm = (mode == MODE_PLAIN && depth <= 1)
-                                                 ? bin_rays(ctx, s_bounds, t->s_ray, n, cnt_s, 0u, st, &s_reordered)
+                                                 ? bin_rays(ctx, s_bounds, t->s_ray, n, cnt_s, 0u, BIN_MIN_ANY, st, &s_reordered)
                                                  : nullptr;
                 const bool by_count = can_group && !groups && depth > 0 && !s_perm;
                 auto shadow = [&](auto kern) {

@@ -220,7 +220,6 @@ void launch_simple(bool small_stack, uint32_t grid, cudaStream_t st, const vkg_b
 constexpr int BIN_CELL_BITS = 3;                                            // per axis
 constexpr int BIN_DIR_BITS = 3;                                             // per octahedral axis
 constexpr uint32_t NUM_BINS = 1u << (3 * BIN_CELL_BITS + 2 * BIN_DIR_BITS); // 32,768
-constexpr uint32_t BIN_MIN_RAYS = 1u << 19;
 constexpr int BIN_THREADS = 1024;                                           // per tile CTA
 constexpr uint32_t BIN_MAX_TILE = 40u * BIN_THREADS;                        // ranks fit 16 bits
 // slot NUM_BINS (KEEP_BIN): the rays of tiles that keep their order; the count rows are padded to
@@ -520,7 +519,7 @@ vkg_status launch_trace(vkg_ctx *ctx, const vkg_bvh *bvh, const vkg_ray *d_rays,
     }
     // reordered: device word, the number of tiles the binning reordered (0: trace in the given order)
     const uint32_t *reordered = nullptr;
-    const uint32_t *perm = bin_rays(ctx, bvh, d_rays, n, nullptr, flags, st, &reordered);
+    const uint32_t *perm = bin_rays(ctx, bvh, d_rays, n, nullptr, flags, d_occ ? BIN_MIN_ANY : BIN_MIN_CLOSEST, st, &reordered);
     if(use_persistent())
     {
         if(d_occ)
@@ -563,10 +562,10 @@ vkg_status check_common(vkg_ctx *ctx, const vkg_bvh *bvh, const void *rays, cons
 }// namespace
 
 const uint32_t *bin_rays(vkg_ctx *ctx, const vkg_bvh *bvh, const vkg_ray *d_rays, uint32_t n, const uint32_t *d_n,
-                         uint32_t flags, cudaStream_t st, const uint32_t **reordered_out)
+                         uint32_t flags, uint32_t min_rays, cudaStream_t st, const uint32_t **reordered_out)
 {
     *reordered_out = nullptr;
-    if((flags & VKG_RAY_KEEP_ORDER) || n < BIN_MIN_RAYS || !bvh) return nullptr;
+    if((flags & VKG_RAY_KEEP_ORDER) || n < min_rays || !bvh) return nullptr;
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     if(cudaStreamIsCapturing(st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone)
     {
