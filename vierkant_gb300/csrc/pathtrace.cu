@@ -1239,6 +1239,11 @@ vkg_status vkg_tracer_render(vkg_tracer *t, const vkg_scene *sc, const vkg_camer
         P.s0 = s0;
         P.train_base = last && train_paths ? n_render : 0xFFFFFFFFu;
         const uint32_t grid = (uint32_t)std::min<size_t>((n + PT_THREADS - 1) / PT_THREADS, (size_t)ctx->num_sms * 16);
+        // The tracers' and shaders' entries differ widely in cost: four to eight times the blocks that fit leave
+        // the balancing to the block scheduler (1280x720 at 16 samples: 17,580 us with 16 blocks a SM, 16,610
+        // with 36, 16,140 with 72, 16,160 with 288; the shaders alone 0.8-1.5 % of a frame).
+        const uint32_t wide_grid =
+                (uint32_t)std::min<size_t>((n + PT_THREADS - 1) / PT_THREADS, (size_t)ctx->num_sms * 72);
         const single_scene SS{P};
         // Short queues of scenes without alpha-tested materials are traced by groups of eight
         // lanes (k_pt_extend_group). A wave of at most PT_GROUP_MAX_WAVE paths is always; a larger wave's
@@ -1279,7 +1284,7 @@ vkg_status vkg_tracer_render(vkg_tracer *t, const vkg_scene *sc, const vkg_camer
                         bin_queue ? bin_rays(ctx, bounds, t->q_ray[a], n, cnt_in, 0u, BIN_MIN_CLOSEST, st, &reordered) : nullptr;
                 const bool by_count = can_group && !groups && depth > 0 && !perm;
                 auto extend = [&](auto kern) {
-                    kern<<<grid, PT_THREADS, 0, st>>>(SS, t->q_ray[a], t->q_pid[a], cnt_in, t->hits, t->hit_inst, perm,
+                    kern<<<wide_grid, PT_THREADS, 0, st>>>(SS, t->q_ray[a], t->q_pid[a], cnt_in, t->hits, t->hit_inst, perm,
                                                       reordered, t->rng, depth, by_count ? PT_GROUP_MAX_QUEUE : 0u);
                 };
                 auto extend_group = [&](auto kern) {
@@ -1319,7 +1324,7 @@ vkg_status vkg_tracer_render(vkg_tracer *t, const vkg_scene *sc, const vkg_camer
                 order = t->order;
             }
 #define VKG_SHADE(M, F, MD, TX)                                                                                        \
-    k_pt_shade<M, single_scene, F, MD, TX><<<grid, PT_THREADS, 0, st>>>(SS, depth, t->q_ray[a], t->q_pid[a], t->hits, t->hit_inst, cnt_in,    \
+    k_pt_shade<M, single_scene, F, MD, TX><<<wide_grid, PT_THREADS, 0, st>>>(SS, depth, t->q_ray[a], t->q_pid[a], t->hits, t->hit_inst, cnt_in,    \
                                                t->q_ray[1 - a],                                                          \
                                                t->q_pid[1 - a], cnt_out, t->s_ray, t->s_pid, t->s_contrib, cnt_s,         \
                                                t->rng, t->beta_pdf, t->radiance, io, lq, order)
@@ -1353,7 +1358,7 @@ vkg_status vkg_tracer_render(vkg_tracer *t, const vkg_scene *sc, const vkg_camer
                                                  : nullptr;
                 const bool by_count = can_group && !groups && depth > 0 && !s_perm;
                 auto shadow = [&](auto kern) {
-                    kern<<<grid, PT_THREADS, 0, st>>>(SS, t->s_ray, t->s_pid, t->s_contrib, cnt_s, t->radiance, s_perm,
+                    kern<<<wide_grid, PT_THREADS, 0, st>>>(SS, t->s_ray, t->s_pid, t->s_contrib, cnt_s, t->radiance, s_perm,
                                                       s_reordered, t->rng, by_count ? PT_GROUP_MAX_QUEUE : 0u);
                 };
                 auto shadow_group = [&](auto kern) {

@@ -396,10 +396,15 @@ __device__ __forceinline__ bool two_level(const pt_params &P)
     return LEVELS == LEVELS_ANY ? P.two_level != 0u : LEVELS == LEVELS_TWO;
 }
 
+// resident blocks the tracers are compiled for: the plain single-level ones fit 56 registers with 8 bytes of
+// spills, and a ninth block gains more (k_trace 1.6 % on a mixed batch); the others 64 or 85 registers
+template<int STACK, bool ALPHA, int LEVELS>
+constexpr int min_blocks = LEVELS == LEVELS_ONE && !ALPHA ? 9 : STACK <= 64 ? 8 : 6;
+
 // ALPHA: the scene has alpha-tested materials (alpha_filter); rng and depth then give each ray its
 // segment's first uniform
 template<class J, int STACK = (int)TRAVERSAL_STACK, bool ALPHA = false, int LEVELS = LEVELS_ANY>
-__global__ void __launch_bounds__(PT_THREADS, STACK <= 64 ? 8 : 6) // 64 / 85 registers
+__global__ void __launch_bounds__(PT_THREADS, min_blocks<STACK, ALPHA, LEVELS>)
         k_pt_extend(J S, const vkg_ray *__restrict__ q_ray, const uint32_t *__restrict__ q_pid,
                     const uint32_t *__restrict__ count, vkg_hit *__restrict__ hits, uint32_t *__restrict__ hit_inst,
                     const uint32_t *__restrict__ perm = nullptr, const uint32_t *__restrict__ reordered = nullptr,
@@ -1272,7 +1277,7 @@ __global__ void __launch_bounds__(PT_THREADS)
 
 // ALPHA: alpha-tested materials (alpha_filter), each candidate's uniform hashed from rng[path]
 template<class J, int STACK = (int)TRAVERSAL_STACK, bool ALPHA = false, int LEVELS = LEVELS_ANY>
-__global__ void __launch_bounds__(PT_THREADS, STACK <= 64 ? 8 : 6) // 64 / 85 registers
+__global__ void __launch_bounds__(PT_THREADS, min_blocks<STACK, ALPHA, LEVELS>)
         k_pt_shadow(J S, const vkg_ray *__restrict__ s_ray, const uint32_t *__restrict__ s_pid,
                     const float4 *__restrict__ s_contrib, const uint32_t *__restrict__ count,
                     float4 *__restrict__ radiance, const uint32_t *__restrict__ perm = nullptr,
