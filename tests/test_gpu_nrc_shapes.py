@@ -75,3 +75,21 @@ def test_inference(ctx, n):
     # the emulated BF16 network: only FP32 sums and a rounding flip of a BF16 activation (2^-8 of it) differ
     assert np.abs(got - want).max() <= 0.05 * max(1.0, np.abs(want).max())
     cache.close()
+
+
+def test_binned_batches_equal_their_parts(ctx):
+    """a batch of 2^19 records or more is encoded in the order of its cells; its predictions are those of
+    the same records in smaller batches, records outside the box and repeated ones among them"""
+    cache, _, _ = _cache(ctx, 16)
+    n = (1 << 19) + 1077
+    feats = random_features(n, 3)
+    feats[::17, 0:3] *= 3.0
+    feats[5::1000] = feats[4]
+    whole = cache.infer(feats)
+    half = n // 2
+    assert torch.equal(whole, torch.cat([cache.infer(feats[:half]), cache.infer(feats[half:])]))
+    # all in one cell: the batch keeps its order
+    feats[:, 0:3] = feats[:, 0:3] * 0.01 + 0.013
+    whole = cache.infer(feats)
+    assert torch.equal(whole, torch.cat([cache.infer(feats[:half]), cache.infer(feats[half:])]))
+    cache.close()

@@ -132,6 +132,11 @@ const uint32_t *bin_rays(vkg_ctx *ctx, const vkg_bvh *bvh, const vkg_ray *d_rays
 // traversal, which ends at the first hit, from about 1.5 million (600,000: 164 -> 184 us, 784,000: 209 ->
 // 218 us, 1,200,000: 351 either way, 1,800,000: 551 -> 534 us).
 constexpr uint32_t BIN_MIN_CLOSEST = 1u << 19, BIN_MIN_ANY = 3u << 19;
+// the same for points (the first three floats of records of `stride` floats) over a 32^3 grid of the box
+// lo, 1 / scale: neighbouring positions of the order are neighbouring in space
+const uint32_t *bin_points(vkg_ctx *ctx, const float *d_points, uint32_t stride, uint32_t n, const uint32_t *d_n,
+                           const float lo[3], const float scale[3], uint32_t min_points, cudaStream_t st,
+                           const uint32_t **reordered_out);
 // after the launch that reads the order: the scratch may be reused once the stream reaches here
 inline void bin_rays_done(vkg_ctx *ctx, cudaStream_t st) { cudaEventRecord(ctx->bins.done, st); }
 }// namespace vkg

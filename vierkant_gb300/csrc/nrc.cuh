@@ -65,6 +65,7 @@ struct grid_config
     float growth;
     float smin[3], sinv[3]; // position normalisation: p = (x - smin) * sinv
     uint32_t res[16];       // level_res() of every level
+    uint32_t dense;         // bit l: level l's (res + 1)^3 corners fit its table
 };
 
 __host__ __device__ inline uint32_t level_res(const grid_config &g, uint32_t l)

@@ -39,9 +39,9 @@ __device__ __forceinline__ void sh4(float x, float y, float z, float *o)
 
 struct corner_iter
 {
-    uint32_t res, table;
+    uint32_t res, mask;
     bool dense;
-    int cx, cy, cz;
+    uint32_t cx, cy, cz;
     float fx, fy, fz;
 };
 
@@ -49,35 +49,53 @@ __device__ __forceinline__ corner_iter level_setup(const grid_config &gc, uint32
 {
     corner_iter c;
     c.res = gc.res[l];
-    c.table = 1u << gc.log2_t;
-    const uint64_t r1 = (uint64_t)c.res + 1;
-    c.dense = r1 * r1 * r1 <= (uint64_t)c.table;
+    c.mask = (1u << gc.log2_t) - 1u;
+    c.dense = (gc.dense >> l) & 1u;
     const float x = px * (float)c.res, y = py * (float)c.res, z = pz * (float)c.res;
     // the cell is clamped so p = 1 interpolates inside the last cell (every corner stays in range)
     const float top = (float)(c.res - 1);
     const float flx = fminf(floorf(x), top), fly = fminf(floorf(y), top), flz = fminf(floorf(z), top);
-    c.cx = (int)flx;
-    c.cy = (int)fly;
-    c.cz = (int)flz;
+    c.cx = (uint32_t)(int)flx;
+    c.cy = (uint32_t)(int)fly;
+    c.cz = (uint32_t)(int)flz;
     c.fx = x - flx;
     c.fy = y - fly;
     c.fz = z - flz;
     return c;
 }
 
-__device__ __forceinline__ uint32_t corner_index(const corner_iter &c, int k, float &w)
+// table entries and trilinear weights of the cell's corners; corner k is at x + (k & 1), y + (k >> 1 & 1),
+// z + (k >> 2 & 1). Dense levels are indexed, the others hashed (x ^ y 2654435761 ^ z 805459861)
+__device__ __forceinline__ void corners(const corner_iter &c, uint32_t (&idx)[8], float (&w)[8])
 {
-    const uint32_t x = (uint32_t)(c.cx + (k & 1)), y = (uint32_t)(c.cy + ((k >> 1) & 1)),
-                   z = (uint32_t)(c.cz + ((k >> 2) & 1));
-    w = ((k & 1) ? c.fx : 1.f - c.fx) * ((k & 2) ? c.fy : 1.f - c.fy) * ((k & 4) ? c.fz : 1.f - c.fz);
-    if(c.dense) return x + y * (c.res + 1) + z * (c.res + 1) * (c.res + 1);
-    return (x * 1u ^ y * 2654435761u ^ z * 805459861u) & (c.table - 1u);
+    if(c.dense)
+    {
+        const uint32_t s = c.res + 1, base = c.cx + (c.cy + c.cz * s) * s;
+#pragma unroll
+        for(int k = 0; k < 8; ++k) idx[k] = base + (k & 1) + ((k & 2) ? s : 0u) + ((k & 4) ? s * s : 0u);
+    }
+    else
+    {
+        const uint32_t hy = c.cy * 2654435761u, hz = c.cz * 805459861u;
+#pragma unroll
+        for(int k = 0; k < 8; ++k)
+            idx[k] = ((c.cx + (k & 1)) ^ ((k & 2) ? hy + 2654435761u : hy) ^ ((k & 4) ? hz + 805459861u : hz)) & c.mask;
+    }
+#pragma unroll
+    for(int k = 0; k < 8; ++k)
+        w[k] = ((k & 1) ? c.fx : 1.f - c.fx) * ((k & 2) ? c.fy : 1.f - c.fy) * ((k & 4) ? c.fz : 1.f - c.fz);
 }
 
 __device__ __forceinline__ uint32_t quad_word(const uint4 &q, uint32_t i)
 {
     const uint32_t a = (i & 1u) ? q.y : q.x, b = (i & 1u) ? q.w : q.z;
     return (i & 2u) ? b : a;
+}
+
+// v = *p if cond, as a predicated load (a branch per entry costs its reconvergence)
+__device__ __forceinline__ void ld_if(uint32_t cond, const uint32_t *p, uint32_t &v)
+{
+    asm("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %2, 0;\n\t@q ld.global.nc.u32 %0, [%1];\n}" : "+r"(v) : "l"(p), "r"(cond));
 }
 
 // BF16 feature pair of one level: the eight corners' entries interpolated. The gathers are bound by
@@ -92,8 +110,7 @@ __device__ __forceinline__ uint32_t encode_level(const grid_config &gc, const __
     float w[8];
     uint32_t idx[8], e[8];
     uint4 q[4];
-#pragma unroll
-    for(int k = 0; k < 8; ++k) idx[k] = corner_index(c, k, w[k]);
+    corners(c, idx, w);
 #pragma unroll
     for(int p = 0; p < 4; ++p) q[p] = __ldg(reinterpret_cast<const uint4 *>(tab) + (idx[2 * p] >> 2));
 #pragma unroll
@@ -101,7 +118,7 @@ __device__ __forceinline__ uint32_t encode_level(const grid_config &gc, const __
     {
         e[2 * p] = quad_word(q[p], idx[2 * p]);
         e[2 * p + 1] = quad_word(q[p], idx[2 * p + 1]);
-        if((idx[2 * p] ^ idx[2 * p + 1]) >> 2) e[2 * p + 1] = __ldg(tab + idx[2 * p + 1]);
+        ld_if((idx[2 * p] ^ idx[2 * p + 1]) >> 2, tab + idx[2 * p + 1], e[2 * p + 1]);
     }
     float f0 = 0.f, f1 = 0.f;
 #pragma unroll

@@ -280,6 +280,24 @@ __global__ void __launch_bounds__(256)
     bins[i] = (uint16_t)ray_bin(__ldg(rp), __ldg(rp + 1), lo, scale);
 }
 
+// bins of points instead of rays: the Morton index of a point's cell in a 32 x 32 x 32 grid over the box
+// lo, 1 / scale (points outside count to the border cells); `stride` floats from point to point
+__global__ void __launch_bounds__(256)
+        k_bin_point_keys(const float *__restrict__ pts, uint32_t stride, uint32_t n_cap, const uint32_t *__restrict__ d_n,
+                         float3 lo, float3 scale, uint16_t *__restrict__ bins, uint32_t *__restrict__ reordered)
+{
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if(i == 0) *reordered = 0u;
+    const uint32_t n = d_n ? min(*d_n, n_cap) : n_cap;
+    if(i >= n) return;
+    const float *p = pts + (size_t)stride * i;
+    auto cell = [](float x, float l, float s) {
+        return (uint32_t)min(max(__float2int_rz((x - l) * s * 32.f), 0), 31);
+    };
+    bins[i] = (uint16_t)((expand10(cell(__ldg(p), lo.x, scale.x)) << 2) | (expand10(cell(__ldg(p + 1), lo.y, scale.y)) << 1) |
+                         expand10(cell(__ldg(p + 2), lo.z, scale.z)));
+}
+
 // Each warp walks its own contiguous 1/32 of the tile, 32 rays a step. Steps whose rays all share
 // one bin extend a run of that bin; a run takes its ranks with one atomic when it ends (its keys are
 // written then), so a stretch of coherent rays costs one atomic instead of one per step and warp
@@ -561,11 +579,14 @@ vkg_status check_common(vkg_ctx *ctx, const vkg_bvh *bvh, const void *rays, cons
 
 }// namespace
 
-const uint32_t *bin_rays(vkg_ctx *ctx, const vkg_bvh *bvh, const vkg_ray *d_rays, uint32_t n, const uint32_t *d_n,
-                         uint32_t flags, uint32_t min_rays, cudaStream_t st, const uint32_t **reordered_out)
+namespace
+{
+// the order of n elements whose 16-bit bins write_bins(bins, reordered) computes on the stream
+template<class WriteBins>
+const uint32_t *bin_order(vkg_ctx *ctx, uint32_t n, const uint32_t *d_n, cudaStream_t st, const uint32_t **reordered_out,
+                          WriteBins write_bins)
 {
     *reordered_out = nullptr;
-    if((flags & VKG_RAY_KEEP_ORDER) || n < min_rays || !bvh) return nullptr;
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     if(cudaStreamIsCapturing(st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone)
     {
@@ -629,6 +650,26 @@ const uint32_t *bin_rays(vkg_ctx *ctx, const vkg_bvh *bvh, const vkg_ray *d_rays
         b.cap = n;
         b.tiles_cap = tiles;
     }
+    uint32_t *S = b.bin_totals, *F = b.bin_totals + BIN_SLOTS;
+    // the 16-bit bins live in the first half of perm's storage until k_bin_place overwrites it
+    // (k_bin_tiles reads them before; k_bin_place reads only keys)
+    uint16_t *bins16 = reinterpret_cast<uint16_t *>(b.perm);
+    uint32_t *reordered = b.bin_totals + 2 * BIN_SLOTS;
+    write_bins(bins16, reordered);
+    k_bin_tiles<<<tiles, BIN_THREADS, BIN_SMEM, st>>>(bins16, n, d_n, tile, b.keys, b.tile_counts, reordered);
+    k_bin_columns<<<BIN_SLOTS / 32, 1024, 0, st>>>(b.tile_counts, tiles, S, reordered);
+    k_bin_offsets<<<1, BIN_THREADS, BIN_SCAN_SMEM, st>>>(S, F, reordered);
+    k_bin_place<<<(n + 255) / 256, 256, 0, st>>>(b.keys, n, d_n, tile, b.tile_counts, F, b.perm, reordered);
+    *reordered_out = reordered;
+    return b.perm;
+}
+}// namespace
+
+const uint32_t *bin_rays(vkg_ctx *ctx, const vkg_bvh *bvh, const vkg_ray *d_rays, uint32_t n, const uint32_t *d_n,
+                         uint32_t flags, uint32_t min_rays, cudaStream_t st, const uint32_t **reordered_out)
+{
+    *reordered_out = nullptr;
+    if((flags & VKG_RAY_KEEP_ORDER) || n < min_rays || !bvh) return nullptr;
     float3 lo, scale;
     float *plo = &lo.x, *ps = &scale.x;
     for(int a = 0; a < 3; ++a)
@@ -637,18 +678,21 @@ const uint32_t *bin_rays(vkg_ctx *ctx, const vkg_bvh *bvh, const vkg_ray *d_rays
         const float ext = bvh->scene_max[a] - bvh->scene_min[a];
         ps[a] = ext > 0.f ? (float)(1 << BIN_CELL_BITS) / ext : 0.f;
     }
-    uint32_t *S = b.bin_totals, *F = b.bin_totals + BIN_SLOTS;
-    // the 16-bit bins live in the first half of perm's storage until k_bin_place overwrites it
-    // (k_bin_tiles reads them before; k_bin_place reads only keys)
-    uint16_t *bins16 = reinterpret_cast<uint16_t *>(b.perm);
-    uint32_t *reordered = b.bin_totals + 2 * BIN_SLOTS;
-    k_bin_keys<<<(n + 255) / 256, 256, 0, st>>>(d_rays, n, d_n, lo, scale, bins16, reordered);
-    k_bin_tiles<<<tiles, BIN_THREADS, BIN_SMEM, st>>>(bins16, n, d_n, tile, b.keys, b.tile_counts, reordered);
-    k_bin_columns<<<BIN_SLOTS / 32, 1024, 0, st>>>(b.tile_counts, tiles, S, reordered);
-    k_bin_offsets<<<1, BIN_THREADS, BIN_SCAN_SMEM, st>>>(S, F, reordered);
-    k_bin_place<<<(n + 255) / 256, 256, 0, st>>>(b.keys, n, d_n, tile, b.tile_counts, F, b.perm, reordered);
-    *reordered_out = reordered;
-    return b.perm;
+    return bin_order(ctx, n, d_n, st, reordered_out, [&](uint16_t *bins, uint32_t *reordered) {
+        k_bin_keys<<<(n + 255) / 256, 256, 0, st>>>(d_rays, n, d_n, lo, scale, bins, reordered);
+    });
+}
+
+const uint32_t *bin_points(vkg_ctx *ctx, const float *d_points, uint32_t stride, uint32_t n, const uint32_t *d_n,
+                           const float lo[3], const float scale[3], uint32_t min_points, cudaStream_t st,
+                           const uint32_t **reordered_out)
+{
+    *reordered_out = nullptr;
+    if(n < min_points) return nullptr;
+    return bin_order(ctx, n, d_n, st, reordered_out, [&](uint16_t *bins, uint32_t *reordered) {
+        k_bin_point_keys<<<(n + 255) / 256, 256, 0, st>>>(d_points, stride, n, d_n, make_float3(lo[0], lo[1], lo[2]),
+                                                          make_float3(scale[0], scale[1], scale[2]), bins, reordered);
+    });
 }
 
 }// namespace vkg
