@@ -266,16 +266,29 @@ __global__ void __launch_bounds__(TC_THREADS)
 }
 
 // ---- pipelined inference: independent warpgroups ------------------------------------------------
-// The single-tile kernel above leaves the tensor core idle while a layer's epilogue (TMEM -> registers
-// -> ReLU / BF16 -> shared memory) runs, and the epilogue, not the MMA, sets its time. Here a CTA of
-// NWG warpgroups (128 threads each) runs NWG tiles at once: warpgroup g owns 64 TMEM columns
-// [64 g, 64 g + 64), one A operand in shared memory, one mbarrier and named barrier g + 1, and its
-// thread 0 issues its own MMAs; so while one warpgroup drains its accumulator the tensor core works
-// on another's layer. The weights (all six layers, 45 KB) are shared. Thread r of a warpgroup owns
-// row r of its tile (TMEM lane r: warp w reads lanes 32 (w mod 4) .. + 31). Inputs are the encoded
-// BF16 records of k_encode.
+// The single-tile kernel above leaves the tensor core idle while a layer's epilogue runs, and the
+// epilogue, not the MMA, sets its time. Here a CTA of NWG warpgroups (128 threads each) runs NWG tiles
+// at once, each with 96 TMEM columns, an mbarrier and a named barrier of its own, and its thread 0
+// issues its own MMAs; so while one warpgroup drains its accumulator the tensor core works on
+// another's layer. The weights (all six layers, 45 KB) are shared. Thread r of a warpgroup owns row r of
+// its tile (TMEM lane r: warp w reads lanes 32 (w mod 4) .. + 31).
+// Layer 0 reads the encoded BF16 records of k_encode from shared memory (canonical K-major), copied there
+// by cp.async while the tile before runs its later layers. The hidden layers read their operand from
+// TMEM: the epilogue (64 columns in, ReLU, BF16) stores 32 columns back with tcgen05.st, which takes the
+// 16 KB a layer and tile of shared-memory stores and reads out of the way. 2,073,600 queries: 222 us
+// with operands in shared memory and eight warpgroups, 183 us with four this way; as the training forward of
+// 262,144 records 32 -> 26 us (it stores 168 MB).
 // TRAIN: also store the hidden activations H1..H5 (BF16, 5 x 64 per record in natural column order,
 // the layout the backward reads) as the training forward.
+// TMEM columns a CTA of g warpgroups allocates when each uses `per`: a power of two of at least 32
+__host__ __device__ constexpr uint32_t tmem_columns(uint32_t per, uint32_t g)
+{
+    uint32_t c = 32;
+    while(c < per * g) c *= 2;
+    return c;
+}
+constexpr uint32_t TC_WG_COLS = 96; // per warpgroup: 64 of the accumulator, 32 of the next layer's operand
+
 template<int NWG, bool TRAIN>
 __global__ void __launch_bounds__(NWG * 128)
         k_infer_tc_wg(const uint32_t *__restrict__ X, uint32_t n_cap, const uint32_t *__restrict__ d_n,
@@ -287,31 +300,40 @@ __global__ void __launch_bounds__(NWG * 128)
     __shared__ uint32_t tslot;
     const uint32_t tid = threadIdx.x, warp = tid >> 5, g = tid >> 7, r = tid & 127u;
     uint8_t *sw = smem, *sa = smem + TC_W_BYTES + g * TC_A_BYTES;
+    const uint32_t sw_addr = tc::smem_addr(sw), sa_addr = tc::smem_addr(sa);
+    const uint32_t n = eff_n(n_cap, d_n), tiles = (n + TC_TILE - 1) / TC_TILE;
+    // this thread's row of a tile's layer-0 operand (zeros past n)
+    auto load = [&](uint32_t tile) {
+        const uint32_t q = tile * TC_TILE + r;
+        const uint32_t *src = X + (size_t)(IN / 2) * (q < n ? q : 0u);
+#pragma unroll
+        for(int j = 0; j < IN / 8; ++j)
+            tc::cp_async16(sa_addr + tc::canon_offset(r, 8 * j, IN), src + 4 * j, q < n);
+    };
+    const uint32_t first = blockIdx.x * NWG + g;
+    if(first < tiles) load(first);
     for(uint32_t i = tid; i < TC_W_BYTES / 16; i += NWG * 128)
-        reinterpret_cast<uint4 *>(sw)[i] = reinterpret_cast<const uint4 *>(wtc)[i];
-    // TMEM columns: 64 per warpgroup, allocated as a power of two of at least 32
-    static_assert(NWG >= 1 && NWG <= 8, "at most 512 TMEM columns");
-    constexpr uint32_t COLS = NWG * 64 <= 64 ? 64 : (NWG * 64 <= 128 ? 128 : (NWG * 64 <= 256 ? 256 : 512));
+        tc::cp_async16(sw_addr + 16u * i, reinterpret_cast<const uint4 *>(wtc) + i, true);
+    static_assert(NWG >= 1 && NWG * TC_WG_COLS <= 512, "at most 512 TMEM columns");
+    constexpr uint32_t COLS = tmem_columns(TC_WG_COLS, NWG);
     if(warp == 0) tc::tmem_alloc(&tslot, COLS);
     if(tid < NWG) tc::mbar_init(&mbar[tid], 1);
+    tc::cp_async_commit();
+    tc::cp_async_wait<0>();
     tc::fence_async_smem();
     tc::fence_before_sync();
     __syncthreads();
     tc::fence_after_sync();
-    const uint32_t tmem = tslot + 64u * g, lane_base = ((warp & 3u) * 32u) << 16;
-    const uint32_t sw_addr = tc::smem_addr(sw), sa_addr = tc::smem_addr(sa);
-    const uint32_t n = eff_n(n_cap, d_n), tiles = (n + TC_TILE - 1) / TC_TILE;
+    const uint32_t tmem = tslot + TC_WG_COLS * g, ta = tmem + 64u, lane_base = ((warp & 3u) * 32u) << 16;
     const uint32_t bar_id = g + 1;
     uint32_t phase = 0;
     bool failed = false;
 
-    for(uint32_t tile = blockIdx.x * NWG + g; tile < tiles && !failed; tile += gridDim.x * NWG)
+    for(uint32_t tile = first; tile < tiles && !failed; tile += gridDim.x * NWG)
     {
         const uint32_t q = tile * TC_TILE + r;
-        const uint4 *src = reinterpret_cast<const uint4 *>(X + (size_t)(IN / 2) * q);
-#pragma unroll
-        for(int j = 0; j < IN / 8; ++j)
-            *reinterpret_cast<uint4 *>(sa + tc::canon_offset(r, 8 * j, IN)) = q < n ? src[j] : make_uint4(0u, 0u, 0u, 0u);
+        // the tile's rows were loaded during the tile before
+        tc::cp_async_wait<0>();
         tc::fence_async_smem();
         tc::fence_before_sync();
         tc::wg_sync(bar_id);
@@ -325,8 +347,11 @@ __global__ void __launch_bounds__(NWG * 128)
                 const uint32_t idesc = tc::idesc_bf16(TC_TILE, N);
                 const uint32_t wb = sw_addr + (uint32_t)layer_off(l) * 2u;
                 for(uint32_t s = 0; s < K / 16; ++s)
-                    tc::mma_bf16(tmem, tc::smem_desc(sa_addr + 256u * s, 128u, K * 16u),
-                                 tc::smem_desc(wb + 256u * s, 128u, K * 16u), idesc, s > 0);
+                {
+                    const uint64_t b = tc::smem_desc(wb + 256u * s, 128u, K * 16u);
+                    if(l == 0) tc::mma_bf16(tmem, tc::smem_desc(sa_addr + 256u * s, 128u, K * 16u), b, idesc, s > 0);
+                    else tc::mma_bf16_ts(tmem, ta + 8u * s, b, idesc, s > 0);
+                }
                 tc::mma_commit(&mbar[g]);
             }
             const bool ok = tc::mbar_wait(&mbar[g], phase);
@@ -337,6 +362,11 @@ __global__ void __launch_bounds__(NWG * 128)
             }
             phase ^= 1u;
             tc::fence_after_sync();
+            if(l == 0 && tile + gridDim.x * NWG < tiles)
+            {
+                load(tile + gridDim.x * NWG); // layer 0 is done with the operand
+                tc::cp_async_commit();
+            }
             if(l + 1 < NLAYER)
             {
                 // two TMEM loads in flight per wait
@@ -347,27 +377,19 @@ __global__ void __launch_bounds__(NWG * 128)
                     tc::tmem_ld16(tmem + lane_base + 32u * c2, v[0]);
                     tc::tmem_ld16(tmem + lane_base + 32u * c2 + 16u, v[1]);
                     tc::tmem_ld_wait();
+                    uint32_t hv[16];
 #pragma unroll
-                    for(int cc = 0; cc < 2; ++cc)
+                    for(int j = 0; j < 16; ++j)
+                        hv[j] = pack_bf16(fmaxf(v[j >> 3][2 * (j & 7)], 0.f), fmaxf(v[j >> 3][2 * (j & 7) + 1], 0.f));
+                    tc::tmem_st16(ta + lane_base + 16u * c2, hv);
+                    if(TRAIN && q < n)
                     {
-                        const int c = 2 * c2 + cc;
-                        uint32_t hv[8];
+                        uint4 *hp = reinterpret_cast<uint4 *>(H + (size_t)q * (5 * HID / 2) + l * (HID / 2) + 16 * c2);
 #pragma unroll
-                        for(int j = 0; j < 8; ++j)
-                            hv[j] = pack_bf16(fmaxf(v[cc][2 * j], 0.f), fmaxf(v[cc][2 * j + 1], 0.f));
-                        *reinterpret_cast<uint4 *>(sa + tc::canon_offset(r, 16 * c, HID)) =
-                                make_uint4(hv[0], hv[1], hv[2], hv[3]);
-                        *reinterpret_cast<uint4 *>(sa + tc::canon_offset(r, 16 * c + 8, HID)) =
-                                make_uint4(hv[4], hv[5], hv[6], hv[7]);
-                        if(TRAIN && q < n)
-                        {
-                            uint4 *hp = reinterpret_cast<uint4 *>(H + (size_t)q * (5 * HID / 2) + l * (HID / 2) + 8 * c);
-                            hp[0] = make_uint4(hv[0], hv[1], hv[2], hv[3]);
-                            hp[1] = make_uint4(hv[4], hv[5], hv[6], hv[7]);
-                        }
+                        for(int j = 0; j < 4; ++j) hp[j] = make_uint4(hv[4 * j], hv[4 * j + 1], hv[4 * j + 2], hv[4 * j + 3]);
                     }
                 }
-                tc::fence_async_smem();
+                tc::tmem_st_wait();
             }
             else
             {
@@ -385,6 +407,7 @@ __global__ void __launch_bounds__(NWG * 128)
             tc::wg_sync(bar_id);
         }
     }
+    tc::cp_async_wait<0>();
     if(failed)
     {
         if(r == 0) atomicOr(err, TC_TIMEOUT);
@@ -402,11 +425,12 @@ __global__ void __launch_bounds__(NWG * 128)
 //   dy = dL/dy of the relative L2 loss (|y - t|^2 / (y^2 + 0.01), mean over 3n) -> G block 5 and the
 //   BF16 A operand (128 x 16);
 //   for l = 5 .. 1: D = G_l W_l^T (UMMA, TMEM), G_{l-1} = D * [H_l > 0] rounded to BF16 -> G block
-//   l - 1 and the next A operand (128 x 64);
+//   l - 1 and the next A operand (128 x 64), in TMEM as in the forward; H_l is fetched during the MMAs;
+//   262,144 records: 47 us with operands in shared memory and eight warpgroups, 31 us (343 MB) this way;
 //   dX (the 32 hash-grid features) = G_0 W_0^T (N = 32) -> dXg in FP32.
 // Quantisation points equal k_backward's (FP32 sums, mask in FP32, BF16 rounding of each G); only
 // the summation order inside an MMA differs. Weights: wtc_t (k_pack_tc_t), resident in shared memory.
-constexpr uint32_t TC_G_BYTES = TC_TILE * HID * 2; // one A operand of the backward (16,384 B)
+constexpr uint32_t TC_G_BYTES = TC_TILE * OUTP * 2; // the backward's first A operand (4,096 B)
 template<int NWG>
 __global__ void __launch_bounds__(NWG * 128)
         k_backward_tc_wg(const uint32_t *__restrict__ H, const float *__restrict__ Y, const float *__restrict__ T,
@@ -420,16 +444,18 @@ __global__ void __launch_bounds__(NWG * 128)
     const uint32_t tid = threadIdx.x, warp = tid >> 5, g = tid >> 7, r = tid & 127u;
     uint8_t *sw = smem, *sa = smem + TC_W_BYTES + g * TC_G_BYTES;
     for(uint32_t i = tid; i < TC_W_BYTES / 16; i += NWG * 128)
-        reinterpret_cast<uint4 *>(sw)[i] = reinterpret_cast<const uint4 *>(wtc_t)[i];
-    static_assert(NWG >= 1 && NWG <= 8, "at most 512 TMEM columns");
-    constexpr uint32_t COLS = NWG * 64 <= 64 ? 64 : (NWG * 64 <= 128 ? 128 : (NWG * 64 <= 256 ? 256 : 512));
+        tc::cp_async16(tc::smem_addr(sw) + 16u * i, reinterpret_cast<const uint4 *>(wtc_t) + i, true);
+    tc::cp_async_commit();
+    static_assert(NWG >= 1 && NWG * TC_WG_COLS <= 512, "at most 512 TMEM columns");
+    constexpr uint32_t COLS = tmem_columns(TC_WG_COLS, NWG);
     if(warp == 0) tc::tmem_alloc(&tslot, COLS);
     if(tid < NWG) tc::mbar_init(&mbar[tid], 1);
+    tc::cp_async_wait<0>();
     tc::fence_async_smem();
     tc::fence_before_sync();
     __syncthreads();
     tc::fence_after_sync();
-    const uint32_t tmem = tslot + 64u * g, lane_base = ((warp & 3u) * 32u) << 16;
+    const uint32_t tmem = tslot + TC_WG_COLS * g, ta = tmem + 64u, lane_base = ((warp & 3u) * 32u) << 16;
     const uint32_t sw_addr = tc::smem_addr(sw), sa_addr = tc::smem_addr(sa);
     const uint32_t n = eff_n(n_cap, d_n), tiles = (n + TC_TILE - 1) / TC_TILE;
     const float inv_count = n ? 1.f / (3.f * (float)n) : 0.f;
@@ -477,10 +503,19 @@ __global__ void __launch_bounds__(NWG * 128)
                 const uint32_t idesc = tc::idesc_bf16(TC_TILE, rows);
                 const uint32_t wb = sw_addr + (uint32_t)layer_off(l) * 2u;
                 for(uint32_t s = 0; s < Kp / 16; ++s)
-                    tc::mma_bf16(tmem, tc::smem_desc(sa_addr + 256u * s, 128u, Kp * 16u),
-                                 tc::smem_desc(wb + 256u * s, 128u, Kp * 16u), idesc, s > 0);
+                {
+                    const uint64_t b = tc::smem_desc(wb + 256u * s, 128u, Kp * 16u);
+                    if(l == NLAYER - 1) tc::mma_bf16(tmem, tc::smem_desc(sa_addr + 256u * s, 128u, Kp * 16u), b, idesc, s > 0);
+                    else tc::mma_bf16_ts(tmem, ta + 8u * s, b, idesc, s > 0);
+                }
                 tc::mma_commit(&mbar[g]);
             }
+            // H_l (block l - 1 of H), on its way while the MMAs run
+            uint4 h[8];
+#pragma unroll
+            for(int j = 0; j < 8; ++j)
+                h[j] = valid && l > 0 ? __ldg(reinterpret_cast<const uint4 *>(H + (size_t)q * 160 + (l - 1) * 32) + j)
+                                      : make_uint4(0u, 0u, 0u, 0u);
             const bool ok = tc::mbar_wait(&mbar[g], phase);
             if(tc::wg_sync_or(bar_id, !ok))
             {
@@ -491,35 +526,32 @@ __global__ void __launch_bounds__(NWG * 128)
             tc::fence_after_sync();
             if(l > 0)
             {
-                // G_{l-1} = dH_l * [H_l > 0]; H_l is block l - 1 of H
-                const uint4 *hp = reinterpret_cast<const uint4 *>(H + (size_t)q * 160 + (l - 1) * 32);
+                // G_{l-1} = dH_l * [H_l > 0]
 #pragma unroll
-                for(int c = 0; c < 4; ++c)
+                for(int c = 0; c < 2; ++c)
                 {
-                    float v[16];
-                    tc::tmem_ld16(tmem + lane_base + 16u * c, v);
+                    float v[2][16];
+                    tc::tmem_ld16(tmem + lane_base + 32u * c, v[0]);
+                    tc::tmem_ld16(tmem + lane_base + 32u * c + 16u, v[1]);
                     tc::tmem_ld_wait();
-                    const uint4 h0 = valid ? hp[2 * c] : make_uint4(0u, 0u, 0u, 0u);
-                    const uint4 h1 = valid ? hp[2 * c + 1] : make_uint4(0u, 0u, 0u, 0u);
-                    const uint32_t hw[8] = {h0.x, h0.y, h0.z, h0.w, h1.x, h1.y, h1.z, h1.w};
-                    uint32_t gv[8];
+                    uint32_t gv[16];
 #pragma unroll
-                    for(int j = 0; j < 8; ++j)
+                    for(int j = 0; j < 16; ++j)
                     {
-                        const float m0 = (hw[j] & 0x7FFFu) ? 1.f : 0.f, m1 = ((hw[j] >> 16) & 0x7FFFu) ? 1.f : 0.f;
-                        gv[j] = pack_bf16(v[2 * j] * m0, v[2 * j + 1] * m1);
+                        const uint4 &hq = h[4 * c + (j >> 2)];
+                        const uint32_t hw = (j & 3) == 0 ? hq.x : (j & 3) == 1 ? hq.y : (j & 3) == 2 ? hq.z : hq.w;
+                        const float m0 = (hw & 0x7FFFu) ? 1.f : 0.f, m1 = ((hw >> 16) & 0x7FFFu) ? 1.f : 0.f;
+                        gv[j] = pack_bf16(v[j >> 3][2 * (j & 7)] * m0, v[j >> 3][2 * (j & 7) + 1] * m1);
                     }
-                    *reinterpret_cast<uint4 *>(sa + tc::canon_offset(r, 16 * c, HID)) = make_uint4(gv[0], gv[1], gv[2], gv[3]);
-                    *reinterpret_cast<uint4 *>(sa + tc::canon_offset(r, 16 * c + 8, HID)) =
-                            make_uint4(gv[4], gv[5], gv[6], gv[7]);
+                    tc::tmem_st16(ta + lane_base + 16u * c, gv);
                     if(valid)
                     {
-                        uint4 *gp = reinterpret_cast<uint4 *>(G + (size_t)q * 168 + (l - 1) * 32 + 8 * c);
-                        gp[0] = make_uint4(gv[0], gv[1], gv[2], gv[3]);
-                        gp[1] = make_uint4(gv[4], gv[5], gv[6], gv[7]);
+                        uint4 *gp = reinterpret_cast<uint4 *>(G + (size_t)q * 168 + (l - 1) * 32 + 16 * c);
+#pragma unroll
+                        for(int j = 0; j < 4; ++j) gp[j] = make_uint4(gv[4 * j], gv[4 * j + 1], gv[4 * j + 2], gv[4 * j + 3]);
                     }
                 }
-                tc::fence_async_smem();
+                tc::tmem_st_wait();
             }
             else
             {
@@ -758,8 +790,8 @@ vkg_status launch_forward_tc(vkg_ctx *ctx, const uint16_t *wtc, const uint32_t *
     VKG_TRY_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     int per_sm = 0;
     VKG_TRY_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, NWG * 128, smem));
-    // TMEM: a resident CTA holds NWG x 64 of the SM's 512 columns
-    per_sm = std::max(1, std::min(per_sm, 512 / (NWG * 64)));
+    // TMEM: a resident CTA holds its share of the SM's 512 columns
+    per_sm = std::max(1, std::min(per_sm, (int)(512 / tmem_columns(TC_WG_COLS, NWG))));
     const uint32_t tiles = (n + TC_TILE - 1) / TC_TILE;
     const uint32_t grid_n = std::min<uint32_t>((tiles + NWG - 1) / NWG, (uint32_t)(ctx->num_sms * per_sm));
     kern<<<grid_n, NWG * 128, smem, st>>>(X, n, d_n, wtc, Y, err, H);
@@ -770,10 +802,12 @@ vkg_status nrc_forward_tc(vkg_ctx *ctx, const uint16_t *wtc, const uint32_t *X, 
                           float *Y, uint32_t *H, uint32_t *err, cudaStream_t st)
 {
     if(n == 0) return VKG_OK;
-    // as many tiles in flight per SM as the batch fills: eight warpgroups once every SM gets eight tiles
+    // tiles in flight per SM (inference with the encoding, 4,096 / 20,000 / 65,536 / 2,073,600 queries: one
+    // warpgroup a CTA 19 / 28 / 46 / 908 us, two 21 / 25 / 42 / 751, four 24 / 29 / 40 / 643, five 26 / 31 /
+    // 42 / 684)
     const uint32_t tiles = (n + TC_TILE - 1) / TC_TILE, sms = (uint32_t)ctx->num_sms;
-    if(tiles >= 8 * sms) return launch_forward_tc<8>(ctx, wtc, X, n, d_n, Y, H, err, st);
-    if(tiles >= 4 * sms) return launch_forward_tc<4>(ctx, wtc, X, n, d_n, Y, H, err, st);
+    if(tiles >= 3 * sms) return launch_forward_tc<4>(ctx, wtc, X, n, d_n, Y, H, err, st);
+    if(tiles <= sms / 2) return launch_forward_tc<1>(ctx, wtc, X, n, d_n, Y, H, err, st);
     return launch_forward_tc<2>(ctx, wtc, X, n, d_n, Y, H, err, st);
 }
 
@@ -786,7 +820,7 @@ vkg_status launch_backward_tc(vkg_ctx *ctx, const uint16_t *wtc_t, const uint32_
     VKG_TRY_CUDA(ctx, cudaFuncSetAttribute(k_backward_tc_wg<NWG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     int per_sm = 0;
     VKG_TRY_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_backward_tc_wg<NWG>, NWG * 128, smem));
-    per_sm = std::max(1, std::min(per_sm, 512 / (NWG * 64)));
+    per_sm = std::max(1, std::min(per_sm, (int)(512 / tmem_columns(TC_WG_COLS, NWG))));
     const uint32_t tiles = (n + TC_TILE - 1) / TC_TILE;
     const uint32_t grid_n = std::min<uint32_t>((tiles + NWG - 1) / NWG, (uint32_t)(ctx->num_sms * per_sm));
     k_backward_tc_wg<NWG><<<grid_n, NWG * 128, smem, st>>>(H, Y, T, n, d_n, wtc_t, G, dXg, loss, err);
@@ -799,8 +833,7 @@ vkg_status nrc_backward_tc(vkg_ctx *ctx, const uint16_t *wtc_t, const uint32_t *
 {
     if(n == 0) return VKG_OK;
     const uint32_t tiles = (n + TC_TILE - 1) / TC_TILE, sms = (uint32_t)ctx->num_sms;
-    if(tiles >= 8 * sms) return launch_backward_tc<8>(ctx, wtc_t, H, Y, T, n, d_n, G, dXg, loss, err, st);
-    if(tiles >= 4 * sms) return launch_backward_tc<4>(ctx, wtc_t, H, Y, T, n, d_n, G, dXg, loss, err, st);
+    if(tiles >= 3 * sms) return launch_backward_tc<4>(ctx, wtc_t, H, Y, T, n, d_n, G, dXg, loss, err, st);
     return launch_backward_tc<2>(ctx, wtc_t, H, Y, T, n, d_n, G, dXg, loss, err, st);
 }
 
