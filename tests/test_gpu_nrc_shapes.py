@@ -93,3 +93,56 @@ def test_binned_batches_equal_their_parts(ctx):
     whole = cache.infer(feats)
     assert torch.equal(whole, torch.cat([cache.infer(feats[:half]), cache.infer(feats[half:])]))
     cache.close()
+
+
+def _write(address, values):
+    torch.cuda.synchronize()
+    assert _cudart().cudaMemcpy(C.c_void_p(address), C.c_void_p(values.data_ptr()), C.c_size_t(4 * values.numel()), 3) == 0
+
+
+@pytest.mark.parametrize("steps", [1, 2, 5])
+@pytest.mark.parametrize("levels, kernel", [(1, 1), (16, 1), (16, 2)])
+def test_adam_steps(ctx, steps, levels, kernel):
+    """parameters after some steps against the formula in 64 bits. Gradients keep their sign, so nothing
+    cancels: each step adds 3 roundings (2^-24) to m and 4 to v (halved by the root), the update has 8
+    (4 of its own, at most 4 of the shared factor), each 1 - beta^t is off by at most 4 units of 2^-24
+    (powf is good to 2 ulp), and the sum rounds the parameter. A third of the gradients is always zero and
+    a third zero in every other step. The packed weights and the FP16 grid are those of the parameters."""
+    cfg = NeuralRadianceCache.default_config()
+    cfg.levels, cfg.log2_table_size, cfg.infer_kernel = levels, 12, kernel
+    cache = NeuralRadianceCache(ctx, cfg)
+    i = cache.info()
+    mlp, grid = _read(i.d_mlp_params, i.num_mlp_params), _read(i.d_grid_params, i.num_grid_params)
+    gen = torch.Generator(device="cuda").manual_seed(steps)
+    state = []
+    for p in (mlp, grid):
+        base = (torch.rand(p.numel(), generator=gen, device="cuda") + 0.25) * torch.where(p < 0, -1e-3, 1e-3)
+        state.append({"p": p.double(), "g": base, "kind": torch.arange(p.numel(), device="cuda") // 7 % 3,
+                      "m": torch.zeros_like(p, dtype=torch.float64), "v": torch.zeros_like(p, dtype=torch.float64),
+                      "tol": torch.zeros_like(p, dtype=torch.float64)})
+    b1, b2, lr, eps = (float(np.float32(x)) for x in (cfg.beta1, cfg.beta2, cfg.learning_rate, cfg.epsilon))
+    u = 2.0 ** -24
+    for t in range(1, steps + 1):
+        c1, c2 = 1 - b1 ** t, 1 - b2 ** t
+        for s, address in zip(state, (i.d_mlp_grads, i.d_grid_grads)):
+            g = torch.where((s["kind"] == 0) | ((s["kind"] == 1) & (t % 2 == 0)), 0.0, s["g"]) * (1 + 0.1 * t)
+            _write(address, g)
+            g = g.double()
+            s["m"] = b1 * s["m"] + (1 - b1) * g
+            s["v"] = b2 * s["v"] + (1 - b2) * g * g
+            d = lr * (s["m"] / c1) / (torch.sqrt(s["v"] / c2) + eps)
+            s["p"] = s["p"] - d
+            s["tol"] += u * (d.abs() * (4 / c1 + 2 / c2 + 3 * t + 2 * t + 8) + s["p"].abs())
+        cache.adam_step()
+        torch.cuda.synchronize()
+    i = cache.info()
+    assert i.step == steps and i.kernel_error == 0
+    got = [_read(i.d_mlp_params, i.num_mlp_params), _read(i.d_grid_params, i.num_grid_params)]
+    for s, p in zip(state, got):
+        assert torch.all((p.double() - s["p"]).abs() <= s["tol"])
+    for address, count in ((i.d_mlp_grads, i.num_mlp_params), (i.d_grid_grads, i.num_grid_params)):
+        assert torch.count_nonzero(_read(address, count)) == 0
+    feats = random_features(300, 1)
+    other = NeuralRadianceCache(ctx, cfg)
+    other.load_params(*got)
+    assert torch.equal(cache.infer(feats), other.infer(feats))

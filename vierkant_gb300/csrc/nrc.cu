@@ -8,6 +8,7 @@
 // memory. This mma.sync path is the correctness twin of the tcgen05 inference kernel
 // (nrc_tc.cu) and the training path.
 #include "nrc_encode.cuh"
+#include "tc.cuh"
 
 #include <cmath>
 #include <cstdio>
@@ -22,7 +23,7 @@ struct vkg_nrc
     uint32_t table = 0;          // entries per level
     size_t ngrid = 0;            // grid parameters (levels * table * 2)
     float lr = 1e-2f, b1 = 0.9f, b2 = 0.99f, eps = 1e-15f;
-    uint32_t *d_state = nullptr; // [0] Adam steps taken, [1] 1 if the current step has records
+    uint32_t *d_state = nullptr; // [0] Adam steps taken, [1] blocks of the current step that are done
     float *grid = nullptr, *grid_g = nullptr, *grid_m = nullptr, *grid_v = nullptr;
     __half2 *grid_h = nullptr;
     float *w = nullptr, *w_g = nullptr, *w_m = nullptr, *w_v = nullptr;
@@ -479,42 +480,135 @@ __global__ void __launch_bounds__(256)
     }
 }
 
-// An optimiser step starts on the device: it counts (and runs) only if its batch has records, so a
-// frame whose training paths all escaped leaves the parameters and the moments untouched.
-__global__ void k_adam_begin(const uint32_t *__restrict__ d_n, uint32_t *__restrict__ state)
+// One FP32 master weight ([in][out] row-major per layer), rounded to BF16, into every layout the MLP
+// kernels read: the per-lane B fragments of mma.sync (forward, and transposed for the backward) and the
+// canonical K-major operands of tcgen05 (wtc: layer l as N x K; wtc_t: layer l as K_l x N_l, rows = the
+// layer's inputs, so that D (128 x K_l) = G_l (128 x N_l) W_l^T is one MMA chain).
+struct packed_weights
 {
-    const bool active = d_n == nullptr || *d_n > 0;
-    state[1] = active ? 1u : 0u;
-    if(active) state[0] += 1u;
+    uint16_t *frag, *fragT, *wtc, *wtc_t;
+};
+
+__device__ __forceinline__ int fragment_slot(int k, int n, int width) // of a K x width operand, in 16-bit values
+{
+    const int lane = (n & 7) * 4 + ((k & 7) >> 1);
+    return ((((k >> 4) * (width / 8) + (n >> 3)) * 32 + lane) << 2) + (((k >> 3) & 1) << 1) + (k & 1);
 }
 
-// Adam (Kingma & Ba 2015) with bias correction 1 - beta^t, t the device step count; gradients are
-// consumed (zeroed). Each thread updates one pair of parameters so the FP16 copy (feature pairs) is
-// written from values it owns.
-__global__ void k_adam(float *__restrict__ p, float *__restrict__ g, float *__restrict__ m, float *__restrict__ v,
-                       size_t n, float lr, float b1, float b2, float eps, const uint32_t *__restrict__ state,
-                       __half2 *__restrict__ half_copy)
+__device__ __forceinline__ void pack_weight(int e, float w, const packed_weights &pk)
 {
-    if(state[1] == 0) return;
-    const float t = (float)state[0];
-    const float c1 = 1.f - powf(b1, t), c2 = 1.f - powf(b2, t);
-    const size_t stride = (size_t)gridDim.x * blockDim.x;
-    for(size_t i2 = (size_t)blockIdx.x * blockDim.x + threadIdx.x; 2 * i2 < n; i2 += stride)
+    int l = 0;
+    while(l + 1 < NLAYER && e >= layer_off(l + 1)) ++l;
+    const int K = layer_in(l), N = layer_out(l), local = e - layer_off(l);
+    const int k = local / N, n = local - k * N;
+    const uint16_t b = __bfloat16_as_ushort(__float2bfloat16_rn(w));
+    pk.frag[4 * frag_off(l) + fragment_slot(k, n, N)] = b;
+    pk.fragT[4 * fragT_off(l) + fragment_slot(n, k, K)] = b;
+    pk.wtc[layer_off(l) + tc::canon_offset(n, k, K) / 2] = b;
+    pk.wtc_t[layer_off(l) + tc::canon_offset(k, n, N) / 2] = b;
+}
+
+__global__ void k_pack(const float *__restrict__ W, packed_weights pk)
+{
+    const int e = blockIdx.x * blockDim.x + threadIdx.x;
+    if(e < NPARAM) pack_weight(e, W[e], pk);
+}
+
+struct adam_arrays
+{
+    float *p, *g, *m, *v;
+};
+
+// Adam (Kingma & Ba 2015) with bias correction c = 1 - beta^t, t the device step count:
+//   p -= lr (m / c1) / (sqrt(v / c2) + eps) = s m / (sqrt(v) + e),  s = lr sqrt(c2) / c1, e = eps sqrt(c2).
+// s is carried in two floats, so that an update has four roundings (product, root, sum, quotient) where
+// the first form has six; two of its three divisions leave the inner loop, which was bound by them.
+struct adam_step
+{
+    float b1, b2, s_hi, s_lo, e;
+    bool keeps_zero; // a parameter with no gradient and no moments keeps its value
+    __device__ adam_step(float lr, float b1_, float b2_, float eps, float t) : b1(b1_), b2(b2_)
     {
-        const float2 gi = reinterpret_cast<const float2 *>(g)[i2];
-        float2 mi = reinterpret_cast<const float2 *>(m)[i2], vi = reinterpret_cast<const float2 *>(v)[i2];
-        float2 pi = reinterpret_cast<const float2 *>(p)[i2];
-        mi.x = b1 * mi.x + (1.f - b1) * gi.x;
-        mi.y = b1 * mi.y + (1.f - b1) * gi.y;
-        vi.x = b2 * vi.x + (1.f - b2) * gi.x * gi.x;
-        vi.y = b2 * vi.y + (1.f - b2) * gi.y * gi.y;
-        pi.x = pi.x - lr * (mi.x / c1) / (sqrtf(vi.x / c2) + eps);
-        pi.y = pi.y - lr * (mi.y / c1) / (sqrtf(vi.y / c2) + eps);
-        reinterpret_cast<float2 *>(m)[i2] = mi;
-        reinterpret_cast<float2 *>(v)[i2] = vi;
-        reinterpret_cast<float2 *>(p)[i2] = pi;
-        reinterpret_cast<float2 *>(g)[i2] = make_float2(0.f, 0.f);
-        if(half_copy) half_copy[i2] = __floats2half2_rn(pi.x, pi.y);
+        const float c1 = 1.f - powf(b1, t), c2 = fabsf(1.f - powf(b2, t));
+        const float q = lr / c1, ql = fmaf(-q, c1, lr) / c1;
+        const float h = sqrtf(c2), hl = h > 0.f ? fmaf(-h, h, c2) / (2.f * h) : 0.f;
+        const float s = q * h, sl = fmaf(q, h, -s) + fmaf(q, hl, ql * h);
+        s_hi = s + sl;
+        s_lo = sl - (s_hi - s);
+        e = eps * h;
+        keeps_zero = e > 0.f && isfinite(s_hi);
+    }
+    __device__ __forceinline__ float operator()(float p, float g, float &m, float &v) const
+    {
+        m = b1 * m + (1.f - b1) * g;
+        v = b2 * v + (1.f - b2) * g * g;
+        return p - fmaf(s_hi, m, s_lo * m) / (sqrtf(fabsf(v)) + e);
+    }
+};
+
+// One optimiser step; gradients are consumed (zeroed). The first ADAM_W blocks take one MLP weight a
+// thread and write its packed copies; the others take pairs of grid parameters, so that the FP16 copy
+// (feature pairs) is written from values the thread owns. A pair with no gradient and no moments keeps
+// them and its parameters: nothing but the FP16 copy is written (a level whose cells do not fill its
+// table leaves most of it so). The last block to finish counts the step; a batch with no records takes
+// none, so a frame whose training paths all escaped leaves the parameters and the moments untouched.
+// Bound by memory: 16.8 million grid parameters in 74 us (34 bytes each where all are written, 570 MB; the dense
+// levels leave a quarter untouched); with the three divisions, a launch for the weights, one for the count and
+// three that packed the weights it was 132 us.
+constexpr uint32_t ADAM_THREADS = 256, ADAM_W = (NPARAM + ADAM_THREADS - 1) / ADAM_THREADS;
+__global__ void __launch_bounds__(ADAM_THREADS)
+        k_adam(adam_arrays grid, size_t n, adam_arrays w, float lr, float b1, float b2, float eps,
+               const uint32_t *__restrict__ d_n, uint32_t *__restrict__ state, __half2 *__restrict__ half_copy,
+               packed_weights pk)
+{
+    if(d_n && *d_n == 0) return;
+    const uint32_t step = state[0] + 1u;
+    const adam_step adam(lr, b1, b2, eps, (float)step);
+    if(blockIdx.x < ADAM_W)
+    {
+        const uint32_t i = blockIdx.x * ADAM_THREADS + threadIdx.x;
+        if(i < NPARAM)
+        {
+            float m = w.m[i], v = w.v[i];
+            const float p = adam(w.p[i], w.g[i], m, v);
+            w.m[i] = m;
+            w.v[i] = v;
+            w.p[i] = p;
+            w.g[i] = 0.f;
+            pack_weight((int)i, p, pk);
+        }
+    }
+    else
+    {
+        const size_t stride = (size_t)(gridDim.x - ADAM_W) * ADAM_THREADS;
+        for(size_t i2 = (size_t)(blockIdx.x - ADAM_W) * ADAM_THREADS + threadIdx.x; 2 * i2 < n; i2 += stride)
+        {
+            const float2 gi = reinterpret_cast<const float2 *>(grid.g)[i2];
+            float2 mi = reinterpret_cast<const float2 *>(grid.m)[i2], vi = reinterpret_cast<const float2 *>(grid.v)[i2];
+            float2 pi = reinterpret_cast<const float2 *>(grid.p)[i2];
+            const uint32_t any = __float_as_uint(gi.x) | __float_as_uint(gi.y) | __float_as_uint(mi.x) |
+                                 __float_as_uint(mi.y) | __float_as_uint(vi.x) | __float_as_uint(vi.y);
+            if(any || !adam.keeps_zero)
+            {
+                pi.x = adam(pi.x, gi.x, mi.x, vi.x);
+                pi.y = adam(pi.y, gi.y, mi.y, vi.y);
+                reinterpret_cast<float2 *>(grid.m)[i2] = mi;
+                reinterpret_cast<float2 *>(grid.v)[i2] = vi;
+                reinterpret_cast<float2 *>(grid.p)[i2] = pi;
+                reinterpret_cast<float2 *>(grid.g)[i2] = make_float2(0.f, 0.f);
+            }
+            half_copy[i2] = __floats2half2_rn(pi.x, pi.y);
+        }
+    }
+    __syncthreads(); // the block has read the step count
+    if(threadIdx.x == 0)
+    {
+        __threadfence();
+        if(atomicAdd(&state[1], 1u) == gridDim.x - 1)
+        {
+            state[0] = step;
+            state[1] = 0;
+        }
     }
 }
 
@@ -526,30 +620,6 @@ __global__ void k_to_half(const float *__restrict__ p, size_t n, __half2 *__rest
     {
         const float2 v = reinterpret_cast<const float2 *>(p)[i2];
         half_copy[i2] = __floats2half2_rn(v.x, v.y);
-    }
-}
-
-// pack the FP32 master weights into per-lane B fragments (forward) and transposed fragments (backward)
-__global__ void k_pack(const float *__restrict__ W, uint2 *__restrict__ frag, uint2 *__restrict__ fragT)
-{
-    const int e = blockIdx.x * blockDim.x + threadIdx.x;
-    if(e >= NFRAG) return;
-    int l = 0;
-    while(l + 1 < NLAYER && e >= frag_off(l + 1)) ++l;
-    const int K = layer_in(l), N = layer_out(l), lane = e & 31, g = lane >> 2, tig = lane & 3;
-    const float *w = W + layer_off(l);
-    {
-        const int idx = (e - frag_off(l)) >> 5;
-        const int kt = idx / (N / 8), j = idx % (N / 8);
-        const int n = 8 * j + g, k = 16 * kt + 2 * tig;
-        frag[e] = make_uint2(pack_bf16(w[k * N + n], w[(k + 1) * N + n]), pack_bf16(w[(k + 8) * N + n], w[(k + 9) * N + n]));
-    }
-    {
-        // transposed: B' = W^T (K' = N, N' = K)
-        const int idx = (e - fragT_off(l)) >> 5;
-        const int kt = idx / (K / 8), j = idx % (K / 8);
-        const int n = 8 * j + g, k = 16 * kt + 2 * tig; // n indexes W rows (inputs), k W columns (outputs)
-        fragT[e] = make_uint2(pack_bf16(w[n * N + k], w[n * N + k + 1]), pack_bf16(w[n * N + k + 8], w[n * N + k + 9]));
     }
 }
 
@@ -578,6 +648,11 @@ __global__ void k_init(float *__restrict__ grid, __half2 *__restrict__ grid_h, s
 }
 
 }// namespace
+
+static packed_weights packed(const vkg_nrc *c)
+{
+    return {reinterpret_cast<uint16_t *>(c->frag), reinterpret_cast<uint16_t *>(c->fragT), c->wtc, c->wtc_t};
+}
 
 vkg_status nrc_ensure(vkg_nrc *c, uint32_t n)
 {
@@ -665,13 +740,9 @@ vkg_status nrc_backward(vkg_nrc *c, const float *feats, const float *targets, ui
 // d_n: optional device-side record count of the batch; an empty batch takes no step
 vkg_status nrc_adam(vkg_nrc *c, const uint32_t *d_n, cudaStream_t st)
 {
-    const uint32_t blocks = (uint32_t)c->ctx->num_sms * 8;
-    k_adam_begin<<<1, 1, 0, st>>>(d_n, c->d_state);
-    k_adam<<<blocks, 256, 0, st>>>(c->grid, c->grid_g, c->grid_m, c->grid_v, c->ngrid, c->lr, c->b1, c->b2, c->eps,
-                                   c->d_state, c->grid_h);
-    k_adam<<<64, 256, 0, st>>>(c->w, c->w_g, c->w_m, c->w_v, NPARAM, c->lr, c->b1, c->b2, c->eps, c->d_state, nullptr);
-    k_pack<<<(NFRAG + 255) / 256, 256, 0, st>>>(c->w, c->frag, c->fragT);
-    if(vkg_status s = nrc_pack_tc(c->ctx, c->w, c->wtc, st, c->wtc_t); s != VKG_OK) return s;
+    const adam_arrays grid{c->grid, c->grid_g, c->grid_m, c->grid_v}, w{c->w, c->w_g, c->w_m, c->w_v};
+    k_adam<<<ADAM_W + (uint32_t)c->ctx->num_sms * 8, ADAM_THREADS, 0, st>>>(
+            grid, c->ngrid, w, c->lr, c->b1, c->b2, c->eps, d_n, c->d_state, c->grid_h, packed(c));
     return cuda_check(c->ctx, cudaGetLastError(), "nrc adam");
 }
 
@@ -813,12 +884,7 @@ vkg_status vkg_nrc_create(vkg_ctx *ctx, const vkg_nrc_config *cfg, vkg_nrc **out
         return cuda_check(ctx, e, "vkg_nrc_create");
     }
     k_init<<<ctx->num_sms * 8, 256>>>(c->grid, c->grid_h, c->ngrid, c->w, cfg->seed);
-    k_pack<<<(NFRAG + 255) / 256, 256>>>(c->w, c->frag, c->fragT);
-    if(vkg_status s = nrc_pack_tc(ctx, c->w, c->wtc, nullptr, c->wtc_t); s != VKG_OK)
-    {
-        vkg_nrc_destroy(c);
-        return s;
-    }
+    k_pack<<<(NPARAM + 255) / 256, 256>>>(c->w, packed(c));
     e = cudaDeviceSynchronize();
     if(e != cudaSuccess)
     {
@@ -923,8 +989,7 @@ vkg_status vkg_nrc_load_params(vkg_nrc *c, const float *d_mlp, const float *d_gr
         // refresh the FP16 copy the encoder reads
         k_to_half<<<c->ctx->num_sms * 8, 256, 0, st>>>(c->grid, c->ngrid, c->grid_h);
     }
-    k_pack<<<(NFRAG + 255) / 256, 256, 0, st>>>(c->w, c->frag, c->fragT);
-    if(vkg_status s = nrc_pack_tc(c->ctx, c->w, c->wtc, st, c->wtc_t); s != VKG_OK) return s;
+    k_pack<<<(NPARAM + 255) / 256, 256, 0, st>>>(c->w, packed(c));
     return cuda_check(c->ctx, cudaGetLastError(), "vkg_nrc_load_params");
 }
 
@@ -1069,8 +1134,7 @@ vkg_status vkg_nrc_load(vkg_nrc *c, const char *path, void *stream)
     VKG_TRY_CUDA(c->ctx, cudaMemcpyAsync(c->d_state, &h.step, sizeof(uint32_t), cudaMemcpyHostToDevice, st));
     // the operand copies the kernels read
     k_to_half<<<c->ctx->num_sms * 8, 256, 0, st>>>(c->grid, c->ngrid, c->grid_h);
-    k_pack<<<(NFRAG + 255) / 256, 256, 0, st>>>(c->w, c->frag, c->fragT);
-    if(vkg_status s = nrc_pack_tc(c->ctx, c->w, c->wtc, st, c->wtc_t); s != VKG_OK) return s;
+    k_pack<<<(NPARAM + 255) / 256, 256, 0, st>>>(c->w, packed(c));
     VKG_TRY_CUDA(c->ctx, cudaStreamSynchronize(st));
     return cuda_check(c->ctx, cudaGetLastError(), "vkg_nrc_load");
 }

@@ -36,33 +36,6 @@ namespace
 
 __device__ __forceinline__ uint32_t eff_n(uint32_t n, const uint32_t *d_n) { return d_n ? min(*d_n, n) : n; }
 
-// FP32 master weights ([in][out] row-major per layer) -> BF16 B operands: layer l as N x K, K-major
-__global__ void k_pack_tc(const float *__restrict__ W, uint16_t *__restrict__ wtc)
-{
-    const int e = blockIdx.x * blockDim.x + threadIdx.x;
-    if(e >= NPARAM) return;
-    int l = 0;
-    while(l + 1 < NLAYER && e >= layer_off(l + 1)) ++l;
-    const int K = layer_in(l), N = layer_out(l), local = e - layer_off(l);
-    const int k = local / N, n = local - k * N;
-    const __nv_bfloat16 b = __float2bfloat16_rn(W[e]);
-    wtc[(layer_off(l) * 2 + tc::canon_offset(n, k, K)) / 2] = *reinterpret_cast<const uint16_t *>(&b);
-}
-
-// FP32 master weights -> BF16 operands of the backward: layer l as K_l x N_l (rows = the layer's
-// inputs, K = its outputs), K-major, so that D (128 x K_l) = G_l (128 x N_l) W_l^T is one UMMA chain
-__global__ void k_pack_tc_t(const float *__restrict__ W, uint16_t *__restrict__ wtc_t)
-{
-    const int e = blockIdx.x * blockDim.x + threadIdx.x;
-    if(e >= NPARAM) return;
-    int l = 0;
-    while(l + 1 < NLAYER && e >= layer_off(l + 1)) ++l;
-    const int N = layer_out(l), local = e - layer_off(l);
-    const int k = local / N, n = local - k * N;
-    const __nv_bfloat16 b = __float2bfloat16_rn(W[e]);
-    wtc_t[(layer_off(l) * 2 + tc::canon_offset(k, n, N)) / 2] = *reinterpret_cast<const uint16_t *>(&b);
-}
-
 // FUSED: encode the feature records here; else read the encoded inputs X (n x 40 u32) written by k_encode
 template<bool FUSED>
 __global__ void __launch_bounds__(TC_INFER_THREADS)
@@ -429,7 +402,7 @@ __global__ void __launch_bounds__(NWG * 128)
 //   262,144 records: 47 us with operands in shared memory and eight warpgroups, 31 us (343 MB) this way;
 //   dX (the 32 hash-grid features) = G_0 W_0^T (N = 32) -> dXg in FP32.
 // Quantisation points equal k_backward's (FP32 sums, mask in FP32, BF16 rounding of each G); only
-// the summation order inside an MMA differs. Weights: wtc_t (k_pack_tc_t), resident in shared memory.
+// the summation order inside an MMA differs. Weights: wtc_t (pack_weight), resident in shared memory.
 constexpr uint32_t TC_G_BYTES = TC_TILE * OUTP * 2; // the backward's first A operand (4,096 B)
 template<int NWG>
 __global__ void __launch_bounds__(NWG * 128)
@@ -770,13 +743,6 @@ vkg_status nrc_wgrad_tc(vkg_ctx *ctx, const uint32_t *X, const uint32_t *H, cons
     const uint32_t grid = std::min<uint32_t>(chunks, (uint32_t)ctx->num_sms);
     k_wgrad_tc<<<grid, WG_TC_THREADS, WG_TC_SMEM, st>>>(X, H, G, n, d_n, dW, err);
     return cuda_check(ctx, cudaGetLastError(), "k_wgrad_tc");
-}
-
-vkg_status nrc_pack_tc(vkg_ctx *ctx, const float *W, uint16_t *wtc, cudaStream_t st, uint16_t *wtc_t)
-{
-    k_pack_tc<<<(NPARAM + 255) / 256, 256, 0, st>>>(W, wtc);
-    if(wtc_t) k_pack_tc_t<<<(NPARAM + 255) / 256, 256, 0, st>>>(W, wtc_t);
-    return cuda_check(ctx, cudaGetLastError(), "k_pack_tc");
 }
 
 // the pipelined MLP over encoded inputs X: inference (H null) or the training forward (H receives the
