@@ -146,3 +146,30 @@ def test_adam_steps(ctx, steps, levels, kernel):
     other = NeuralRadianceCache(ctx, cfg)
     other.load_params(*got)
     assert torch.equal(cache.infer(feats), other.infer(feats))
+
+
+@pytest.mark.parametrize("n", [127, 128, 129, 128 * 152 + 1, 128 * 304 + 1, 45_000, 70_001])
+def test_training_tiles_match_mma(ctx, n):
+    """the fused tcgen05 training pass, whose intermediates are stored by tiles, against the mma.sync kernels, which
+    store them by records: tiles and warpgroups at their edges. Both round every activation and layer
+    gradient to BF16 (2^-8) from FP32 sums of another order; the bounds are those of the full-size comparison"""
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    feats = random_features(n, n)
+    targets = torch.rand((n, 3), device="cuda", generator=gen)
+    got = {}
+    for kernel in (2, 3):
+        cfg = NeuralRadianceCache.default_config()
+        cfg.log2_table_size, cfg.train_kernel = 12, kernel
+        cache = NeuralRadianceCache(ctx, cfg)
+        i = cache.info()
+        gen.manual_seed(5)
+        cache.load_params(torch.randn(i.num_mlp_params, device="cuda", generator=gen) * 0.2,
+                          torch.randn(i.num_grid_params, device="cuda", generator=gen) * 0.5)
+        cache.backward(feats, targets)
+        i = cache.info()
+        assert i.kernel_error == 0 and i.train_kernel == kernel
+        got[kernel] = _read(i.d_mlp_grads, i.num_mlp_params), _read(i.d_grid_grads, i.num_grid_params)
+        cache.close()
+    for a, b in zip(got[2], got[3]):
+        assert float((a * b).sum() / (a.norm() * b.norm())) > 0.9999
+    assert (got[2][0] - got[3][0]).abs().max().item() <= 2e-2 * got[2][0].abs().max().item()

@@ -449,11 +449,13 @@ __global__ void __launch_bounds__(WG_THREADS)
 // one four-wide atomic, 6 per level on average.
 __global__ void __launch_bounds__(256)
         k_grid_backward(const float *__restrict__ feats, uint32_t n, const uint32_t *__restrict__ d_n, grid_config gc,
-                        const float *__restrict__ dXg, float *__restrict__ grid_g)
+                        const float *__restrict__ dXg, bool tiled, float *__restrict__ grid_g)
 {
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x, i = t >> 4, l = t & 15u;
     if(i >= eff_count(n, d_n) || l >= gc.levels) return;
-    const float2 g = *reinterpret_cast<const float2 *>(dXg + (size_t)i * 32 + 2 * l);
+    // dXg by records, or by tiles as the tcgen05 backward stores it
+    const size_t group = tiled ? tiled_group(i, 8, l >> 1) : (size_t)i * 8 + (l >> 1);
+    const float2 g = *reinterpret_cast<const float2 *>(dXg + 4 * group + 2 * (l & 1u));
     if(g.x == 0.f && g.y == 0.f) return;
     float px, py, pz;
     normalised_pos(gc, feats + (size_t)FEAT * i, px, py, pz);
@@ -669,11 +671,12 @@ vkg_status nrc_ensure(vkg_nrc *c, uint32_t n)
     auto al = [&](void **p, size_t b) {
         if(e == cudaSuccess) e = cudaMalloc(p, b);
     };
+    const size_t whole = ((size_t)n + 127) / 128 * 128; // H, G and dXg may be stored by tiles of 128 records
     al((void **)&c->X, (size_t)n * 40 * 4);
-    al((void **)&c->H, (size_t)n * 160 * 4);
-    al((void **)&c->G, (size_t)n * 168 * 4);
+    al((void **)&c->H, whole * 160 * 4);
+    al((void **)&c->G, whole * 168 * 4);
     al((void **)&c->Y, (size_t)n * 3 * 4);
-    al((void **)&c->dXg, (size_t)n * 32 * 4);
+    al((void **)&c->dXg, whole * 32 * 4);
     if(e != cudaSuccess) return cuda_check(c->ctx, e, "nrc buffers");
     c->cap = n;
     return VKG_OK;
@@ -706,34 +709,31 @@ vkg_status nrc_backward(vkg_nrc *c, const float *feats, const float *targets, ui
     if(n == 0) return VKG_OK;
     if(vkg_status s = nrc_ensure(c, n); s != VKG_OK) return s;
     if(vkg_status s = nrc_encode(c, feats, n, d_n, c->X, st); s != VKG_OK) return s;
-    const uint32_t tiles = (n + 15) / 16, per_cta = MLP_THREADS / 32;
-    const uint32_t grid = std::min<uint32_t>((tiles + per_cta - 1) / per_cta, (uint32_t)c->ctx->num_sms * 8);
     // the training forward and backward: on tcgen05 (train_kernel 3), else the mma.sync twins
     if(c->tc_forward)
     {
-        if(vkg_status s = nrc_forward_tc(c->ctx, c->wtc, c->X, n, d_n, c->Y, c->H, c->d_err, st); s != VKG_OK) return s;
-    }
-    else
-        k_forward<true><<<grid, MLP_THREADS, 0, st>>>(c->X, n, d_n, c->frag, c->Y, c->H);
-    if(c->tc_forward)
-    {
-        if(vkg_status s = nrc_backward_tc(c->ctx, c->wtc_t, c->H, c->Y, targets, n, d_n, c->G, c->dXg, c->loss,
-                                          c->d_err, st);
+        if(vkg_status s = nrc_train_tc(c->ctx, c->wtc, c->wtc_t, c->X, targets, n, d_n, c->H, c->G, c->dXg, c->loss,
+                                       c->d_err, st);
            s != VKG_OK)
             return s;
     }
     else
+    {
+        const uint32_t tiles = (n + 15) / 16, per_cta = MLP_THREADS / 32;
+        const uint32_t grid = std::min<uint32_t>((tiles + per_cta - 1) / per_cta, (uint32_t)c->ctx->num_sms * 8);
+        k_forward<true><<<grid, MLP_THREADS, 0, st>>>(c->X, n, d_n, c->frag, c->Y, c->H);
         k_backward<<<grid, MLP_THREADS, 0, st>>>(c->H, c->Y, targets, n, d_n, c->fragT, c->G, c->dXg, c->loss);
+    }
     if(c->tc_train)
     {
-        if(vkg_status s = nrc_wgrad_tc(c->ctx, c->X, c->H, c->G, n, d_n, c->w_g, c->d_err, st); s != VKG_OK) return s;
+        if(vkg_status s = nrc_wgrad_tc(c->ctx, c->X, c->H, c->G, n, d_n, c->tc_forward, c->w_g, c->d_err, st); s != VKG_OK) return s;
     }
     else
     {
         const uint32_t wg = std::min<uint32_t>((n + WG_CHUNK - 1) / WG_CHUNK, (uint32_t)c->ctx->num_sms * 2);
         k_wgrad<<<wg, WG_THREADS, 0, st>>>(c->X, c->H, c->G, n, d_n, c->w_g);
     }
-    k_grid_backward<<<(n + 15) / 16, 256, 0, st>>>(feats, n, d_n, c->gc, c->dXg, c->grid_g);
+    k_grid_backward<<<(n + 15) / 16, 256, 0, st>>>(feats, n, d_n, c->gc, c->dXg, c->tc_forward, c->grid_g);
     return cuda_check(c->ctx, cudaGetLastError(), "nrc backward");
 }
 

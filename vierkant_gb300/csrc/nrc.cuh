@@ -83,20 +83,26 @@ constexpr size_t ENCODED_BYTES = IN * 2;
 // predictions (n x 3 fp32) for n feature records (n x FEAT fp32); X is caller-owned scratch of n x ENCODED_BYTES
 vkg_status nrc_predict(vkg_nrc *c, const float *feats, uint32_t n, const uint32_t *d_n, uint32_t *X, float *Y,
                        cudaStream_t st);
+// 16-byte group p of a record's `groups`, in an array stored by tiles of 128 records: a tile's records side by side
+__host__ __device__ constexpr size_t tiled_group(size_t record, uint32_t groups, uint32_t p)
+{
+    return ((record >> 7) * groups + p) * 128 + (record & 127u);
+}
 // tcgen05 inference (nrc_tc.cu): BF16 B operands of all layers (NPARAM x 2 bytes, canonical K-major)
-vkg_status nrc_backward_tc(vkg_ctx *ctx, const uint16_t *wtc_t, const uint32_t *H, const float *Y, const float *T,
-                           uint32_t n, const uint32_t *d_n, uint32_t *G, float *dXg, float *loss, uint32_t *err,
-                           cudaStream_t st);
 // MLP on tcgen05 over the encoded inputs X (n x 40 u32), or, with X == nullptr, encoding + MLP fused;
 // err receives 1 if a tensor-core wait ran out
 vkg_status nrc_infer_tc(vkg_ctx *ctx, const grid_config &gc, const __half2 *grid, const uint16_t *wtc,
                         const float *feats, const uint32_t *X, uint32_t n, const uint32_t *d_n, float *Y, uint32_t *err,
                         cudaStream_t st);
-// weight gradients of n records on tcgen05 (accumulated into dW); err receives 1 if a wait ran out
-vkg_status nrc_forward_tc(vkg_ctx *ctx, const uint16_t *wtc, const uint32_t *X, uint32_t n, const uint32_t *d_n,
-                          float *Y, uint32_t *H, uint32_t *err, cudaStream_t st);
+// training forward and backward of n encoded records on tcgen05: activations H, gradients G and dXg by tiles of
+// 128 records (capacity: n rounded up to 128), the loss added to *loss; err receives 1 if a wait ran out
+vkg_status nrc_train_tc(vkg_ctx *ctx, const uint16_t *wtc, const uint16_t *wtc_t, const uint32_t *X, const float *T,
+                        uint32_t n, const uint32_t *d_n, uint32_t *H, uint32_t *G, float *dXg, float *loss,
+                        uint32_t *err, cudaStream_t st);
+// weight gradients of n records on tcgen05 (accumulated into dW), H and G by tiles or by records; err receives 1 if a
+// wait ran out
 vkg_status nrc_wgrad_tc(vkg_ctx *ctx, const uint32_t *X, const uint32_t *H, const uint32_t *G, uint32_t n,
-                        const uint32_t *d_n, float *dW, uint32_t *err, cudaStream_t st);
+                        const uint32_t *d_n, bool tiled, float *dW, uint32_t *err, cudaStream_t st);
 // one optimiser step (backward + Adam) on n records; records past *d_n contribute nothing
 vkg_status nrc_train(vkg_nrc *c, const float *feats, const float *targets, uint32_t n, const uint32_t *d_n,
                      cudaStream_t st);

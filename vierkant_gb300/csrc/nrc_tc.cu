@@ -249,10 +249,7 @@ __global__ void __launch_bounds__(TC_THREADS)
 // by cp.async while the tile before runs its later layers. The hidden layers read their operand from
 // TMEM: the epilogue (64 columns in, ReLU, BF16) stores 32 columns back with tcgen05.st, which takes the
 // 16 KB a layer and tile of shared-memory stores and reads out of the way. 2,073,600 queries: 222 us
-// with operands in shared memory and eight warpgroups, 183 us with four this way; as the training forward of
-// 262,144 records 32 -> 26 us (it stores 168 MB).
-// TRAIN: also store the hidden activations H1..H5 (BF16, 5 x 64 per record in natural column order,
-// the layout the backward reads) as the training forward.
+// with operands in shared memory and eight warpgroups, 183 us with four this way.
 // TMEM columns a CTA of g warpgroups allocates when each uses `per`: a power of two of at least 32
 __host__ __device__ constexpr uint32_t tmem_columns(uint32_t per, uint32_t g)
 {
@@ -262,11 +259,10 @@ __host__ __device__ constexpr uint32_t tmem_columns(uint32_t per, uint32_t g)
 }
 constexpr uint32_t TC_WG_COLS = 96; // per warpgroup: 64 of the accumulator, 32 of the next layer's operand
 
-template<int NWG, bool TRAIN>
+template<int NWG>
 __global__ void __launch_bounds__(NWG * 128)
         k_infer_tc_wg(const uint32_t *__restrict__ X, uint32_t n_cap, const uint32_t *__restrict__ d_n,
-                      const uint16_t *__restrict__ wtc, float *__restrict__ Y, uint32_t *__restrict__ err,
-                      uint32_t *__restrict__ H)
+                      const uint16_t *__restrict__ wtc, float *__restrict__ Y, uint32_t *__restrict__ err)
 {
     extern __shared__ __align__(1024) uint8_t smem[];
     __shared__ uint64_t mbar[NWG];
@@ -355,12 +351,6 @@ __global__ void __launch_bounds__(NWG * 128)
                     for(int j = 0; j < 16; ++j)
                         hv[j] = pack_bf16(fmaxf(v[j >> 3][2 * (j & 7)], 0.f), fmaxf(v[j >> 3][2 * (j & 7) + 1], 0.f));
                     tc::tmem_st16(ta + lane_base + 16u * c2, hv);
-                    if(TRAIN && q < n)
-                    {
-                        uint4 *hp = reinterpret_cast<uint4 *>(H + (size_t)q * (5 * HID / 2) + l * (HID / 2) + 16 * c2);
-#pragma unroll
-                        for(int j = 0; j < 4; ++j) hp[j] = make_uint4(hv[4 * j], hv[4 * j + 1], hv[4 * j + 2], hv[4 * j + 3]);
-                    }
                 }
                 tc::tmem_st_wait();
             }
@@ -392,111 +382,196 @@ __global__ void __launch_bounds__(NWG * 128)
     if(warp == 0) tc::tmem_dealloc(tslot, COLS);
 }
 
-// ---- backward through the layers on tcgen05 ------------------------------------------------------
-// The mma.sync k_backward restated on the tensor cores with the warpgroup pipeline of k_infer_tc_wg:
-// per tile of 128 records, thread r owns record q = 128 tile + r:
+// ---- training forward and backward on tcgen05 ---------------------------------------------------
+// The mma.sync k_forward<true> and k_backward as one pass over the tiles, with the warpgroup pipeline of
+// k_infer_tc_wg: per tile of 128 records, thread r owns record q = 128 tile + r:
+//   forward as in k_infer_tc_wg; H_1..H_5 go to memory for the weight gradients, and one bit an
+//   activation, H > 0, stays in registers;
 //   dy = dL/dy of the relative L2 loss (|y - t|^2 / (y^2 + 0.01), mean over 3n) -> G block 5 and the
-//   BF16 A operand (128 x 16);
+//   BF16 A operand (128 x 16, shared memory);
 //   for l = 5 .. 1: D = G_l W_l^T (UMMA, TMEM), G_{l-1} = D * [H_l > 0] rounded to BF16 -> G block
-//   l - 1 and the next A operand (128 x 64), in TMEM as in the forward; H_l is fetched during the MMAs;
-//   262,144 records: 47 us with operands in shared memory and eight warpgroups, 31 us (343 MB) this way;
+//   l - 1 and the next A operand (128 x 64), in TMEM as in the forward;
 //   dX (the 32 hash-grid features) = G_0 W_0^T (N = 32) -> dXg in FP32.
-// Quantisation points equal k_backward's (FP32 sums, mask in FP32, BF16 rounding of each G); only
-// the summation order inside an MMA differs. Weights: wtc_t (pack_weight), resident in shared memory.
+// Quantisation points equal the mma.sync kernels' (FP32 sums, BF16 rounding of each H and G); only the
+// summation order inside an MMA differs. Both weight layouts (wtc, and wtc_t transposed) are resident.
+// H, G and dXg are stored by tiles: 16-byte group p of a record's P groups at group (tile P + p) 128 + r,
+// so that a warp's stores are whole lines (by records each 16-byte store touched 32).
+// Bound by the chain of twelve layers and its stores (1.4 KB a record, to L2): 65,536 records in 25 us; as two
+// kernels with the records' rows, the activations read back, 56 us.
 constexpr uint32_t TC_G_BYTES = TC_TILE * OUTP * 2; // the backward's first A operand (4,096 B)
 template<int NWG>
 __global__ void __launch_bounds__(NWG * 128)
-        k_backward_tc_wg(const uint32_t *__restrict__ H, const float *__restrict__ Y, const float *__restrict__ T,
-                         uint32_t n_cap, const uint32_t *__restrict__ d_n, const uint16_t *__restrict__ wtc_t,
-                         uint32_t *__restrict__ G, float *__restrict__ dXg, float *__restrict__ loss_sum,
-                         uint32_t *__restrict__ err)
+        k_train_tc_wg(const uint32_t *__restrict__ X, const float *__restrict__ T, uint32_t n_cap,
+                      const uint32_t *__restrict__ d_n, const uint16_t *__restrict__ wtc,
+                      const uint16_t *__restrict__ wtc_t, uint4 *__restrict__ H, uint4 *__restrict__ G,
+                      float4 *__restrict__ dXg, float *__restrict__ loss_sum, uint32_t *__restrict__ err)
 {
     extern __shared__ __align__(1024) uint8_t smem[];
     __shared__ uint64_t mbar[NWG];
     __shared__ uint32_t tslot;
     const uint32_t tid = threadIdx.x, warp = tid >> 5, g = tid >> 7, r = tid & 127u;
-    uint8_t *sw = smem, *sa = smem + TC_W_BYTES + g * TC_G_BYTES;
+    uint8_t *sg = smem + 2 * TC_W_BYTES + NWG * TC_A_BYTES + g * TC_G_BYTES;
+    const uint32_t sw_addr = tc::smem_addr(smem), sa_addr = sw_addr + 2 * TC_W_BYTES + g * TC_A_BYTES;
+    const uint32_t sg_addr = tc::smem_addr(sg);
+    const uint32_t n = eff_n(n_cap, d_n), tiles = (n + TC_TILE - 1) / TC_TILE;
+    // this thread's row of a tile's layer-0 operand (zeros past n)
+    auto load = [&](uint32_t tile) {
+        const uint32_t q = tile * TC_TILE + r;
+        const uint32_t *src = X + (size_t)(IN / 2) * (q < n ? q : 0u);
+#pragma unroll
+        for(int j = 0; j < IN / 8; ++j)
+            tc::cp_async16(sa_addr + tc::canon_offset(r, 8 * j, IN), src + 4 * j, q < n);
+    };
+    const uint32_t first = blockIdx.x * NWG + g;
+    if(first < tiles) load(first);
     for(uint32_t i = tid; i < TC_W_BYTES / 16; i += NWG * 128)
-        tc::cp_async16(tc::smem_addr(sw) + 16u * i, reinterpret_cast<const uint4 *>(wtc_t) + i, true);
-    tc::cp_async_commit();
+    {
+        tc::cp_async16(sw_addr + 16u * i, reinterpret_cast<const uint4 *>(wtc) + i, true);
+        tc::cp_async16(sw_addr + TC_W_BYTES + 16u * i, reinterpret_cast<const uint4 *>(wtc_t) + i, true);
+    }
     static_assert(NWG >= 1 && NWG * TC_WG_COLS <= 512, "at most 512 TMEM columns");
     constexpr uint32_t COLS = tmem_columns(TC_WG_COLS, NWG);
     if(warp == 0) tc::tmem_alloc(&tslot, COLS);
     if(tid < NWG) tc::mbar_init(&mbar[tid], 1);
+    tc::cp_async_commit();
     tc::cp_async_wait<0>();
     tc::fence_async_smem();
     tc::fence_before_sync();
     __syncthreads();
     tc::fence_after_sync();
     const uint32_t tmem = tslot + TC_WG_COLS * g, ta = tmem + 64u, lane_base = ((warp & 3u) * 32u) << 16;
-    const uint32_t sw_addr = tc::smem_addr(sw), sa_addr = tc::smem_addr(sa);
-    const uint32_t n = eff_n(n_cap, d_n), tiles = (n + TC_TILE - 1) / TC_TILE;
     const float inv_count = n ? 1.f / (3.f * (float)n) : 0.f;
     const uint32_t bar_id = g + 1;
     uint32_t phase = 0;
     bool failed = false;
     float loss = 0.f;
 
-    for(uint32_t tile = blockIdx.x * NWG + g; tile < tiles && !failed; tile += gridDim.x * NWG)
+    // D (128 x rows) = A (128 x K) * B^T, the A operand in shared memory (at a, else 0) or TMEM; false if the
+    // wait ran out
+    auto multiply = [&](uint32_t a, uint32_t b, uint32_t K, uint32_t rows) {
+        if(r == 0)
+        {
+            tc::fence_after_sync();
+            const uint32_t idesc = tc::idesc_bf16(TC_TILE, rows);
+            for(uint32_t s = 0; s < K / 16; ++s)
+            {
+                const uint64_t bd = tc::smem_desc(b + 256u * s, 128u, K * 16u);
+                if(a) tc::mma_bf16(tmem, tc::smem_desc(a + 256u * s, 128u, K * 16u), bd, idesc, s > 0);
+                else tc::mma_bf16_ts(tmem, ta + 8u * s, bd, idesc, s > 0);
+            }
+            tc::mma_commit(&mbar[g]);
+        }
+        const bool ok = tc::mbar_wait(&mbar[g], phase);
+        if(tc::wg_sync_or(bar_id, !ok)) return false;
+        phase ^= 1u;
+        tc::fence_after_sync();
+        return true;
+    };
+
+    for(uint32_t tile = first; tile < tiles && !failed; tile += gridDim.x * NWG)
     {
         const uint32_t q = tile * TC_TILE + r;
         const bool valid = q < n;
+        float t[3] = {0.f, 0.f, 0.f}, y[3] = {0.f, 0.f, 0.f};
+        if(valid)
+            for(int c = 0; c < 3; ++c) t[c] = T[(size_t)q * 3 + c];
+        uint4 *hp = H + tiled_group(q, ACT / 8, 0), *gp = G + tiled_group(q, GRAD / 8, 0);
+        // H_l > 0 of the last layers first: bits j and 16 + j of word c are columns 32 c + 2 j and 32 c + 2 j + 1
+        uint32_t pos[NLAYER - 1][2];
+        // the tile's rows were loaded during the tile before
+        tc::cp_async_wait<0>();
+        tc::fence_async_smem();
+        tc::fence_before_sync();
+        tc::wg_sync(bar_id);
+#pragma unroll 1
+        for(int l = 0; l < NLAYER; ++l)
+        {
+            if(!multiply(l == 0 ? sa_addr : 0u, sw_addr + (uint32_t)layer_off(l) * 2u, layer_in(l), layer_out(l)))
+            {
+                failed = true;
+                break;
+            }
+            if(l == 0 && tile + gridDim.x * NWG < tiles)
+            {
+                load(tile + gridDim.x * NWG); // layer 0 is done with the operand
+                tc::cp_async_commit();
+            }
+            if(l + 1 < NLAYER)
+            {
+#pragma unroll
+                for(int i = NLAYER - 2; i > 0; --i)
+                {
+                    pos[i][0] = pos[i - 1][0];
+                    pos[i][1] = pos[i - 1][1];
+                }
+#pragma unroll
+                for(int c = 0; c < 2; ++c)
+                {
+                    // two TMEM loads in flight per wait
+                    float v[2][16];
+                    tc::tmem_ld16(tmem + lane_base + 32u * c, v[0]);
+                    tc::tmem_ld16(tmem + lane_base + 32u * c + 16u, v[1]);
+                    tc::tmem_ld_wait();
+                    uint32_t hv[16], bits = 0;
+#pragma unroll
+                    for(int j = 0; j < 16; ++j)
+                    {
+                        hv[j] = pack_bf16(fmaxf(v[j >> 3][2 * (j & 7)], 0.f), fmaxf(v[j >> 3][2 * (j & 7) + 1], 0.f));
+                        // the sum carries into a half's top bit unless its value is zero
+                        bits = (bits >> 1) | (((hv[j] & 0x7FFF7FFFu) + 0x7FFF7FFFu) & 0x80008000u);
+                    }
+                    pos[0][c] = bits;
+                    tc::tmem_st16(ta + lane_base + 16u * c, hv);
+                    if(valid)
+#pragma unroll
+                        for(int j = 0; j < 4; ++j)
+                            hp[(8 * l + 4 * c + j) * TC_TILE] = make_uint4(hv[4 * j], hv[4 * j + 1], hv[4 * j + 2], hv[4 * j + 3]);
+                }
+                tc::tmem_st_wait();
+                tc::fence_before_sync();
+                tc::wg_sync(bar_id);
+            }
+            else
+            {
+                float v[16];
+                tc::tmem_ld16(tmem + lane_base, v);
+                tc::tmem_ld_wait();
+                for(int c = 0; c < 3; ++c) y[c] = v[c];
+            }
+        }
+        if(failed) break;
         // dL/dy (raw columns 0..2 of 16)
         float dy[3] = {0.f, 0.f, 0.f};
         if(valid)
             for(int c = 0; c < 3; ++c)
             {
-                const float y = Y[(size_t)q * 3 + c], t = T[(size_t)q * 3 + c];
-                const float den = y * y + 0.01f;
-                const float e = y - t;
+                const float den = y[c] * y[c] + 0.01f;
+                const float e = y[c] - t[c];
                 loss += e * e / den;
                 dy[c] = 2.f * e / den * inv_count;
             }
-        const uint32_t gy0 = pack_bf16(dy[0], dy[1]), gy1 = pack_bf16(dy[2], 0.f);
+        const uint4 gy = make_uint4(pack_bf16(dy[0], dy[1]), pack_bf16(dy[2], 0.f), 0u, 0u), zero = make_uint4(0u, 0u, 0u, 0u);
         if(valid)
         {
-            uint4 *gp = reinterpret_cast<uint4 *>(G + (size_t)q * 168 + 160);
-            gp[0] = make_uint4(gy0, gy1, 0u, 0u);
-            gp[1] = make_uint4(0u, 0u, 0u, 0u);
+            gp[8 * (NLAYER - 1) * TC_TILE] = gy;
+            gp[(8 * (NLAYER - 1) + 1) * TC_TILE] = zero;
         }
         // A operand 128 x 16 (K = 16): columns 0..7 and 8..15
-        *reinterpret_cast<uint4 *>(sa + tc::canon_offset(r, 0, 16)) = make_uint4(gy0, gy1, 0u, 0u);
-        *reinterpret_cast<uint4 *>(sa + tc::canon_offset(r, 8, 16)) = make_uint4(0u, 0u, 0u, 0u);
+        *reinterpret_cast<uint4 *>(sg + tc::canon_offset(r, 0, 16)) = gy;
+        *reinterpret_cast<uint4 *>(sg + tc::canon_offset(r, 8, 16)) = zero;
         tc::fence_async_smem();
         tc::fence_before_sync();
         tc::wg_sync(bar_id);
 #pragma unroll 1
         for(int l = NLAYER - 1; l >= 0; --l)
         {
-            // D (128 x rows) = A (128 x K') * B^T with B = W_l as rows = inputs, K' = outputs
-            const uint32_t Kp = layer_out(l), rows = l == 0 ? 32u : (uint32_t)layer_in(l);
-            if(r == 0)
-            {
-                tc::fence_after_sync();
-                const uint32_t idesc = tc::idesc_bf16(TC_TILE, rows);
-                const uint32_t wb = sw_addr + (uint32_t)layer_off(l) * 2u;
-                for(uint32_t s = 0; s < Kp / 16; ++s)
-                {
-                    const uint64_t b = tc::smem_desc(wb + 256u * s, 128u, Kp * 16u);
-                    if(l == NLAYER - 1) tc::mma_bf16(tmem, tc::smem_desc(sa_addr + 256u * s, 128u, Kp * 16u), b, idesc, s > 0);
-                    else tc::mma_bf16_ts(tmem, ta + 8u * s, b, idesc, s > 0);
-                }
-                tc::mma_commit(&mbar[g]);
-            }
-            // H_l (block l - 1 of H), on its way while the MMAs run
-            uint4 h[8];
-#pragma unroll
-            for(int j = 0; j < 8; ++j)
-                h[j] = valid && l > 0 ? __ldg(reinterpret_cast<const uint4 *>(H + (size_t)q * 160 + (l - 1) * 32) + j)
-                                      : make_uint4(0u, 0u, 0u, 0u);
-            const bool ok = tc::mbar_wait(&mbar[g], phase);
-            if(tc::wg_sync_or(bar_id, !ok))
+            // B = W_l as rows = inputs, K = outputs
+            if(!multiply(l == NLAYER - 1 ? sg_addr : 0u, sw_addr + TC_W_BYTES + (uint32_t)layer_off(l) * 2u, layer_out(l),
+                         l == 0 ? 32u : (uint32_t)layer_in(l)))
             {
                 failed = true;
                 break;
             }
-            phase ^= 1u;
-            tc::fence_after_sync();
             if(l > 0)
             {
                 // G_{l-1} = dH_l * [H_l > 0]
@@ -510,25 +585,26 @@ __global__ void __launch_bounds__(NWG * 128)
                     uint32_t gv[16];
 #pragma unroll
                     for(int j = 0; j < 16; ++j)
-                    {
-                        const uint4 &hq = h[4 * c + (j >> 2)];
-                        const uint32_t hw = (j & 3) == 0 ? hq.x : (j & 3) == 1 ? hq.y : (j & 3) == 2 ? hq.z : hq.w;
-                        const float m0 = (hw & 0x7FFFu) ? 1.f : 0.f, m1 = ((hw >> 16) & 0x7FFFu) ? 1.f : 0.f;
-                        gv[j] = pack_bf16(v[j >> 3][2 * (j & 7)] * m0, v[j >> 3][2 * (j & 7) + 1] * m1);
-                    }
+                        gv[j] = pack_bf16(v[j >> 3][2 * (j & 7)], v[j >> 3][2 * (j & 7) + 1]) &
+                                (((pos[0][c] >> j) & 0x00010001u) * 0xFFFFu);
                     tc::tmem_st16(ta + lane_base + 16u * c, gv);
                     if(valid)
-                    {
-                        uint4 *gp = reinterpret_cast<uint4 *>(G + (size_t)q * 168 + (l - 1) * 32 + 16 * c);
 #pragma unroll
-                        for(int j = 0; j < 4; ++j) gp[j] = make_uint4(gv[4 * j], gv[4 * j + 1], gv[4 * j + 2], gv[4 * j + 3]);
-                    }
+                        for(int j = 0; j < 4; ++j)
+                            gp[(8 * (l - 1) + 4 * c + j) * TC_TILE] = make_uint4(gv[4 * j], gv[4 * j + 1], gv[4 * j + 2], gv[4 * j + 3]);
+                }
+#pragma unroll
+                for(int i = 0; i < NLAYER - 2; ++i)
+                {
+                    pos[i][0] = pos[i + 1][0];
+                    pos[i][1] = pos[i + 1][1];
                 }
                 tc::tmem_st_wait();
             }
             else
             {
                 // dX of the 32 hash-grid features, FP32
+                float4 *dp = dXg + tiled_group(q, 8, 0);
 #pragma unroll
                 for(int c = 0; c < 2; ++c)
                 {
@@ -536,23 +612,22 @@ __global__ void __launch_bounds__(NWG * 128)
                     tc::tmem_ld16(tmem + lane_base + 16u * c, v);
                     tc::tmem_ld_wait();
                     if(valid)
-                    {
-                        float4 *dp = reinterpret_cast<float4 *>(dXg + (size_t)q * 32 + 16 * c);
 #pragma unroll
-                        for(int j = 0; j < 4; ++j) dp[j] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
-                    }
+                        for(int j = 0; j < 4; ++j)
+                            dp[(4 * c + j) * TC_TILE] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
                 }
             }
             tc::fence_before_sync();
             tc::wg_sync(bar_id);
         }
     }
+    tc::cp_async_wait<0>();
     for(int o = 16; o > 0; o >>= 1) loss += __shfl_down_sync(0xffffffffu, loss, o);
     if((tid & 31u) == 0 && loss_sum) atomicAdd(loss_sum, loss * inv_count);
     if(failed)
     {
         if(r == 0) atomicOr(err, TC_TIMEOUT);
-        tc::mbar_wait(&mbar[g], phase);
+        tc::mbar_wait(&mbar[g], phase); // this warpgroup's MMAs in flight, if any
     }
     tc::fence_before_sync();
     __syncthreads();
@@ -603,8 +678,8 @@ __global__ void __launch_bounds__(TC_THREADS)
 // still reads 128 rows: rows past its inputs are the following groups' data, and the accumulator
 // lanes that they give are never read. The six accumulators (336 TMEM columns) stay resident while
 // the CTA walks its chunks.
-// Bound by the loads (1.47 KB a record from L2). 65,536 records took 121 us when each record's features
-// were scattered into K-major operands with 2-byte shared-memory stores.
+// Bound by the loads (1.47 KB a record from L2): 65,536 records in 29 us; 39 us with H and G by records, 121 us
+// when each record's features were scattered into K-major operands with 2-byte shared-memory stores.
 constexpr uint32_t WG_TC_THREADS = 256, WG_TC_CHUNK = 64, WG_TC_TMEM = 512;
 constexpr uint32_t WG_X = IN / 8, WG_H = ACT / 8, WG_G = GRAD / 8; // 16-byte groups of a record: 10, 40, 42
 // a group's records, and 16 bytes that spread the groups of a record over the banks
@@ -614,18 +689,21 @@ static_assert(WG_X + 8 * 4 + 16 <= WG_X + WG_H + WG_G, "the last layer's 128 ope
 
 __device__ __forceinline__ uint32_t tmem_col(int l) { return l < NLAYER - 1 ? 64u * (uint32_t)l : 320u; }
 
-// groups [g0, g0 + GROUPS) of a stage: rows [r0, r0 + 64) of src (GROUPS x 16 bytes each), zeros past n
-template<uint32_t GROUPS>
+// groups [g0, g0 + GROUPS) of a stage: rows [r0, r0 + 64) of src (GROUPS x 16 bytes each, by records or by
+// tiles as k_train_tc_wg stores them), zeros past n
+template<uint32_t GROUPS, bool TILED>
 __device__ __forceinline__ void wg_load(const uint32_t *__restrict__ src, uint32_t r0, uint32_t n, uint32_t dst)
 {
     for(uint32_t i = threadIdx.x; i < GROUPS * WG_TC_CHUNK; i += WG_TC_THREADS)
     {
-        const uint32_t s = i / GROUPS, p = i - s * GROUPS;
+        const uint32_t s = TILED ? i % WG_TC_CHUNK : i / GROUPS, p = TILED ? i / WG_TC_CHUNK : i - s * GROUPS;
         const bool valid = r0 + s < n;
-        tc::cp_async16(dst + p * WG_GROUP + s * 16u, src + (valid ? ((size_t)(r0 + s) * GROUPS + p) * 4u : 0u), valid);
+        const size_t group = TILED ? tiled_group(r0 + s, GROUPS, p) : (size_t)(r0 + s) * GROUPS + p;
+        tc::cp_async16(dst + p * WG_GROUP + s * 16u, src + (valid ? group * 4u : 0u), valid);
     }
 }
 
+template<bool TILED> // H and G by tiles
 __global__ void __launch_bounds__(WG_TC_THREADS)
         k_wgrad_tc(const uint32_t *__restrict__ X, const uint32_t *__restrict__ H, const uint32_t *__restrict__ G,
                    uint32_t n_cap, const uint32_t *__restrict__ d_n, float *__restrict__ dW, uint32_t *__restrict__ err)
@@ -639,9 +717,9 @@ __global__ void __launch_bounds__(WG_TC_THREADS)
     const uint32_t base = tc::smem_addr(smem);
     auto load = [&](uint32_t c, uint32_t b) {
         const uint32_t r0 = c * WG_TC_CHUNK, st = base + b * WG_STAGE;
-        wg_load<WG_X>(X, r0, n, st);
-        wg_load<WG_H>(H, r0, n, st + WG_X * WG_GROUP);
-        wg_load<WG_G>(G, r0, n, st + (WG_X + WG_H) * WG_GROUP);
+        wg_load<WG_X, false>(X, r0, n, st);
+        wg_load<WG_H, TILED>(H, r0, n, st + WG_X * WG_GROUP);
+        wg_load<WG_G, TILED>(G, r0, n, st + (WG_X + WG_H) * WG_GROUP);
     };
     if(blockIdx.x < chunks) load(blockIdx.x, 0);
     tc::cp_async_commit();
@@ -735,72 +813,80 @@ __global__ void __launch_bounds__(WG_TC_THREADS)
 }// namespace
 
 vkg_status nrc_wgrad_tc(vkg_ctx *ctx, const uint32_t *X, const uint32_t *H, const uint32_t *G, uint32_t n,
-                        const uint32_t *d_n, float *dW, uint32_t *err, cudaStream_t st)
+                        const uint32_t *d_n, bool tiled, float *dW, uint32_t *err, cudaStream_t st)
 {
     if(n == 0) return VKG_OK;
-    VKG_TRY_CUDA(ctx, cudaFuncSetAttribute(k_wgrad_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)WG_TC_SMEM));
+    auto kern = tiled ? k_wgrad_tc<true> : k_wgrad_tc<false>;
+    VKG_TRY_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)WG_TC_SMEM));
     const uint32_t chunks = (n + WG_TC_CHUNK - 1) / WG_TC_CHUNK;
     const uint32_t grid = std::min<uint32_t>(chunks, (uint32_t)ctx->num_sms);
-    k_wgrad_tc<<<grid, WG_TC_THREADS, WG_TC_SMEM, st>>>(X, H, G, n, d_n, dW, err);
+    kern<<<grid, WG_TC_THREADS, WG_TC_SMEM, st>>>(X, H, G, n, d_n, dW, err);
     return cuda_check(ctx, cudaGetLastError(), "k_wgrad_tc");
 }
 
-// the pipelined MLP over encoded inputs X: inference (H null) or the training forward (H receives the
-// activations)
-template<int NWG>
-vkg_status launch_forward_tc(vkg_ctx *ctx, const uint16_t *wtc, const uint32_t *X, uint32_t n, const uint32_t *d_n,
-                             float *Y, uint32_t *H, uint32_t *err, cudaStream_t st)
+// grid of a warpgroup kernel: a CTA per NWG tiles, at most as many as are resident
+template<int NWG, class K>
+vkg_status warpgroup_grid(vkg_ctx *ctx, K kern, uint32_t smem, uint32_t n, uint32_t &grid)
 {
-    const uint32_t smem = TC_W_BYTES + NWG * TC_A_BYTES;
-    auto kern = H ? k_infer_tc_wg<NWG, true> : k_infer_tc_wg<NWG, false>;
     VKG_TRY_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     int per_sm = 0;
     VKG_TRY_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, NWG * 128, smem));
     // TMEM: a resident CTA holds its share of the SM's 512 columns
     per_sm = std::max(1, std::min(per_sm, (int)(512 / tmem_columns(TC_WG_COLS, NWG))));
     const uint32_t tiles = (n + TC_TILE - 1) / TC_TILE;
-    const uint32_t grid_n = std::min<uint32_t>((tiles + NWG - 1) / NWG, (uint32_t)(ctx->num_sms * per_sm));
-    kern<<<grid_n, NWG * 128, smem, st>>>(X, n, d_n, wtc, Y, err, H);
+    grid = std::min<uint32_t>((tiles + NWG - 1) / NWG, (uint32_t)(ctx->num_sms * per_sm));
+    return VKG_OK;
+}
+
+template<int NWG>
+vkg_status launch_forward_tc(vkg_ctx *ctx, const uint16_t *wtc, const uint32_t *X, uint32_t n, const uint32_t *d_n,
+                             float *Y, uint32_t *err, cudaStream_t st)
+{
+    const uint32_t smem = TC_W_BYTES + NWG * TC_A_BYTES;
+    uint32_t grid = 0;
+    if(vkg_status s = warpgroup_grid<NWG>(ctx, k_infer_tc_wg<NWG>, smem, n, grid); s != VKG_OK) return s;
+    k_infer_tc_wg<NWG><<<grid, NWG * 128, smem, st>>>(X, n, d_n, wtc, Y, err);
     return cuda_check(ctx, cudaGetLastError(), "k_infer_tc_wg");
 }
 
-vkg_status nrc_forward_tc(vkg_ctx *ctx, const uint16_t *wtc, const uint32_t *X, uint32_t n, const uint32_t *d_n,
-                          float *Y, uint32_t *H, uint32_t *err, cudaStream_t st)
+// the pipelined MLP over encoded inputs X
+static vkg_status nrc_forward_tc(vkg_ctx *ctx, const uint16_t *wtc, const uint32_t *X, uint32_t n, const uint32_t *d_n,
+                                 float *Y, uint32_t *err, cudaStream_t st)
 {
-    if(n == 0) return VKG_OK;
     // tiles in flight per SM (inference with the encoding, 4,096 / 20,000 / 65,536 / 2,073,600 queries: one
     // warpgroup a CTA 19 / 28 / 46 / 908 us, two 21 / 25 / 42 / 751, four 24 / 29 / 40 / 643, five 26 / 31 /
     // 42 / 684)
     const uint32_t tiles = (n + TC_TILE - 1) / TC_TILE, sms = (uint32_t)ctx->num_sms;
-    if(tiles >= 3 * sms) return launch_forward_tc<4>(ctx, wtc, X, n, d_n, Y, H, err, st);
-    if(tiles <= sms / 2) return launch_forward_tc<1>(ctx, wtc, X, n, d_n, Y, H, err, st);
-    return launch_forward_tc<2>(ctx, wtc, X, n, d_n, Y, H, err, st);
+    if(tiles >= 3 * sms) return launch_forward_tc<4>(ctx, wtc, X, n, d_n, Y, err, st);
+    if(tiles <= sms / 2) return launch_forward_tc<1>(ctx, wtc, X, n, d_n, Y, err, st);
+    return launch_forward_tc<2>(ctx, wtc, X, n, d_n, Y, err, st);
 }
 
 template<int NWG>
-vkg_status launch_backward_tc(vkg_ctx *ctx, const uint16_t *wtc_t, const uint32_t *H, const float *Y, const float *T,
-                              uint32_t n, const uint32_t *d_n, uint32_t *G, float *dXg, float *loss, uint32_t *err,
-                              cudaStream_t st)
+vkg_status launch_train_tc(vkg_ctx *ctx, const uint16_t *wtc, const uint16_t *wtc_t, const uint32_t *X, const float *T,
+                           uint32_t n, const uint32_t *d_n, uint32_t *H, uint32_t *G, float *dXg, float *loss,
+                           uint32_t *err, cudaStream_t st)
 {
-    const uint32_t smem = TC_W_BYTES + NWG * TC_G_BYTES;
-    VKG_TRY_CUDA(ctx, cudaFuncSetAttribute(k_backward_tc_wg<NWG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    int per_sm = 0;
-    VKG_TRY_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_backward_tc_wg<NWG>, NWG * 128, smem));
-    per_sm = std::max(1, std::min(per_sm, (int)(512 / tmem_columns(TC_WG_COLS, NWG))));
-    const uint32_t tiles = (n + TC_TILE - 1) / TC_TILE;
-    const uint32_t grid_n = std::min<uint32_t>((tiles + NWG - 1) / NWG, (uint32_t)(ctx->num_sms * per_sm));
-    k_backward_tc_wg<NWG><<<grid_n, NWG * 128, smem, st>>>(H, Y, T, n, d_n, wtc_t, G, dXg, loss, err);
-    return cuda_check(ctx, cudaGetLastError(), "k_backward_tc_wg");
+    const uint32_t smem = 2 * TC_W_BYTES + NWG * (TC_A_BYTES + TC_G_BYTES);
+    uint32_t grid = 0;
+    if(vkg_status s = warpgroup_grid<NWG>(ctx, k_train_tc_wg<NWG>, smem, n, grid); s != VKG_OK) return s;
+    k_train_tc_wg<NWG><<<grid, NWG * 128, smem, st>>>(X, T, n, d_n, wtc, wtc_t, reinterpret_cast<uint4 *>(H),
+                                                      reinterpret_cast<uint4 *>(G), reinterpret_cast<float4 *>(dXg), loss,
+                                                      err);
+    return cuda_check(ctx, cudaGetLastError(), "k_train_tc_wg");
 }
 
-vkg_status nrc_backward_tc(vkg_ctx *ctx, const uint16_t *wtc_t, const uint32_t *H, const float *Y, const float *T,
-                           uint32_t n, const uint32_t *d_n, uint32_t *G, float *dXg, float *loss, uint32_t *err,
-                           cudaStream_t st)
+vkg_status nrc_train_tc(vkg_ctx *ctx, const uint16_t *wtc, const uint16_t *wtc_t, const uint32_t *X, const float *T,
+                        uint32_t n, const uint32_t *d_n, uint32_t *H, uint32_t *G, float *dXg, float *loss,
+                        uint32_t *err, cudaStream_t st)
 {
     if(n == 0) return VKG_OK;
     const uint32_t tiles = (n + TC_TILE - 1) / TC_TILE, sms = (uint32_t)ctx->num_sms;
-    if(tiles >= 3 * sms) return launch_backward_tc<4>(ctx, wtc_t, H, Y, T, n, d_n, G, dXg, loss, err, st);
-    return launch_backward_tc<2>(ctx, wtc_t, H, Y, T, n, d_n, G, dXg, loss, err, st);
+    // a wave that holds every tile, with as few tiles per SM as that takes (backward of 12,000 / 30,000 / 40,000 /
+    // 65,536 records: one warpgroup a CTA 56 / 98 / 119 / 152 us, two 58 / 88 / 112 / 132, four 62 / 94 / 106 / 127)
+    if(tiles > 2 * sms) return launch_train_tc<4>(ctx, wtc, wtc_t, X, T, n, d_n, H, G, dXg, loss, err, st);
+    if(tiles > sms) return launch_train_tc<2>(ctx, wtc, wtc_t, X, T, n, d_n, H, G, dXg, loss, err, st);
+    return launch_train_tc<1>(ctx, wtc, wtc_t, X, T, n, d_n, H, G, dXg, loss, err, st);
 }
 
 vkg_status nrc_infer_tc(vkg_ctx *ctx, const grid_config &gc, const __half2 *grid, const uint16_t *wtc,
@@ -808,7 +894,7 @@ vkg_status nrc_infer_tc(vkg_ctx *ctx, const grid_config &gc, const __half2 *grid
                         cudaStream_t st)
 {
     if(n == 0) return VKG_OK;
-    if(X) return nrc_forward_tc(ctx, wtc, X, n, d_n, Y, nullptr, err, st);
+    if(X) return nrc_forward_tc(ctx, wtc, X, n, d_n, Y, err, st);
     auto kern = X ? k_infer_tc<false> : k_infer_tc<true>;
     VKG_TRY_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_SMEM));
     int per_sm = 0;
