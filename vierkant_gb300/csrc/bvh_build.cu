@@ -609,44 +609,26 @@ struct blas_box
     const node8 *nodes; // the BLAS's nodes: its upper levels give a tighter instance box than its bounds
 };
 
-// child box k of a node, dequantised (the quantised boxes contain their geometry)
-__device__ __forceinline__ void node_child_box(const node8 *nd, int k, double lo[3], double hi[3])
+// corner of child k of a node (words w): coordinate c, the box's high side or its low one. Layout
+// (traverse.cuh, node_keys): origin in words 0-2, scales in 3, lo x / y / z in words 4-5 / 6-7 / 8-9, hi in 10-15
+__device__ __forceinline__ uint32_t child_quant(const uint32_t *w, int k, int c, bool high)
 {
-    const uint32_t *w = reinterpret_cast<const uint32_t *>(nd);
-    const float ox = __uint_as_float(w[0]), oy = __uint_as_float(w[1]), oz = __uint_as_float(w[2]);
-    const uint32_t meta = w[3];
-    const double sx = exp_scale(meta & 0xFFu), sy = exp_scale((meta >> 8) & 0xFFu), sz = exp_scale((meta >> 16) & 0xFFu);
-    auto q = [&](int word, int kk) { return (double)((w[word + (kk >> 2)] >> (8 * (kk & 3))) & 0xFFu); };
-    // layout (traverse.cuh, node_keys): lo x / y / z in words 4-5 / 6-7 / 8-9, hi x / y / z in 10-11 / 12-13 / 14-15
-    lo[0] = ox + q(4, k) * sx;
-    lo[1] = oy + q(6, k) * sy;
-    lo[2] = oz + q(8, k) * sz;
-    hi[0] = ox + q(10, k) * sx;
-    hi[1] = oy + q(12, k) * sy;
-    hi[2] = oz + q(14, k) * sz;
+    return (w[(high ? 10 : 4) + 2 * c + (k >> 2)] >> (8 * (k & 3))) & 0xFFu;
 }
+__device__ __forceinline__ float child_scale(const uint32_t *w, int c) { return exp_scale((w[3] >> (8 * c)) & 0xFFu); }
 
-// [wlo, whi] grown by the transformed box [lo, hi]. Of the box's eight corners the one whose products are
-// all the smallest (largest) gives the smallest (largest) rounded sum, as rounding is monotone.
-__device__ __forceinline__ void grow_transformed(const float *T, const double lo[3], const double hi[3], double wlo[3],
-                                                 double whi[3])
+// box slot s (0..63) of a BLAS, two levels below its root: child s & 7 of root child s >> 3, or a leaf of the
+// root at s & 7 = 0. The words of the node that holds the box and its child there; false if there is none
+__device__ __forceinline__ bool box_slot(const node8 *nodes, uint32_t s, const uint32_t *&w, int &k)
 {
-    for(int a = 0; a < 3; ++a)
-    {
-        double p[3], q[3];
-        for(int k = 0; k < 3; ++k)
-        {
-            const bool neg = T[4 * a + k] < 0.f;
-            p[k] = neg ? hi[k] : lo[k];
-            q[k] = neg ? lo[k] : hi[k];
-        }
-        auto at = [&](const double c[3]) {
-            return (double)T[4 * a] * c[0] + (double)T[4 * a + 1] * c[1] + (double)T[4 * a + 2] * c[2] +
-                   (double)T[4 * a + 3];
-        };
-        wlo[a] = fmin(wlo[a], at(p));
-        whi[a] = fmax(whi[a], at(q));
-    }
+    w = reinterpret_cast<const uint32_t *>(nodes);
+    k = (int)(s >> 3);
+    if((uint32_t)k >= w[3] >> 24) return false;
+    const uint32_t c = w[16 + k];
+    if(c & LEAF_BIT) return (s & 7u) == 0u;
+    w = reinterpret_cast<const uint32_t *>(nodes + c);
+    k = (int)(s & 7u);
+    return (uint32_t)k < w[3] >> 24;
 }
 
 // world -> object transform of an object -> world 3x4 transform: inverse of the 3x3 part by the
@@ -680,8 +662,11 @@ __device__ __forceinline__ bool invert_3x4(const float *m, float *inv)
 
 // World boxes of the instances, one warp each: the union of the transformed boxes two levels below the
 // BLAS root (a rotated mesh's own bounds would be loose: a sphere's rotated bounding cube holds up to 5x
-// its volume), two of them per lane. One thread per instance walked its 64 boxes, eight corners each in
-// FP64: 606 us for 20,000 instances, now 225 us (FP64 issue).
+// its volume), two of them per lane. A side of the union is the smallest (largest) of 64 sums in FP64, and
+// of a box's eight corners the one whose products are all the smallest gives it, as rounding is monotone.
+// The sums in FP32, with a bound of their error, leave one or a few boxes that can hold the extreme; FP64
+// (two operations a clock and SM) evaluates those alone, five lanes a side.
+// 20,000 instances: 68 us; 225 us with every sum in FP64.
 __global__ void __launch_bounds__(256)
         k_instance_boxes(const vkg_instance *__restrict__ inst, uint32_t n, const blas_box *__restrict__ bb,
                          uint32_t nblas, box6 *__restrict__ tbox, uint32_t *__restrict__ scene_enc,
@@ -707,50 +692,89 @@ __global__ void __launch_bounds__(256)
         const blas_box B = bb[bl];
         float inv[12];
         if(lane == 0 && !invert_3x4(I.transform, inv)) atomicOr(err, BUILD_ERR_SINGULAR);
-        double lo[3] = {1e300, 1e300, 1e300}, hi[3] = {-1e300, -1e300, -1e300};
+        // sides 0..2: the lows, 3..5: the highs negated; lane l evaluates side l mod 6 (lanes 30, 31: none)
+        const uint32_t side = lane % 6u;
+        uint64_t cand = 0;
         if(B.num_tris)
         {
-            const node8 *root = B.nodes;
-            const uint32_t *rw = reinterpret_cast<const uint32_t *>(root);
-            const uint32_t nch = rw[3] >> 24, g = lane & 7u;
-            for(uint32_t k = lane >> 3; k < nch; k += 4)
+            float low[2][6], up[6]; // bounds of this lane's two boxes, and of the least of them from above
+            bool have[2];
+#pragma unroll
+            for(int d = 0; d < 6; ++d) up[d] = __int_as_float(0x7f800000);
+#pragma unroll
+            for(int it = 0; it < 2; ++it)
             {
-                const uint32_t c = rw[16 + k];
-                double clo[3], chi[3];
-                if(c & LEAF_BIT)
+                const uint32_t *w;
+                int k;
+                have[it] = box_slot(B.nodes, lane + 32u * it, w, k);
+                if(!have[it]) continue;
+                float lo[3], hi[3];
+#pragma unroll
+                for(int c = 0; c < 3; ++c)
                 {
-                    if(g) continue;
-                    node_child_box(root, (int)k, clo, chi);
+                    const float o = __uint_as_float(w[c]), sc = child_scale(w, c);
+                    lo[c] = fmaf((float)child_quant(w, k, c, false), sc, o);
+                    hi[c] = fmaf((float)child_quant(w, k, c, true), sc, o);
                 }
-                else
+#pragma unroll
+                for(int d = 0; d < 6; ++d)
                 {
-                    const node8 *ch = B.nodes + c;
-                    if(g >= reinterpret_cast<const uint32_t *>(ch)[3] >> 24) continue;
-                    node_child_box(ch, (int)g, clo, chi);
+                    const float *T = I.transform + 4 * (d % 3);
+                    float v = T[3], mag = fabsf(T[3]);
+#pragma unroll
+                    for(int c = 0; c < 3; ++c)
+                    {
+                        const float x = (T[c] < 0.f) != (d >= 3) ? hi[c] : lo[c];
+                        v = fmaf(T[c], x, v);
+                        mag = fmaf(fabsf(T[c]), fabsf(x), mag);
+                    }
+                    // at most 6 roundings of 2^-24, each of at most mag; 2^-20 also covers mag's own
+                    const float e = fmaf(mag, 0x1p-20f, 0x1p-120f), key = d < 3 ? v : -v;
+                    low[it][d] = key - e;
+                    up[d] = fminf(up[d], key + e);
                 }
-                grow_transformed(I.transform, clo, chi, lo, hi);
             }
+            __syncwarp();
+#pragma unroll
+            for(int d = 0; d < 6; ++d)
+            {
+                // a box is out if it cannot reach the least upper bound; one that is not a number stays in
+                const float least = fdec(__reduce_min_sync(0xffffffffu, fenc(up[d])));
+                const uint32_t m0 = __ballot_sync(0xffffffffu, have[0] && !(low[0][d] > least));
+                const uint32_t m1 = __ballot_sync(0xffffffffu, have[1] && !(low[1][d] > least));
+                if(side == (uint32_t)d) cand = m0 | ((uint64_t)m1 << 32);
+            }
+            if(lane >= 30) cand = 0;
+            for(uint32_t k = lane / 6u; k; --k) cand &= cand - 1; // every fifth candidate, from the (l / 6)th on
+        }
+        const uint32_t axis = side % 3u;
+        const bool high = side >= 3u;
+        const float *T = inst[i].transform + 4 * axis;
+        double best = 1e300;
+        while(cand)
+        {
+            const uint32_t *w;
+            int k;
+            box_slot(B.nodes, (uint32_t)__ffsll(cand) - 1u, w, k);
+            double c[3];
+            for(int a = 0; a < 3; ++a)
+                c[a] = (double)__uint_as_float(w[a]) +
+                       (double)child_quant(w, k, a, (T[a] < 0.f) != high) * (double)child_scale(w, a);
+            const double v = (double)T[0] * c[0] + (double)T[1] * c[1] + (double)T[2] * c[2] + (double)T[3];
+            best = fmin(best, high ? -v : v);
+            for(int t = 0; t < 5; ++t) cand &= cand - 1;
         }
         __syncwarp();
-        for(int a = 0; a < 3; ++a)
-            for(int o = 16; o; o >>= 1)
-            {
-                lo[a] = fmin(lo[a], __shfl_xor_sync(0xffffffffu, lo[a], o));
-                hi[a] = fmax(hi[a], __shfl_xor_sync(0xffffffffu, hi[a], o));
-            }
-        if(lane == 0)
+        double least = best;
+        for(uint32_t d = 6; d < 30; d += 6) least = fmin(least, __shfl_sync(0xffffffffu, best, lane + d));
+        if(lane < 6)
         {
-            box6 b;
-            for(int a = 0; a < 3; ++a)
-            {
-                // rounded outward; the collapse grows every box by its margin on top. An empty mesh: a
-                // point box at the instance origin (the traversal skips it)
-                b.lo[a] = B.num_tris ? __double2float_rd(lo[a]) : I.transform[4 * a + 3];
-                b.hi[a] = B.num_tris ? __double2float_ru(hi[a]) : I.transform[4 * a + 3];
-                atomicMin(&s_lo[a], fenc(b.lo[a]));
-                atomicMax(&s_hi[a], fenc(b.hi[a]));
-            }
-            tbox[i] = b;
+            // rounded outward; the collapse grows every box by its margin on top. An empty mesh: a
+            // point box at the instance origin (the traversal skips it)
+            const float f = !B.num_tris ? T[3] : (high ? __double2float_ru(-least) : __double2float_rd(least));
+            (high ? tbox[i].hi : tbox[i].lo)[axis] = f;
+            if(high) atomicMax(&s_hi[axis], fenc(f));
+            else atomicMin(&s_lo[axis], fenc(f));
         }
     }
     __syncthreads();
