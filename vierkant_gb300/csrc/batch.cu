@@ -85,7 +85,11 @@ __global__ void __launch_bounds__(PT_THREADS)
         beta_pdf[p] = make_float4(1.f, 1.f, 1.f, 0.f);
         radiance[p] = make_float4(0.f, 0.f, 0.f, 0.f);
     }
-    if(blockIdx.x == 0 && threadIdx.x == 0) counters[0] = n;
+    if(blockIdx.x == 0 && threadIdx.x == 0)
+    {
+        counters[0] = n;
+        counters[1] = counters[2] = counters[4] = 0; // the other queue, the shadow and the light-shadow queue
+    }
 }
 
 // the wave's radiance into the job pixels' sums: one thread per (chunk, pixel), samples in order
@@ -167,7 +171,7 @@ struct vkg_batch
     batch_job_dev *d_jd = nullptr;
     float *sum = nullptr, *accum = nullptr;
     uint32_t *d_batch = nullptr;
-    uint32_t *counters = nullptr; // [0..1] queues, [2] shadow queue, [3] persistent work counter
+    uint32_t *counters = nullptr; // [0..1] queues, [2] shadow queue, [3] persistent work counter, [4] light-shadow queue
     unsigned long long *totals = nullptr;
     // plan for the current tuning
     struct wave
@@ -378,9 +382,6 @@ vkg_status enqueue(vkg_batch *b, const std::vector<vkg_batch::wave> &waves, cuda
                 k_pt_extend<job_table, 64><<<grid, bs, 0, st>>>(J, b->q_ray[a], b->q_pid[a], cnt_in, b->hits, b->hit_inst);
             else
                 k_pt_extend<<<grid, bs, 0, st>>>(J, b->q_ray[a], b->q_pid[a], cnt_in, b->hits, b->hit_inst);
-            VKG_TRY_CUDA(ctx, cudaMemsetAsync(cnt_out, 0, sizeof(uint32_t), st));
-            VKG_TRY_CUDA(ctx, cudaMemsetAsync(cnt_s, 0, sizeof(uint32_t), st));
-            if(cnt_l) VKG_TRY_CUDA(ctx, cudaMemsetAsync(cnt_l, 0, sizeof(uint32_t), st));
             // the shade variant: the full material set and the lights or metal-roughness only, each
             // with the texture terms when a job has textures
 #define VKG_BATCH_SHADE(F, TX, LQ)                                                                                     \

@@ -1257,6 +1257,8 @@ vkg_status vkg_tracer_render(vkg_tracer *t, const vkg_scene *sc, const vkg_camer
         k_pt_generate<<<grid, PT_THREADS, 0, st>>>(P, n, t->q_ray[0], t->q_pid[0], t->rng, t->beta_pdf, t->radiance,
                                                    t->counters, t->vcount);
         int a = 0;
+        bool paired = false; // this bounce's short ray queue was traced with the last one's shadow rays
+        auto bins_queue = [&](uint32_t depth) { return depth == 1 || (sc->tlas && depth == 2); };
         for(uint32_t depth = 0; depth < depths; ++depth)
         {
             uint32_t *cnt_in = t->counters + a, *cnt_out = t->counters + (1 - a), *cnt_s = t->counters + 2;
@@ -1279,18 +1281,16 @@ vkg_status vkg_tracer_render(vkg_tracer *t, const vkg_scene *sc, const vkg_camer
                 // costlier two-level traversal still gains: the stress frame 1,334 -> 1,268 ms with the
                 // shadow queues below, 1,233 -> 1,215 ms with the second bounce)
                 const vkg_bvh *bounds = sc->bvh ? sc->bvh : (sc->tlas ? &sc->tlas->top : nullptr);
-                const bool bin_queue = depth == 1 || (sc->tlas && depth == 2);
                 const uint32_t *perm =
-                        bin_queue ? bin_rays(ctx, bounds, t->q_ray[a], n, cnt_in, 0u, BIN_MIN_CLOSEST, st, &reordered) : nullptr;
+                        bins_queue(depth) ? bin_rays(ctx, bounds, t->q_ray[a], n, cnt_in, 0u, BIN_MIN_CLOSEST, st, &reordered) : nullptr;
                 const bool by_count = can_group && !groups && depth > 0 && !perm;
                 auto extend = [&](auto kern) {
                     kern<<<wide_grid, PT_THREADS, 0, st>>>(SS, t->q_ray[a], t->q_pid[a], cnt_in, t->hits, t->hit_inst, perm,
                                                       reordered, t->rng, depth, by_count ? PT_GROUP_MAX_QUEUE : 0u);
                 };
-                auto extend_group = [&](auto kern) {
-                    kern<<<group_grid, PT_THREADS, 0, st>>>(SS, t->q_ray[a], cnt_in, t->hits, t->hit_inst,
-                                                            by_count ? PT_GROUP_MAX_QUEUE : 0xFFFFFFFFu);
-                };
+                const extend_queue eq{t->q_ray[a], cnt_in, t->hits, t->hit_inst,
+                                      by_count ? PT_GROUP_MAX_QUEUE : 0xFFFFFFFFu, group_grid};
+                auto extend_group = [&](auto kern) { kern<<<group_grid, PT_THREADS, 0, st>>>(SS, eq); };
                 constexpr int BIG = (int)TRAVERSAL_STACK;
                 using T1 = single_scene;
                 if(sc->tlas && !groups)
@@ -1301,7 +1301,9 @@ vkg_status vkg_tracer_render(vkg_tracer *t, const vkg_scene *sc, const vkg_camer
                 else if(!groups)
                     small_stack ? extend(k_pt_extend<T1, 64, false, LEVELS_ONE>)
                                 : extend(k_pt_extend<T1, BIG, false, LEVELS_ONE>);
-                if((groups || by_count) && sc->tlas)
+                if(paired)
+                    ; // traced with the last bounce's shadow rays
+                else if((groups || by_count) && sc->tlas)
                     tl_small_stack ? extend_group(k_pt_extend_group<TL_GROUP_SMALL_STACK, LEVELS_TWO>)
                                    : extend_group(k_pt_extend_group<TL_GROUP_STACK, LEVELS_TWO>);
                 else if(groups || by_count)
@@ -1309,9 +1311,6 @@ vkg_status vkg_tracer_render(vkg_tracer *t, const vkg_scene *sc, const vkg_camer
                                 : extend_group(k_pt_extend_group<BIG, LEVELS_ONE>);
                 if(perm) bin_rays_done(ctx, st);
             }
-            VKG_TRY_CUDA(ctx, cudaMemsetAsync(cnt_out, 0, sizeof(uint32_t), st));
-            VKG_TRY_CUDA(ctx, cudaMemsetAsync(cnt_s, 0, sizeof(uint32_t), st));
-            if(cnt_l) VKG_TRY_CUDA(ctx, cudaMemsetAsync(cnt_l, 0, sizeof(uint32_t), st));
             // the full material set: group the queue by material class first, so that warps shade
             // coherently (k_pt_bin_count / k_pt_bin_scatter, two light passes over the hits)
             const uint32_t *order = nullptr;
@@ -1361,10 +1360,13 @@ vkg_status vkg_tracer_render(vkg_tracer *t, const vkg_scene *sc, const vkg_camer
                     kern<<<wide_grid, PT_THREADS, 0, st>>>(SS, t->s_ray, t->s_pid, t->s_contrib, cnt_s, t->radiance, s_perm,
                                                       s_reordered, t->rng, by_count ? PT_GROUP_MAX_QUEUE : 0u);
                 };
-                auto shadow_group = [&](auto kern) {
-                    kern<<<group_grid, PT_THREADS, 0, st>>>(SS, t->s_ray, t->s_pid, t->s_contrib, cnt_s, t->radiance,
-                                                            by_count ? PT_GROUP_MAX_QUEUE : 0xFFFFFFFFu);
-                };
+                const shadow_queue sq{t->s_ray, t->s_pid, t->s_contrib, cnt_s, t->radiance,
+                                      by_count ? PT_GROUP_MAX_QUEUE : 0xFFFFFFFFu, group_grid};
+                auto shadow_group = [&](auto kern) { kern<<<group_grid, PT_THREADS, 0, st>>>(SS, sq); };
+                // with the next bounce's rays, unless those are traced in another way
+                paired = (groups || (by_count && !bins_queue(depth + 1))) && depth + 1 < depths;
+                const extend_queue eq{t->q_ray[1 - a], cnt_out, t->hits, t->hit_inst, sq.up_to, group_grid};
+                auto pair = [&](auto kern) { kern<<<2 * group_grid, PT_THREADS, 0, st>>>(SS, eq, sq); };
                 constexpr int BIG = (int)TRAVERSAL_STACK;
                 using T1 = single_scene;
                 if(sc->tlas && !groups)
@@ -1375,7 +1377,12 @@ vkg_status vkg_tracer_render(vkg_tracer *t, const vkg_scene *sc, const vkg_camer
                 else if(!groups)
                     small_stack ? shadow(k_pt_shadow<T1, 64, false, LEVELS_ONE>)
                                 : shadow(k_pt_shadow<T1, BIG, false, LEVELS_ONE>);
-                if((groups || by_count) && sc->tlas)
+                if(paired && sc->tlas)
+                    tl_small_stack ? pair(k_pt_pair_group<TL_GROUP_SMALL_STACK, LEVELS_TWO>)
+                                   : pair(k_pt_pair_group<TL_GROUP_STACK, LEVELS_TWO>);
+                else if(paired)
+                    small_stack ? pair(k_pt_pair_group<64, LEVELS_ONE>) : pair(k_pt_pair_group<BIG, LEVELS_ONE>);
+                else if((groups || by_count) && sc->tlas)
                     tl_small_stack ? shadow_group(k_pt_shadow_group<TL_GROUP_SMALL_STACK, LEVELS_TWO>)
                                    : shadow_group(k_pt_shadow_group<TL_GROUP_STACK, LEVELS_TWO>);
                 else if(groups || by_count)

@@ -378,7 +378,11 @@ __global__ void __launch_bounds__(PT_THREADS)
         if(P.mstack)
             P.mstack[p] = P.cam_medium != 0xFFFFFFFFu ? make_uint4(1u, P.cam_medium, 0u, 0u) : make_uint4(0u, 0u, 0u, 0u);
     }
-    if(blockIdx.x == 0 && threadIdx.x == 0) counters[0] = n;
+    if(blockIdx.x == 0 && threadIdx.x == 0)
+    {
+        counters[0] = n;
+        counters[1] = counters[2] = counters[7] = 0; // the other queue, the shadow and the light-shadow queue
+    }
 }
 
 // The levels of a scene's BVH that a tracer is compiled for: one that holds both traversals spills in
@@ -449,17 +453,29 @@ __global__ void __launch_bounds__(PT_THREADS, min_blocks<STACK, ALPHA, LEVELS>)
 // queues are faster with a thread per ray and the later ones by groups (1,478 us; none 1,654, all 1,517).
 // Incoherent queues break even at 64,000 to 190,000 rays.
 constexpr uint32_t PT_GROUP_MAX_WAVE = 1u << 18, PT_GROUP_MAX_QUEUE = 1u << 17;
-template<int STACK, int LEVELS>
-__global__ void __launch_bounds__(PT_THREADS)
-        k_pt_extend_group(single_scene S, const vkg_ray *__restrict__ q_ray, const uint32_t *__restrict__ count,
-                          vkg_hit *__restrict__ hits, uint32_t *__restrict__ hit_inst, uint32_t up_to)
+struct extend_queue
 {
-    __shared__ uint2 stack[PT_THREADS / GROUP_LANES][group_stack_entries<STACK>];
+    const vkg_ray *ray;
+    const uint32_t *count;
+    vkg_hit *hits;
+    uint32_t *hit_inst;
+    uint32_t up_to, blocks; // a longer queue is left to k_pt_extend
+};
+template<int STACK>
+using group_stacks = uint2[PT_THREADS / GROUP_LANES][group_stack_entries<STACK>];
+
+// block `block` of q.blocks
+template<int STACK, int LEVELS>
+__device__ __forceinline__ void extend_group(const pt_params &P, const extend_queue &q, uint32_t block,
+                                             group_stacks<STACK> &stack)
+{
     constexpr uint32_t PER = PT_THREADS / GROUP_LANES;
-    const pt_params &P = S.params(0u);
-    const uint32_t n = *count, group = threadIdx.x / GROUP_LANES;
-    if(n > up_to) return;
-    for(uint32_t base = blockIdx.x * PER; base < n; base += gridDim.x * PER)
+    const vkg_ray *__restrict__ q_ray = q.ray;
+    vkg_hit *__restrict__ hits = q.hits;
+    uint32_t *__restrict__ hit_inst = q.hit_inst;
+    const uint32_t n = *q.count, group = threadIdx.x / GROUP_LANES;
+    if(n > q.up_to) return;
+    for(uint32_t base = block * PER; base < n; base += q.blocks * PER)
     {
         const uint32_t i = base + group;
         const bool active = i < n;
@@ -486,6 +502,13 @@ __global__ void __launch_bounds__(PT_THREADS)
         const uint4 h = trace();
         if(writes) reinterpret_cast<uint4 *>(hits)[i] = h;
     }
+}
+
+template<int STACK, int LEVELS>
+__global__ void __launch_bounds__(PT_THREADS) k_pt_extend_group(single_scene S, extend_queue q)
+{
+    __shared__ group_stacks<STACK> stack;
+    extend_group<STACK, LEVELS>(S.params(0u), q, blockIdx.x, stack);
 }
 
 // surface point, unit geometric normal (world space) and material of a hit: the triangle's vertices,
@@ -1325,18 +1348,27 @@ __global__ void __launch_bounds__(PT_THREADS, min_blocks<STACK, ALPHA, LEVELS>)
 }
 
 // the same for short queues, eight lanes per ray (k_pt_extend_group)
-template<int STACK, int LEVELS>
-__global__ void __launch_bounds__(PT_THREADS)
-        k_pt_shadow_group(single_scene S, const vkg_ray *__restrict__ s_ray, const uint32_t *__restrict__ s_pid,
-                          const float4 *__restrict__ s_contrib, const uint32_t *__restrict__ count,
-                          float4 *__restrict__ radiance, uint32_t up_to)
+struct shadow_queue
 {
-    __shared__ uint2 stack[PT_THREADS / GROUP_LANES][group_stack_entries<STACK>];
+    const vkg_ray *ray;
+    const uint32_t *pid;
+    const float4 *contrib;
+    const uint32_t *count;
+    float4 *radiance;
+    uint32_t up_to, blocks;
+};
+template<int STACK, int LEVELS>
+__device__ __forceinline__ void shadow_group(const pt_params &P, const shadow_queue &q, uint32_t block,
+                                             group_stacks<STACK> &stack)
+{
     constexpr uint32_t PER = PT_THREADS / GROUP_LANES;
-    const pt_params &P = S.params(0u);
-    const uint32_t n = *count, group = threadIdx.x / GROUP_LANES;
-    if(n > up_to) return;
-    for(uint32_t base = blockIdx.x * PER; base < n; base += gridDim.x * PER)
+    const vkg_ray *__restrict__ s_ray = q.ray;
+    const uint32_t *__restrict__ s_pid = q.pid;
+    const float4 *__restrict__ s_contrib = q.contrib;
+    float4 *__restrict__ radiance = q.radiance;
+    const uint32_t n = *q.count, group = threadIdx.x / GROUP_LANES;
+    if(n > q.up_to) return;
+    for(uint32_t base = block * PER; base < n; base += q.blocks * PER)
     {
         const bool active = base + group < n;
         const uint32_t i = active ? base + group : base;
@@ -1363,6 +1395,24 @@ __global__ void __launch_bounds__(PT_THREADS)
             radiance[pid] = L;
         }
     }
+}
+
+template<int STACK, int LEVELS>
+__global__ void __launch_bounds__(PT_THREADS) k_pt_shadow_group(single_scene S, shadow_queue q)
+{
+    __shared__ group_stacks<STACK> stack;
+    shadow_group<STACK, LEVELS>(S.params(0u), q, blockIdx.x, stack);
+}
+
+// A bounce's shadow queue and the next bounce's ray queue in one launch: both come from the same shading pass
+// and neither reads what the other writes. Short queues are bound by the slowest rays of each launch, which
+// here run side by side: NNNPAIR
+template<int STACK, int LEVELS>
+__global__ void __launch_bounds__(PT_THREADS) k_pt_pair_group(single_scene S, extend_queue e, shadow_queue s)
+{
+    __shared__ group_stacks<STACK> stack;
+    if(blockIdx.x < e.blocks) extend_group<STACK, LEVELS>(S.params(0u), e, blockIdx.x, stack);
+    else shadow_group<STACK, LEVELS>(S.params(0u), s, blockIdx.x - e.blocks, stack);
 }
 
 // light-NEE visibility (transmittance_test, visibility_test.slang:94-131): 0 at the first opaque
@@ -1657,11 +1707,14 @@ __global__ void k_fill_miss_queue(const uint32_t *__restrict__ count, vkg_hit *_
         reinterpret_cast<uint4 *>(hits)[i] = make_uint4(VKG_MISS, 0u, 0u, 0u);
 }
 
-__global__ void k_pt_tally(const uint32_t *__restrict__ ext_count, const uint32_t *__restrict__ s_count,
-                           const uint32_t *__restrict__ l_count, unsigned long long *__restrict__ totals)
+// a bounce's rays into the totals; its queues start the next one empty
+__global__ void k_pt_tally(uint32_t *__restrict__ ext_count, uint32_t *__restrict__ s_count,
+                           uint32_t *__restrict__ l_count, unsigned long long *__restrict__ totals)
 {
     totals[0] += *ext_count;
     totals[1] += *s_count + (l_count ? *l_count : 0u);
+    *ext_count = *s_count = 0;
+    if(l_count) *l_count = 0;
 }
 
 // rendering with a cache: path radiance += throughput x prediction (negative outputs clamped)
