@@ -1293,7 +1293,9 @@ vkg_status vkg_tracer_render(vkg_tracer *t, const vkg_scene *sc, const vkg_camer
                 auto extend_group = [&](auto kern) { kern<<<group_grid, PT_THREADS, 0, st>>>(SS, eq); };
                 constexpr int BIG = (int)TRAVERSAL_STACK;
                 using T1 = single_scene;
-                if(sc->tlas && !groups)
+                if(paired)
+                    ; // traced with the last bounce's shadow rays
+                else if(sc->tlas && !groups)
                     alpha ? extend(k_pt_extend<T1, BIG, true, LEVELS_TWO>) : extend(k_pt_extend<T1, BIG, false, LEVELS_TWO>);
                 else if(alpha)
                     small_stack ? extend(k_pt_extend<T1, 64, true, LEVELS_ONE>)
@@ -1361,15 +1363,25 @@ vkg_status vkg_tracer_render(vkg_tracer *t, const vkg_scene *sc, const vkg_camer
                                                       s_reordered, t->rng, by_count ? PT_GROUP_MAX_QUEUE : 0u);
                 };
                 const shadow_queue sq{t->s_ray, t->s_pid, t->s_contrib, cnt_s, t->radiance,
-                                      by_count ? PT_GROUP_MAX_QUEUE : 0xFFFFFFFFu, group_grid};
+                                      groups ? 0xFFFFFFFFu : (by_count ? PT_GROUP_MAX_QUEUE : 0u), group_grid};
                 auto shadow_group = [&](auto kern) { kern<<<group_grid, PT_THREADS, 0, st>>>(SS, sq); };
                 // with the next bounce's rays, unless those are traced in another way
-                paired = (groups || (by_count && !bins_queue(depth + 1))) && depth + 1 < depths;
-                const extend_queue eq{t->q_ray[1 - a], cnt_out, t->hits, t->hit_inst, sq.up_to, group_grid};
+                paired = (groups || (can_group && depth > 0 && !bins_queue(depth + 1))) && depth + 1 < depths;
+                const extend_queue eq{t->q_ray[1 - a], cnt_out, t->hits, t->hit_inst,
+                                      groups ? 0xFFFFFFFFu : PT_GROUP_MAX_QUEUE, group_grid};
                 auto pair = [&](auto kern) { kern<<<2 * group_grid, PT_THREADS, 0, st>>>(SS, eq, sq); };
                 constexpr int BIG = (int)TRAVERSAL_STACK;
                 using T1 = single_scene;
-                if(sc->tlas && !groups)
+                if(paired && !groups)
+                {
+                    extend_queue el = eq;
+                    shadow_queue sl = sq;
+                    el.blocks = sl.blocks = wide_grid;
+                    auto pair_long = [&](auto kern) { kern<<<2 * wide_grid, PT_THREADS, 0, st>>>(SS, el, sl, s_perm, s_reordered); };
+                    sc->tlas ? pair_long(k_pt_pair<BIG, LEVELS_TWO>)
+                    : small_stack ? pair_long(k_pt_pair<64, LEVELS_ONE>) : pair_long(k_pt_pair<BIG, LEVELS_ONE>);
+                }
+                else if(sc->tlas && !groups)
                     alpha ? shadow(k_pt_shadow<T1, BIG, true, LEVELS_TWO>) : shadow(k_pt_shadow<T1, BIG, false, LEVELS_TWO>);
                 else if(alpha)
                     small_stack ? shadow(k_pt_shadow<T1, 64, true, LEVELS_ONE>)
