@@ -85,11 +85,7 @@ __global__ void __launch_bounds__(PT_THREADS)
         beta_pdf[p] = make_float4(1.f, 1.f, 1.f, 0.f);
         radiance[p] = make_float4(0.f, 0.f, 0.f, 0.f);
     }
-    if(blockIdx.x == 0 && threadIdx.x == 0)
-    {
-        counters[0] = n;
-        counters[1] = counters[2] = counters[4] = 0; // the other queue, the shadow and the light-shadow queue
-    }
+    if(blockIdx.x == 0) start_queues(counters, n);
 }
 
 // the wave's radiance into the job pixels' sums: one thread per (chunk, pixel), samples in order
@@ -171,7 +167,7 @@ struct vkg_batch
     batch_job_dev *d_jd = nullptr;
     float *sum = nullptr, *accum = nullptr;
     uint32_t *d_batch = nullptr;
-    uint32_t *counters = nullptr; // [0..1] queues, [2] shadow queue, [3] persistent work counter, [4] light-shadow queue
+    uint32_t *counters = nullptr; // queue lengths (start_queues), then the persistent work counter
     unsigned long long *totals = nullptr;
     // plan for the current tuning
     struct wave
@@ -345,8 +341,6 @@ vkg_status enqueue(vkg_batch *b, const std::vector<vkg_batch::wave> &waves, cuda
     // a 64-entry stack serves BVHs of depth <= 10 (7 (depth - 1) + 1 entries at most)
     if(b->max_bvh_depth > 10) T.stack_depth = 128;
     const job_table J{b->d_params, b->pjob, b->pinc};
-    uint32_t *cnt_l = b->any_lights ? b->counters + 4 : nullptr;
-    const light_queue lq{b->l_ray, b->l_pid, b->l_contrib, cnt_l};
     VKG_TRY_CUDA(ctx, cudaMemsetAsync(b->sum, 0, (size_t)b->total_pix * 3 * sizeof(float), st));
     cache_io io{};
     const uint32_t bs = T.block_size;
@@ -361,16 +355,18 @@ vkg_status enqueue(vkg_batch *b, const std::vector<vkg_batch::wave> &waves, cuda
         int a = 0;
         for(uint32_t depth = 0; depth < w.depths; ++depth)
         {
-            uint32_t *cnt_in = b->counters + a, *cnt_out = b->counters + (1 - a), *cnt_s = b->counters + 2;
+            uint32_t *cnt_in = b->counters + 3 * depth, *cnt_s = cnt_in + 1, *cnt_out = cnt_in + 3;
+            uint32_t *cnt_l = b->any_lights ? cnt_in + 2 : nullptr;
+            const light_queue lq{b->l_ray, b->l_pid, b->l_contrib, cnt_l};
             if(T.extend_kernel == 2)
             {
-                VKG_TRY_CUDA(ctx, cudaMemsetAsync(b->counters + 3, 0, sizeof(uint32_t), st));
+                VKG_TRY_CUDA(ctx, cudaMemsetAsync(b->counters + PT_QUEUE_COUNTS, 0, sizeof(uint32_t), st));
                 if(T.stack_depth == 64)
                     k_pt_trace_persistent<false, job_table, 64><<<grid, bs, 0, st>>>(
-                            J, b->q_ray[a], b->q_pid[a], cnt_in, b->hits, b->hit_inst, nullptr, nullptr, b->counters + 3);
+                            J, b->q_ray[a], b->q_pid[a], cnt_in, b->hits, b->hit_inst, nullptr, nullptr, b->counters + PT_QUEUE_COUNTS);
                 else
                     k_pt_trace_persistent<false, job_table><<<grid, bs, 0, st>>>(
-                            J, b->q_ray[a], b->q_pid[a], cnt_in, b->hits, b->hit_inst, nullptr, nullptr, b->counters + 3);
+                            J, b->q_ray[a], b->q_pid[a], cnt_in, b->hits, b->hit_inst, nullptr, nullptr, b->counters + PT_QUEUE_COUNTS);
             }
             else if(b->any_alpha && T.stack_depth == 64)
                 k_pt_extend<job_table, 64, true><<<grid, bs, 0, st>>>(J, b->q_ray[a], b->q_pid[a], cnt_in, b->hits,
@@ -396,13 +392,13 @@ vkg_status enqueue(vkg_batch *b, const std::vector<vkg_batch::wave> &waves, cuda
 #undef VKG_BATCH_SHADE
             if(T.extend_kernel == 2)
             {
-                VKG_TRY_CUDA(ctx, cudaMemsetAsync(b->counters + 3, 0, sizeof(uint32_t), st));
+                VKG_TRY_CUDA(ctx, cudaMemsetAsync(b->counters + PT_QUEUE_COUNTS, 0, sizeof(uint32_t), st));
                 if(T.stack_depth == 64)
                     k_pt_trace_persistent<true, job_table, 64><<<grid, bs, 0, st>>>(
-                            J, b->s_ray, b->s_pid, cnt_s, nullptr, nullptr, b->s_contrib, b->radiance, b->counters + 3);
+                            J, b->s_ray, b->s_pid, cnt_s, nullptr, nullptr, b->s_contrib, b->radiance, b->counters + PT_QUEUE_COUNTS);
                 else
                     k_pt_trace_persistent<true, job_table><<<grid, bs, 0, st>>>(
-                            J, b->s_ray, b->s_pid, cnt_s, nullptr, nullptr, b->s_contrib, b->radiance, b->counters + 3);
+                            J, b->s_ray, b->s_pid, cnt_s, nullptr, nullptr, b->s_contrib, b->radiance, b->counters + PT_QUEUE_COUNTS);
             }
             else if(b->any_alpha && T.stack_depth == 64)
                 k_pt_shadow<job_table, 64, true><<<grid, bs, 0, st>>>(J, b->s_ray, b->s_pid, b->s_contrib, cnt_s,
@@ -423,9 +419,9 @@ vkg_status enqueue(vkg_batch *b, const std::vector<vkg_batch::wave> &waves, cuda
                 k_pt_light_shadow<job_table, 64><<<grid, bs, 0, st>>>(J, lq, b->radiance);
             else if(cnt_l)
                 k_pt_light_shadow<job_table><<<grid, bs, 0, st>>>(J, lq, b->radiance);
-            k_pt_tally<<<1, 1, 0, st>>>(cnt_in, cnt_s, cnt_l, b->totals);
             a = 1 - a;
         }
+        k_pt_tally<<<1, 32, 0, st>>>(b->counters, w.depths, b->totals);
         k_batch_accumulate<<<(w.npix + 255) / 256, 256, 0, st>>>(ch, w.nchunks, w.npix, b->d_jd, b->radiance, b->sum);
     }
     k_batch_finalize<<<(3 * b->total_pix + 255) / 256, 256, 0, st>>>(b->d_jd, b->njobs, b->total_pix, b->d_batch,
@@ -576,7 +572,7 @@ vkg_status vkg_batch_create(vkg_ctx *ctx, const vkg_batch_job *jobs, uint32_t nj
     al((void **)&b->sum, (size_t)off * 3 * sizeof(float));
     al((void **)&b->accum, (size_t)off * 3 * sizeof(float));
     al((void **)&b->d_batch, sizeof(uint32_t));
-    al((void **)&b->counters, 5 * sizeof(uint32_t));
+    al((void **)&b->counters, (PT_QUEUE_COUNTS + 1) * sizeof(uint32_t));
     al((void **)&b->totals, 2 * sizeof(unsigned long long));
     b->any_lights = !all_lights.empty();
     if(b->any_lights)

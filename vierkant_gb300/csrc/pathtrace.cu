@@ -74,9 +74,9 @@ struct vkg_tracer
     size_t mstack_cap = 0;
     float *cone = nullptr;          // per-path ray-cone widths (scenes with textures)
     size_t cone_cap = 0;
-    uint32_t *counters = nullptr;           // [0..1] queue lengths, [2] shadow queue length, [3] cache queries,
+    uint32_t *counters = nullptr;           // [3] cache queries,
                                             // [4] training records, [5] training batch length, [6] work
-                                            // counter, [7] light shadow queue length
+                                            // counter, from [8] queue lengths (start_queues)
     unsigned long long *totals = nullptr;   // [0] extension rays, [1] shadow rays, [2] cache queries
     cudaEvent_t ev0 = nullptr, ev1 = nullptr, ev_train = nullptr;
     uint64_t last_paths = 0;
@@ -1014,7 +1014,7 @@ vkg_status vkg_tracer_create(vkg_ctx *ctx, const vkg_tracer_create_info *info, v
     t->seed = info->seed;
     t->ref_engine.seed(info->seed);
     t->settings = info->settings;
-    if(cudaMalloc(&t->counters, 8 * sizeof(uint32_t)) != cudaSuccess ||
+    if(cudaMalloc(&t->counters, (8 + PT_QUEUE_COUNTS) * sizeof(uint32_t)) != cudaSuccess ||
        cudaMalloc(&t->totals, 3 * sizeof(unsigned long long)) != cudaSuccess ||
        cudaEventCreate(&t->ev0) != cudaSuccess || cudaEventCreate(&t->ev1) != cudaSuccess ||
        cudaEventCreate(&t->ev_train) != cudaSuccess)
@@ -1122,8 +1122,7 @@ vkg_status vkg_tracer_render(vkg_tracer *t, const vkg_scene *sc, const vkg_camer
     P.dbg_stride = 2 + DBG_U_PER_SEGMENT * t->dbg_segments;
     P.lights = lights.empty() ? nullptr : t->d_lights;
     P.num_lights = (uint32_t)lights.size();
-    uint32_t *cnt_l = lights.empty() ? nullptr : t->counters + 7;
-    const light_queue lq{t->l_ray, t->l_pid, t->l_contrib, cnt_l};
+    const bool lit = !lights.empty();
     // the camera's medium (raypipeline.slang:128-135, PBRPathTracer.cpp:598-605): given, or the
     // medium of the smallest volume instance around the eye; its record follows the scene's
     uint32_t cam_mat = 0xFFFFFFFFu;
@@ -1223,7 +1222,6 @@ vkg_status vkg_tracer_render(vkg_tracer *t, const vkg_scene *sc, const vkg_camer
     }
     cache_io io{t->q_feat, t->q_beta, cnt_q, t->rec, t->vcount};
 
-    VKG_TRY_CUDA(ctx, cudaMemsetAsync(t->sum, 0, (size_t)npix * 3 * sizeof(float), st));
     VKG_TRY_CUDA(ctx, cudaMemsetAsync(t->gbuf, 0, (size_t)npix * sizeof(vkg_pixel_data), st));
     VKG_TRY_CUDA(ctx, cudaMemsetAsync(t->totals, 0, 3 * sizeof(unsigned long long), st));
     VKG_TRY_CUDA(ctx, cudaEventRecord(t->ev0, st));
@@ -1245,6 +1243,7 @@ vkg_status vkg_tracer_render(vkg_tracer *t, const vkg_scene *sc, const vkg_camer
         const uint32_t wide_grid =
                 (uint32_t)std::min<size_t>((n + PT_THREADS - 1) / PT_THREADS, (size_t)ctx->num_sms * 72);
         const single_scene SS{P};
+        uint32_t *queues = t->counters + 8;
         // Short queues of scenes without alpha-tested materials are traced by groups of eight
         // lanes (k_pt_extend_group). A wave of at most PT_GROUP_MAX_WAVE paths is always; a larger wave's
         // later queues may be short, which only the device knows: both kernels are launched from the
@@ -1255,13 +1254,14 @@ vkg_status vkg_tracer_render(vkg_tracer *t, const vkg_scene *sc, const vkg_camer
                                                                (size_t)ctx->num_sms * 64);
         if(cache_render) VKG_TRY_CUDA(ctx, cudaMemsetAsync(cnt_q, 0, sizeof(uint32_t), st));
         k_pt_generate<<<grid, PT_THREADS, 0, st>>>(P, n, t->q_ray[0], t->q_pid[0], t->rng, t->beta_pdf, t->radiance,
-                                                   t->counters, t->vcount);
+                                                   queues, t->vcount);
         int a = 0;
         bool paired = false; // this bounce's short ray queue was traced with the last one's shadow rays
         auto bins_queue = [&](uint32_t depth) { return depth == 1 || (sc->tlas && depth == 2); };
         for(uint32_t depth = 0; depth < depths; ++depth)
         {
-            uint32_t *cnt_in = t->counters + a, *cnt_out = t->counters + (1 - a), *cnt_s = t->counters + 2;
+            uint32_t *cnt_in = queues + 3 * depth, *cnt_s = cnt_in + 1, *cnt_out = cnt_in + 3;
+            const light_queue lq{t->l_ray, t->l_pid, t->l_contrib, lit ? cnt_in + 2 : nullptr};
             if(empty)
                 k_fill_miss_queue<<<grid, PT_THREADS, 0, st>>>(cnt_in, t->hits);
             else if(tl_persistent)
@@ -1402,7 +1402,7 @@ vkg_status vkg_tracer_render(vkg_tracer *t, const vkg_scene *sc, const vkg_camer
                                 : shadow_group(k_pt_shadow_group<BIG, LEVELS_ONE>);
                 if(s_perm) bin_rays_done(ctx, st);
             }
-            if(cnt_l && !empty)
+            if(lit && !empty)
             {
                 auto light = [&](auto kern) { kern<<<grid, PT_THREADS, 0, st>>>(SS, lq, t->radiance, t->rng); };
                 constexpr int BIG = (int)TRAVERSAL_STACK;
@@ -1417,9 +1417,9 @@ vkg_status vkg_tracer_render(vkg_tracer *t, const vkg_scene *sc, const vkg_camer
                     small_stack ? light(k_pt_light_shadow<T1, 64, false, LEVELS_ONE>)
                                 : light(k_pt_light_shadow<T1, BIG, false, LEVELS_ONE>);
             }
-            k_pt_tally<<<1, 1, 0, st>>>(cnt_in, cnt_s, cnt_l, t->totals);
             a = 1 - a;
         }
+        k_pt_tally<<<1, 32, 0, st>>>(queues, depths, t->totals);
         if(cache_render)
         {
             if(vkg_status s = nrc::nrc_predict(t->cache, t->q_feat, n_render, cnt_q, t->q_x, t->q_y, st); s != VKG_OK)
@@ -1427,7 +1427,7 @@ vkg_status vkg_tracer_render(vkg_tracer *t, const vkg_scene *sc, const vkg_camer
             const uint32_t rg = (uint32_t)std::min<size_t>((n_render + 255) / 256, (size_t)ctx->num_sms * 8);
             k_cache_resolve<<<rg, 256, 0, st>>>(t->q_beta, t->q_y, cnt_q, t->radiance, t->totals);
         }
-        k_pt_accumulate<<<(npix + 255) / 256, 256, 0, st>>>(npix, ns, t->radiance, t->sum);
+        k_pt_accumulate<<<(npix + 255) / 256, 256, 0, st>>>(npix, ns, t->radiance, s0 == 0, t->sum);
         if(last && train_paths)
         {
             VKG_TRY_CUDA(ctx, cudaEventRecord(t->ev_train, st));
@@ -1454,8 +1454,8 @@ vkg_status vkg_tracer_render(vkg_tracer *t, const vkg_scene *sc, const vkg_camer
     }
     if(!train_paths) VKG_TRY_CUDA(ctx, cudaEventRecord(t->ev_train, st));
     t->trained = train_paths > 0;
-    k_pt_finalize<<<(3 * npix + 255) / 256, 256, 0, st>>>(npix, S.num_samples, t->batch, t->sum, t->accum, d_rgb_out);
-    k_pixel_radiance<<<(npix + 255) / 256, 256, 0, st>>>(t->accum, npix, t->gbuf);
+    k_pt_finalize<<<(3 * npix + 255) / 256, 256, 0, st>>>(npix, S.num_samples, t->batch, t->sum, t->accum, d_rgb_out,
+                                                         t->gbuf);
     if(S.denoising && d_rgb_out)
         if(vkg_status s = denoise_run(ctx, t->gbuf, cw, ch, nullptr, d_rgb_out, nullptr, st); s != VKG_OK) return s;
     VKG_TRY_CUDA(ctx, cudaEventRecord(t->ev1, st));

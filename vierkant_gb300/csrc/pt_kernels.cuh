@@ -309,6 +309,14 @@ __device__ __forceinline__ void camera_ray(const vkg_camera &c, uint32_t x, uint
     o[1] = make_float4(fmul(d[0], inv), fmul(d[1], inv), fmul(d[2], inv), PT_TMAX);
 }
 
+// queue lengths of a wave: of bounce d the rays at 3 d, the shadow rays at 3 d + 1, the light-shadow rays at
+// 3 d + 2. Each bounce has its own, so that a wave is cleared and tallied once
+constexpr uint32_t PT_MAX_DEPTH = 64, PT_QUEUE_COUNTS = 3 * (PT_MAX_DEPTH + 1);
+__device__ __forceinline__ void start_queues(uint32_t *counts, uint32_t n) // one block
+{
+    for(uint32_t i = threadIdx.x; i < PT_QUEUE_COUNTS; i += blockDim.x) counts[i] = i == 0 ? n : 0u;
+}
+
 __global__ void __launch_bounds__(PT_THREADS)
         k_pt_generate(pt_params P, uint32_t n, vkg_ray *__restrict__ q_ray, uint32_t *__restrict__ q_pid,
                       uint64_t *__restrict__ rng, float4 *__restrict__ beta_pdf, float4 *__restrict__ radiance,
@@ -378,11 +386,7 @@ __global__ void __launch_bounds__(PT_THREADS)
         if(P.mstack)
             P.mstack[p] = P.cam_medium != 0xFFFFFFFFu ? make_uint4(1u, P.cam_medium, 0u, 0u) : make_uint4(0u, 0u, 0u, 0u);
     }
-    if(blockIdx.x == 0 && threadIdx.x == 0)
-    {
-        counters[0] = n;
-        counters[1] = counters[2] = counters[7] = 0; // the other queue, the shadow and the light-shadow queue
-    }
+    if(blockIdx.x == 0) start_queues(counters, n);
 }
 
 // The levels of a scene's BVH that a tracer is compiled for: one that holds both traversals spills in
@@ -1744,14 +1748,25 @@ __global__ void k_fill_miss_queue(const uint32_t *__restrict__ count, vkg_hit *_
         reinterpret_cast<uint4 *>(hits)[i] = make_uint4(VKG_MISS, 0u, 0u, 0u);
 }
 
-// a bounce's rays into the totals; its queues start the next one empty
-__global__ void k_pt_tally(uint32_t *__restrict__ ext_count, uint32_t *__restrict__ s_count,
-                           uint32_t *__restrict__ l_count, unsigned long long *__restrict__ totals)
+// a wave's rays into the totals (one warp)
+__global__ void k_pt_tally(const uint32_t *__restrict__ counts, uint32_t depths, unsigned long long *__restrict__ totals)
 {
-    totals[0] += *ext_count;
-    totals[1] += *s_count + (l_count ? *l_count : 0u);
-    *ext_count = *s_count = 0;
-    if(l_count) *l_count = 0;
+    unsigned long long rays = 0, shadow = 0;
+    for(uint32_t d = threadIdx.x; d < depths; d += 32)
+    {
+        rays += counts[3 * d];
+        shadow += counts[3 * d + 1] + counts[3 * d + 2];
+    }
+    for(int o = 16; o; o >>= 1)
+    {
+        rays += __shfl_xor_sync(0xffffffffu, rays, o);
+        shadow += __shfl_xor_sync(0xffffffffu, shadow, o);
+    }
+    if(threadIdx.x == 0)
+    {
+        totals[0] += rays;
+        totals[1] += shadow;
+    }
 }
 
 // rendering with a cache: path radiance += throughput x prediction (negative outputs clamped)
@@ -1821,11 +1836,19 @@ __global__ void k_cache_window(const uint32_t *__restrict__ t_count, uint32_t k,
     *b_count = cnt > lo ? (uint32_t)std::min<uint64_t>(cnt - lo, B) : 0u;
 }
 
-__global__ void k_pt_accumulate(uint32_t npix, uint32_t ns, const float4 *__restrict__ radiance, float *__restrict__ sum)
+// sum of a wave's samples per pixel, after those of the waves before it
+__global__ void k_pt_accumulate(uint32_t npix, uint32_t ns, const float4 *__restrict__ radiance, bool first,
+                                float *__restrict__ sum)
 {
     uint32_t pix = blockIdx.x * blockDim.x + threadIdx.x;
     if(pix >= npix) return;
-    float sx = sum[3 * (size_t)pix], sy = sum[3 * (size_t)pix + 1], sz = sum[3 * (size_t)pix + 2];
+    float sx = 0.f, sy = 0.f, sz = 0.f;
+    if(!first)
+    {
+        sx = sum[3 * (size_t)pix];
+        sy = sum[3 * (size_t)pix + 1];
+        sz = sum[3 * (size_t)pix + 2];
+    }
     for(uint32_t k = 0; k < ns; ++k)
     {
         const float4 L = radiance[(size_t)k * npix + pix];
@@ -1838,8 +1861,9 @@ __global__ void k_pt_accumulate(uint32_t npix, uint32_t ns, const float4 *__rest
     sum[3 * (size_t)pix + 2] = sz;
 }
 
+// the batch's mean into the accumulation, the output and the pixel records
 __global__ void k_pt_finalize(uint32_t npix, uint32_t spp, uint32_t batch, const float *__restrict__ sum,
-                              float *__restrict__ accum, float *__restrict__ out)
+                              float *__restrict__ accum, float *__restrict__ out, vkg_pixel_data *__restrict__ px)
 {
     uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
     if(k >= 3 * npix) return;
@@ -1847,16 +1871,7 @@ __global__ void k_pt_finalize(uint32_t npix, uint32_t spp, uint32_t batch, const
     const float a = batch == 0 ? mean : (mean + (float)batch * accum[k]) / (float)(batch + 1);
     accum[k] = a;
     if(out) out[k] = a;
-}
-
-// the accumulated radiance into the pixel records
-__global__ void k_pixel_radiance(const float *__restrict__ accum, uint32_t npix, vkg_pixel_data *__restrict__ px)
-{
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if(i >= npix) return;
-    px[i].radiance[0] = accum[3 * (size_t)i];
-    px[i].radiance[1] = accum[3 * (size_t)i + 1];
-    px[i].radiance[2] = accum[3 * (size_t)i + 2];
+    px[k / 3].radiance[k % 3] = a;
 }
 
 __global__ void k_tri_flags(tri_rec *__restrict__ tris, uint32_t n, const uint32_t *__restrict__ tri_mat,
