@@ -339,10 +339,12 @@ enum
     VKG_RAY_COUNT_STATS = 2u,     /* also count node visits / triangle tests (slower; see vkg_ray_stats_get) */
     VKG_RAY_KEEP_ORDER = 4u       /* trace in the given order: no binning of large batches (below) */
 };
-/* Batches of 2^19 rays or more are traced in bins: rays are grouped by the cell of the scene box
- * (8 x 8 x 8) that holds their origin and by their direction (64 octahedral bins), and each group is
- * traced together; tiles of rays that are coherent already (most runs of 32 consecutive rays in one
- * bin, as camera rays are) keep their order. Results, counters and error flags are those of tracing
+/* Closest-hit batches of 2^19 rays or more, and any-hit batches of 3 * 2^19 or more, are traced in
+ * bins: rays are grouped by the cell of the scene box (8 x 8 x 8) that holds their origin and by their
+ * direction (64 octahedral bins), and each group is traced together; tiles of rays that are coherent
+ * already (most runs of 32 consecutive rays in one bin, as camera rays are) keep their order. Small
+ * batches (up to 65,536 rays, two-level ones up to 131,072) are traced by eight lanes per ray, unless
+ * node visits are counted. Results, counters and error flags are those of tracing
  * in the given order; only the speed differs. The context keeps the scratch (8 B per ray plus 128 KB
  * per SM-sized tile, grown on demand; calls on different streams are ordered by an event). Calls made
  * while the stream is being captured into a CUDA graph, calls with VKG_RAY_KEEP_ORDER, calls whose

@@ -817,11 +817,11 @@ vkg_status vkg_nrc_create(vkg_ctx *ctx, const vkg_nrc_config *cfg, vkg_nrc **out
     auto *c = new vkg_nrc();
     c->ctx = ctx;
     c->cfg = *cfg;
-    // default inference: the pipelined tcgen05 MLP after the shared encoding (2,073,600 queries: 1.152 ms,
-    // the mma.sync twin 1.138 ms; the encoding is ~85 % of either)
+    // default inference: the pipelined tcgen05 MLP after the shared encoding (2,073,600 queries: 0.642 ms,
+    // the mma.sync twin 0.671 ms; the encoding is ~60 % of either)
     c->tc_infer = cfg->infer_kernel ? cfg->infer_kernel : 2u;
-    // default: everything on tcgen05 (per 65,536-record step 0.479 ms, against 0.482 ms with the mma.sync
-    // forward / backward and 0.574 ms with the FP32 weight gradients)
+    // default: everything on tcgen05 (per 65,536-record step 0.228 ms, against 0.290 ms with the mma.sync
+    // forward / backward and 0.464 ms with the FP32 weight gradients)
     c->tc_train = cfg->train_kernel != 1;
     c->tc_forward = cfg->train_kernel == 3 || cfg->train_kernel == 0;
     c->gc.levels = cfg->levels;

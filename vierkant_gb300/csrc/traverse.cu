@@ -24,8 +24,13 @@ namespace
 constexpr int TRACE_THREADS = 128;
 
 // STACK: traversal stack entries; 64 serve BVHs up to 10 levels deep (7 (depth - 1) + 1 entries)
-template<bool ANY, bool STATS, int STACK>
-__global__ void __launch_bounds__(TRACE_THREADS, 9) // 56 registers, 24 bytes spilled: 1,398 -> 1,375 us
+// BLOCKS: resident blocks the kernel is compiled for. Nine take 56 registers with 24 bytes spilled: a large
+// closest-hit batch gains (3.7 M rays 1,398 -> 1,375 us, 340,054 rays 0.5 %), one whose blocks are all resident
+// at once anyway loses (147,768 rays 97.8 -> 101.7 us, 74,298 rays 53.8 -> 55.6); any-hit batches of these
+// sizes take the same time either way.
+constexpr uint32_t TRACE_FULL_MIN = 1u << 18;
+template<bool ANY, bool STATS, int STACK, int BLOCKS>
+__global__ void __launch_bounds__(TRACE_THREADS, BLOCKS)
         k_trace(const node8 *__restrict__ nodes, const tri_rec *__restrict__ tris, const vkg_ray *__restrict__ rays,
                 uint32_t n, vkg_hit *__restrict__ hits, uint32_t *__restrict__ occluded, int cull,
                 unsigned long long *__restrict__ counters, const uint32_t *__restrict__ perm,
@@ -192,12 +197,16 @@ void launch_simple(bool small_stack, uint32_t grid, cudaStream_t st, const vkg_b
                    uint32_t n, vkg_hit *hits, uint32_t *occ, int cull, unsigned long long *counters,
                    const uint32_t *perm, const uint32_t *reordered)
 {
-    if(small_stack)
-        k_trace<ANY, STATS, 64><<<grid, TRACE_THREADS, 0, st>>>(bvh->d_nodes, bvh->d_tris, rays, n, hits, occ, cull,
-                                                                counters, perm, reordered);
-    else
-        k_trace<ANY, STATS, (int)TRAVERSAL_STACK><<<grid, TRACE_THREADS, 0, st>>>(
-                bvh->d_nodes, bvh->d_tris, rays, n, hits, occ, cull, counters, perm, reordered);
+    auto go = [&](auto kern) {
+        kern<<<grid, TRACE_THREADS, 0, st>>>(bvh->d_nodes, bvh->d_tris, rays, n, hits, occ, cull, counters, perm, reordered);
+    };
+    if constexpr(!ANY)
+        if(n < TRACE_FULL_MIN)
+        {
+            small_stack ? go(k_trace<ANY, STATS, 64, 1>) : go(k_trace<ANY, STATS, (int)TRAVERSAL_STACK, 1>);
+            return;
+        }
+    small_stack ? go(k_trace<ANY, STATS, 64, 9>) : go(k_trace<ANY, STATS, (int)TRAVERSAL_STACK, 9>);
 }
 
 // ---- ray binning -------------------------------------------------------------------------------
