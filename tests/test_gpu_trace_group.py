@@ -81,3 +81,28 @@ def test_images_do_not_depend_on_the_wave(ctx, lit):
     assert torch.isfinite(images[0]).all() and float(images[0].mean()) > 0.01
     assert torch.equal(images[0], images[1]) and torch.equal(images[0], images[2])
     scene.close()
+
+
+@pytest.mark.parametrize("segments", [1, 6])
+def test_alpha_images_do_not_depend_on_the_wave(ctx, segments):
+    """masked and blended materials: groups trace waves of 8,643 and 259,290 paths, a thread per ray one of 553,152"""
+    sc = geometry.cornell_scene(11, 2, 16, 8)
+    scene = Scene(ctx, sc["xyz"], sc["indices"], sc["tri_material"], geometry.alpha_materials(sc["materials"]),
+                  torch.full((16, 32, 3), 0.7, device="cuda"))
+    uv, tangents = geometry.cornell_texcoords(sc)
+    scene.set_normals(geometry.cornell_vertex_normals(sc))
+    scene.set_texcoords(uv)
+    scene.set_tangents(tangents)
+    scene.set_textures(geometry.alpha_textures())
+    cam = geometry.camera_lookat((0, 0, 3.4), (0, 0, 0), (0, 1, 0), 45.0, 129, 67)
+    images = []
+    for per_wave in (1, 30, 64):
+        s = PBRPathTracer.default_settings()
+        s.num_samples, s.max_trace_depth, s.rr_start_depth, s.samples_per_wave = 64, segments, 2, per_wave
+        s.resolution[0], s.resolution[1] = 129, 67
+        pt = PBRPathTracer(ctx, seed=5, settings=s)
+        images.append(pt.render_scene(scene, cam).clone())
+        pt.close()
+    assert torch.isfinite(images[0]).all() and float(images[0].mean()) > 0.01
+    assert torch.equal(images[0], images[1]) and torch.equal(images[0], images[2])
+    scene.close()

@@ -1245,11 +1245,13 @@ vkg_status vkg_tracer_render(vkg_tracer *t, const vkg_scene *sc, const vkg_camer
         const single_scene SS{P};
         uint32_t *queues = t->counters + 8;
         // Short queues of scenes without alpha-tested materials are traced by groups of eight
-        // lanes (k_pt_extend_group). A wave of at most PT_GROUP_MAX_WAVE paths is always; a larger wave's
+        // lanes (k_pt_extend_group), those of single-level scenes with them in waves of the first kind below
+        // (six segments, 58,101 paths: 2,033 us a thread per ray, 643 us by groups; 232,404: 2,393 and 1,183). A wave of at most PT_GROUP_MAX_WAVE paths is always; a larger wave's
         // later queues may be short, which only the device knows: both kernels are launched from the
         // first bounce on (a binned queue is long), and the queue's count picks the one that runs.
-        const bool can_group = !alpha && !empty && !tl_persistent;
-        const bool groups = can_group && n <= PT_GROUP_MAX_WAVE;
+        const bool small_wave = n <= PT_GROUP_MAX_WAVE;
+        const bool can_group = !empty && !tl_persistent && (!alpha || (small_wave && !sc->tlas));
+        const bool groups = can_group && small_wave;
         const uint32_t group_grid = (uint32_t)std::min<size_t>(((size_t)n * GROUP_LANES + PT_THREADS - 1) / PT_THREADS,
                                                                (size_t)ctx->num_sms * 64);
         if(cache_render) VKG_TRY_CUDA(ctx, cudaMemsetAsync(cnt_q, 0, sizeof(uint32_t), st));
@@ -1289,7 +1291,7 @@ vkg_status vkg_tracer_render(vkg_tracer *t, const vkg_scene *sc, const vkg_camer
                                                       reordered, t->rng, depth, by_count ? PT_GROUP_MAX_QUEUE : 0u);
                 };
                 const extend_queue eq{t->q_ray[a], cnt_in, t->hits, t->hit_inst,
-                                      by_count ? PT_GROUP_MAX_QUEUE : 0xFFFFFFFFu, group_grid};
+                                      by_count ? PT_GROUP_MAX_QUEUE : 0xFFFFFFFFu, group_grid, t->q_pid[a], t->rng, depth};
                 auto extend_group = [&](auto kern) { kern<<<group_grid, PT_THREADS, 0, st>>>(SS, eq); };
                 constexpr int BIG = (int)TRAVERSAL_STACK;
                 using T1 = single_scene;
@@ -1297,7 +1299,7 @@ vkg_status vkg_tracer_render(vkg_tracer *t, const vkg_scene *sc, const vkg_camer
                     ; // traced with the last bounce's shadow rays
                 else if(sc->tlas && !groups)
                     alpha ? extend(k_pt_extend<T1, BIG, true, LEVELS_TWO>) : extend(k_pt_extend<T1, BIG, false, LEVELS_TWO>);
-                else if(alpha)
+                else if(alpha && !groups)
                     small_stack ? extend(k_pt_extend<T1, 64, true, LEVELS_ONE>)
                                 : extend(k_pt_extend<T1, BIG, true, LEVELS_ONE>);
                 else if(!groups)
@@ -1308,6 +1310,8 @@ vkg_status vkg_tracer_render(vkg_tracer *t, const vkg_scene *sc, const vkg_camer
                 else if((groups || by_count) && sc->tlas)
                     tl_small_stack ? extend_group(k_pt_extend_group<TL_GROUP_SMALL_STACK, LEVELS_TWO>)
                                    : extend_group(k_pt_extend_group<TL_GROUP_STACK, LEVELS_TWO>);
+                else if(groups && alpha)
+                    extend_group(k_pt_extend_group<BIG, LEVELS_ONE, true>);
                 else if(groups || by_count)
                     small_stack ? extend_group(k_pt_extend_group<64, LEVELS_ONE>)
                                 : extend_group(k_pt_extend_group<BIG, LEVELS_ONE>);
@@ -1363,12 +1367,12 @@ vkg_status vkg_tracer_render(vkg_tracer *t, const vkg_scene *sc, const vkg_camer
                                                       s_reordered, t->rng, by_count ? PT_GROUP_MAX_QUEUE : 0u);
                 };
                 const shadow_queue sq{t->s_ray, t->s_pid, t->s_contrib, cnt_s, t->radiance,
-                                      groups ? 0xFFFFFFFFu : (by_count ? PT_GROUP_MAX_QUEUE : 0u), group_grid};
+                                      groups ? 0xFFFFFFFFu : (by_count ? PT_GROUP_MAX_QUEUE : 0u), group_grid, t->rng};
                 auto shadow_group = [&](auto kern) { kern<<<group_grid, PT_THREADS, 0, st>>>(SS, sq); };
                 // with the next bounce's rays, unless those are traced in another way
                 paired = (groups || (can_group && depth > 0 && !bins_queue(depth + 1))) && depth + 1 < depths;
                 const extend_queue eq{t->q_ray[1 - a], cnt_out, t->hits, t->hit_inst,
-                                      groups ? 0xFFFFFFFFu : PT_GROUP_MAX_QUEUE, group_grid};
+                                      groups ? 0xFFFFFFFFu : PT_GROUP_MAX_QUEUE, group_grid, t->q_pid[1 - a], t->rng, depth + 1};
                 auto pair = [&](auto kern) { kern<<<2 * group_grid, PT_THREADS, 0, st>>>(SS, eq, sq); };
                 constexpr int BIG = (int)TRAVERSAL_STACK;
                 using T1 = single_scene;
@@ -1383,7 +1387,7 @@ vkg_status vkg_tracer_render(vkg_tracer *t, const vkg_scene *sc, const vkg_camer
                 }
                 else if(sc->tlas && !groups)
                     alpha ? shadow(k_pt_shadow<T1, BIG, true, LEVELS_TWO>) : shadow(k_pt_shadow<T1, BIG, false, LEVELS_TWO>);
-                else if(alpha)
+                else if(alpha && !groups)
                     small_stack ? shadow(k_pt_shadow<T1, 64, true, LEVELS_ONE>)
                                 : shadow(k_pt_shadow<T1, BIG, true, LEVELS_ONE>);
                 else if(!groups)
@@ -1392,11 +1396,15 @@ vkg_status vkg_tracer_render(vkg_tracer *t, const vkg_scene *sc, const vkg_camer
                 if(paired && sc->tlas)
                     tl_small_stack ? pair(k_pt_pair_group<TL_GROUP_SMALL_STACK, LEVELS_TWO>)
                                    : pair(k_pt_pair_group<TL_GROUP_STACK, LEVELS_TWO>);
+                else if(paired && alpha)
+                    pair(k_pt_pair_group<BIG, LEVELS_ONE, true>);
                 else if(paired)
                     small_stack ? pair(k_pt_pair_group<64, LEVELS_ONE>) : pair(k_pt_pair_group<BIG, LEVELS_ONE>);
                 else if((groups || by_count) && sc->tlas)
                     tl_small_stack ? shadow_group(k_pt_shadow_group<TL_GROUP_SMALL_STACK, LEVELS_TWO>)
                                    : shadow_group(k_pt_shadow_group<TL_GROUP_STACK, LEVELS_TWO>);
+                else if(groups && alpha)
+                    shadow_group(k_pt_shadow_group<BIG, LEVELS_ONE, true>);
                 else if(groups || by_count)
                     small_stack ? shadow_group(k_pt_shadow_group<64, LEVELS_ONE>)
                                 : shadow_group(k_pt_shadow_group<BIG, LEVELS_ONE>);

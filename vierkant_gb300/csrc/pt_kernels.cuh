@@ -462,7 +462,7 @@ __global__ void __launch_bounds__(PT_THREADS, min_blocks<STACK, ALPHA, LEVELS>)
 }
 
 // The same for short queues, eight lanes per ray (traverse_group.cuh, tlas_group.cuh); scenes without
-// alpha-tested materials, queues of at most `up_to` rays (k_pt_extend traces longer ones).
+// alpha-tested materials or of one level, queues of at most `up_to` rays (k_pt_extend traces longer ones).
 // The bounds: a 720p-like Cornell frame of one sample and six segments takes 542 against 1,065 us at 58,101
 // paths, 921 against 1,283 us at 256,000 with every queue traced by groups; at 516,000 the first two
 // queues are faster with a thread per ray and the later ones by groups (1,478 us; none 1,654, all 1,517).
@@ -475,19 +475,24 @@ struct extend_queue
     vkg_hit *hits;
     uint32_t *hit_inst;
     uint32_t up_to, blocks; // a longer queue is left to k_pt_extend
+    // scenes with alpha-tested materials
+    const uint32_t *pid;
+    const uint64_t *rng;
+    uint32_t depth;
 };
 template<int STACK>
 using group_stacks = uint2[PT_THREADS / GROUP_LANES][group_stack_entries<STACK>];
 
 // block `block` of q.blocks
-template<int STACK, int LEVELS>
-__device__ __forceinline__ void extend_group(const pt_params &P, const extend_queue &q, uint32_t block,
+template<int STACK, int LEVELS, bool ALPHA>
+__device__ __forceinline__ void extend_group(const single_scene &S, const extend_queue &q, uint32_t block,
                                              group_stacks<STACK> &stack)
 {
     constexpr uint32_t PER = PT_THREADS / GROUP_LANES;
     const vkg_ray *__restrict__ q_ray = q.ray;
     vkg_hit *__restrict__ hits = q.hits;
     uint32_t *__restrict__ hit_inst = q.hit_inst;
+    const pt_params &P = S.params(0u);
     const uint32_t n = *q.count, group = threadIdx.x / GROUP_LANES;
     if(n > q.up_to) return;
     for(uint32_t base = block * PER; base < n; base += q.blocks * PER)
@@ -508,9 +513,16 @@ __device__ __forceinline__ void extend_group(const pt_params &P, const extend_qu
             }
             else
             {
-                const trace_result r = trace_group<false, STACK>(active, P.nodes, P.tris, r0.x, r0.y, r0.z, r0.w, r1.x,
-                                                                 r1.y, r1.z, r1.w, CULL_BACK_UNLESS_TWOSIDED,
-                                                                 stack[group], nullptr);
+                using F = std::conditional_t<ALPHA, alpha_filter, no_filter>;
+                F f{};
+                if constexpr(ALPHA)
+                {
+                    const uint32_t pid = q.pid[active ? i : base];
+                    f = alpha_filter{&P, 0ull, peek_uniform(P, q.rng[pid], S.inc(pid), q.depth), 0u, false};
+                }
+                const trace_result r = trace_group<false, STACK, F>(active, P.nodes, P.tris, r0.x, r0.y, r0.z, r0.w,
+                                                                    r1.x, r1.y, r1.z, r1.w, CULL_BACK_UNLESS_TWOSIDED,
+                                                                    stack[group], nullptr, f);
                 return make_uint4(r.prim, __float_as_uint(r.t), __float_as_uint(r.u), __float_as_uint(r.v));
             }
         };
@@ -519,11 +531,11 @@ __device__ __forceinline__ void extend_group(const pt_params &P, const extend_qu
     }
 }
 
-template<int STACK, int LEVELS>
+template<int STACK, int LEVELS, bool ALPHA = false>
 __global__ void __launch_bounds__(PT_THREADS) k_pt_extend_group(single_scene S, extend_queue q)
 {
     __shared__ group_stacks<STACK> stack;
-    extend_group<STACK, LEVELS>(S.params(0u), q, blockIdx.x, stack);
+    extend_group<STACK, LEVELS, ALPHA>(S, q, blockIdx.x, stack);
 }
 
 // surface point, unit geometric normal (world space) and material of a hit: the triangle's vertices,
@@ -1382,9 +1394,10 @@ struct shadow_queue
     const uint32_t *count;
     float4 *radiance;
     uint32_t up_to, blocks;
+    const uint64_t *rng; // scenes with alpha-tested materials
 };
-template<int STACK, int LEVELS>
-__device__ __forceinline__ void shadow_group(const pt_params &P, const shadow_queue &q, uint32_t block,
+template<int STACK, int LEVELS, bool ALPHA>
+__device__ __forceinline__ void shadow_group(const single_scene &S, const shadow_queue &q, uint32_t block,
                                              group_stacks<STACK> &stack)
 {
     constexpr uint32_t PER = PT_THREADS / GROUP_LANES;
@@ -1392,6 +1405,7 @@ __device__ __forceinline__ void shadow_group(const pt_params &P, const shadow_qu
     const uint32_t *__restrict__ s_pid = q.pid;
     const float4 *__restrict__ s_contrib = q.contrib;
     float4 *__restrict__ radiance = q.radiance;
+    const pt_params &P = S.params(0u);
     const uint32_t n = *q.count, group = threadIdx.x / GROUP_LANES;
     if(n > q.up_to) return;
     for(uint32_t base = block * PER; base < n; base += q.blocks * PER)
@@ -1408,9 +1422,14 @@ __device__ __forceinline__ void shadow_group(const pt_params &P, const shadow_qu
                                                      r0.w, r1.x, r1.y, r1.z, r1.w, cull, stack[group])
                                .occluded;
         else
-            occluded = trace_group<true, STACK>(active, P.nodes, P.tris, r0.x, r0.y, r0.z, r0.w, r1.x, r1.y, r1.z, r1.w,
-                                                cull, stack[group], nullptr)
+        {
+            using F = std::conditional_t<ALPHA, alpha_filter, no_filter>;
+            F f{};
+            if constexpr(ALPHA) f = alpha_filter{&P, q.rng[s_pid[i]], 0.f, ALPHA_SALT_SHADOW, false};
+            occluded = trace_group<true, STACK, F>(active, P.nodes, P.tris, r0.x, r0.y, r0.z, r0.w, r1.x, r1.y, r1.z,
+                                                   r1.w, cull, stack[group], nullptr, f)
                                .occluded;
+        }
         if(active && !occluded && !(threadIdx.x & (GROUP_LANES - 1)))
         {
             const uint32_t pid = s_pid[i];
@@ -1423,22 +1442,22 @@ __device__ __forceinline__ void shadow_group(const pt_params &P, const shadow_qu
     }
 }
 
-template<int STACK, int LEVELS>
+template<int STACK, int LEVELS, bool ALPHA = false>
 __global__ void __launch_bounds__(PT_THREADS) k_pt_shadow_group(single_scene S, shadow_queue q)
 {
     __shared__ group_stacks<STACK> stack;
-    shadow_group<STACK, LEVELS>(S.params(0u), q, blockIdx.x, stack);
+    shadow_group<STACK, LEVELS, ALPHA>(S, q, blockIdx.x, stack);
 }
 
 // A bounce's shadow queue and the next bounce's ray queue in one launch: both come from the same shading pass
 // and neither reads what the other writes. Short queues are bound by the slowest rays of each launch, which
 // here run side by side: a frame of 58,101 paths and six segments 520 us with two launches, 412 us with one.
-template<int STACK, int LEVELS>
+template<int STACK, int LEVELS, bool ALPHA = false>
 __global__ void __launch_bounds__(PT_THREADS) k_pt_pair_group(single_scene S, extend_queue e, shadow_queue s)
 {
     __shared__ group_stacks<STACK> stack;
-    if(blockIdx.x < e.blocks) extend_group<STACK, LEVELS>(S.params(0u), e, blockIdx.x, stack);
-    else shadow_group<STACK, LEVELS>(S.params(0u), s, blockIdx.x - e.blocks, stack);
+    if(blockIdx.x < e.blocks) extend_group<STACK, LEVELS, ALPHA>(S, e, blockIdx.x, stack);
+    else shadow_group<STACK, LEVELS, ALPHA>(S, s, blockIdx.x - e.blocks, stack);
 }
 
 // the same for long queues, a thread per ray: queues of at most `up_to` rays are left to k_pt_pair_group. A binned

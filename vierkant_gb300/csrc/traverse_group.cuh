@@ -31,11 +31,13 @@ constexpr uint32_t GROUP_MAX_RAYS = 1u << 16;
 
 // All 32 lanes of a warp call this together; `active`, the ray and `st` are uniform over a group's
 // lanes. The result is uniform over the group.
-template<bool ANY, int STACK>
+// f: the candidate filter (no_filter, traverse.cuh); what it accepts does not depend on the order of the tests.
+template<bool ANY, int STACK, class F = no_filter>
 __device__ __forceinline__ trace_result trace_group(bool active, const node8 *__restrict__ nodes,
                                                     const tri_rec *__restrict__ tris, float ox, float oy, float oz,
                                                     float tmin, float dx, float dy, float dz, float tmax, int cull,
-                                                    uint2 *st, unsigned long long *__restrict__ counters)
+                                                    uint2 *st, unsigned long long *__restrict__ counters,
+                                                    const F &f = F())
 {
     constexpr uint32_t ALL = 0xffffffffu, GROUP = 0xFFu;
     const uint32_t lane = threadIdx.x & 31u, k = lane & 7u, g0 = lane & 24u;
@@ -103,6 +105,7 @@ __device__ __forceinline__ trace_result trace_group(bool active, const node8 *__
                 if(!(t > tmin && t < tmax)) return;
                 const uint32_t prim = __float_as_uint(c.y);
                 if(!ANY && !(t < ct || (t == ct && prim < cp))) return;
+                if(F::active && (__float_as_uint(c.z) & TRI_FLAG_ALPHA) && !f.accept(0u, prim, u, v)) return;
                 better = true;
                 ct = t;
                 cp = prim;
