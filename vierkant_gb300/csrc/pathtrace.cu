@@ -13,7 +13,9 @@
 //                 Queues are compacted with warp ballots (one atomic per warp).
 //   k_pt_shadow   any-hit visibility of the NEE rays (no culling, visibility_test.slang:45-87);
 //                 visible contributions are added to the path radiance
-// then k_pt_accumulate sums the wave's samples per pixel, and k_pt_finalize blends the batch into
+// A bounce's shadow rays and the next bounce's rays may share a launch (k_pt_pair, k_pt_pair_group): both come from
+// one shading pass, and neither writes what the other reads.
+// Then k_pt_accumulate sums the wave's samples per pixel, and k_pt_finalize blends the batch into
 // the running mean (raypipeline.slang:258-266). No host synchronisation inside a render: queue
 // lengths live in device memory and every queue kernel is a grid-stride loop over them.
 //

@@ -25,7 +25,7 @@ constexpr int TRACE_THREADS = 128;
 
 // STACK: traversal stack entries; 64 serve BVHs up to 10 levels deep (7 (depth - 1) + 1 entries)
 // BLOCKS: resident blocks the kernel is compiled for. Nine take 56 registers with 24 bytes spilled: a large
-// closest-hit batch gains (3.7 M rays 1,398 -> 1,375 us, 340,054 rays 0.5 %), one whose blocks are all resident
+// closest-hit batch gains (5.5 M rays 1,398 -> 1,375 us, 340,054 rays 0.5 %), one whose blocks are all resident
 // at once anyway loses (147,768 rays 97.8 -> 101.7 us, 74,298 rays 53.8 -> 55.6); any-hit batches of these
 // sizes take the same time either way.
 constexpr uint32_t TRACE_FULL_MIN = 1u << 18;
