@@ -317,8 +317,8 @@ def run_ours(args):
     e2e_ok = bool(torch.equal(dev_hits, hits_host))
     hits_digest = batch_digest(dev_hits.numpy())
 
-    # per call: five ray-binning kernels (batches of 2^19 rays or more) and the traversal kernel
-    launches_per_call = 6 if n >= BIN_MIN_RAYS else 1
+    # per call: four ray-binning kernels (batches of 2^19 rays or more) and the traversal kernel
+    launches_per_call = 5 if n >= BIN_MIN_RAYS else 1
     peak, peak_kind = measured_peaks()
     achieved = bytes_per_launch / (ms_step * 1e-3) / 1e9
     prof = profiled_counters()

@@ -36,8 +36,8 @@ struct vkg_ctx
     cudaEvent_t pipe_ev[7] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
     // ray-binning scratch of the bulk queries (calls on different streams are ordered by `done`). keys: bin | rank in its tile << 16 per ray; perm: traced position -> ray
     // index (its first half holds the 16-bit bins before that); tile_counts: rays per (tile, bin);
-    // bin_totals: rays per bin and the bins' first positions; done: recorded after the last use,
-    // waited for by the next
+    // bin_totals: first positions of runs of 32 bins and of the bins within them, the counters of the
+    // binning; done: recorded after the last use, waited for by the next
     struct ray_bins
     {
         uint32_t *keys = nullptr;

@@ -223,9 +223,9 @@ void launch_simple(bool small_stack, uint32_t grid, cudaStream_t st, const vkg_b
 //                  counters) and the tile's bin histogram -> M[t][bin]; a tile whose rays are
 //                  coherent already (most 32-ray steps in one bin: camera rays) keeps its order as
 //                  one run in an extra bin placed after all others
-//   k_bin_columns  per bin, M[.][bin] scanned over the tiles in place (exclusive); S[bin] = total
-//   k_bin_offsets  F = exclusive scan of S: the bins' first positions
-//   k_bin_place    perm[F[bin] + M[t][bin] + rank] = ray
+//   k_bin_columns  per bin, M[.][bin] scanned over the tiles in place (exclusive); F = exclusive scan of
+//                  the totals within a run of 32 bins, O of the runs' totals (by the last CTA to have its own)
+//   k_bin_place    perm[O[bin / 32] + F[bin] + M[t][bin] + rank] = ray
 constexpr int BIN_CELL_BITS = 3;                                            // per axis
 constexpr int BIN_DIR_BITS = 3;                                             // per octahedral axis
 constexpr uint32_t NUM_BINS = 1u << (3 * BIN_CELL_BITS + 2 * BIN_DIR_BITS); // 32,768
@@ -236,7 +236,7 @@ constexpr uint32_t BIN_MAX_TILE = 40u * BIN_THREADS;                        // r
 constexpr uint32_t KEEP_BIN = NUM_BINS;
 constexpr uint32_t BIN_SLOTS = NUM_BINS + 32;
 constexpr size_t BIN_SMEM = sizeof(uint32_t) * BIN_SLOTS;                    // 128 KB + 128 B
-static_assert(NUM_BINS == BIN_THREADS * 32, "32 bins per thread");
+static_assert(NUM_BINS == BIN_THREADS * 32, "k_bin_columns: a total per thread and that of the kept slots");
 static_assert(BIN_SLOTS <= 65536 && BIN_MAX_TILE <= 65536, "bin and rank are packed in 16 bits each");
 
 __device__ __forceinline__ uint32_t spread3(uint32_t v) { return (v & 1u) | ((v & 2u) << 2) | ((v & 4u) << 4); }
@@ -282,7 +282,8 @@ __global__ void __launch_bounds__(256)
                    float3 scale, uint16_t *__restrict__ bins, uint32_t *__restrict__ reordered)
 {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if(i == 0) *reordered = 0u; // k_bin_tiles counts the tiles that do not keep their order
+    // k_bin_tiles counts the tiles that do not keep their order, k_bin_columns its CTAs
+    if(i == 0) reordered[0] = reordered[1] = 0u;
     const uint32_t n = d_n ? min(*d_n, n_cap) : n_cap;
     if(i >= n) return;
     const float4 *rp = reinterpret_cast<const float4 *>(rays + i);
@@ -296,7 +297,7 @@ __global__ void __launch_bounds__(256)
                          float3 lo, float3 scale, uint16_t *__restrict__ bins, uint32_t *__restrict__ reordered)
 {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if(i == 0) *reordered = 0u;
+    if(i == 0) reordered[0] = reordered[1] = 0u;
     const uint32_t n = d_n ? min(*d_n, n_cap) : n_cap;
     if(i >= n) return;
     const float *p = pts + (size_t)stride * i;
@@ -417,13 +418,16 @@ __global__ void __launch_bounds__(BIN_THREADS)
 }
 
 // CTA = 32 bins (lanes) x 32 chunks of consecutive tiles (warps): chunk sums, their scan per bin in
-// shared memory, then the chunk's entries rewritten as the bin's running count before the tile
+// shared memory, then the chunk's entries rewritten as the bin's running count before the tile. The CTA
+// that is the last to publish its bins' total scans the totals (a launch of one CTA for that took 10 us)
 __global__ void __launch_bounds__(1024)
-        k_bin_columns(uint32_t *__restrict__ M, uint32_t tiles, uint32_t *__restrict__ S,
-                      const uint32_t *__restrict__ reordered)
+        k_bin_columns(uint32_t *__restrict__ M, uint32_t tiles, uint32_t *__restrict__ F, uint32_t *__restrict__ O,
+                      uint32_t *__restrict__ reordered)
 {
     if(*reordered == 0u) return; // every tile keeps its order: the batch is traced as given
     __shared__ uint32_t part[32][33];
+    __shared__ uint32_t warp_sum[32];
+    __shared__ bool last;
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     const uint32_t b = blockIdx.x * 32u + lane;
     const uint32_t per = (tiles + 31u) / 32u;
@@ -441,7 +445,19 @@ __global__ void __launch_bounds__(1024)
             part[w][lane] = run;
             run += c;
         }
-        S[b] = run;
+        uint32_t x = run;
+        for(int o = 1; o < 32; o <<= 1)
+        {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+            if(lane >= (uint32_t)o) x += y;
+        }
+        F[b] = x - run;
+        if(lane == 31)
+        {
+            __stcg(O + blockIdx.x, x);
+            __threadfence();
+            last = atomicAdd(reordered + 1, 1u) == gridDim.x - 1;
+        }
     }
     __syncthreads();
     uint32_t run = part[warp][lane];
@@ -452,23 +468,10 @@ __global__ void __launch_bounds__(1024)
         *p = run;
         run += c;
     }
-}
-
-// F = exclusive scan of S, one CTA: S staged in shared memory (a pad word after every 32 keeps the
-// per-thread runs of 32 consecutive bins free of bank conflicts), 32 bins per thread
-constexpr size_t BIN_SCAN_SMEM = sizeof(uint32_t) * (NUM_BINS + NUM_BINS / 32);
-__global__ void __launch_bounds__(BIN_THREADS)
-        k_bin_offsets(const uint32_t *__restrict__ S, uint32_t *__restrict__ F, const uint32_t *__restrict__ reordered)
-{
-    if(*reordered == 0u) return;
-    extern __shared__ uint32_t sm[];
-    __shared__ uint32_t warp_sum[32];
-    const uint32_t t = threadIdx.x, lane = t & 31u, warp = t >> 5;
-    for(uint32_t b = t; b < NUM_BINS; b += BIN_THREADS) sm[b + (b >> 5)] = __ldg(S + b);
-    __syncthreads();
-    uint32_t *mine = sm + t * 33u; // bins t*32 .. t*32+31
-    uint32_t total = 0;
-    for(int k = 0; k < 32; ++k) total += mine[k];
+    if(!last) return;
+    // exclusive scan of the runs' totals, one a thread; the slots of kept rays follow all bins
+    __threadfence();
+    const uint32_t total = __ldcg(O + threadIdx.x);
     uint32_t x = total;
     for(int o = 1; o < 32; o <<= 1)
     {
@@ -477,32 +480,15 @@ __global__ void __launch_bounds__(BIN_THREADS)
     }
     if(lane == 31) warp_sum[warp] = x;
     __syncthreads();
-    if(warp == 0)
-    {
-        uint32_t w = warp_sum[lane];
-        for(int o = 1; o < 32; o <<= 1)
-        {
-            const uint32_t y = __shfl_up_sync(0xffffffffu, w, o);
-            if(lane >= (uint32_t)o) w += y;
-        }
-        warp_sum[lane] = w;
-    }
-    __syncthreads();
-    uint32_t acc = (warp ? warp_sum[warp - 1] : 0u) + x - total;
-    for(int k = 0; k < 32; ++k)
-    {
-        const uint32_t c = mine[k];
-        mine[k] = acc;
-        acc += c;
-    }
-    __syncthreads();
-    for(uint32_t b = t; b < NUM_BINS; b += BIN_THREADS) F[b] = sm[b + (b >> 5)];
-    if(t == BIN_THREADS - 1) F[KEEP_BIN] = acc; // the kept rays follow all bins
+    for(uint32_t w = 0; w < warp; ++w) x += warp_sum[w];
+    O[threadIdx.x] = x - total;
+    if(threadIdx.x == 1023) O[1024] = x;
 }
 
 __global__ void __launch_bounds__(256)
         k_bin_place(const uint32_t *__restrict__ keys, uint32_t n_cap, const uint32_t *__restrict__ d_n, uint32_t tile,
-                    const uint32_t *__restrict__ M, const uint32_t *__restrict__ F, uint32_t *__restrict__ perm,
+                    const uint32_t *__restrict__ M, const uint32_t *__restrict__ F, const uint32_t *__restrict__ O,
+                    uint32_t *__restrict__ perm,
                     const uint32_t *__restrict__ reordered)
 {
     if(*reordered == 0u) return;
@@ -510,7 +496,7 @@ __global__ void __launch_bounds__(256)
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if(i >= n) return;
     const uint32_t k = keys[i], bin = k & 0xFFFFu, t = i / tile;
-    perm[__ldg(F + bin) + M[(size_t)t * BIN_SLOTS + bin] + (k >> 16)] = i;
+    perm[__ldg(O + (bin >> 5)) + __ldg(F + bin) + M[(size_t)t * BIN_SLOTS + bin] + (k >> 16)] = i;
 }
 
 
@@ -607,9 +593,7 @@ const uint32_t *bin_order(vkg_ctx *ctx, uint32_t n, const uint32_t *d_n, cudaStr
     const uint64_t dev_bit = 1ull << (ctx->device & 63);
     if(!(smem_set & dev_bit))
     {
-        if(cudaFuncSetAttribute(k_bin_tiles, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)BIN_SMEM) != cudaSuccess ||
-           cudaFuncSetAttribute(k_bin_offsets, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)BIN_SCAN_SMEM) !=
-                   cudaSuccess)
+        if(cudaFuncSetAttribute(k_bin_tiles, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)BIN_SMEM) != cudaSuccess)
         {
             cudaGetLastError();
             return nullptr;
@@ -642,11 +626,11 @@ const uint32_t *bin_order(vkg_ctx *ctx, uint32_t n, const uint32_t *d_n, cudaStr
         cudaFree(b.tile_counts);
         cudaFree(b.bin_totals);
         b = vkg_ctx::ray_bins{nullptr, nullptr, nullptr, nullptr, 0, 0, b.done};
-        // bin_totals: S, F, the count of reordered tiles
+        // bin_totals: O, F, the count of reordered tiles, the CTAs of k_bin_columns that are done
         if(cudaMalloc(&b.keys, sizeof(uint32_t) * (size_t)n) != cudaSuccess ||
            cudaMalloc(&b.perm, sizeof(uint32_t) * (size_t)n) != cudaSuccess ||
            cudaMalloc(&b.tile_counts, sizeof(uint32_t) * (size_t)BIN_SLOTS * tiles) != cudaSuccess ||
-           cudaMalloc(&b.bin_totals, sizeof(uint32_t) * (2 * (size_t)BIN_SLOTS + 1)) != cudaSuccess)
+           cudaMalloc(&b.bin_totals, sizeof(uint32_t) * (2 * (size_t)BIN_SLOTS + 2)) != cudaSuccess)
         {
             cudaFree(b.keys);
             cudaFree(b.perm);
@@ -659,16 +643,15 @@ const uint32_t *bin_order(vkg_ctx *ctx, uint32_t n, const uint32_t *d_n, cudaStr
         b.cap = n;
         b.tiles_cap = tiles;
     }
-    uint32_t *S = b.bin_totals, *F = b.bin_totals + BIN_SLOTS;
+    uint32_t *O = b.bin_totals, *F = b.bin_totals + BIN_SLOTS;
     // the 16-bit bins live in the first half of perm's storage until k_bin_place overwrites it
     // (k_bin_tiles reads them before; k_bin_place reads only keys)
     uint16_t *bins16 = reinterpret_cast<uint16_t *>(b.perm);
     uint32_t *reordered = b.bin_totals + 2 * BIN_SLOTS;
     write_bins(bins16, reordered);
     k_bin_tiles<<<tiles, BIN_THREADS, BIN_SMEM, st>>>(bins16, n, d_n, tile, b.keys, b.tile_counts, reordered);
-    k_bin_columns<<<BIN_SLOTS / 32, 1024, 0, st>>>(b.tile_counts, tiles, S, reordered);
-    k_bin_offsets<<<1, BIN_THREADS, BIN_SCAN_SMEM, st>>>(S, F, reordered);
-    k_bin_place<<<(n + 255) / 256, 256, 0, st>>>(b.keys, n, d_n, tile, b.tile_counts, F, b.perm, reordered);
+    k_bin_columns<<<BIN_SLOTS / 32, 1024, 0, st>>>(b.tile_counts, tiles, F, O, reordered);
+    k_bin_place<<<(n + 255) / 256, 256, 0, st>>>(b.keys, n, d_n, tile, b.tile_counts, F, O, b.perm, reordered);
     *reordered_out = reordered;
     return b.perm;
 }
