@@ -59,7 +59,10 @@ __device__ __forceinline__ tlas_result trace_tlas_group(bool active, const node8
     {
         uint32_t ni = 0;    // the node, or the first instance of an opened leaf
         uint32_t boxes = 0; // instances of an opened leaf (at most 8); 0: a node
-        bool have = false;
+        // what goes back on the stack in the place of the popped entry. Lane 0 writes it after the vote below:
+        // until then the group's other lanes may still have to read that place
+        uint2 back = make_uint2(0u, 0u);
+        bool have = false, put = false;
         while(sp > 0 && !have)
         {
             const uint2 e = st[--sp];
@@ -87,8 +90,8 @@ __device__ __forceinline__ tlas_result trace_tlas_group(bool active, const node8
                 boxes = min(cnt, (uint32_t)GROUP_LANES);
                 if(cnt > GROUP_LANES) // the rest of a large leaf waits below
                 {
-                    if(k == 0) st[sp] = make_uint2(LEAF_BIT | ((cnt - GROUP_LANES - 1u) << 27) | (ni + GROUP_LANES), e.y);
-                    ++sp;
+                    back = make_uint2(LEAF_BIT | ((cnt - GROUP_LANES - 1u) << 27) | (ni + GROUP_LANES), e.y);
+                    put = true;
                 }
                 have = true;
                 continue;
@@ -104,12 +107,17 @@ __device__ __forceinline__ tlas_result trace_tlas_group(bool active, const node8
             tris = B.tris;
             cur_inst = meta.y;
             in_blas = true;
-            if(k == 0) st[sp] = make_uint2(TL_RETURN, __float_as_uint(tmin));
-            ++sp;
+            back = make_uint2(TL_RETURN, __float_as_uint(tmin));
+            put = true;
             ni = 0;
             have = true;
         }
         if(!__any_sync(ALL, have)) break;
+        if(put)
+        {
+            if(k == 0) st[sp] = back;
+            ++sp;
+        }
         float tn, tf;
         uint32_t word;
         bool hit;
