@@ -114,7 +114,9 @@ typedef struct vkg_ctx vkg_ctx;
 
 /* library version string, e.g. "vkg 0.1 sm_103a" */
 const char *vkg_version(void);
-/* create a context bound to CUDA device `device` */
+/* create a context bound to CUDA device `device`. Builds, vkg_denoise and vkg_post_fx take their memory from
+ * a pool of the context, which keeps up to 512 MiB of it between calls; destroying the context gives
+ * that back (trees built with the context stay valid) */
 vkg_status vkg_ctx_create(int device, vkg_ctx **out);
 vkg_status vkg_ctx_destroy(vkg_ctx *ctx);
 /* last error message of this context ("" if none); valid until the next call on ctx */
@@ -327,6 +329,8 @@ vkg_status vkg_bvh_info_get(const vkg_bvh *bvh, vkg_bvh_info *out);
 vkg_status vkg_bvh_build_noalloc(const float *d_xyz, uint32_t num_vertices, const uint32_t *d_indices,
                                  uint32_t num_tris, uint32_t leaf_max, void *d_nodes, uint32_t node_capacity,
                                  void *d_tris, uint32_t *d_info, void *stream);
+/* Waits for all work on the tree's device (a query may still read it on any stream), then frees it; not
+ * during a stream capture. ctx may be NULL. */
 vkg_status vkg_bvh_destroy(vkg_ctx *ctx, vkg_bvh *bvh);
 
 /* ---- bulk ray queries (replaces TraceRay / RayQuery, raypipeline.slang:182, visibility_test.slang:45-87)
@@ -397,6 +401,7 @@ typedef struct vkg_tlas_info
 vkg_status vkg_tlas_build(vkg_ctx *ctx, const vkg_bvh *const *blas, uint32_t num_blas, const vkg_instance *d_instances,
                           uint32_t num_instances, const vkg_bvh_build_options *opts, vkg_tlas **out, void *stream);
 vkg_status vkg_tlas_info_get(const vkg_tlas *tlas, vkg_tlas_info *out);
+/* waits as vkg_bvh_destroy does */
 vkg_status vkg_tlas_destroy(vkg_ctx *ctx, vkg_tlas *tlas);
 /* flags: VKG_RAY_CULL_BACK_FACES (object-space facing) */
 vkg_status vkg_tlas_closest_hit(vkg_ctx *ctx, const vkg_tlas *tlas, const vkg_ray *d_rays, uint32_t n,

@@ -972,6 +972,7 @@ extern "C" vkg_status vkg_bvh_build(vkg_ctx *ctx, const float *d_xyz, uint32_t n
 
     cudaStream_t st = static_cast<cudaStream_t>(stream_);
     auto *bvh = new vkg_bvh();
+    bvh->device = ctx->device;
     bvh->num_tris = num_tris;
     bvh->leaf_max = leaf_max;
     if(num_tris == 0)
@@ -1032,19 +1033,6 @@ extern "C" vkg_status vkg_bvh_info_get(const vkg_bvh *bvh, vkg_bvh_info *out)
     return VKG_OK;
 }
 
-extern "C" vkg_status vkg_bvh_destroy(vkg_ctx *ctx, vkg_bvh *bvh)
-{
-    if(!bvh) return VKG_OK;
-    if(ctx) bind_device(ctx);
-    cudaDeviceSynchronize(); // cudaFree does not wait for work that still reads stream-ordered memory
-    cudaFree(bvh->d_nodes);
-    cudaFree(bvh->d_tris);
-    cudaFree(bvh->d_morton);
-    cudaFree(bvh->d_sorted);
-    delete bvh;
-    return VKG_OK;
-}
-
 // ---- two-level BVH -----------------------------------------------------------------------------
 // The top level is the same 8-wide quantised BVH, built by the same core over the instances' world
 // boxes (the 8 transformed corners of the mesh's bounds, rounded outward); its leaves index
@@ -1070,6 +1058,7 @@ extern "C" vkg_status vkg_tlas_build(vkg_ctx *ctx, const vkg_bvh *const *blas, u
     if(vkg_status s = bind_device(ctx); s != VKG_OK) return s;
     cudaStream_t st = static_cast<cudaStream_t>(stream_);
     auto *t = new vkg_tlas();
+    t->top.device = ctx->device;
     t->num_instances = num_instances;
     t->num_blas = num_blas;
     t->top.leaf_max = leaf_max;
@@ -1165,22 +1154,6 @@ extern "C" vkg_status vkg_tlas_info_get(const vkg_tlas *t, vkg_tlas_info *out)
     out->d_instances = t->d_inst;
     out->d_instances_by_id = t->d_inst_by_id;
     out->build_ms = t->top.build_ms;
-    return VKG_OK;
-}
-
-extern "C" vkg_status vkg_tlas_destroy(vkg_ctx *ctx, vkg_tlas *t)
-{
-    if(!t) return VKG_OK;
-    if(ctx) bind_device(ctx);
-    cudaDeviceSynchronize(); // as in vkg_bvh_destroy
-    cudaFree(t->top.d_nodes);
-    cudaFree(t->top.d_morton);
-    cudaFree(t->top.d_sorted);
-    cudaFree(t->d_inst);
-    cudaFree(t->d_inst_by_id);
-    cudaFree(t->d_inst_box);
-    cudaFree(t->d_blas);
-    delete t;
     return VKG_OK;
 }
 

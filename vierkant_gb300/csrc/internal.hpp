@@ -52,6 +52,7 @@ struct vkg_ctx
 
 struct vkg_bvh
 {
+    int device = 0; // where its memory lies
     uint32_t num_tris = 0, num_nodes = 0, depth = 0, leaf_max = 4;
     float scene_min[3] = {0, 0, 0}, scene_max[3] = {0, 0, 0}, margin = 0.f;
     vkg::node8 *d_nodes = nullptr;
