@@ -26,6 +26,13 @@ vkg_status vkg_diag_tc_gemm(vkg_ctx *ctx, const uint16_t *d_a, const uint16_t *d
 vkg_status vkg_diag_wait_timeout(vkg_ctx *ctx, uint32_t num_ctas, uint64_t limit_ns, uint32_t *d_err,
                                  uint64_t *d_elapsed_ns, void *stream);
 
+/* the error path of a BVH build's grid barriers, run to its end: vkg_bvh_build (more than 2,048 triangles) whose
+ * barriers expect one block more than there are, with a limit of limit_ns (<= 1e8) instead of the builds'
+ * 4 s. Returns VKG_ERR_TIMEOUT once the first barrier has run out and every block has returned; nothing
+ * is kept. */
+vkg_status vkg_diag_build_timeout(vkg_ctx *ctx, const float *d_xyz, uint32_t num_vertices, const uint32_t *d_indices,
+                                  uint32_t num_tris, uint64_t limit_ns, void *stream);
+
 /* record the random numbers the tracer's kernels draw (d_buf NULL: stop). From the next render on,
  * the path of sample s through window pixel p writes record r = s * pixels + p of d_buf (floats):
  * [0..1] the camera jitter, then per segment i < max_segments the segment's uniforms at

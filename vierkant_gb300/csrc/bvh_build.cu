@@ -17,6 +17,7 @@
 // with 16-byte vector loads by the traversal kernels.
 #include "internal.hpp"
 #include "radix_sort.cuh"
+#include "tc.cuh"
 
 #include <algorithm>
 #include <cstring>
@@ -239,6 +240,15 @@ __global__ void k_refit(const uint32_t *__restrict__ lparent, const uint32_t *__
 }
 
 // ---- breadth-first collapse to 8-wide nodes (deterministic numbering) -----------------------------
+// how long a grid barrier waits for the other blocks (they are all resident, so it never runs out in a build);
+// `absent`: arrivals it expects beyond the grid's, which never come (vkg_diag_build_timeout)
+struct grid_wait
+{
+    uint64_t limit_ns = 4000000000ull;
+    uint32_t absent = 0;
+};
+constexpr uint32_t GRID_WAIT_TRIES = 1u << 26; // and at most so many looks
+
 struct collapse_args
 {
     const bvh2_node *tree;
@@ -251,6 +261,7 @@ struct collapse_args
     uint32_t *out_info;  // [0] num_nodes, [1] depth, [2] error flags, [3] grid barrier (zero at launch)
     uint32_t *block_sum; // [grid] children of a block's nodes in the current level
     float *out_margin;
+    grid_wait wait;
 };
 
 __device__ __forceinline__ uint32_t ref_count(const collapse_args &A, uint32_t r)
@@ -258,25 +269,34 @@ __device__ __forceinline__ uint32_t ref_count(const collapse_args &A, uint32_t r
     return (r & LEAF_BIT) ? 1u : A.tree[r].count;
 }
 
-// Grid barrier of a cooperative launch: arrival `target` = grid size x barriers so far. false when
-// the others did not arrive within the try limit (a few seconds), which it reports to them.
-__device__ bool grid_barrier(uint32_t *arrived, uint32_t target, uint32_t *err)
+// Grid barrier of a cooperative launch, the `barrier`-th of the kernel: every block adds one to *arrived. false
+// when the others did not arrive within the limit, which it reports to them.
+__device__ bool grid_barrier(uint32_t *arrived, uint32_t barrier, uint32_t *err, const grid_wait &wait)
 {
     __shared__ uint32_t s_ok;
     __syncthreads();
     if(threadIdx.x == 0)
     {
+        const uint32_t target = gridDim.x * barrier + wait.absent;
         s_ok = 1u;
         __threadfence();
         atomicAdd(arrived, 1u);
-        uint32_t tries = 0;
-        while(*reinterpret_cast<volatile uint32_t *>(arrived) < target)
-            if(++tries > (1u << 23) || (*reinterpret_cast<volatile uint32_t *>(err) & BUILD_ERR_WAIT))
+        uint64_t start = 0;
+        for(uint32_t tries = 0; *reinterpret_cast<volatile uint32_t *>(arrived) < target; ++tries)
+        {
+            // (the clock is read now and then: a look at the counter is what the barrier's latency consists of)
+            bool out = tries > GRID_WAIT_TRIES || (*reinterpret_cast<volatile uint32_t *>(err) & BUILD_ERR_WAIT);
+            if((tries & 255u) == 255u)
             {
-                atomicOr(err, BUILD_ERR_WAIT);
-                s_ok = 0u;
-                break;
+                const uint64_t now = tc::global_ns();
+                if(!start) start = now;
+                out = out || now - start > wait.limit_ns;
             }
+            if(!out) continue;
+            atomicOr(err, BUILD_ERR_WAIT);
+            s_ok = 0u;
+            break;
+        }
         __threadfence();
     }
     __syncthreads();
@@ -420,7 +440,7 @@ __global__ void __launch_bounds__(COLLAPSE_THREADS) k_topology(collapse_args A)
         if(gridDim.x > 1)
         {
             if(tid == 0) __stcg(&A.block_sum[blockIdx.x], carry);
-            if(!grid_barrier(&A.out_info[3], gridDim.x * ++barriers, &A.out_info[2])) return;
+            if(!grid_barrier(&A.out_info[3], ++barriers, &A.out_info[2], A.wait)) return;
             uint32_t b = 0, t = 0;
             for(uint32_t k = tid; k < gridDim.x; k += COLLAPSE_THREADS)
             {
@@ -455,7 +475,7 @@ __global__ void __launch_bounds__(COLLAPSE_THREADS) k_topology(collapse_args A)
         end += next;
         if(gridDim.x > 1 && begin < end)
         {
-            if(!grid_barrier(&A.out_info[3], gridDim.x * ++barriers, &A.out_info[2])) return;
+            if(!grid_barrier(&A.out_info[3], ++barriers, &A.out_info[2], A.wait)) return;
         }
         else
             __syncthreads();
@@ -834,7 +854,7 @@ cudaError_t launch_collapse(const collapse_args &A, uint32_t max_blocks, cudaStr
 // records in sorted order (lbox: the boxes in that order). On success bvh holds the nodes, Morton codes, sorted order, scene box, margin and depth, and
 // err_bits the error bits that make_boxes raised. The caller frees bvh on failure.
 template<class MakeBoxes, class MakeRecords>
-vkg_status build_core(vkg_ctx *ctx, vkg_bvh *bvh, uint32_t n, uint32_t leaf_max, cudaStream_t st,
+vkg_status build_core(vkg_ctx *ctx, vkg_bvh *bvh, uint32_t n, uint32_t leaf_max, const grid_wait &wait, cudaStream_t st,
                       MakeBoxes make_boxes, MakeRecords make_records, uint32_t &err_bits)
 {
     cudaEvent_t ev0, ev1;
@@ -905,7 +925,8 @@ vkg_status build_core(vkg_ctx *ctx, vkg_bvh *bvh, uint32_t n, uint32_t leaf_max,
         k_refit<<<g, T, 0, st>>>(lparent, iparent, tree, lbox, ibox, visits, n);
     }
     collapse_args A{tree,     first,     ibox,      lbox,      n,        leaf_max, capacity, small,
-                    node_ref, nodes_tmp, small + 8, block_sum, reinterpret_cast<float *>(small + 12)};
+                    node_ref, nodes_tmp, small + 8, block_sum, reinterpret_cast<float *>(small + 12),
+                    wait};
     chk(launch_collapse(A, (uint32_t)ctx->num_sms, st));
     make_records(static_cast<const uint32_t *>(vin), lbox, reinterpret_cast<const float *>(small + 12));
     chk(cudaGetLastError());
@@ -953,9 +974,9 @@ vkg_status build_core(vkg_ctx *ctx, vkg_bvh *bvh, uint32_t n, uint32_t leaf_max,
 
 using namespace vkg;
 
-extern "C" vkg_status vkg_bvh_build(vkg_ctx *ctx, const float *d_xyz, uint32_t num_vertices,
-                                    const uint32_t *d_indices, uint32_t num_tris, const vkg_bvh_build_options *opts,
-                                    vkg_bvh **out, void *stream_)
+static vkg_status bvh_build(vkg_ctx *ctx, const float *d_xyz, uint32_t num_vertices, const uint32_t *d_indices,
+                            uint32_t num_tris, const vkg_bvh_build_options *opts, const grid_wait &wait, vkg_bvh **out,
+                            void *stream_)
 {
     if(!ctx) return VKG_ERR_INVALID_ARGUMENT;
     if(!out) return set_error(ctx, VKG_ERR_INVALID_ARGUMENT, "vkg_bvh_build: out is NULL");
@@ -990,7 +1011,7 @@ extern "C" vkg_status vkg_bvh_build(vkg_ctx *ctx, const float *d_xyz, uint32_t n
     const uint32_t g = (n + T - 1) / T;
     uint32_t err_bits = 0;
     vkg_status s = build_core(
-            ctx, bvh, n, leaf_max, st,
+            ctx, bvh, n, leaf_max, wait, st,
             [&](box6 *tbox, uint32_t *scene_enc, uint32_t *err) {
                 k_tri_boxes<<<g, T, 0, st>>>(d_xyz, num_vertices, d_indices, n, tbox, scene_enc, err);
             },
@@ -1008,6 +1029,27 @@ extern "C" vkg_status vkg_bvh_build(vkg_ctx *ctx, const float *d_xyz, uint32_t n
     bvh->bytes = sizeof(node8) * bvh->num_nodes + sizeof(tri_rec) * n + 8 * (size_t)n;
     *out = bvh;
     return VKG_OK;
+}
+
+extern "C" vkg_status vkg_bvh_build(vkg_ctx *ctx, const float *d_xyz, uint32_t num_vertices,
+                                    const uint32_t *d_indices, uint32_t num_tris, const vkg_bvh_build_options *opts,
+                                    vkg_bvh **out, void *stream)
+{
+    return bvh_build(ctx, d_xyz, num_vertices, d_indices, num_tris, opts, grid_wait{}, out, stream);
+}
+
+extern "C" vkg_status vkg_diag_build_timeout(vkg_ctx *ctx, const float *d_xyz, uint32_t num_vertices,
+                                             const uint32_t *d_indices, uint32_t num_tris, uint64_t limit_ns,
+                                             void *stream)
+{
+    if(!ctx) return VKG_ERR_INVALID_ARGUMENT;
+    if(num_tris <= COLLAPSE_PRIMS_PER_BLOCK || limit_ns == 0 || limit_ns > 100000000ull)
+        return set_error(ctx, VKG_ERR_INVALID_ARGUMENT, "vkg_diag_build_timeout: need more than %u triangles and 0 < limit_ns <= 1e8",
+                         COLLAPSE_PRIMS_PER_BLOCK);
+    vkg_bvh *bvh = nullptr;
+    const vkg_status s = bvh_build(ctx, d_xyz, num_vertices, d_indices, num_tris, nullptr, grid_wait{limit_ns, 1u}, &bvh, stream);
+    vkg_bvh_destroy(ctx, bvh);
+    return s;
 }
 
 extern "C" vkg_status vkg_bvh_info_get(const vkg_bvh *bvh, vkg_bvh_info *out)
@@ -1110,7 +1152,7 @@ extern "C" vkg_status vkg_tlas_build(vkg_ctx *ctx, const vkg_bvh *const *blas, u
     const uint32_t g = (n + T - 1) / T;
     uint32_t err_bits = 0;
     vkg_status s = build_core(
-            ctx, &t->top, n, leaf_max, st,
+            ctx, &t->top, n, leaf_max, grid_wait{}, st,
             [&](box6 *tbox, uint32_t *scene_enc, uint32_t *err) {
                 k_instance_boxes<<<(n + 7) / 8, 256, 0, st>>>(d_instances, n, d_bb, num_blas, tbox, scene_enc, err);
             },
@@ -1270,7 +1312,8 @@ extern "C" vkg_status vkg_bvh_build_noalloc(const float *d_xyz, uint32_t num_ver
     }
     const uint32_t capacity = std::min<uint32_t>(node_capacity, NOALLOC_MAX_TRIS + 8);
     collapse_args A{s->tree, s->first, s->ibox, s->lbox, n, leaf_max, capacity, s->small, s->node_ref,
-                    static_cast<node8 *>(d_nodes), s->small + 8, nullptr, reinterpret_cast<float *>(s->small + 12)};
+                    static_cast<node8 *>(d_nodes), s->small + 8, nullptr, reinterpret_cast<float *>(s->small + 12),
+                    grid_wait{}};
     if(launch_collapse(A, 1, st) != cudaSuccess) return VKG_ERR_CUDA;
     k_tri_records<<<g, T, 0, st>>>(d_xyz, num_vertices, d_indices, vin, n, static_cast<tri_rec *>(d_tris));
     k_noalloc_info<<<1, 1, 0, st>>>(s, n, d_info);
