@@ -78,7 +78,8 @@ __global__ void __launch_bounds__(128, 6)
         k_dn_filter(const float4 *__restrict__ dm, const float4 *__restrict__ geo, const float4 *__restrict__ alb,
                     uint32_t w, uint32_t h, int step, float4 *__restrict__ out)
 {
-    const int x = blockIdx.x * blockDim.x + threadIdx.x, g = blockIdx.y * blockDim.y + threadIdx.y;
+    const int x = blockIdx.x * blockDim.x + threadIdx.x;
+    const int g = (blockIdx.z * gridDim.y + blockIdx.y) * blockDim.y + threadIdx.y; // (grids are 65,535 blocks high at most)
     const int y0 = g / step * (DN_ROWS * step) + g % step;
     if(x >= (int)w || y0 >= (int)h) return;
     const float color_phi = 1.f / .9f, normal_phi = 1.f / .3f, position_phi = 1.f;
@@ -171,7 +172,8 @@ vkg_status denoise_run(vkg_ctx *ctx, const vkg_pixel_data *px, uint32_t w, uint3
     for(int pass = 0; pass < 5; ++pass)
     {
         const uint32_t step = ATROUS_STEPS[pass], groups = (h + DN_ROWS * step - 1) / (DN_ROWS * step) * step;
-        const dim3 grid((w + blk.x - 1) / blk.x, (groups + blk.y - 1) / blk.y);
+        const uint32_t rows = (groups + blk.y - 1) / blk.y, layers = (rows + 65534u) / 65535u;
+        const dim3 grid((w + blk.x - 1) / blk.x, (rows + layers - 1) / layers, layers);
         if(pass + 1 < 5)
             k_dn_filter<false><<<grid, blk, 0, st>>>(ping, geo, alb, w, h, (int)step, pong);
         else
