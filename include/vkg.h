@@ -871,7 +871,8 @@ vkg_status vkg_nrc_config_default(vkg_nrc_config *out);
 vkg_status vkg_nrc_create(vkg_ctx *ctx, const vkg_nrc_config *cfg, vkg_nrc **out);
 vkg_status vkg_nrc_destroy(vkg_nrc *nrc);
 vkg_status vkg_nrc_info(const vkg_nrc *nrc, vkg_nrc_info_t *out);
-/* prediction for n feature records -> n x 3 fp32 */
+/* prediction for n feature records -> n x 3 fp32. The cache keeps scratch for its largest call (1.6 KB a record); a
+ * call of a new largest size allocates it, which waits for the device. */
 vkg_status vkg_nrc_infer(vkg_nrc *nrc, const float *d_features, uint32_t n, float *d_rgb, void *stream);
 /* accumulate the gradients of the relative-L2 loss against n x 3 targets (no parameter update) */
 vkg_status vkg_nrc_backward(vkg_nrc *nrc, const float *d_features, const float *d_targets, uint32_t n, void *stream);

@@ -96,11 +96,7 @@ vkg_status vkg_ctx_destroy(vkg_ctx *ctx)
         if(s) cudaStreamDestroy(s);
     for(cudaEvent_t e: ctx->pipe_ev)
         if(e) cudaEventDestroy(e);
-    cudaFree(ctx->bins.keys);
-    cudaFree(ctx->bins.perm);
-    cudaFree(ctx->bins.tile_counts);
-    cudaFree(ctx->bins.bin_totals);
-    if(ctx->bins.done) cudaEventDestroy(ctx->bins.done);
+    ctx->bins.release();
     if(ctx->pool) cudaMemPoolDestroy(ctx->pool); // (memory still allocated from it stays valid until freed)
     delete ctx;
     return VKG_OK;

@@ -3,8 +3,6 @@
 // waited for first. The tree knows its device: a call without a context may come with another one current.
 #include "internal.hpp"
 
-#include <initializer_list>
-
 namespace
 {
 

@@ -9,7 +9,42 @@
 
 #include <cstdarg>
 #include <cstdio>
+#include <initializer_list>
 #include <string>
+
+namespace vkg
+{
+// Scratch of the binnings (traverse.cu): the context's, grown on demand, whose uses on different streams are ordered
+// by an event; or a view of memory whose owner's calls follow one another anyway (bin_view, no event).
+// keys: bin | rank in its tile << 16 per element; perm: position -> element (its first half holds the
+// 16-bit bins before that); tile_counts: elements per (tile, bin); bin_totals: first positions of runs of
+// 32 bins and of the bins within them, the counters of the binning; done: recorded after the last use,
+// waited for by the next
+struct bin_scratch
+{
+    uint32_t *keys = nullptr;
+    uint32_t *perm = nullptr;
+    uint32_t *tile_counts = nullptr;
+    uint32_t *bin_totals = nullptr;
+    size_t cap = 0;
+    uint32_t tiles_cap = 0;
+    cudaEvent_t done = nullptr;
+    bool view = false;
+    void release_buffers() // cudaFree waits for the device, so nothing in flight still uses them
+    {
+        for(uint32_t *p: {keys, perm, tile_counts, bin_totals}) cudaFree(p);
+        keys = perm = tile_counts = bin_totals = nullptr;
+        cap = 0;
+        tiles_cap = 0;
+    }
+    void release()
+    {
+        release_buffers();
+        if(done) cudaEventDestroy(done);
+        done = nullptr;
+    }
+};
+}// namespace vkg
 
 struct vkg_ctx
 {
@@ -34,20 +69,7 @@ struct vkg_ctx
     // upload done, [6] a chunk's trace done
     cudaStream_t pipe[4] = {nullptr, nullptr, nullptr, nullptr};
     cudaEvent_t pipe_ev[7] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
-    // ray-binning scratch of the bulk queries (calls on different streams are ordered by `done`). keys: bin | rank in its tile << 16 per ray; perm: traced position -> ray
-    // index (its first half holds the 16-bit bins before that); tile_counts: rays per (tile, bin);
-    // bin_totals: first positions of runs of 32 bins and of the bins within them, the counters of the
-    // binning; done: recorded after the last use, waited for by the next
-    struct ray_bins
-    {
-        uint32_t *keys = nullptr;
-        uint32_t *perm = nullptr;
-        uint32_t *tile_counts = nullptr;
-        uint32_t *bin_totals = nullptr;
-        size_t cap = 0;
-        uint32_t tiles_cap = 0;
-        cudaEvent_t done = nullptr;
-    } bins;
+    vkg::bin_scratch bins; // of the ray queries and the path tracer
 };
 
 struct vkg_bvh
@@ -125,7 +147,7 @@ constexpr uint32_t TRAVERSAL_STACK = 128;
 // perm[position] = ray, valid when *reordered_out (a device word) is non-zero; otherwise the rays
 // are to be traced as given. Returns nullptr (trace as given) for VKG_RAY_KEEP_ORDER, batches below
 // min_rays, a stream being captured, or scratch that cannot be allocated. The scratch is the
-// context's; calls on different streams are ordered by an event recorded by bin_rays_done().
+// context's (ctx->bins); calls on different streams are ordered by an event recorded by bins_done().
 const uint32_t *bin_rays(vkg_ctx *ctx, const vkg_bvh *bvh, const vkg_ray *d_rays, uint32_t n, const uint32_t *d_n,
                          uint32_t flags, uint32_t min_rays, cudaStream_t st, const uint32_t **reordered_out);
 // Batches from which binning pays. The binning itself takes 40-90 us; a closest-hit traversal of incoherent
@@ -134,12 +156,17 @@ const uint32_t *bin_rays(vkg_ctx *ctx, const vkg_bvh *bvh, const vkg_ray *d_rays
 // 218 us, 1,200,000: 351 either way, 1,800,000: 551 -> 534 us).
 constexpr uint32_t BIN_MIN_CLOSEST = 1u << 19, BIN_MIN_ANY = 3u << 19;
 // the same for points (the first three floats of records of `stride` floats) over a 32^3 grid of the box
-// lo, 1 / scale: neighbouring positions of the order are neighbouring in space
-const uint32_t *bin_points(vkg_ctx *ctx, const float *d_points, uint32_t stride, uint32_t n, const uint32_t *d_n,
-                           const float lo[3], const float scale[3], uint32_t min_points, cudaStream_t st,
-                           const uint32_t **reordered_out);
+// lo, 1 / scale: neighbouring positions of the order are neighbouring in space; `bins` is the caller's scratch
+const uint32_t *bin_points(vkg_ctx *ctx, bin_scratch &bins, const float *d_points, uint32_t stride, uint32_t n,
+                           const uint32_t *d_n, const float lo[3], const float scale[3], uint32_t min_points,
+                           cudaStream_t st, const uint32_t **reordered_out);
 // after the launch that reads the order: the scratch may be reused once the stream reaches here
-inline void bin_rays_done(vkg_ctx *ctx, cudaStream_t st) { cudaEventRecord(ctx->bins.done, st); }
+inline void bins_done(const bin_scratch &bins, cudaStream_t st)
+{
+    if(!bins.view) cudaEventRecord(bins.done, st);
+}
+// scratch for n elements in `bytes` bytes at mem (256-byte aligned); of no use to bin_points if they are too few
+bin_scratch bin_view(const vkg_ctx *ctx, uint32_t n, void *mem, size_t bytes);
 }// namespace vkg
 
 #define VKG_TRY_CUDA(ctx, expr)                                                                                      \

@@ -682,16 +682,25 @@ vkg_status nrc_ensure(vkg_nrc *c, uint32_t n)
     return VKG_OK;
 }
 
-// n: capacity (host); d_n: optional device-side count (<= n) of the valid records
-vkg_status nrc_encode(vkg_nrc *c, const float *feats, uint32_t n, const uint32_t *d_n, uint32_t *X, cudaStream_t st)
+// n: capacity (host); d_n: optional device-side count (<= n) of the valid records; bins: scratch of the order
+vkg_status nrc_encode(vkg_nrc *c, const float *feats, uint32_t n, const uint32_t *d_n, uint32_t *X, bin_scratch &bins,
+                      cudaStream_t st)
 {
     if(n == 0) return VKG_OK;
     const uint32_t *reordered = nullptr;
-    const uint32_t *perm = bin_points(c->ctx, feats, FEAT, n, d_n, c->gc.smin, c->gc.sinv,
+    const uint32_t *perm = bin_points(c->ctx, bins, feats, FEAT, n, d_n, c->gc.smin, c->gc.sinv,
                                       ENC_BIN_MIN, st, &reordered);
     k_encode<<<(n + ENC_ROWS - 1) / ENC_ROWS, ENC_THREADS, 0, st>>>(feats, n, d_n, c->gc, c->grid_h, X, perm, reordered);
-    if(perm) bin_rays_done(c->ctx, st);
+    if(perm) bins_done(bins, st);
     return cuda_check(c->ctx, cudaGetLastError(), "k_encode");
+}
+
+// The cache's own calls order their records in the memory of H, which nrc_ensure sized for them and which holds
+// nothing until the forward pass that follows on the same stream: no memory of its own, and no scratch
+// shared with the context's ray queries, which may be under way on another stream.
+static bin_scratch own_bins(vkg_nrc *c, uint32_t n)
+{
+    return bin_view(c->ctx, n, c->H, (size_t)n * 160 * 4);
 }
 
 vkg_status nrc_forward(vkg_nrc *c, const uint32_t *X, uint32_t n, const uint32_t *d_n, float *Y, cudaStream_t st)
@@ -708,7 +717,8 @@ vkg_status nrc_backward(vkg_nrc *c, const float *feats, const float *targets, ui
 {
     if(n == 0) return VKG_OK;
     if(vkg_status s = nrc_ensure(c, n); s != VKG_OK) return s;
-    if(vkg_status s = nrc_encode(c, feats, n, d_n, c->X, st); s != VKG_OK) return s;
+    bin_scratch bins = own_bins(c, n);
+    if(vkg_status s = nrc_encode(c, feats, n, d_n, c->X, bins, st); s != VKG_OK) return s;
     // the training forward and backward: on tcgen05 (train_kernel 3), else the mma.sync twins
     if(c->tc_forward)
     {
@@ -748,16 +758,12 @@ vkg_status nrc_adam(vkg_nrc *c, const uint32_t *d_n, cudaStream_t st)
 
 const vkg_nrc_config &nrc_config(const vkg_nrc *c) { return c->cfg; }
 
-vkg_status nrc_predict(vkg_nrc *c, const float *feats, uint32_t n, const uint32_t *d_n, uint32_t *X, float *Y,
-                       cudaStream_t st)
+vkg_status nrc_predict(vkg_nrc *c, const float *feats, uint32_t n, const uint32_t *d_n, uint32_t *X, bin_scratch &bins,
+                       float *Y, cudaStream_t st)
 {
     if(c->tc_infer == 3) return nrc_infer_tc(c->ctx, c->gc, c->grid_h, c->wtc, feats, nullptr, n, d_n, Y, c->d_err, st);
-    if(c->tc_infer == 2)
-    {
-        if(vkg_status s = nrc_encode(c, feats, n, d_n, X, st); s != VKG_OK) return s;
-        return nrc_infer_tc(c->ctx, c->gc, c->grid_h, c->wtc, feats, X, n, d_n, Y, c->d_err, st);
-    }
-    if(vkg_status s = nrc_encode(c, feats, n, d_n, X, st); s != VKG_OK) return s;
+    if(vkg_status s = nrc_encode(c, feats, n, d_n, X, bins, st); s != VKG_OK) return s;
+    if(c->tc_infer == 2) return nrc_infer_tc(c->ctx, c->gc, c->grid_h, c->wtc, feats, X, n, d_n, Y, c->d_err, st);
     return nrc_forward(c, X, n, d_n, Y, st);
 }
 
@@ -940,7 +946,8 @@ vkg_status vkg_nrc_infer(vkg_nrc *c, const float *d_feats, uint32_t n, float *d_
     if(c->tc_infer == 3)
         return nrc_infer_tc(c->ctx, c->gc, c->grid_h, c->wtc, d_feats, nullptr, n, nullptr, d_rgb, c->d_err, st);
     if(vkg_status s = nrc_ensure(c, n); s != VKG_OK) return s;
-    if(vkg_status s = nrc_encode(c, d_feats, n, nullptr, c->X, st); s != VKG_OK) return s;
+    bin_scratch bins = own_bins(c, n);
+    if(vkg_status s = nrc_encode(c, d_feats, n, nullptr, c->X, bins, st); s != VKG_OK) return s;
     if(c->tc_infer == 2) return nrc_infer_tc(c->ctx, c->gc, c->grid_h, c->wtc, d_feats, c->X, n, nullptr, d_rgb, c->d_err, st);
     return nrc_forward(c, c->X, n, nullptr, d_rgb, st);
 }

@@ -80,9 +80,10 @@ __host__ __device__ inline uint32_t level_res(const grid_config &g, uint32_t l)
 const vkg_nrc_config &nrc_config(const vkg_nrc *c);
 // encoded inputs of n records: n x 40 u32 (80 BF16 values per record)
 constexpr size_t ENCODED_BYTES = IN * 2;
-// predictions (n x 3 fp32) for n feature records (n x FEAT fp32); X is caller-owned scratch of n x ENCODED_BYTES
-vkg_status nrc_predict(vkg_nrc *c, const float *feats, uint32_t n, const uint32_t *d_n, uint32_t *X, float *Y,
-                       cudaStream_t st);
+// predictions (n x 3 fp32) for n feature records (n x FEAT fp32); X is caller-owned scratch of n x ENCODED_BYTES, bins
+// the caller's scratch of the records' order
+vkg_status nrc_predict(vkg_nrc *c, const float *feats, uint32_t n, const uint32_t *d_n, uint32_t *X, bin_scratch &bins,
+                       float *Y, cudaStream_t st);
 // 16-byte group p of a record's `groups`, in an array stored by tiles of 128 records: a tile's records side by side
 __host__ __device__ constexpr size_t tiled_group(size_t record, uint32_t groups, uint32_t p)
 {

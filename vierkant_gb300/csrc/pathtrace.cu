@@ -1317,7 +1317,7 @@ vkg_status vkg_tracer_render(vkg_tracer *t, const vkg_scene *sc, const vkg_camer
                 else if(groups || by_count)
                     small_stack ? extend_group(k_pt_extend_group<64, LEVELS_ONE>)
                                 : extend_group(k_pt_extend_group<BIG, LEVELS_ONE>);
-                if(perm) bin_rays_done(ctx, st);
+                if(perm) bins_done(ctx->bins, st);
             }
             // the full material set: group the queue by material class first, so that warps shade
             // coherently (k_pt_bin_count / k_pt_bin_scatter, two light passes over the hits)
@@ -1410,7 +1410,7 @@ vkg_status vkg_tracer_render(vkg_tracer *t, const vkg_scene *sc, const vkg_camer
                 else if(groups || by_count)
                     small_stack ? shadow_group(k_pt_shadow_group<64, LEVELS_ONE>)
                                 : shadow_group(k_pt_shadow_group<BIG, LEVELS_ONE>);
-                if(s_perm) bin_rays_done(ctx, st);
+                if(s_perm) bins_done(ctx->bins, st);
             }
             if(lit && !empty)
             {
@@ -1432,7 +1432,7 @@ vkg_status vkg_tracer_render(vkg_tracer *t, const vkg_scene *sc, const vkg_camer
         k_pt_tally<<<1, 32, 0, st>>>(queues, depths, t->totals);
         if(cache_render)
         {
-            if(vkg_status s = nrc::nrc_predict(t->cache, t->q_feat, n_render, cnt_q, t->q_x, t->q_y, st); s != VKG_OK)
+            if(vkg_status s = nrc::nrc_predict(t->cache, t->q_feat, n_render, cnt_q, t->q_x, ctx->bins, t->q_y, st); s != VKG_OK)
                 return s;
             const uint32_t rg = (uint32_t)std::min<size_t>((n_render + 255) / 256, (size_t)ctx->num_sms * 8);
             k_cache_resolve<<<rg, 256, 0, st>>>(t->q_beta, t->q_y, cnt_q, t->radiance, t->totals);

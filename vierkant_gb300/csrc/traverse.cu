@@ -545,7 +545,7 @@ vkg_status launch_trace(vkg_ctx *ctx, const vkg_bvh *bvh, const vkg_ray *d_rays,
             if(stats) launch_persistent<false, true>(ctx, bvh, d_rays, n, d_hits, nullptr, cull, st, perm, reordered);
             else launch_persistent<false, false>(ctx, bvh, d_rays, n, d_hits, nullptr, cull, st, perm, reordered);
         }
-        if(perm) bin_rays_done(ctx, st);
+        if(perm) bins_done(ctx->bins, st);
         return cuda_check(ctx, cudaGetLastError(), "k_trace_persistent");
     }
     if(d_occ)
@@ -558,7 +558,7 @@ vkg_status launch_trace(vkg_ctx *ctx, const vkg_bvh *bvh, const vkg_ray *d_rays,
         if(stats) launch_simple<false, true>(small, grid, st, bvh, d_rays, n, d_hits, nullptr, cull, ctx->d_counters, perm, reordered);
         else launch_simple<false, false>(small, grid, st, bvh, d_rays, n, d_hits, nullptr, cull, ctx->d_counters, perm, reordered);
     }
-    if(perm) bin_rays_done(ctx, st);
+    if(perm) bins_done(ctx->bins, st);
     return cuda_check(ctx, cudaGetLastError(), "k_trace");
 }
 
@@ -576,10 +576,19 @@ vkg_status check_common(vkg_ctx *ctx, const vkg_bvh *bvh, const void *rays, cons
 
 namespace
 {
+// tiles of whole 1024-ray rounds: one per SM, or more of BIN_MAX_TILE rays each for larger batches
+uint32_t bin_tile(const vkg_ctx *ctx, uint32_t n)
+{
+    const size_t per_sm = ((size_t)n + (size_t)ctx->num_sms - 1) / (size_t)ctx->num_sms;
+    return (uint32_t)std::min<size_t>(BIN_MAX_TILE, (per_sm + BIN_THREADS - 1) / BIN_THREADS * BIN_THREADS);
+}
+// words of bin_totals: O, F, the count of reordered tiles, the CTAs of k_bin_columns that are done
+constexpr size_t BIN_TOTALS = 2 * (size_t)BIN_SLOTS + 2;
+
 // the order of n elements whose 16-bit bins write_bins(bins, reordered) computes on the stream
 template<class WriteBins>
-const uint32_t *bin_order(vkg_ctx *ctx, uint32_t n, const uint32_t *d_n, cudaStream_t st, const uint32_t **reordered_out,
-                          WriteBins write_bins)
+const uint32_t *bin_order(vkg_ctx *ctx, bin_scratch &b, uint32_t n, const uint32_t *d_n, cudaStream_t st,
+                          const uint32_t **reordered_out, WriteBins write_bins)
 {
     *reordered_out = nullptr;
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
@@ -600,43 +609,29 @@ const uint32_t *bin_order(vkg_ctx *ctx, uint32_t n, const uint32_t *d_n, cudaStr
         }
         smem_set |= dev_bit;
     }
-    // tiles of whole 1024-ray rounds: one per SM, or more of BIN_MAX_TILE rays each for larger batches
-    const size_t per_sm = ((size_t)n + (size_t)ctx->num_sms - 1) / (size_t)ctx->num_sms;
-    const uint32_t tile =
-            (uint32_t)std::min<size_t>(BIN_MAX_TILE, (per_sm + BIN_THREADS - 1) / BIN_THREADS * BIN_THREADS);
-    const uint32_t tiles = (uint32_t)(((size_t)n + tile - 1) / tile);
-    auto &b = ctx->bins;
-    if(!b.done && cudaEventCreateWithFlags(&b.done, cudaEventDisableTiming) != cudaSuccess)
+    const uint32_t tile = bin_tile(ctx, n), tiles = (uint32_t)(((size_t)n + tile - 1) / tile);
+    if(b.view && (b.cap < n || b.tiles_cap < tiles)) return nullptr;
+    if(!b.view && !b.done && cudaEventCreateWithFlags(&b.done, cudaEventDisableTiming) != cudaSuccess)
     {
         b.done = nullptr;
         cudaGetLastError();
         return nullptr;
     }
     // the previous call's kernels may still use the scratch (another stream)
-    if(cudaStreamWaitEvent(st, b.done, 0) != cudaSuccess)
+    if(!b.view && cudaStreamWaitEvent(st, b.done, 0) != cudaSuccess)
     {
         cudaGetLastError();
         return nullptr;
     }
     if(b.cap < n || b.tiles_cap < tiles)
     {
-        // cudaFree waits for the device, so nothing in flight still uses the old buffers
-        cudaFree(b.keys);
-        cudaFree(b.perm);
-        cudaFree(b.tile_counts);
-        cudaFree(b.bin_totals);
-        b = vkg_ctx::ray_bins{nullptr, nullptr, nullptr, nullptr, 0, 0, b.done};
-        // bin_totals: O, F, the count of reordered tiles, the CTAs of k_bin_columns that are done
+        b.release_buffers();
         if(cudaMalloc(&b.keys, sizeof(uint32_t) * (size_t)n) != cudaSuccess ||
            cudaMalloc(&b.perm, sizeof(uint32_t) * (size_t)n) != cudaSuccess ||
            cudaMalloc(&b.tile_counts, sizeof(uint32_t) * (size_t)BIN_SLOTS * tiles) != cudaSuccess ||
-           cudaMalloc(&b.bin_totals, sizeof(uint32_t) * (2 * (size_t)BIN_SLOTS + 2)) != cudaSuccess)
+           cudaMalloc(&b.bin_totals, sizeof(uint32_t) * BIN_TOTALS) != cudaSuccess)
         {
-            cudaFree(b.keys);
-            cudaFree(b.perm);
-            cudaFree(b.tile_counts);
-            cudaFree(b.bin_totals);
-            b = vkg_ctx::ray_bins{nullptr, nullptr, nullptr, nullptr, 0, 0, b.done};
+            b.release_buffers();
             cudaGetLastError();
             return nullptr;
         }
@@ -657,6 +652,27 @@ const uint32_t *bin_order(vkg_ctx *ctx, uint32_t n, const uint32_t *d_n, cudaStr
 }
 }// namespace
 
+bin_scratch bin_view(const vkg_ctx *ctx, uint32_t n, void *mem, size_t bytes)
+{
+    const uint32_t tile = bin_tile(ctx, n), tiles = (uint32_t)(((size_t)n + tile - 1) / tile);
+    size_t used = 0;
+    auto take = [&](size_t words) {
+        auto *p = reinterpret_cast<uint32_t *>(static_cast<char *>(mem) + used);
+        used += (words * sizeof(uint32_t) + 255) & ~size_t(255);
+        return p;
+    };
+    bin_scratch b;
+    b.view = true;
+    b.keys = take(n);
+    b.perm = take(n);
+    b.tile_counts = take((size_t)BIN_SLOTS * tiles);
+    b.bin_totals = take(BIN_TOTALS);
+    if(used > bytes) return bin_scratch{.view = true};
+    b.cap = n;
+    b.tiles_cap = tiles;
+    return b;
+}
+
 const uint32_t *bin_rays(vkg_ctx *ctx, const vkg_bvh *bvh, const vkg_ray *d_rays, uint32_t n, const uint32_t *d_n,
                          uint32_t flags, uint32_t min_rays, cudaStream_t st, const uint32_t **reordered_out)
 {
@@ -670,18 +686,18 @@ const uint32_t *bin_rays(vkg_ctx *ctx, const vkg_bvh *bvh, const vkg_ray *d_rays
         const float ext = bvh->scene_max[a] - bvh->scene_min[a];
         ps[a] = ext > 0.f ? (float)(1 << BIN_CELL_BITS) / ext : 0.f;
     }
-    return bin_order(ctx, n, d_n, st, reordered_out, [&](uint16_t *bins, uint32_t *reordered) {
+    return bin_order(ctx, ctx->bins, n, d_n, st, reordered_out, [&](uint16_t *bins, uint32_t *reordered) {
         k_bin_keys<<<(n + 255) / 256, 256, 0, st>>>(d_rays, n, d_n, lo, scale, bins, reordered);
     });
 }
 
-const uint32_t *bin_points(vkg_ctx *ctx, const float *d_points, uint32_t stride, uint32_t n, const uint32_t *d_n,
-                           const float lo[3], const float scale[3], uint32_t min_points, cudaStream_t st,
-                           const uint32_t **reordered_out)
+const uint32_t *bin_points(vkg_ctx *ctx, bin_scratch &scratch, const float *d_points, uint32_t stride, uint32_t n,
+                           const uint32_t *d_n, const float lo[3], const float scale[3], uint32_t min_points,
+                           cudaStream_t st, const uint32_t **reordered_out)
 {
     *reordered_out = nullptr;
     if(n < min_points) return nullptr;
-    return bin_order(ctx, n, d_n, st, reordered_out, [&](uint16_t *bins, uint32_t *reordered) {
+    return bin_order(ctx, scratch, n, d_n, st, reordered_out, [&](uint16_t *bins, uint32_t *reordered) {
         k_bin_point_keys<<<(n + 255) / 256, 256, 0, st>>>(d_points, stride, n, d_n, make_float3(lo[0], lo[1], lo[2]),
                                                           make_float3(scale[0], scale[1], scale[2]), bins, reordered);
     });
