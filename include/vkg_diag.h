@@ -33,6 +33,12 @@ vkg_status vkg_diag_wait_timeout(vkg_ctx *ctx, uint32_t num_ctas, uint64_t limit
 vkg_status vkg_diag_build_timeout(vkg_ctx *ctx, const float *d_xyz, uint32_t num_vertices, const uint32_t *d_indices,
                                   uint32_t num_tris, uint64_t limit_ns, void *stream);
 
+/* predictions as a cached frame asks for them: a batch of capacity n (> 0) with *d_n (device, <= n) records.
+ * *d_reordered (device) receives 0 if the records were encoded in the given order, else the number of tiles
+ * that the order by cells changed */
+vkg_status vkg_diag_nrc_predict(vkg_nrc *nrc, const float *d_features, uint32_t n, const uint32_t *d_n, float *d_rgb,
+                                uint32_t *d_reordered, void *stream);
+
 /* record the random numbers the tracer's kernels draw (d_buf NULL: stop). From the next render on,
  * the path of sample s through window pixel p writes record r = s * pixels + p of d_buf (floats):
  * [0..1] the camera jitter, then per segment i < max_segments the segment's uniforms at

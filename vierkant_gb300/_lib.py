@@ -308,6 +308,7 @@ SIGNATURES = {
     "vkg_diag_tc_gemm": (I32, [P, P, P, U32, U32, P, P, P]),
     "vkg_diag_wait_timeout": (I32, [P, U32, U64, P, P, P]),
     "vkg_diag_build_timeout": (I32, [P, P, U32, P, U32, U64, P]),
+    "vkg_diag_nrc_predict": (I32, [P, P, U32, P, P, P, P]),
     "vkg_diag_tracer_uniforms": (I32, [P, P, U32]),
     "vkg_nrc_config_default": (I32, [C.POINTER(vkg_nrc_config)]),
     "vkg_nrc_create": (I32, [P, C.POINTER(vkg_nrc_config), C.POINTER(P)]),

@@ -156,7 +156,8 @@ const uint32_t *bin_rays(vkg_ctx *ctx, const vkg_bvh *bvh, const vkg_ray *d_rays
 // 218 us, 1,200,000: 351 either way, 1,800,000: 551 -> 534 us).
 constexpr uint32_t BIN_MIN_CLOSEST = 1u << 19, BIN_MIN_ANY = 3u << 19;
 // the same for points (the first three floats of records of `stride` floats) over a 32^3 grid of the box
-// lo, 1 / scale: neighbouring positions of the order are neighbouring in space; `bins` is the caller's scratch
+// lo, 1 / scale: neighbouring positions of the order are neighbouring in space; `bins` is the caller's scratch.
+// Fewer than min_points points, by n or by *d_n, keep their order
 const uint32_t *bin_points(vkg_ctx *ctx, bin_scratch &bins, const float *d_points, uint32_t stride, uint32_t n,
                            const uint32_t *d_n, const float lo[3], const float scale[3], uint32_t min_points,
                            cudaStream_t st, const uint32_t **reordered_out);

@@ -682,9 +682,11 @@ vkg_status nrc_ensure(vkg_nrc *c, uint32_t n)
     return VKG_OK;
 }
 
-// n: capacity (host); d_n: optional device-side count (<= n) of the valid records; bins: scratch of the order
+// n: capacity (host); d_n: optional device-side count (<= n) of the valid records; bins: scratch of the order.
+// order: optional, receives the device word that is non-zero if the records are encoded in the order of their
+// cells (nullptr: never)
 vkg_status nrc_encode(vkg_nrc *c, const float *feats, uint32_t n, const uint32_t *d_n, uint32_t *X, bin_scratch &bins,
-                      cudaStream_t st)
+                      cudaStream_t st, const uint32_t **order = nullptr)
 {
     if(n == 0) return VKG_OK;
     const uint32_t *reordered = nullptr;
@@ -692,6 +694,7 @@ vkg_status nrc_encode(vkg_nrc *c, const float *feats, uint32_t n, const uint32_t
                                       ENC_BIN_MIN, st, &reordered);
     k_encode<<<(n + ENC_ROWS - 1) / ENC_ROWS, ENC_THREADS, 0, st>>>(feats, n, d_n, c->gc, c->grid_h, X, perm, reordered);
     if(perm) bins_done(bins, st);
+    if(order) *order = perm ? reordered : nullptr;
     return cuda_check(c->ctx, cudaGetLastError(), "k_encode");
 }
 
@@ -950,6 +953,25 @@ vkg_status vkg_nrc_infer(vkg_nrc *c, const float *d_feats, uint32_t n, float *d_
     if(vkg_status s = nrc_encode(c, d_feats, n, nullptr, c->X, bins, st); s != VKG_OK) return s;
     if(c->tc_infer == 2) return nrc_infer_tc(c->ctx, c->gc, c->grid_h, c->wtc, d_feats, c->X, n, nullptr, d_rgb, c->d_err, st);
     return nrc_forward(c, c->X, n, nullptr, d_rgb, st);
+}
+
+vkg_status vkg_diag_nrc_predict(vkg_nrc *c, const float *d_feats, uint32_t n, const uint32_t *d_n, float *d_rgb,
+                                uint32_t *d_reordered, void *stream)
+{
+    if(!c) return VKG_ERR_INVALID_ARGUMENT;
+    if(n == 0 || !d_feats || !d_n || !d_rgb || !d_reordered)
+        return set_error(c->ctx, VKG_ERR_INVALID_ARGUMENT, "vkg_diag_nrc_predict: NULL buffer or no records");
+    if(c->tc_infer == 3) return set_error(c->ctx, VKG_ERR_NOT_SUPPORTED, "vkg_diag_nrc_predict: infer_kernel 3 has no encoding pass");
+    if(vkg_status s = bind_device(c->ctx); s != VKG_OK) return s;
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    if(vkg_status s = nrc_ensure(c, n); s != VKG_OK) return s;
+    const uint32_t *order = nullptr;
+    bin_scratch bins = own_bins(c, n);
+    if(vkg_status s = nrc_encode(c, d_feats, n, d_n, c->X, bins, st, &order); s != VKG_OK) return s;
+    if(order) VKG_TRY_CUDA(c->ctx, cudaMemcpyAsync(d_reordered, order, sizeof(uint32_t), cudaMemcpyDeviceToDevice, st));
+    else VKG_TRY_CUDA(c->ctx, cudaMemsetAsync(d_reordered, 0, sizeof(uint32_t), st));
+    if(c->tc_infer == 2) return nrc_infer_tc(c->ctx, c->gc, c->grid_h, c->wtc, d_feats, c->X, n, d_n, d_rgb, c->d_err, st);
+    return nrc_forward(c, c->X, n, d_n, d_rgb, st);
 }
 
 vkg_status vkg_nrc_backward(vkg_nrc *c, const float *d_feats, const float *d_targets, uint32_t n, void *stream)

@@ -291,15 +291,17 @@ __global__ void __launch_bounds__(256)
 }
 
 // bins of points instead of rays: the Morton index of a point's cell in a 32 x 32 x 32 grid over the box
-// lo, 1 / scale (points outside count to the border cells); `stride` floats from point to point
+// lo, 1 / scale (points outside count to the border cells); `stride` floats from point to point. Fewer than n_min
+// points (a device-side count far below the capacity) are left in their order: no tile of k_bin_tiles counts
 __global__ void __launch_bounds__(256)
         k_bin_point_keys(const float *__restrict__ pts, uint32_t stride, uint32_t n_cap, const uint32_t *__restrict__ d_n,
-                         float3 lo, float3 scale, uint16_t *__restrict__ bins, uint32_t *__restrict__ reordered)
+                         uint32_t n_min, float3 lo, float3 scale, uint16_t *__restrict__ bins,
+                         uint32_t *__restrict__ reordered)
 {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if(i == 0) reordered[0] = reordered[1] = 0u;
     const uint32_t n = d_n ? min(*d_n, n_cap) : n_cap;
-    if(i >= n) return;
+    if(i >= n || n < n_min) return;
     const float *p = pts + (size_t)stride * i;
     auto cell = [](float x, float l, float s) {
         return (uint32_t)min(max(__float2int_rz((x - l) * s * 32.f), 0), 31);
@@ -314,10 +316,11 @@ __global__ void __launch_bounds__(256)
 // (all warps of a camera tile would otherwise queue on the same few counters). In other steps each
 // ray takes its rank with its own atomic.
 __global__ void __launch_bounds__(BIN_THREADS)
-        k_bin_tiles(const uint16_t *__restrict__ bins, uint32_t n_cap, const uint32_t *__restrict__ d_n, uint32_t tile,
-                    uint32_t *__restrict__ keys, uint32_t *__restrict__ M, uint32_t *__restrict__ reordered)
+        k_bin_tiles(const uint16_t *__restrict__ bins, uint32_t n_cap, const uint32_t *__restrict__ d_n, uint32_t n_min,
+                    uint32_t tile, uint32_t *__restrict__ keys, uint32_t *__restrict__ M, uint32_t *__restrict__ reordered)
 {
     const uint32_t n = d_n ? min(*d_n, n_cap) : n_cap;
+    if(n < n_min) return;
     extern __shared__ uint32_t h[];
     __shared__ uint32_t uniform_steps;
     for(uint32_t b = threadIdx.x; b < BIN_SLOTS; b += BIN_THREADS) h[b] = 0u;
@@ -585,9 +588,10 @@ uint32_t bin_tile(const vkg_ctx *ctx, uint32_t n)
 // words of bin_totals: O, F, the count of reordered tiles, the CTAs of k_bin_columns that are done
 constexpr size_t BIN_TOTALS = 2 * (size_t)BIN_SLOTS + 2;
 
-// the order of n elements whose 16-bit bins write_bins(bins, reordered) computes on the stream
+// the order of n elements whose 16-bit bins write_bins(bins, reordered) computes on the stream; the given order if
+// there are fewer than n_min of them (d_n)
 template<class WriteBins>
-const uint32_t *bin_order(vkg_ctx *ctx, bin_scratch &b, uint32_t n, const uint32_t *d_n, cudaStream_t st,
+const uint32_t *bin_order(vkg_ctx *ctx, bin_scratch &b, uint32_t n, const uint32_t *d_n, uint32_t n_min, cudaStream_t st,
                           const uint32_t **reordered_out, WriteBins write_bins)
 {
     *reordered_out = nullptr;
@@ -644,7 +648,7 @@ const uint32_t *bin_order(vkg_ctx *ctx, bin_scratch &b, uint32_t n, const uint32
     uint16_t *bins16 = reinterpret_cast<uint16_t *>(b.perm);
     uint32_t *reordered = b.bin_totals + 2 * BIN_SLOTS;
     write_bins(bins16, reordered);
-    k_bin_tiles<<<tiles, BIN_THREADS, BIN_SMEM, st>>>(bins16, n, d_n, tile, b.keys, b.tile_counts, reordered);
+    k_bin_tiles<<<tiles, BIN_THREADS, BIN_SMEM, st>>>(bins16, n, d_n, n_min, tile, b.keys, b.tile_counts, reordered);
     k_bin_columns<<<BIN_SLOTS / 32, 1024, 0, st>>>(b.tile_counts, tiles, F, O, reordered);
     k_bin_place<<<(n + 255) / 256, 256, 0, st>>>(b.keys, n, d_n, tile, b.tile_counts, F, O, b.perm, reordered);
     *reordered_out = reordered;
@@ -686,7 +690,7 @@ const uint32_t *bin_rays(vkg_ctx *ctx, const vkg_bvh *bvh, const vkg_ray *d_rays
         const float ext = bvh->scene_max[a] - bvh->scene_min[a];
         ps[a] = ext > 0.f ? (float)(1 << BIN_CELL_BITS) / ext : 0.f;
     }
-    return bin_order(ctx, ctx->bins, n, d_n, st, reordered_out, [&](uint16_t *bins, uint32_t *reordered) {
+    return bin_order(ctx, ctx->bins, n, d_n, 0u, st, reordered_out, [&](uint16_t *bins, uint32_t *reordered) {
         k_bin_keys<<<(n + 255) / 256, 256, 0, st>>>(d_rays, n, d_n, lo, scale, bins, reordered);
     });
 }
@@ -697,8 +701,9 @@ const uint32_t *bin_points(vkg_ctx *ctx, bin_scratch &scratch, const float *d_po
 {
     *reordered_out = nullptr;
     if(n < min_points) return nullptr;
-    return bin_order(ctx, scratch, n, d_n, st, reordered_out, [&](uint16_t *bins, uint32_t *reordered) {
-        k_bin_point_keys<<<(n + 255) / 256, 256, 0, st>>>(d_points, stride, n, d_n, make_float3(lo[0], lo[1], lo[2]),
+    return bin_order(ctx, scratch, n, d_n, min_points, st, reordered_out, [&](uint16_t *bins, uint32_t *reordered) {
+        k_bin_point_keys<<<(n + 255) / 256, 256, 0, st>>>(d_points, stride, n, d_n, min_points,
+                                                          make_float3(lo[0], lo[1], lo[2]),
                                                           make_float3(scale[0], scale[1], scale[2]), bins, reordered);
     });
 }
