@@ -36,12 +36,11 @@ namespace
 
 __device__ __forceinline__ uint32_t eff_n(uint32_t n, const uint32_t *d_n) { return d_n ? min(*d_n, n) : n; }
 
-// FUSED: encode the feature records here; else read the encoded inputs X (n x 40 u32) written by k_encode
-template<bool FUSED>
+// encodes the feature records of a tile and runs them through the MLP
 __global__ void __launch_bounds__(TC_INFER_THREADS)
-        k_infer_tc(const float *__restrict__ feats, const uint32_t *__restrict__ X, uint32_t n_cap,
-                   const uint32_t *__restrict__ d_n, grid_config gc, const __half2 *__restrict__ grid,
-                   const uint16_t *__restrict__ wtc, float *__restrict__ Y, uint32_t *__restrict__ err)
+        k_infer_tc(const float *__restrict__ feats, uint32_t n_cap, const uint32_t *__restrict__ d_n, grid_config gc,
+                   const __half2 *__restrict__ grid, const uint16_t *__restrict__ wtc, float *__restrict__ Y,
+                   uint32_t *__restrict__ err)
 {
     extern __shared__ __align__(1024) uint8_t smem[];
     __shared__ uint64_t mbar;
@@ -70,16 +69,7 @@ __global__ void __launch_bounds__(TC_INFER_THREADS)
     for(uint32_t tile = blockIdx.x; tile < tiles && !failed; tile += gridDim.x)
     {
         const uint32_t q = tile * TC_TILE + r;
-        if constexpr(!FUSED)
-        {
-            // half h copies 16-byte groups h, h + 2, ... of row r
-            const uint4 *src = reinterpret_cast<const uint4 *>(X + (size_t)(IN / 2) * q);
-#pragma unroll
-            for(int j = h; j < IN / 8; j += 2)
-                *reinterpret_cast<uint4 *>(sa + tc::canon_offset(r, 8 * j, IN)) =
-                        q < n ? src[j] : make_uint4(0u, 0u, 0u, 0u);
-        }
-        else if(h == 0)
+        if(h == 0)
         {
             uint32_t x[8];
             if(q < n)
@@ -895,15 +885,14 @@ vkg_status nrc_infer_tc(vkg_ctx *ctx, const grid_config &gc, const __half2 *grid
 {
     if(n == 0) return VKG_OK;
     if(X) return nrc_forward_tc(ctx, wtc, X, n, d_n, Y, err, st);
-    auto kern = X ? k_infer_tc<false> : k_infer_tc<true>;
-    VKG_TRY_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_SMEM));
+    VKG_TRY_CUDA(ctx, cudaFuncSetAttribute(k_infer_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_SMEM));
     int per_sm = 0;
-    VKG_TRY_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, TC_INFER_THREADS, TC_SMEM));
+    VKG_TRY_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_infer_tc, TC_INFER_THREADS, TC_SMEM));
     // TMEM: every resident CTA holds 64 of the SM's 512 columns
     per_sm = std::max(1, std::min(per_sm, (int)(512 / TC_TMEM_COLS)));
     const uint32_t tiles = (n + TC_TILE - 1) / TC_TILE;
     const uint32_t grid_n = std::min<uint32_t>(tiles, (uint32_t)(ctx->num_sms * per_sm));
-    kern<<<grid_n, TC_INFER_THREADS, TC_SMEM, st>>>(feats, X, n, d_n, gc, grid, wtc, Y, err);
+    k_infer_tc<<<grid_n, TC_INFER_THREADS, TC_SMEM, st>>>(feats, n, d_n, gc, grid, wtc, Y, err);
     return cuda_check(ctx, cudaGetLastError(), "k_infer_tc");
 }
 
