@@ -88,11 +88,19 @@ __device__ __forceinline__ bool tl_step(tl_state &s, const node8 *__restrict__ t
                                         const float4 *__restrict__ box, const blas_ref *__restrict__ blas, int cull,
                                         const F &f = F())
 {
-    while(s.sp > 0 && !s.done)
+    // The next node, or the next instance that the ray hits. The search and the node below it have one exit each, so
+    // that the lanes of a warp meet again after either: a `continue` past the own-box test with the node inside
+    // the loop left them apart for good, which cost more than the test saves wherever many instances
+    // overlap. 518,400 rays, closest hit, us: without the test / with the `continue` / so. Camera rays over 50,
+    // 4,000 and 40,000 instances of a flat scene 118 / 90 / 91, 891 / 773 / 707 and 1,366 / 1,308 / 1,134;
+    // random rays over 20,000 instances that overlap a lot 12,811 / 18,067 / 11,597.
+    uint32_t e = 0;
+    bool have = false;
+    while(s.sp > 0 && !have)
     {
         --s.sp;
         const uint2 ent = s.st[s.sp];
-        const uint32_t e = ent.x;
+        e = ent.x;
         if(e == TL_RETURN)
         {
             for(int a = 0; a < 3; ++a)
@@ -103,25 +111,33 @@ __device__ __forceinline__ bool tl_step(tl_state &s, const node8 *__restrict__ t
             }
             s.nodes = tnodes;
             s.in_blas = false;
-            continue;
         }
-        if(__uint_as_float(ent.y) > s.best_t) continue;
-        if(!s.in_blas && (e & INST_BIT))
+        else if(!(__uint_as_float(ent.y) > s.best_t))
         {
-            // a leaf's instances were pushed for the box they share: each is entered only if the ray hits
-            // its own (20,000 spheres, 518,400 camera rays: 1,175 -> 1,095 us)
-            const float4 b0 = __ldg(box + 2 * (e & ~INST_BIT)), b1 = __ldg(box + 2 * (e & ~INST_BIT) + 1);
-            const float x0 = (b0.x - s.wo[0]) * s.wi[0], x1 = (b0.w - s.wo[0]) * s.wi[0];
-            const float y0 = (b0.y - s.wo[1]) * s.wi[1], y1 = (b1.x - s.wo[1]) * s.wi[1];
-            const float z0 = (b0.z - s.wo[2]) * s.wi[2], z1 = (b1.y - s.wo[2]) * s.wi[2];
-            const float tn = fmaxf(fmaxf(fminf(x0, x1), fminf(y0, y1)), fmaxf(fminf(z0, z1), s.tmin));
-            const float tf = fminf(fminf(fmaxf(x0, x1), fmaxf(y0, y1)), fminf(fmaxf(z0, z1), s.best_t));
-            if(!(tn <= tf)) continue;
-            // enter an instance: object-space ray, RETURN marker, BLAS root
-            const float4 *mp = reinterpret_cast<const float4 *>(inst + (e & ~INST_BIT));
-            const uint4 meta = __ldg(reinterpret_cast<const uint4 *>(mp + 6));
-            const blas_ref B = blas[meta.x];
-            if(B.num_tris == 0 || s.sp + 2 > (int)TL_STACK) continue;
+            have = true;
+            if(!s.in_blas && (e & INST_BIT))
+            {
+                // a leaf's instances were pushed for the box they share: each is entered only if the ray
+                // hits its own
+                const float4 b0 = __ldg(box + 2 * (e & ~INST_BIT)), b1 = __ldg(box + 2 * (e & ~INST_BIT) + 1);
+                const float x0 = (b0.x - s.wo[0]) * s.wi[0], x1 = (b0.w - s.wo[0]) * s.wi[0];
+                const float y0 = (b0.y - s.wo[1]) * s.wi[1], y1 = (b1.x - s.wo[1]) * s.wi[1];
+                const float z0 = (b0.z - s.wo[2]) * s.wi[2], z1 = (b1.y - s.wo[2]) * s.wi[2];
+                const float tn = fmaxf(fmaxf(fminf(x0, x1), fminf(y0, y1)), fmaxf(fminf(z0, z1), s.tmin));
+                const float tf = fminf(fminf(fmaxf(x0, x1), fmaxf(y0, y1)), fminf(fmaxf(z0, z1), s.best_t));
+                have = tn <= tf;
+            }
+        }
+    }
+    if(have && !s.in_blas && (e & INST_BIT))
+    {
+        // enter it: object-space ray, RETURN marker, and on with the BLAS root
+        const float4 *mp = reinterpret_cast<const float4 *>(inst + (e & ~INST_BIT));
+        const uint4 meta = __ldg(reinterpret_cast<const uint4 *>(mp + 6));
+        const blas_ref B = blas[meta.x];
+        have = B.num_tris != 0 && s.sp + 2 <= (int)TL_STACK;
+        if(have)
+        {
             const float4 m[3] = {__ldg(mp), __ldg(mp + 1), __ldg(mp + 2)};
             to_object(m, s.wo[0], s.wo[1], s.wo[2], s.wd[0], s.wd[1], s.wd[2], s.o, s.d);
             for(int a = 0; a < 3; ++a) s.inv[a] = safe_rcp(s.d[a]);
@@ -131,10 +147,12 @@ __device__ __forceinline__ bool tl_step(tl_state &s, const node8 *__restrict__ t
             if(F::active) s.cur_alpha = f.tests_material(meta.z);
             s.in_blas = true;
             s.st[s.sp] = make_uint2(TL_RETURN, __float_as_uint(s.tmin));
-            s.st[s.sp + 1] = make_uint2(0u, __float_as_uint(s.tmin));
-            s.sp += 2;
-            continue;
+            ++s.sp;
+            e = 0;
         }
+    }
+    if(have)
+    {
         uint32_t key[8];
         uint4 w4, w5;
         node_keys<false, POS>(s.nodes, e, s.o[0], s.o[1], s.o[2], s.inv[0], s.inv[1], s.inv[2], s.tmin, s.best_t, key,
@@ -183,9 +201,10 @@ __device__ __forceinline__ bool tl_step(tl_state &s, const node8 *__restrict__ t
                     }
                 }
             }
-            if(s.done) break;
         }
         // push far-to-near: internal children, and at the top level the instance leaves as entries
+        if(ANY && s.done) s.sp = 0;
+        else
 #pragma unroll
         for(int h = 7; h >= 0; --h)
         {
@@ -211,9 +230,8 @@ __device__ __forceinline__ bool tl_step(tl_state &s, const node8 *__restrict__ t
                 ++s.sp;
             }
         }
-        return true;
     }
-    return false;
+    return s.sp > 0;
 }
 
 template<bool ANY, class F = no_filter>
