@@ -613,7 +613,8 @@ struct arena
 };
 
 // what a build starts from: [0..5] the empty scene box (ordered uints: +inf, -inf), [6] error bits of the
-// primitives, [8..10] the collapse's info, [11] its grid barrier, [12] the margin
+// primitives, [8..10] the collapse's info, [11] its grid barrier, [12] the margin, [13] half the surface areas of the
+// instances' boxes (0 for triangles)
 __global__ void k_build_init(uint32_t *__restrict__ visits, uint32_t n, uint32_t *__restrict__ small)
 {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -690,9 +691,11 @@ __device__ __forceinline__ bool invert_3x4(const float *m, float *inv)
 __global__ void __launch_bounds__(256)
         k_instance_boxes(const vkg_instance *__restrict__ inst, uint32_t n, const blas_box *__restrict__ bb,
                          uint32_t nblas, box6 *__restrict__ tbox, uint32_t *__restrict__ scene_enc,
-                         uint32_t *__restrict__ err)
+                         uint32_t *__restrict__ err, float *__restrict__ area)
 {
     __shared__ uint32_t s_lo[3], s_hi[3];
+    __shared__ float s_area; // half the surface areas of the block's boxes
+    if(threadIdx.x == 0) s_area = 0.f;
     if(threadIdx.x < 3)
     {
         s_lo[threadIdx.x] = fenc(__int_as_float(0x7f800000));
@@ -787,11 +790,14 @@ __global__ void __launch_bounds__(256)
         __syncwarp();
         double least = best;
         for(uint32_t d = 6; d < 30; d += 6) least = fmin(least, __shfl_sync(0xffffffffu, best, lane + d));
+        // rounded outward; the collapse grows every box by its margin on top. An empty mesh: a
+        // point box at the instance origin (the traversal skips it)
+        const float f = !B.num_tris ? T[3] : (high ? __double2float_ru(-least) : __double2float_rd(least));
+        const float g = __shfl_down_sync(0xffffffffu, f, 3) - f; // lanes 0..2: the box's extents
+        const float gy = __shfl_sync(0xffffffffu, g, 1), gz = __shfl_sync(0xffffffffu, g, 2);
+        if(lane == 0) atomicAdd(&s_area, g * gy + gy * gz + gz * g);
         if(lane < 6)
         {
-            // rounded outward; the collapse grows every box by its margin on top. An empty mesh: a
-            // point box at the instance origin (the traversal skips it)
-            const float f = !B.num_tris ? T[3] : (high ? __double2float_ru(-least) : __double2float_rd(least));
             (high ? tbox[i].hi : tbox[i].lo)[axis] = f;
             if(high) atomicMax(&s_hi[axis], fenc(f));
             else atomicMin(&s_lo[axis], fenc(f));
@@ -803,6 +809,7 @@ __global__ void __launch_bounds__(256)
         atomicMin(&scene_enc[threadIdx.x], s_lo[threadIdx.x]);
         atomicMax(&scene_enc[3 + threadIdx.x], s_hi[threadIdx.x]);
     }
+    if(threadIdx.x == 0) atomicAdd(area, s_area);
 }
 
 // instance records in leaf (sorted) order and in input order
@@ -855,7 +862,7 @@ cudaError_t launch_collapse(const collapse_args &A, uint32_t max_blocks, cudaStr
 // err_bits the error bits that make_boxes raised. The caller frees bvh on failure.
 template<class MakeBoxes, class MakeRecords>
 vkg_status build_core(vkg_ctx *ctx, vkg_bvh *bvh, uint32_t n, uint32_t leaf_max, const grid_wait &wait, cudaStream_t st,
-                      MakeBoxes make_boxes, MakeRecords make_records, uint32_t &err_bits)
+                      MakeBoxes make_boxes, MakeRecords make_records, uint32_t &err_bits, float &box_area)
 {
     cudaEvent_t ev0, ev1;
     cudaEventCreate(&ev0);
@@ -939,6 +946,7 @@ vkg_status build_core(vkg_ctx *ctx, vkg_bvh *bvh, uint32_t n, uint32_t leaf_max,
         bvh->num_nodes = info[8];
         bvh->depth = info[9];
         std::memcpy(&bvh->margin, &info[12], 4);
+        std::memcpy(&box_area, &info[13], 4);
         for(int a = 0; a < 3; ++a)
         {
             uint32_t lo = info[a], hi = info[3 + a];
@@ -1010,6 +1018,7 @@ static vkg_status bvh_build(vkg_ctx *ctx, const float *d_xyz, uint32_t num_verti
     const int T = 256;
     const uint32_t g = (n + T - 1) / T;
     uint32_t err_bits = 0;
+    float box_area = 0.f;
     vkg_status s = build_core(
             ctx, bvh, n, leaf_max, wait, st,
             [&](box6 *tbox, uint32_t *scene_enc, uint32_t *err) {
@@ -1018,7 +1027,7 @@ static vkg_status bvh_build(vkg_ctx *ctx, const float *d_xyz, uint32_t num_verti
             [&](const uint32_t *sorted, const box6 *, const float *) {
                 k_tri_records<<<g, T, 0, st>>>(d_xyz, num_vertices, d_indices, sorted, n, bvh->d_tris);
             },
-            err_bits);
+            err_bits, box_area);
     if(s == VKG_OK && (err_bits & BUILD_ERR_INDEX))
         s = set_error(ctx, VKG_ERR_INVALID_ARGUMENT, "vkg_bvh_build: triangle index >= num_vertices (%u)", num_vertices);
     if(s != VKG_OK)
@@ -1151,18 +1160,23 @@ extern "C" vkg_status vkg_tlas_build(vkg_ctx *ctx, const vkg_bvh *const *blas, u
     const int T = 256;
     const uint32_t g = (n + T - 1) / T;
     uint32_t err_bits = 0;
+    float box_area = 0.f;
     vkg_status s = build_core(
             ctx, &t->top, n, leaf_max, grid_wait{}, st,
             [&](box6 *tbox, uint32_t *scene_enc, uint32_t *err) {
-                k_instance_boxes<<<(n + 7) / 8, 256, 0, st>>>(d_instances, n, d_bb, num_blas, tbox, scene_enc, err);
+                k_instance_boxes<<<(n + 7) / 8, 256, 0, st>>>(d_instances, n, d_bb, num_blas, tbox, scene_enc, err,
+                                                              reinterpret_cast<float *>(scene_enc + 13));
             },
             [&](const uint32_t *sorted, const box6 *lbox, const float *margin) {
                 k_instance_records<<<g, T, 0, st>>>(d_instances, sorted, n, num_blas, lbox, margin, t->d_inst,
                                                     t->d_inst_by_id, t->d_inst_box);
             },
-            err_bits);
+            err_bits, box_area);
     if(d_bb) cudaFreeAsync(d_bb, st);
     t->top.num_tris = n;
+    const float ex = t->top.scene_max[0] - t->top.scene_min[0], ey = t->top.scene_max[1] - t->top.scene_min[1],
+                ez = t->top.scene_max[2] - t->top.scene_min[2], half = ex * ey + ey * ez + ez * ex;
+    t->overlap = half > 0.f ? box_area / half : 0.f;
     if(s == VKG_OK && (err_bits & BUILD_ERR_INDEX))
         s = set_error(ctx, VKG_ERR_INVALID_ARGUMENT, "vkg_tlas_build: an instance's BLAS index >= %u", num_blas);
     if(s == VKG_OK && (err_bits & BUILD_ERR_SINGULAR))

@@ -120,6 +120,7 @@ struct vkg_tlas
     vkg::blas_ref *d_blas = nullptr;
     uint32_t num_instances = 0, num_blas = 0;
     uint32_t max_blas_depth = 0; // depth of the deepest mesh BVH
+    float overlap = 0.f; // instance boxes that a random line through the scene crosses, on average
 };
 
 namespace vkg

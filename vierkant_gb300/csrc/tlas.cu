@@ -83,7 +83,7 @@ vkg_status launch(vkg_ctx *ctx, const vkg_tlas *t, const vkg_ray *rays, uint32_t
             kern<<<(n * lanes + TLAS_THREADS - 1) / TLAS_THREADS, TLAS_THREADS, 0, st>>>(
                     t->top.d_nodes, t->d_inst, t->d_inst_box, t->d_blas, rays, n, hits, occ, cull);
         };
-        if(n > TL_GROUP_MAX_RAYS) go(k_tlas_trace<ANY>, 1u);
+        if(n > tl_group_max_rays(t, ANY)) go(k_tlas_trace<ANY>, 1u);
         else if(tl_group_small_stack(t)) go(k_tlas_trace_group<ANY, TL_GROUP_SMALL_STACK>, GROUP_LANES);
         else go(k_tlas_trace_group<ANY, TL_GROUP_STACK>, GROUP_LANES);
     }

@@ -17,10 +17,19 @@
 namespace vkg
 {
 
-// Largest batch traced by groups: 131,072 camera rays take 61 / 298 / 474 / 496 us against 80 / 320 / 578 /
-// 624 us over 50 / 2,000 / 20,000 / 40,000 instances (4,000 rays 23 / 64 / 72 / 88 against 42 / 206 /
-// 253 / 340), 260,000 break even, 518,400 lose up to a quarter.
-constexpr uint32_t TL_GROUP_MAX_RAYS = 1u << 17;
+// Largest batch traced by groups: 131,072 camera rays take 43 / 278 / 365 / 417 us by groups and 73 / 328 / 413 / 464
+// a thread each over 50 / 4,000 / 20,000 / 40,000 instances of a flat scene (32,768 rays 29 / 108 / 139 / 167 and
+// 60 / 240 / 341 / 342); 260,000 rays gain from a thread each.
+// Closest-hit rays through instances that overlap a lot gain from it earlier, as groups leave them more lanes idle.
+// The time of a thread each over that of groups, for 98,304 / 65,536 / 49,152 random rays: 0.6 / 0.8 / 1.0 where a
+// line crosses 250 instance boxes on average (camera rays 1.0 / 1.2 / 1.4), 0.8 / 1.1 / 1.3 where it crosses 20 to
+// 40 (camera rays 1.2 / 1.5 / 1.7); any-hit rays 0.9 or more at 98,304, 1.1 or more below.
+constexpr uint32_t TL_GROUP_MAX_RAYS = 1u << 17, TL_GROUP_MAX_OVERLAPPING = 3u << 14;
+constexpr float TL_GROUP_OVERLAP = 64.f;
+inline uint32_t tl_group_max_rays(const vkg_tlas *t, bool any)
+{
+    return any || t->overlap <= TL_GROUP_OVERLAP ? TL_GROUP_MAX_RAYS : TL_GROUP_MAX_OVERLAPPING;
+}
 
 // Stack entries of a group. Every level leaves at most 7 entries behind and the last one 8; between the
 // levels an opened leaf adds 8 and the marker 1: 7 (top depth + mesh depth) + 4. The shared memory of
@@ -113,11 +122,8 @@ __device__ __forceinline__ tlas_result trace_tlas_group(bool active, const node8
             have = true;
         }
         if(!__any_sync(ALL, have)) break;
-        if(put)
-        {
-            if(k == 0) st[sp] = back;
-            ++sp;
-        }
+        if(put && k == 0) st[sp] = back;
+        sp += put ? 1 : 0; // (a branch around both lines, or a barrier of the group in the loop, cost 0.7-1.3 % more)
         float tn, tf;
         uint32_t word;
         bool hit;
