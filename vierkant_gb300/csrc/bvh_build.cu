@@ -1086,7 +1086,7 @@ extern "C" vkg_status vkg_bvh_info_get(const vkg_bvh *bvh, vkg_bvh_info *out)
 
 // ---- two-level BVH -----------------------------------------------------------------------------
 // The top level is the same 8-wide quantised BVH, built by the same core over the instances' world
-// boxes (the 8 transformed corners of the mesh's bounds, rounded outward); its leaves index
+// boxes (the union of the transformed boxes two levels below a mesh's root, rounded outward); its leaves index
 // 128-byte instance records (world <-> object transforms, BLAS, input index, material). Mirrors
 // RayBuilder::create_toplevel (RayBuilder.cpp:386-760), which builds the driver TLAS over entries
 // carrying a vk_transform_matrix (:518).

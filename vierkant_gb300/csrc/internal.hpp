@@ -153,8 +153,9 @@ const uint32_t *bin_rays(vkg_ctx *ctx, const vkg_bvh *bvh, const vkg_ray *d_rays
                          uint32_t flags, uint32_t min_rays, cudaStream_t st, const uint32_t **reordered_out);
 // Batches from which binning pays. The binning itself takes 40-90 us; a closest-hit traversal of incoherent
 // rays gains more than that from 2^19 rays on (600,000: 441 -> 414 us, 784,000: 531 -> 494 us), an any-hit
-// traversal, which ends at the first hit, from about 1.5 million (600,000: 164 -> 184 us, 784,000: 209 ->
-// 218 us, 1,200,000: 351 either way, 1,800,000: 551 -> 534 us).
+// traversal, which ends at the first hit, from about 1.5 million (bounce rays, 600,000: 164 -> 184 us, 784,000:
+// 209 -> 218 us, 1,200,000: 351 either way, 1,800,000: 551 -> 534 us; camera rays, 1,048,576: 176 -> 203 us; rays all
+// over the scene's box gain earlier, 700,000: 331 -> 325 us, 1,048,576: 472 -> 439 us).
 constexpr uint32_t BIN_MIN_CLOSEST = 1u << 19, BIN_MIN_ANY = 3u << 19;
 // the same for points (the first three floats of records of `stride` floats) over a 32^3 grid of the box
 // lo, 1 / scale: neighbouring positions of the order are neighbouring in space; `bins` is the caller's scratch.

@@ -405,7 +405,7 @@ __device__ __forceinline__ bool two_level(const pt_params &P)
 }
 
 // resident blocks the tracers are compiled for: the plain single-level ones fit 56 registers with 8 bytes of
-// spills, and a ninth block gains more (k_trace 1.6 % on a mixed batch); the others 64 or 85 registers
+// spills, and a ninth block gains more (1280x720 at 16 samples 15,867 -> 15,752 us); the others 64 or 85 registers
 template<int STACK, bool ALPHA, int LEVELS>
 constexpr int min_blocks = LEVELS == LEVELS_ONE && !ALPHA ? 9 : STACK <= 64 ? 8 : 6;
 

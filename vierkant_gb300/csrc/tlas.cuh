@@ -33,8 +33,8 @@ __device__ __forceinline__ void to_object(const float4 (&m)[3], float ox, float 
 // One stack for both levels. Entries are top-level nodes, instance entries (INST_BIT | instance
 // record) or, above a RETURN sentinel, BLAS nodes of the instance being traversed. Each step
 // processes one node of either level, so the lanes of a warp stay in step whichever level they are
-// in: entering an instance pushes RETURN and the BLAS root and switches the ray to object space;
-// popping RETURN switches back to the world ray and the top level.
+// in: entering an instance pushes RETURN, switches the ray to object space and goes on with the BLAS
+// root; popping RETURN switches back to the world ray and the top level.
 constexpr uint32_t TL_STACK = TLAS_STACK + TRAVERSAL_STACK + 1;
 constexpr uint32_t INST_BIT = 0x80000000u, TL_RETURN = 0xFFFFFFFFu;
 

@@ -24,9 +24,9 @@ namespace vkg
 template<int STACK>
 constexpr int group_stack_entries = STACK + 1;
 constexpr int GROUP_LANES = 8;
-// Largest batch traced by groups. 64,000 rays take 64-80 us either way (64 / 82 in the Cornell box of
-// 196,618 triangles, 80 / 80 on an icosphere, groups / threads); 16,000 take 31-36 against 72 us, 150,000
-// 128-171 against 115-130 us.
+// Largest batch traced by groups, below the first scenes' break-even: over seven scenes (Cornell boxes, an icosphere, a
+// terrain, loose triangles) 16,384 rays are 1.8-3.1 times as fast as with a thread each, 65,536 random rays 1.1-1.5
+// and camera rays 1.6-2.1 times, 81,920 random rays 0.93-1.4 times, 150,000 take 128-171 against 115-130 us.
 constexpr uint32_t GROUP_MAX_RAYS = 1u << 16;
 
 // All 32 lanes of a warp call this together; `active`, the ray and `st` are uniform over a group's
