@@ -106,7 +106,7 @@ __device__ __forceinline__ uint32_t eff_count(uint32_t n, const uint32_t *d_n) {
 // encoded rows go out through shared memory, so that both streams are coalesced (row by row, a warp's
 // 40 stores and 13 loads touched 32 lines each). Rows of 44 words keep the 16-byte stores free of
 // bank conflicts. Large batches are encoded in the order of 32^3 cells (bin_points): the records of a
-// CTA then share the entries of the coarser levels in L1 (5 % -> 30 % hits, less than half the L2 sectors).
+// CTA then share the entries of the coarser levels in L1 (hits 7 % -> 26 % at 600,000 records, less than half the L2 sectors).
 // 2,073,600 / 1,000,000 / 600,000 / 400,000 queries: 810 / 417 / 262 / 192 us in the given order, 683 / 374 /
 // 254 / 198 us binned (encoding and MLP); bound by issue now.
 constexpr uint32_t ENC_BIN_MIN = 1u << 19;

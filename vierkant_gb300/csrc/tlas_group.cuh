@@ -6,7 +6,7 @@
 // object space and goes on with its root, as tl_step does, above a RETURN marker. Hits and ties are those
 // of trace_tlas: the nearest triangle, then the smaller instance, then the smaller triangle index.
 //
-// Two-level rays differ in length far more than single-level ones (7 of 32 lanes were active with one
+// Two-level rays differ in length far more than single-level ones (8 of 32 lanes are active with one
 // thread per ray) and the longest of them set the time; with four rays to a warp and a step split over
 // eight lanes both shrink.
 #pragma once
