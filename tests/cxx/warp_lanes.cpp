@@ -1,7 +1,7 @@
-// The two-level traversal by groups of eight lanes (csrc/tlas_group.cuh), compiled for the host and run by 32
-// emulated lanes. The lanes of a warp meet only in the warp-wide operations: between two of them they may
+// The traversals by groups of eight lanes (csrc/tlas_group.cuh, csrc/traverse_group.cuh), compiled for the host and
+// run by 32 emulated lanes. The lanes of a warp meet only in the warp-wide operations: between two of them they may
 // run in any order. Here every lane runs alone up to the next one, in the order of a permutation of
-// the lanes, and the results have to be those of trace_tlas, one thread per ray, for every order.
+// the lanes, and the results have to be those of trace_tlas and trace_ray, one thread per ray, for every order.
 #include <ucontext.h>
 
 #include <cuda_runtime.h>
@@ -242,15 +242,16 @@ int main()
     }
     const std::vector<node8> tnodes = {make_node(top)};
 
-    int hits = 0, wrong = 0;
+    int hits = 0, single = 0, wrong = 0;
     for(int round = 0; round < 200; ++round)
     {
-        float o[4][3], d[4][3];
+        float o[4][3], d[4][3], m[4][3]; // m: directions towards the mesh
         for(int g = 0; g < 4; ++g)
             for(int a = 0; a < 3; ++a)
             {
                 o[g][a] = uniform(-3.f, 3.f);
                 d[g][a] = uniform(-1.f, 1.f) - 0.3f * o[g][a];
+                m[g][a] = uniform(-1.f, 1.f) - o[g][a];
             }
         // the lanes in order, backwards, and at random
         int order[LANES];
@@ -267,6 +268,16 @@ int main()
         };
         run_warp(order, [&](int l) { trace(l, std::false_type{}); });
         run_warp(order, [&](int l) { trace(l, std::true_type{}); });
+        trace_result one[2][LANES];
+        auto trace_one = [&](int l, auto any) {
+            constexpr bool ANY = decltype(any)::value;
+            const int g = l / GROUP_LANES;
+            one[ANY][l] = trace_group<ANY, TL_GROUP_SMALL_STACK>(true, mesh.data(), tris.data(), o[g][0], o[g][1], o[g][2],
+                                                                 0.f, m[g][0], m[g][1], m[g][2], 1e30f, CULL_NONE,
+                                                                 stack[g], nullptr);
+        };
+        run_warp(order, [&](int l) { trace_one(l, std::false_type{}); });
+        run_warp(order, [&](int l) { trace_one(l, std::true_type{}); });
         for(int l = 0; l < LANES; ++l)
         {
             const int g = l / GROUP_LANES;
@@ -277,8 +288,16 @@ int main()
             hits += want.prim != VKG_MISS;
             wrong += h.prim != want.prim || h.inst != want.inst || h.t != want.t || h.u != want.u || h.v != want.v ||
                      got[1][l].occluded != (want.prim != VKG_MISS);
+            unsigned long long visits = 0, tests = 0;
+            const trace_result w = trace_ray<false, false, TL_GROUP_SMALL_STACK>(
+                    mesh.data(), tris.data(), o[g][0], o[g][1], o[g][2], 0.f, m[g][0], m[g][1], m[g][2], 1e30f, CULL_NONE,
+                    visits, tests, nullptr);
+            const trace_result &s = one[0][l];
+            single += w.prim != VKG_MISS;
+            wrong += s.prim != w.prim || s.t != w.t || s.u != w.u || s.v != w.v ||
+                     one[1][l].occluded != (w.prim != VKG_MISS);
         }
     }
-    std::printf("%d lanes with a hit, %d wrong\n", hits, wrong);
-    return hits > 1000 && wrong == 0 ? 0 : 1;
+    std::printf("%d lanes with a hit in the scene, %d in the mesh, %d wrong\n", hits, single, wrong);
+    return hits > 1000 && single > 1000 && wrong == 0 ? 0 : 1;
 }

@@ -1,5 +1,5 @@
-"""The lanes of a warp may run in any order between two warp-wide operations: the two-level traversal by groups of
-eight lanes, compiled for the host, gives the results of one thread per ray whatever order its lanes take."""
+"""The lanes of a warp may run in any order between two warp-wide operations: the traversals by groups of eight lanes,
+compiled for the host, give the results of one thread per ray whatever order their lanes take."""
 import shutil
 import subprocess
 from pathlib import Path
