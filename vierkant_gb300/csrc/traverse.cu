@@ -24,12 +24,13 @@ namespace
 constexpr int TRACE_THREADS = 128;
 
 // STACK: traversal stack entries; 64 serve BVHs up to 10 levels deep (7 (depth - 1) + 1 entries)
-// BLOCKS: resident blocks the kernel is compiled for. Nine take 56 registers with 24 bytes spilled, which large
+// BLOCKS: resident blocks the kernel is compiled for (0: no minimum, 53 to 64 registers and no spills; a minimum of one
+// makes it 56 to 67, which costs counting launches 3-6 %). Nine take 56 registers with 24 bytes spilled, which large
 // closest-hit batches gain from: 524,288 / 1,048,576 / 4,194,304 random rays in the Cornell box of 196,618 triangles
 // 367 / 629 / 2,164 us without a minimum, 361 / 616 / 2,117 with nine, 5.5 M mixed rays 1,408 / 1,391. Batches whose
 // blocks are all resident at once anyway lose (147,768 rays 97.8 / 101.7 us; 262,144 0.5-1.1 %, but the host variant's
 // chunks start there, and a first chunk on another kernel than the rest cost its pipeline 1,042 -> 1,132 us), as do
-// any-hit batches (784,641 rays 271.0 / 273.1) and launches that count (2,097,152 rays 2,751 / 2,792).
+// any-hit batches (784,641 rays 273.0 / 275.2) and launches that count (2,097,152 rays 2,751 / 2,792).
 constexpr uint32_t TRACE_FULL_MIN = 1u << 18;
 template<bool ANY, bool STATS, int STACK, int BLOCKS>
 __global__ void __launch_bounds__(TRACE_THREADS, BLOCKS)
@@ -208,7 +209,7 @@ void launch_simple(bool small_stack, uint32_t grid, cudaStream_t st, const vkg_b
             small_stack ? go(k_trace<false, false, 64, 9>) : go(k_trace<false, false, (int)TRAVERSAL_STACK, 9>);
             return;
         }
-    small_stack ? go(k_trace<ANY, STATS, 64, 1>) : go(k_trace<ANY, STATS, (int)TRAVERSAL_STACK, 1>);
+    small_stack ? go(k_trace<ANY, STATS, 64, 0>) : go(k_trace<ANY, STATS, (int)TRAVERSAL_STACK, 0>);
 }
 
 // ---- ray binning -------------------------------------------------------------------------------
